@@ -187,8 +187,8 @@ int64_t vsk_schedule_chunk(int64_t seen, int32_t keep, int32_t level);
  * (Acceleration/Metal/MetalThreadConfigurationOptimizer.swift:430-440). */
 typedef enum vsk_peak { VSK_PEAK_FP32_ISSUE = 0, VSK_PEAK_SMEM_GATHER = 1, VSK_PEAK_TMEM_READ = 2 } vsk_peak;
 int32_t vsk_measure_peak(vsk_ctx* ctx, int32_t what, double* per_second);
-/* The checked build variant (libvsk_cuda_checked.so, `python -m vectorstorekit_b200.build --checked`): every global
- * load, store and atomic of every kernel is range-tested against the device buffers the library allocated (with the
+/* The checked build variant (libvsk_cuda_checked.so, `python -m vectorstorekit_b200.build --checked`): the kernels'
+ * read-only global loads and atomics are range-tested against the device buffers the library allocated (with the
  * sizes the calls asked for) and the buffers the caller announced; an access outside them, or one not aligned to its
  * own size, is diverted to a sink and counted instead of being executed - no trap, the context stays usable.  It is
  * what Metal's shader validation layer is to the reference and what compute-sanitizer is to CUDA where that tool can

@@ -29,8 +29,8 @@ def metal_ref():
     return oracle.MetalRef()
 
 
-# Under the checked build variant (VSK_CHECKED=1: every global access of every kernel is range-tested, see
-# vectorstorekit_b200/ptx_check.py) every GPU test also asserts that no access was refused while it ran.
+# Under the checked build variant (VSK_CHECKED=1: the kernels' read-only loads and atomics are range-tested, see
+# vectorstorekit_b200/csrc/checked.cuh) every GPU test also asserts that no access was refused while it ran.
 _checked_dev = None
 
 

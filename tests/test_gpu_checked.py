@@ -1,4 +1,4 @@
-"""The checked build variant (``libvsk_cuda_checked.so``): every global load, store and atomic of every kernel goes
+"""The checked build variant (``libvsk_cuda_checked.so``): the kernels' read-only global loads and atomics go
 through a range test against the buffers the library allocated and the buffers the caller announced.  It stands in
 for compute-sanitizer's memcheck where that tool cannot run.  The first test re-runs the known-answer tests, the odd
 small shapes and the per-kernel parity suites in a child process with VSK_CHECKED=1; tests/conftest.py then fails any

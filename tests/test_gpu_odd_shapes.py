@@ -1,6 +1,6 @@
 """Odd small shapes through every scan: row counts around a warp and a tile edge, dimensions around the vector width and
 the 128-wide k-block, k from one to all rows.  Run under the normal library for parity with the CPU oracle and, from
-tests/test_gpu_checked.py, under the checked build variant, where every global access of every kernel is range-tested."""
+tests/test_gpu_checked.py, under the checked build variant, where read-only loads and atomics are range-tested."""
 import numpy as np
 import pytest
 

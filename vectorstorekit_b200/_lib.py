@@ -10,7 +10,7 @@ import ctypes as C
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-# VSK_CHECKED=1 selects the checked build variant (every global access of every kernel range-tested; see
+# VSK_CHECKED=1 selects the checked build variant (the kernels' read-only loads and atomics range-tested; see
 # ``build.py --checked``).  It is a testing aid: same entry points, several times slower.
 CHECKED = os.environ.get("VSK_CHECKED", "0") not in ("", "0")
 LIB_PATH = os.path.join(HERE, "libvsk_cuda_checked.so" if CHECKED else "libvsk_cuda.so")

@@ -1,9 +1,9 @@
 // Host side of the CHECKED build: the table of device address ranges the instrumented kernels may touch.
 //
 // In a normal build this file only provides the exported entry points as "not a checked build" answers and the
-// allocation hooks as no-ops.  With -DVSK_CHECKED (python -m vectorstorekit_b200.build --checked) every global access
-// of every kernel is routed through vsk_chk_access (checked.cuh, added to the PTX by ptx_check.py), which looks the
-// address up in the table kept here:
+// allocation hooks as no-ops.  With -DVSK_CHECKED (python -m vectorstorekit_b200.build --checked) the kernels' read-only
+// loads and atomics (and the accesses marked VSK_CHK) go through vsk_chk_access (checked.cuh), which looks the address
+// up in the table kept here:
 //   * every device allocation of the library, with the size the call asked for (dev_alloc, scratch),
 //   * device buffers the caller announces with vsk_checked_register (the `_dev` entry points take caller memory; the
 //     Python mirror announces every tensor it passes),
@@ -131,7 +131,7 @@ void chk_remove(const void* p) {
 namespace {
 // Reads one word just past a buffer's announced end: an instrumented build refuses the access (it reads the sink).
 __global__ void selftest_kernel(const int* buf, int words, int* out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) out[0] = buf[words];
+  if (threadIdx.x == 0 && blockIdx.x == 0) out[0] = __ldg(buf + words);
 }
 }  // namespace
 

@@ -1,10 +1,10 @@
-// Device side of the CHECKED build (-DVSK_CHECKED): the range test every instrumented global access calls.
+// Device side of the CHECKED build (-DVSK_CHECKED): the range test of the kernels' global accesses.
 //
-// The build runs a pass over each module's PTX (vectorstorekit_b200/ptx_check.py) that routes the address of every
-// global or generic load, store, atomic and reduction through vsk_chk_access below.  The function and the pointer to
-// the range table are `static`: every module carries its own copy (the library is built without relocatable device
-// code), and every module registers a setter with the host side (checked.cu) so that vsk_open can hand all of them
-// the same table.
+// Works at source level: in a checked build the names __ldg and atomicAdd / Min / Max / Or / CAS stand for the templates
+// below, which pass the address through vsk_chk_access first, and VSK_CHK(p) does the same for a plain load or store
+// (it is p itself in a normal build).  The function and the pointer to the range table are `static`: every module
+// carries its own copy (the library is built without relocatable device code), and every module registers a setter
+// with the host side (checked.cu) so that vsk_open can hand all of them the same table.
 #pragma once
 #ifdef VSK_CHECKED
 #include <cuda_runtime.h>
@@ -71,11 +71,39 @@ static __device__ __noinline__ unsigned long long vsk_chk_access(unsigned long l
   return (reinterpret_cast<unsigned long long>(&s->sink[0]) + 255ull) & ~255ull;
 }
 
-// Keeps the function in modules whose own code never calls it before the PTX pass adds the calls.
-static __global__ void keepalive_kernel(unsigned long long* p, unsigned info) {
-  *p = vsk_chk_access(reinterpret_cast<unsigned long long>(p), info);
+template <typename T>
+static __device__ __forceinline__ T* at(T* p, unsigned flags = 0u) {
+  return reinterpret_cast<T*>(vsk_chk_access(reinterpret_cast<unsigned long long>(p), (unsigned)sizeof(T) | flags));
+}
+template <typename T>
+static __device__ __forceinline__ T load(const T* p) {
+  return __ldg(at(p));
+}
+#define VSK_CHK_ATOMIC(name, op)                              \
+  template <typename T, typename V>                           \
+  static __device__ __forceinline__ T name(T* p, V v) {       \
+    return op(at(p, 0x100u), static_cast<T>(v));              \
+  }
+VSK_CHK_ATOMIC(atomic_add, atomicAdd)
+VSK_CHK_ATOMIC(atomic_min, atomicMin)
+VSK_CHK_ATOMIC(atomic_max, atomicMax)
+VSK_CHK_ATOMIC(atomic_or, atomicOr)
+#undef VSK_CHK_ATOMIC
+template <typename T, typename C, typename V>
+static __device__ __forceinline__ T atomic_cas(T* p, C c, V v) {
+  return atomicCAS(at(p, 0x100u), static_cast<T>(c), static_cast<T>(v));
 }
 
 }  // namespace chk
 }  // namespace vsk
+
+#define __ldg(...) ::vsk::chk::load(__VA_ARGS__)
+#define atomicAdd(...) ::vsk::chk::atomic_add(__VA_ARGS__)
+#define atomicMin(...) ::vsk::chk::atomic_min(__VA_ARGS__)
+#define atomicMax(...) ::vsk::chk::atomic_max(__VA_ARGS__)
+#define atomicOr(...) ::vsk::chk::atomic_or(__VA_ARGS__)
+#define atomicCAS(...) ::vsk::chk::atomic_cas(__VA_ARGS__)
+#define VSK_CHK(p) (::vsk::chk::at(p))
+#else
+#define VSK_CHK(p) (p)
 #endif  // VSK_CHECKED
