@@ -1,0 +1,110 @@
+"""Product-quantised batches on the tensor-core path (code rows decoded to fp16 operand rows, contracted, listed rows
+re-scored from the distance tables): ids and distances equal the CPU oracle's table sums bit for bit."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def vsk():
+    import vectorstorekit_b200 as v
+    return v
+
+
+@pytest.fixture(scope="module")
+def dev(vsk):
+    return vsk.CUDAAcceleratorStrategy(0).initialize()
+
+
+def _index(vsk, dev, cb, codes):
+    m, ksub, ds = cb.shape
+    pq = vsk.ProductQuantizer(dev, m * ds, segments=m, codeSize=int(np.log2(ksub)))
+    pq.set_codebooks(cb)
+    ix = pq.index()
+    ix.add(codes)
+    return ix
+
+
+def _clustered(rng, n, nq, m, ksub, ds, offset=0.0, noise=0.3):
+    """Rows and queries around 64 centres; codewords are segments of sampled rows."""
+    d = m * ds
+    centres = rng.standard_normal((64, d)).astype(np.float32) + np.float32(offset)
+    x = (centres[rng.integers(0, 64, n)] + noise * rng.standard_normal((n, d))).astype(np.float32)
+    q = (centres[rng.integers(0, 64, nq)] + noise * rng.standard_normal((nq, d))).astype(np.float32)
+    cb = np.stack([x[rng.choice(n, ksub, replace=False)][:, s * ds:(s + 1) * ds] for s in range(m)])
+    return q, np.ascontiguousarray(cb), x
+
+
+# (n, m, ds, ksub, nq, k): the smallest batch and index of the path, partial query and row tiles, every segment length
+# with a decode path of its own (2, 4, multiples of 8) and others, operand widths with the row term folded in (inside
+# the padding, d = 40; in a block of its own, d = 64 and 256) and in the epilogue (d = 320), k to the path's limit
+@pytest.mark.parametrize("shape", [(16_384, 8, 8, 256, 64, 10), (16_385, 16, 8, 256, 129, 1), (40_001, 8, 2, 256, 65, 37),
+                                   (30_000, 16, 4, 256, 300, 100), (20_001, 5, 8, 16, 128, 10), (20_000, 16, 16, 256, 70, 10),
+                                   (20_000, 10, 32, 64, 70, 10), (17_000, 7, 3, 256, 200, 5), (17_001, 24, 1, 16, 90, 10),
+                                   (50_000, 8, 8, 256, 64, 1024), (17_777, 32, 24, 16, 100, 10)])
+def test_tensor_batches_equal_table_sums(vsk, dev, cpu_oracle, shape):
+    n, m, ds, ksub, nq, k = shape
+    rng = np.random.default_rng(n + m + nq)
+    q, cb, x = _clustered(rng, n, nq, m, ksub, ds)
+    codes = cpu_oracle.pq_encode(x, cb)
+    ix = _index(vsk, dev, cb, codes)
+    before = dev.stats()["tensor_tiles"]
+    dist, ids = ix.batchSearch(q, k)
+    assert dev.stats()["tensor_tiles"] > before
+    rd, ri = cpu_oracle.pq_search(q, codes, cb, k)
+    assert np.array_equal(ids, ri)
+    assert np.array_equal(dist, rd)
+    # one query fewer than the path takes: the table scan gives the same rows
+    d1, i1 = ix.batchSearch(q[:63], k)
+    assert np.array_equal(i1, ri[:63]) and np.array_equal(d1, rd[:63])
+
+
+@pytest.mark.parametrize("offset", [30.0, 3000.0])
+def test_rows_far_from_the_origin(vsk, dev, cpu_oracle, offset):
+    """The error bound grows with the rows' norms: lists get longer, and where they overflow the table scan answers."""
+    rng = np.random.default_rng(5)
+    q, cb, x = _clustered(rng, 30_000, 80, 8, 256, 4, offset)
+    codes = cpu_oracle.pq_encode(x, cb)
+    ix = _index(vsk, dev, cb, codes)
+    dist, ids = ix.batchSearch(q, 20)
+    rd, ri = cpu_oracle.pq_search(q, codes, cb, 20)
+    assert np.array_equal(ids, ri) and np.array_equal(dist, rd)
+
+
+def test_bulk_ties_and_late_block_fall_back(vsk, dev, cpu_oracle):
+    rng = np.random.default_rng(6)
+    n, m, ds = 60_000, 2, 4
+    cb = rng.standard_normal((m, 16, ds)).astype(np.float32)
+    q = rng.standard_normal((70, m * ds)).astype(np.float32)
+    codes = rng.integers(0, 4, (n, m)).astype(np.uint8)          # 16 distinct rows: thousands tie at every distance
+    dist, ids = _index(vsk, dev, cb, codes).batchSearch(q, 100)
+    rd, ri = cpu_oracle.pq_search(q, codes, cb, 100)
+    assert np.array_equal(ids, ri) and np.array_equal(dist, rd)
+    codes = rng.integers(0, 6, (n, m)).astype(np.uint8)
+    codes[n - 20_000:] = (7, 11)                                  # the nearest row of half the queries, late and in bulk
+    q[::2] = np.concatenate([cb[0, 7], cb[1, 11]]) + 0.01 * rng.standard_normal((35, m * ds)).astype(np.float32)
+    dist, ids = _index(vsk, dev, cb, codes).batchSearch(q, 100)
+    rd, ri = cpu_oracle.pq_search(q, codes, cb, 100)
+    assert np.array_equal(ids, ri) and np.array_equal(dist, rd)
+
+
+def test_non_finite_queries_do_not_disturb_the_others(vsk, dev, cpu_oracle):
+    rng = np.random.default_rng(7)
+    q, cb, x = _clustered(rng, 20_000, 80, 8, 256, 4)
+    codes = cpu_oracle.pq_encode(x, cb)
+    ix = _index(vsk, dev, cb, codes)
+    rd, ri = cpu_oracle.pq_search(q, codes, cb, 10)
+    bad = q.copy()
+    bad[3, 5], bad[70, 0] = np.nan, np.inf
+    dist, ids = ix.batchSearch(bad, 10)
+    keep = [i for i in range(80) if i not in (3, 70)]
+    assert np.array_equal(ids[keep], ri[keep]) and np.array_equal(dist[keep], rd[keep])
+    # a codebook with an infinite entry has no fp16 form: the table scan takes the batch
+    cb2 = cb.copy()
+    cb2[0, 9, 0] = np.inf
+    before = dev.stats()["tensor_tiles"]
+    dist, ids = _index(vsk, dev, cb2, codes).batchSearch(q, 10)
+    assert dev.stats()["tensor_tiles"] == before
+    rd, ri = cpu_oracle.pq_search(q, codes, cb2, 10)
+    assert np.array_equal(ids, ri) and np.array_equal(dist, rd)

@@ -214,6 +214,7 @@ enum Slot : int {
   SLOT_IVF_PROBE_D, SLOT_IVF_PROBE_I, SLOT_IVF_KEYS, SLOT_IVF_ORDER, SLOT_IVF_PAIR_OFF, SLOT_IVF_ITEM_CNT,
   SLOT_IVF_ITEM_OFF, SLOT_IVF_SUBSET, SLOT_IVF_STAGES, SLOT_KM_NSEG, SLOT_KM_SEGOFF, SLOT_KM_PARTIAL, SLOT_FILTER_PERM, SLOT_FILTER_ROWS, SLOT_FILTER_COUNT, SLOT_SQ_A, SLOT_SQ_B, SLOT_TC_A, SLOT_TC_B, SLOT_TC_C, SLOT_TC_D,
   SLOT_PQ_TABLES, SLOT_SH_D, SLOT_SH_I, SLOT_SH_SEND, SLOT_SH_RECV, SLOT_SH_BOUND, SLOT_SH_MERGED, SLOT_SH_ALL,
+  SLOT_PQ_ROWS,
   SLOT_COUNT
 };
 static_assert(SLOT_COUNT <= 64, "grow Ctx::scratch");
@@ -276,6 +277,9 @@ struct Index {
   int32_t pq_m = 0, pq_ksub = 0;   // segments, codewords per segment
   float* pq_codebooks = nullptr;   // [pq_m][pq_ksub][dim / pq_m]
   uint8_t* pq_codes = nullptr;     // [capacity][pq_m]
+  __half* pq_cb16 = nullptr;       // codebooks as fp16 operand values (made at the first tensor-path search) ...
+  float* pq_cw2 = nullptr;         // [pq_m][pq_ksub] ... and the codewords' squared norms
+  int pq_operands = 0;             // 0: not made yet, 1: usable, -1: this codebook has no usable fp16 form
 };
 
 // ---- exact_scan.cu -----------------------------------------------------------------------
@@ -392,6 +396,9 @@ int32_t schedule_max_count(int64_t seen, int64_t chunk, int32_t keep);
 // ---- pq.cu -------------------------------------------------------------------------------
 int32_t pq_search_dev(Index* ix, const float* q, int64_t nq, int32_t k, float* out_dist, int64_t* out_ids);
 int32_t pq_reserve(Index* ix, int64_t need);
+// The table scan of rows [row_begin, row_end): exact distances into the candidate lists (ScanMode `mode`).
+int32_t pq_table_scan(Index* ix, const float* tables, int64_t nq, const int32_t* q_subset, const CandLists& cand, int mode,
+                      int64_t row_begin, int64_t row_end);
 
 // ---- helpers in api.cu ---------------------------------------------------------------------
 vsk_tuning default_tuning();

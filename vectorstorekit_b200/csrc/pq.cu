@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "tensor_scan.cuh"
 
 namespace vsk {
 
@@ -385,6 +386,21 @@ int32_t pq_adopt_rows(Index* ix, int64_t n) {
   return VSK_OK;
 }
 
+int32_t pq_table_scan(Index* ix, const float* tables, int64_t nq, const int32_t* q_subset, const CandLists& cand, int mode,
+                      int64_t row_begin, int64_t row_end) {
+  PqScanArgs a{};
+  a.tables = tables;
+  a.codes = ix->pq_codes;
+  a.m = ix->pq_m;
+  a.ksub = ix->pq_ksub;
+  a.nq = nq;
+  a.q_subset = q_subset;
+  a.cand = cand;
+  a.row_begin = row_begin;
+  a.row_end = row_end;
+  return launch_pq_scan(ix->ctx, a, mode);
+}
+
 int32_t pq_search_dev(Index* ix, const float* q, int64_t nq, int32_t k, float* out_dist, int64_t* out_ids) {
   Ctx* ctx = ix->ctx;
   if (nq <= 0 || ix->n <= 0) return fail(ctx, VSK_ERR_EMPTY_INPUT, "empty queries or empty index");
@@ -400,20 +416,24 @@ int32_t pq_search_dev(Index* ix, const float* q, int64_t nq, int32_t k, float* o
     VSK_TRY(scratch(ctx, SLOT_PQ_TABLES, (size_t)bn * m * ksub * sizeof(float), &tables));
     VSK_TRY(tables_dev(ctx, ix->pq_codebooks, ix->dim, m, ksub, q + b * ix->dim, bn, (float*)tables));
     const ScanBinder bind = [=](const CandLists& cand, int64_t pn, const int32_t* sub) -> ScanFn {
-      PqScanArgs a{};
-      a.tables = (const float*)tables;
-      a.codes = ix->pq_codes;
-      a.m = m;
-      a.ksub = ksub;
-      a.nq = pn;
-      a.q_subset = sub;
-      a.cand = cand;
-      return [ctx, a](int mode, int64_t rb, int64_t re) mutable {
-        a.row_begin = rb;
-        a.row_end = re;
-        return launch_pq_scan(ctx, a, mode);
-      };
+      return [=](int mode, int64_t rb, int64_t re) { return pq_table_scan(ix, (const float*)tables, pn, sub, cand, mode, rb, re); };
     };
+    if (pq_tensor_applicable(ix, bn, k)) {
+      std::vector<int32_t> flagged;
+      bool handled = false;
+      VSK_TRY(pq_tensor_search(ix, q + b * ix->dim, bn, k, (const float*)tables, out_dist + b * k, out_ids + b * k, &flagged, &handled));
+      if (handled && flagged.empty()) continue;
+      if (handled) {
+        void* sub;
+        VSK_TRY(scratch(ctx, SLOT_SUBSET, flagged.size() * sizeof(int32_t), &sub));
+        VSK_CUDA(ctx, cudaMemcpyAsync(sub, flagged.data(), flagged.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
+        VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        ctx->stats.fallback_queries += (int64_t)flagged.size();
+        VSK_TRY(scan_topk(ctx, bind, ix->n, (int64_t)flagged.size(), (const int32_t*)sub, k, ix->id_base, 0, out_dist + b * k,
+                          out_ids + b * k, 0));
+        continue;
+      }
+    }
     VSK_TRY(scan_topk(ctx, bind, ix->n, bn, nullptr, k, ix->id_base, 0, out_dist + b * k, out_ids + b * k, 0));
   }
   VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -2723,6 +2723,329 @@ int32_t ivf_tensor_search(Index* ix, const float* q, int64_t nq, const int64_t* 
   return VSK_OK;
 }
 
+// ---- product-quantised rows on the tensor cores -------------------------------------------------------------
+// The asymmetric distance of a code row is the squared distance between the query and the row the code decodes to,
+// so a batch of queries over m-byte codes is the same contraction as over fp32 rows.  The table scan (pq.cu) does m
+// shared-memory gathers per (query, row) and is bound by them (10 000 queries x 10 000 000 rows x 16 segments: 1.6e12
+// gathers); the contraction costs 2 (d + 16) flop on the tensor cores instead.  Per chunk of rows:
+//   decode     code rows to fp16 operand rows in a bounded work buffer, |x^|^2 / 2 in sixteen folded columns (FoldArgs)
+//   contract   tc_scan_kernel with thresholds that allow for the coarse values' error
+//   re-score   every listed row from the query's table, summed in segment order: the values the table scan forms,
+//              bit for bit; the k best stay and give the next exact threshold
+// The thresholds are exact (as in the list scan above), so no certificate is needed: bulk ties of quantised distances
+// only lengthen a list, and a query whose list overflows is handed back to the table scan.
+constexpr int64_t kPqBlockBytes = 512ll << 20;   // decoded operand rows held at a time
+constexpr int PQ_DEC_ROWS = 64;                  // rows per CTA of the decode kernel
+
+// One CTA decodes PQ_DEC_ROWS rows: codes and |x^|^2 (segment sums of the codewords' norms) are staged in shared
+// memory, then every thread writes 16-byte pieces of the operand rows.  Bound by the 2 dim16 bytes a row writes.
+// DS: 2, 4, 8 = the segment length; 16 = any multiple of 8 (a piece lies inside one codeword); 0 = any length.
+template <int DS>
+__global__ void __launch_bounds__(256) pq_decode16_kernel(const uint8_t* __restrict__ codes, int64_t n, int dim, int dim16, int m,
+                                                          int ksub, int ds_rt, const __half* __restrict__ cb16,
+                                                          const float* __restrict__ cw2, float scale, int fold, int col0,
+                                                          int fold_exp, __half* __restrict__ out, float* __restrict__ aux) {
+  extern __shared__ uint8_t sc[];   // [PQ_DEC_ROWS][m]
+  __shared__ float n2[PQ_DEC_ROWS];
+  const int ds = (DS > 0 && DS <= 8) ? DS : ds_rt;
+  const int64_t r0 = (int64_t)blockIdx.x * PQ_DEC_ROWS;
+  const int rows = (int)min((int64_t)PQ_DEC_ROWS, n - r0);
+  for (int i = threadIdx.x; i < rows * m; i += blockDim.x) sc[i] = __ldg(codes + r0 * m + i);
+  __syncthreads();
+  {
+    // four threads per row
+    const int r = threadIdx.x >> 2, part = threadIdx.x & 3;
+    float s = 0.f;
+    if (r < rows)
+      for (int g = part; g < m; g += 4) s += __ldg(cw2 + (int64_t)g * ksub + sc[r * m + g]);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    if (part == 0 && r < rows) {
+      n2[r] = s;
+      if (aux) aux[r0 + r] = s;
+    }
+  }
+  __syncthreads();
+  const int pieces = dim16 >> 3;
+  for (int t = threadIdx.x; t < rows * pieces; t += blockDim.x) {
+    const int r = t / pieces, c = (t - r * pieces) * 8;
+    __align__(16) __half h[8];
+    if (fold && c >= col0 && c < col0 + kFoldCols) {
+      // pieces of R = s (|x^|^2 / 2) 2^exp as in prep_rows_kernel
+      const float R = ldexpf(0.5f * n2[r] * scale, fold_exp);
+      const __half p0 = __float2half_rn(R * 0.0625f);
+      const float r1 = R - 16.0f * __half2float(p0);
+      const __half p1 = __float2half_rn(r1 * 0.0625f);
+      const __half p2 = __float2half_rn((r1 - 16.0f * __half2float(p1)) * 0.0625f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) h[j] = __hneg(c == col0 ? (j < 4 ? p0 : p1) : p2);
+    } else if (DS > 0 && c + 8 <= dim) {
+      constexpr int W = DS > 0 ? (DS < 8 ? DS : 8) : 1;   // halves taken from one codeword
+#pragma unroll
+      for (int j = 0; j < 8; j += W) {
+        const int g = (c + j) / ds;
+        const __half* w = cb16 + ((int64_t)g * ksub + sc[r * m + g]) * ds + ((c + j) - g * ds);
+        if constexpr (W == 8) *reinterpret_cast<uint4*>(&h[j]) = __ldg(reinterpret_cast<const uint4*>(w));
+        else if constexpr (W == 4) *reinterpret_cast<uint2*>(&h[j]) = __ldg(reinterpret_cast<const uint2*>(w));
+        else if constexpr (W == 2) *reinterpret_cast<uint32_t*>(&h[j]) = __ldg(reinterpret_cast<const uint32_t*>(w));
+        else h[j] = *w;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        __half v = __float2half_rn(0.f);
+        if (c + j < dim) {
+          const int g = (c + j) / ds;
+          v = cb16[((int64_t)g * ksub + sc[r * m + g]) * ds + ((c + j) - g * ds)];
+        }
+        h[j] = v;
+      }
+    }
+    *reinterpret_cast<uint4*>(out + (r0 + r) * dim16 + c) = *reinterpret_cast<const uint4*>(h);
+  }
+}
+
+// Coarse threshold of a query from its exact one (a rooted table sum v).  v <= T means that the fp32 table sum is at
+// most T^2 up to the rounding of the root; the sum's m + ds roundings and those of |q|^2 are covered by the last two
+// terms, and eps covers the coarse value against |x^|^2 - 2 q.x^ itself.
+__global__ void pq_coarse_threshold_kernel(const float* __restrict__ thr_exact, const float* __restrict__ qnorm,
+                                           const float* __restrict__ eps, int64_t nq, float sum_terms, float norm_terms,
+                                           float* __restrict__ thr_coarse) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nq) return;
+  const float t = thr_exact[i];
+  float tc = CUDART_INF_F;
+  if (!(t == CUDART_INF_F)) {
+    const float t2 = t * t, qn2 = qnorm[i] * qnorm[i];
+    tc = (t2 - qn2) + eps[i] + 1.2e-7f * (sum_terms * t2 + norm_terms * qn2);
+  }
+  thr_coarse[i] = tc;
+}
+
+// Entries [kept, count) of a query's list are rows of the decoded block (numbered from its first row): their coarse
+// values are replaced by the table scan's exact ones, summed in segment order and rooted, and the rows get their
+// global numbers.
+__global__ void __launch_bounds__(128) pq_rescore_kernel(const float* __restrict__ tables, const uint8_t* __restrict__ codes, int m,
+                                                         int ksub, int64_t row0, int kept, CandLists cand,
+                                                         unsigned long long* total) {
+  const int64_t qi = blockIdx.x;
+  const int cnt = min(cand.count[qi], kCandCap);
+  uint64_t* keys = cand.keys + qi * kCandCap;
+  const float* tab = tables + qi * m * ksub;
+  if (threadIdx.x == 0 && cnt > kept) atomicAdd(total, (unsigned long long)(cnt - kept));
+  for (int c = kept + threadIdx.x; c < cnt; c += blockDim.x) {
+    const int64_t row = row0 + (int64_t)(uint32_t)keys[c];
+    const uint8_t* src = codes + row * m;
+    float s = 0.f;
+#pragma unroll 4
+    for (int g = 0; g < m; ++g) s = __fadd_rn(s, __ldg(tab + (int64_t)g * ksub + __ldg(src + g)));
+    keys[c] = make_key(__fsqrt_rn(s), (uint32_t)row);
+  }
+}
+
+// Operand constants of a product-quantised index, from its codebooks alone (they never change): fp16 codewords, their
+// squared norms, and upper bounds of the decoded rows' norms and residuals.
+static int32_t pq_tensor_prepare(Index* ix) {
+  Ctx* ctx = ix->ctx;
+  if (ix->pq_operands != 0) return VSK_OK;
+  const int m = ix->pq_m, ksub = ix->pq_ksub, dim = ix->dim, ds = dim / m;
+  const size_t words = (size_t)ksub * dim;
+  std::vector<float> cb(words);
+  VSK_CUDA(ctx, cudaMemcpyAsync(cb.data(), ix->pq_codebooks, words * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
+  VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  ix->pq_operands = -1;   // not usable, unless all of the following holds
+  float absmax = 0.f;
+  bool finite = true;
+  for (float v : cb) {
+    finite = finite && std::isfinite(v);
+    absmax = std::max(absmax, std::fabs(v));
+  }
+  if (!finite || !(absmax < 1e15f) || m > 512) return VSK_OK;   // (the decode kernel stages 64 m bytes of codes)
+  float scale = 1.f;
+  if (absmax > 0.f) {
+    int e;
+    std::frexp(absmax, &e);
+    if (14 - e > 100) return VSK_OK;   // codewords that are all but zero: the table scan
+    scale = std::ldexp(1.f, 14 - e);   // 2^13 <= absmax * scale < 2^14
+  }
+  std::vector<__half> h(words);
+  std::vector<float> cw2((size_t)m * ksub);
+  double norm2 = 0.0, norm16 = 0.0, err16 = 0.0;   // sums over the segments of the largest codeword's
+  for (int g = 0; g < m; ++g) {
+    double a = 0.0, b = 0.0, c = 0.0;
+    for (int w = 0; w < ksub; ++w) {
+      double x2 = 0.0, h2 = 0.0, e2 = 0.0;
+      for (int i = 0; i < ds; ++i) {
+        const size_t at = ((size_t)g * ksub + w) * ds + i;
+        h[at] = __float2half_rn(cb[at] * scale);
+        const double x = cb[at], back = __half2float(h[at]), r = x * scale - back;
+        x2 += x * x;
+        h2 += back * back;
+        e2 += r * r;
+      }
+      cw2[(size_t)g * ksub + w] = (float)x2;
+      a = std::max(a, x2);
+      b = std::max(b, h2);
+      c = std::max(c, e2);
+    }
+    norm2 += a;
+    norm16 += b;
+    err16 += c;
+  }
+  const float up = 1.0f + 1e-5f;
+  ix->dim16 = (int32_t)(ceil_div(dim, TK) * TK);
+  ix->fold16 = ctx->tuning.fold_row_term != 0 && (ix->dim16 / TK <= 4 || ix->dim16 - fold_col0(dim) >= kFoldCols);
+  if (ix->fold16 && ix->dim16 - fold_col0(dim) < kFoldCols) ix->dim16 += TK;
+  const double top = 0.5 * norm2 * scale / 16.0;
+  int e = 0;
+  if (top > 0.0) e = 14 - (int)std::ceil(std::log2(top));
+  ix->fold_exp = std::max(-100, std::min(100, e));
+  ix->fold_bmax = (float)(0.5 * norm2) * up;
+  ix->scale16 = scale;
+  ix->max_xnorm = (float)std::sqrt(norm2) * up;
+  ix->max_xnorm16 = (float)std::sqrt(norm16) * up;
+  ix->max_xerr16 = (float)std::sqrt(err16) * up;
+  ix->min_xnorm_nz = 0.f;
+  if (ix->pq_cb16 == nullptr) VSK_TRY(dev_alloc(ctx, (void**)&ix->pq_cb16, words * sizeof(__half)));
+  if (ix->pq_cw2 == nullptr) VSK_TRY(dev_alloc(ctx, (void**)&ix->pq_cw2, cw2.size() * sizeof(float)));
+  VSK_CUDA(ctx, cudaMemcpyAsync(ix->pq_cb16, h.data(), words * sizeof(__half), cudaMemcpyHostToDevice, ctx->stream));
+  VSK_CUDA(ctx, cudaMemcpyAsync(ix->pq_cw2, cw2.data(), cw2.size() * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
+  VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  ix->pq_operands = 1;
+  return VSK_OK;
+}
+
+bool pq_tensor_applicable(const Index* ix, int64_t nq, int32_t k) {
+  return ix->ctx->search_path == VSK_PATH_TENSOR_RERANK && ix->pq_operands >= 0 && nq >= kPqTensorMinQueries &&
+         ix->n >= kPqTensorMinRows && k <= kCandCap / 4;
+}
+
+int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const float* tables, float* out_dist,
+                         int64_t* out_ids, std::vector<int32_t>* flagged, bool* handled) {
+  VSK_TRACE("vsk:pq_tensor");
+  Ctx* ctx = ix->ctx;
+  *handled = false;
+  flagged->clear();
+  VSK_TRY(pq_tensor_prepare(ix));
+  if (ix->pq_operands < 0) return VSK_OK;
+  const int m = ix->pq_m, ksub = ix->pq_ksub, dim = ix->dim, dim16 = ix->dim16, ds = dim / m;
+  const int64_t n = ix->n;
+  const bool fold = ix->fold16;
+  void* p;
+  // the decoded block; without room for it the table scan takes the batch
+  const int64_t block = std::min(ceil_div(n, TN) * TN, std::max<int64_t>(TN, kPqBlockBytes / ((int64_t)dim16 * 2) / TN * TN));
+  if (scratch(ctx, SLOT_PQ_ROWS, (size_t)block * dim16 * sizeof(__half) + (size_t)block * sizeof(float), &p) != VSK_OK) return VSK_OK;
+  __half* rows16 = (__half*)p;
+  float* aux = (float*)(rows16 + block * dim16);
+  QueryOperands qo;
+  VSK_TRY(prepare_query_operands(ix, q, nq, &qo));
+  const float* qnorm = qo.eps + nq;   // |q| as the operand preparation measured it
+  CUtensorMap mq, mx;
+  VSK_TRY(make_map(ctx, qo.q16, nq, dim16, TM, &mq));
+  CandLists cand;
+  VSK_TRY(cand_lists(ctx, nq, &cand));
+  VSK_TRY(launch_init_cand(ctx, cand, nq));
+  VSK_TRY(scratch(ctx, SLOT_TC_D, (size_t)nq * sizeof(float), &p));
+  CandLists cand_coarse = cand;
+  cand_coarse.thr = (float*)p;
+  TcArgs a{};
+  a.nq = nq;
+  a.kblocks = dim16 / TK;
+  a.k16_last = k16_last_of(fold ? fold_col0(dim) + kFoldCols : dim, dim16);
+  a.mode = SCAN_THRESHOLD;
+  a.alpha = qo.alpha;
+  a.beta = fold ? nullptr : aux;
+  a.cand = cand_coarse;
+  a.cap = kCandCap;
+  a.err = qo.err;
+  SelectArgs sel{};
+  sel.cand = cand;
+  sel.nq = nq;
+  sel.keep = k;
+  sel.k = k;
+  // the first rows by the table scan: exact values, and a threshold to start from
+  int64_t seen = std::min<int64_t>(n, schedule_dense_rows(ctx, k));
+  VSK_TRY(pq_table_scan(ix, tables, nq, nullptr, cand, SCAN_DENSE, 0, seen));
+  sel.dense_count = (int32_t)seen;
+  sel.max_count = (int32_t)seen;
+  VSK_TRY(launch_select(ctx, sel));
+  sel.dense_count = -1;
+  sel.max_count = kCandCap;
+  const int64_t growth = nq <= 2048 ? std::max(16, ctx->tuning.chunk_growth) : std::max(1, ctx->tuning.chunk_growth);
+  PinnedBuf& hb = ctx->host_flags[ctx->lane];
+  VSK_TRY(pinned_reserve(ctx, &hb, (size_t)nq * 4 + 16));
+  char* hbuf = (char*)hb.p;
+  const int32_t* hflags = (const int32_t*)(hbuf + 16);
+  bool looked = false;
+  while (seen < n) {
+    int64_t chunk = std::min(schedule_chunk(seen, k, 0), std::max<int64_t>(1024, growth * seen));
+    chunk = std::max<int64_t>(TN, chunk / TN * TN);
+    chunk = std::min(std::min(chunk, block), n - seen);
+    if (!looked && 16 * seen >= n) {
+      // Most of the work is still ahead: if lists of many queries have overflowed already (rows that tie in bulk), the
+      // table scan, which can pass over a tied row, takes the whole batch.
+      VSK_CUDA(ctx, cudaMemcpyAsync(hbuf + 16, cand.flags, (size_t)nq * 4, cudaMemcpyDeviceToHost, ctx->stream));
+      VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+      int64_t bad = 0;
+      for (int64_t i = 0; i < nq; ++i) bad += hflags[i] != 0;
+      if (4 * bad > nq) return VSK_OK;
+      looked = true;
+    }
+    const unsigned dgrid = (unsigned)ceil_div(chunk, PQ_DEC_ROWS);
+    const size_t dsm = (size_t)PQ_DEC_ROWS * m;
+#define VSK_PQ_DEC(DS_)                                                                                                          \
+    pq_decode16_kernel<DS_><<<dgrid, 256, dsm, ctx->stream>>>(ix->pq_codes + seen * m, chunk, dim, dim16, m, ksub, ds, ix->pq_cb16, \
+                                                              ix->pq_cw2, ix->scale16, fold ? 1 : 0, fold_col0(dim), ix->fold_exp,  \
+                                                              rows16, fold ? nullptr : aux)
+    if (ds == 8) VSK_PQ_DEC(8);
+    else if (ds % 8 == 0) VSK_PQ_DEC(16);
+    else if (ds == 4) VSK_PQ_DEC(4);
+    else if (ds == 2) VSK_PQ_DEC(2);
+    else VSK_PQ_DEC(0);
+#undef VSK_PQ_DEC
+    pq_coarse_threshold_kernel<<<(unsigned)ceil_div(nq, 256), 256, 0, ctx->stream>>>(
+        cand.thr, qnorm, qo.eps, nq, (float)(m + ds + 8), (float)(ceil_div(dim, 32) + 16), cand_coarse.thr);
+    ctx->stats.kernel_launches += 2;
+    VSK_CUDA(ctx, cudaGetLastError());
+    VSK_TRY(make_map(ctx, rows16, chunk, dim16, TN, &mx));
+    a.row_begin = 0;
+    a.row_end = chunk;
+    VSK_TRY(launch_tc<SCAN_THRESHOLD>(ctx, mq, mx, a, !fold));
+    pq_rescore_kernel<<<(unsigned)nq, 128, 0, ctx->stream>>>(tables, ix->pq_codes, m, ksub, seen, (int)std::min<int64_t>(k, seen), cand, qo.rr_total);
+    ctx->stats.kernel_launches++;
+    VSK_CUDA(ctx, cudaGetLastError());
+    tl_mark(ctx, "pq_rescore");
+    VSK_TRY(launch_select(ctx, sel));
+    seen += chunk;
+  }
+  SelectArgs fin{};
+  fin.cand = cand;
+  fin.nq = nq;
+  fin.dense_count = -1;
+  fin.keep = k;
+  fin.out_dist = out_dist;
+  fin.out_ids = out_ids;
+  fin.k = k;
+  fin.id_base = ix->id_base;
+  fin.max_count = k;
+  VSK_TRY(launch_select(ctx, fin));
+  VSK_CUDA(ctx, cudaMemcpyAsync(hbuf, qo.err, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  VSK_CUDA(ctx, cudaMemcpyAsync(hbuf + 8, qo.rr_total, 8, cudaMemcpyDeviceToHost, ctx->stream));
+  VSK_CUDA(ctx, cudaMemcpyAsync(hbuf + 16, cand.flags, (size_t)nq * 4, cudaMemcpyDeviceToHost, ctx->stream));
+  VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  int32_t herr;
+  unsigned long long hrr;
+  memcpy(&herr, hbuf, 4);
+  memcpy(&hrr, hbuf + 8, 8);
+  ctx->stats.reranked_rows += (int64_t)hrr;
+  if (herr != 0)
+    return fail(ctx, VSK_ERR_TIMEOUT, "tensor-core scan: a bounded pipeline wait ran out (role %d)", herr);
+  for (int64_t i = 0; i < nq; ++i)
+    if (hflags[i]) flagged->push_back((int32_t)i);
+  *handled = true;
+  return VSK_OK;
+}
+
 // ---- public: tensor-core nearest-centroid assignment (used by kmeans.cu) ---------------------------
 int32_t tensor_assign_prepare(Ctx* ctx, const float* rows, int64_t n, int32_t dim, TensorAssign* ta) {
   ta->n = n;

@@ -36,6 +36,14 @@ int32_t tensor_coarse_values(Index* ix, const float* q, int64_t nq, int64_t rows
 bool ivf_tensor_applicable(const Index* ix, int64_t nq, int32_t nprobe, int32_t k);
 int32_t ivf_tensor_search(Index* ix, const float* q, int64_t nq, const int64_t* probes, int32_t nprobe, int32_t k,
                           const uint64_t* qmasks, float* out_dist, int64_t* out_ids, std::vector<int32_t>* flagged);
+// A batch over a product-quantised index: code rows decoded block by block into fp16 operand rows, contracted, and the
+// listed rows re-scored from the queries' distance tables (device [nq][m][ksub]), so that results equal the table
+// scan's bit for bit.  *handled = false (nothing written): the table scan takes the batch.  Queries whose list
+// overflowed are returned in `flagged` for the table scan.
+constexpr int64_t kPqTensorMinQueries = 64, kPqTensorMinRows = 16384;
+bool pq_tensor_applicable(const Index* ix, int64_t nq, int32_t k);
+int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const float* tables, float* out_dist,
+                         int64_t* out_ids, std::vector<int32_t>* flagged, bool* handled);
 // Drops the fp16 operand copy after rows were added; makes it (once per index state).
 void tensor_invalidate(Index* ix);
 int32_t tensor_prepare_index(Index* ix);
