@@ -1,0 +1,73 @@
+"""dotProduct batches over int8 codes on the integer contraction (8-bit queries, exact accumulators, listed rows re-scored
+against the dequantised rows): the rows the CPU oracle finds, for operand widths around its K blocks and TMA strides."""
+import numpy as np
+import pytest
+
+import oracle
+from parity import assert_topk_parity
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def vsk():
+    import vectorstorekit_b200 as v
+    return v
+
+
+@pytest.fixture(scope="module")
+def dev(vsk):
+    return vsk.CUDAAcceleratorStrategy(0).initialize()
+
+
+def _quantised(vsk, dev, x):
+    """(index, codes, scale, offset) of the rows, quantised per dimension."""
+    quantizer = vsk.ScalarQuantizer(dev, per_dim=True)
+    quantizer.train(x)
+    codes = quantizer.quantizeBatch(x)
+    ix = vsk.QuantizedFlatIndex(dev, x.shape[1], vsk.DistanceMetric.dotProduct, quantizer.scale, quantizer.offset)
+    ix.add(codes)
+    return ix, np.asarray(codes), np.asarray(quantizer.scale, np.float32), np.asarray(quantizer.offset, np.float32)
+
+
+def _check(cpu_oracle, ix, codes, scale, offset, q, k):
+    d, i = ix.batchSearch(q, k)
+    rd, ri = cpu_oracle.sq8_search(oracle.DOT, q, codes, scale, offset, k)
+    assert_topk_parity(d, i, rd, ri)
+
+
+# one and several K blocks of 128 codes, partial 32-byte steps, rows padded for TMA (dim not a multiple of 16), the
+# smallest index of the path, partial tiles, one query, k up to the path's limit
+@pytest.mark.parametrize("shape", [(16_384, 128, 128, 10), (16_385, 129, 1, 10), (20_000, 16, 300, 37), (20_001, 33, 65, 1),
+                                   (30_000, 384, 200, 10), (17_003, 250, 130, 100), (16_400, 513, 9, 10), (40_000, 64, 64, 1024)])
+def test_integer_contraction_finds_the_oracles_rows(vsk, dev, cpu_oracle, shape):
+    n, d, nq, k = shape
+    rng = np.random.default_rng(n + d + nq)
+    x = rng.standard_normal((n, d)).astype(np.float32) * rng.uniform(0.2, 3.0, d).astype(np.float32) + rng.normal(0, 1, d).astype(np.float32)
+    q = rng.standard_normal((nq, d)).astype(np.float32)
+    ix, codes, scale, offset = _quantised(vsk, dev, x)
+    before = dev.stats()["tensor_tiles"]
+    _check(cpu_oracle, ix, codes, scale, offset, q, k)
+    assert dev.stats()["tensor_tiles"] > before
+    # rows added later are seen
+    ix.add(codes[:257])
+    _check(cpu_oracle, ix, np.concatenate([codes, codes[:257]]), scale, offset, q, k)
+
+
+def test_lists_that_overflow_go_to_the_other_paths(vsk, dev, cpu_oracle):
+    """Rows of one direction and many norms, in ascending order of their products: every later row passes the bar.  The
+    answer is the same, on the batch's first search and on the ones after it."""
+    rng = np.random.default_rng(8)
+    n, d = 30_000, 48
+    base = rng.standard_normal(d).astype(np.float32)
+    x = np.linspace(0.01, 1.0, n, dtype=np.float32)[:, None] * base + 1e-3 * rng.standard_normal((n, d)).astype(np.float32)
+    ix, codes, scale, offset = _quantised(vsk, dev, x)
+    q = (base + 0.1 * rng.standard_normal((300, d))).astype(np.float32)
+    for _ in range(2):
+        _check(cpu_oracle, ix, codes, scale, offset, q, 20)
+    q[7, 3] = np.inf
+    q[9] = 0.0
+    d_, i_ = ix.batchSearch(q, 20)
+    keep = [i for i in range(300) if i not in (7, 9)]
+    rd, ri = cpu_oracle.sq8_search(oracle.DOT, q[keep], codes, scale, offset, 20)
+    assert_topk_parity(d_[keep], i_[keep], rd, ri)

@@ -933,6 +933,7 @@ int32_t vsk_index_destroy(vsk_index* i) {
   dev_free(ix->assign);
   dev_free(ix->pq_codebooks);
   dev_free(ix->pq_codes);
+  dev_free(ix->rows8);
   dev_free(ix->pq_cb16);
   dev_free(ix->pq_cw2);
   if (ix->coarse) {   // shares the centroids: only its derived buffers are its own

@@ -264,6 +264,12 @@ struct Index {
   int8_t* codes = nullptr;     // [capacity][dim]
   float* sq_scale = nullptr;   // [dim]
   float* sq_offset = nullptr;  // [dim]
+  // integer contraction over the codes (tensor_scan.cu: i8_search)
+  int8_t* rows8 = nullptr;     // [n][stride8] padded copy where dim is not a multiple of 16, else null: the codes serve
+  int32_t stride8 = 0;
+  int64_t n8 = -1;             // rows the two norms cover
+  int i8_rest = 0;             // batches still to be left to the fp16 path
+  float max_code_norm = 0.f, max_xnorm8 = 0.f;   // largest norm of a code row / of a decoded row
   // ivf
   int32_t nlist = 0;
   float* centroids = nullptr;      // [nlist][dim]

@@ -218,6 +218,11 @@ int32_t sq8_search_dev(Index* ix, const float* q, int64_t nq, int32_t k, float* 
                       (ix->metric == VSK_METRIC_DOT_PRODUCT || ix->metric == VSK_METRIC_EUCLIDEAN);
   for (int64_t b = 0; b < nq; b += kBatch) {
     const int64_t bn = std::min(kBatch, nq - b);
+    if (i8_search_applicable(ix, k)) {
+      bool handled = false;
+      VSK_TRY(i8_search(ix, q + b * ix->dim, bn, k, out_dist + b * k, out_ids + b * k, &handled));
+      if (handled) continue;
+    }
     if (tensor) {
       VSK_TRY(tensor_search(ix, q + b * ix->dim, bn, k, nullptr, nullptr, out_dist + b * k, out_ids + b * k));
       continue;

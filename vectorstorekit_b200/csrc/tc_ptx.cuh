@@ -103,6 +103,16 @@ __device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t
       : "memory");
 }
 
+// The same tile in 8-bit integers: s8 x s8 -> s32 (exact), K = 32 - the same 32 bytes per row and step
+__device__ __forceinline__ void tc_mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
 // 32 consecutive fp32 columns of this thread's tensor-memory lane
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
   uint32_t r[32];
@@ -222,6 +232,9 @@ __device__ __forceinline__ void tc_commit_a(uint32_t bar) {
 
 // Instruction descriptor: fp32 accumulate, fp16 A and B, both K-major, N = 256, M = 128.
 constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+
+// ... and s32 accumulate, s8 A and B.
+constexpr uint32_t kIdescI8 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
 
 }  // namespace tc
 }  // namespace vsk

@@ -30,6 +30,7 @@
 #include <cuda.h>
 #include <math_constants.h>
 
+#include <climits>
 #include <cmath>
 
 #include "common.cuh"
@@ -111,7 +112,10 @@ struct TcArgs {
 };
 
 
-template <int MODE, bool HAS_BETA, bool HAS_MASK, int EW>
+// I8 (threshold mode, plain grid): both operands are 8-bit integers, 128 to a K block, and the accumulators exact 32-bit
+// integers.  cand.thr then holds, as integer bits, the accumulator a row must reach; a listed key carries the row only
+// (its value is formed by the re-scoring).
+template <int MODE, bool HAS_BETA, bool HAS_MASK, int EW, bool I8 = false>
 __global__ void __launch_bounds__(Epi<EW>::THREADS, 1)
 tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_x, TcArgs a) {
   extern __shared__ uint8_t smem_raw[];
@@ -122,6 +126,8 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   const int64_t unit = blockIdx.x;
   const int64_t units = gridDim.x;
   constexpr int QT = TM;  // queries per tile
+  constexpr int KCOLS = I8 ? 2 * TK : TK;   // operand columns of a K block (128 bytes)
+  static_assert(!I8 || (MODE == SCAN_THRESHOLD && !HAS_BETA && !HAS_MASK), "integer operands: plain threshold scans only");
   const uint32_t wait_limit = a.wait_limit ? a.wait_limit : WAIT_LIMIT;
   const int kps = a.stage_kblocks == 2 ? 2 : 1;   // K blocks per ring stage
   const int nstages = STAGES / kps;
@@ -205,8 +211,8 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           } else {
             mbar_expect_tx(&sm->full[s], (uint32_t)(nkb * STAGE_BYTES));
             for (int j = 0; j < nkb; ++j) {
-              tma_load_2d(st + j * STAGE_BYTES, &map_q, &sm->full[s], (kb + j) * TK, qrow);
-              tma_load_2d(st + j * STAGE_BYTES + A_BYTES, &map_x, &sm->full[s], (kb + j) * TK, xrow);
+              tma_load_2d(st + j * STAGE_BYTES, &map_q, &sm->full[s], (kb + j) * KCOLS, qrow);
+              tma_load_2d(st + j * STAGE_BYTES + A_BYTES, &map_x, &sm->full[s], (kb + j) * KCOLS, xrow);
             }
             issued |= 1u << s;
             issued_ph = (issued_ph & ~(1u << s)) | (ph << s);
@@ -253,8 +259,11 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             const int nk4 = kb == a.kblocks - 1 ? last_nk4 : TK / 16;
 #pragma unroll
             for (int k4 = 0; k4 < TK / 16; ++k4) {
-              // 16 fp16 = 32 bytes further along K inside the swizzle atom: +2 in 16-byte units
-              if (k4 < nk4)
+              // 16 fp16 (32 int8) = 32 bytes further along K inside the swizzle atom: +2 in 16-byte units
+              if (I8 && k4 < nk4)
+                tc_mma_i8(tmem_d, desc_pack(a_lo + (uint32_t)(k4 * 2), kDescHi), desc_pack(b_lo + (uint32_t)(k4 * 2), kDescHi), kIdescI8,
+                          (kb | k4) ? 1u : 0u);
+              else if (k4 < nk4)
                 tc_mma(tmem_d, desc_pack(a_lo + (uint32_t)(k4 * 2), kDescHi), desc_pack(b_lo + (uint32_t)(k4 * 2), kDescHi), kIdesc,
                        (kb | k4) ? 1u : 0u);
             }
@@ -428,7 +437,15 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           // Cheap test first: the smallest of the group's 32 values against the threshold.  Most groups of a late
           // chunk hold no hit for any of the warp's queries and then cost two instructions per value, not five.
           float vmin = CUDART_INF_F;
-          if (!HAS_BETA && alpha < 0.f) {
+          if constexpr (I8) {
+            int top = __float_as_int(v[0]);
+#pragma unroll
+            for (int j = 1; j < 32; ++j) top = max(top, __float_as_int(v[j]));
+            if (left >= 32 && !__any_sync(0xffffffffu, qok && top >= __float_as_int(thr))) {
+              m[c - c0] = 0u;
+              continue;
+            }
+          } else if (!HAS_BETA && alpha < 0.f) {
             // value = alpha * accumulator with alpha < 0: the smallest value is alpha times the largest accumulator
             // (the multiplication is monotone, so this is the same number), one instruction per value; the values
             // themselves are only formed for a group that has a hit
@@ -459,7 +476,7 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             const float val = v[j];
-            const bool hit = val <= thr;
+            const bool hit = I8 ? __float_as_int(val) >= __float_as_int(thr) : val <= thr;
             bits |= hit ? (1u << j) : 0u;
             hv = hit ? val : hv;
           }
@@ -493,7 +510,7 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           if (!HAS_MASK && !__any_sync(0xffffffffu, (bits & (bits - 1u)) != 0u) && n0 + c * 32 + 32 <= row_end) {
             // no query has more than one hit in this (whole) group: its value was kept by pass 1
             const uint32_t ok1 = (bits != 0u && base < cap_here) ? 1u : 0u;
-            const uint64_t key1 = make_key(mv[c - c0], (uint32_t)(n0 + c * 32 + (__ffs((int)bits) - 1)));
+            const uint64_t key1 = make_key(I8 ? 0.f : mv[c - c0], (uint32_t)(n0 + c * 32 + (__ffs((int)bits) - 1)));
             uint64_t* d1 = a.cand.keys + q * a.cap + (owned ? part * cap_here : 0) + base;
             asm volatile(
                 "{\n\t.reg .pred p;\n\t"
@@ -505,7 +522,7 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             continue;
           }
           float v[32];
-          tc_ld32(trow + (uint32_t)(c * 32), v);
+          if constexpr (!I8) tc_ld32(trow + (uint32_t)(c * 32), v);
           const int64_t nc = n0 + c * 32;
           uint64_t* dst = a.cand.keys + q * a.cap + (owned ? part * cap_here : 0) + base;
           // Straight-line code with predicated stores: a branch around every store makes the warp wait out each
@@ -517,7 +534,7 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #pragma unroll
             for (int jj = 0; jj < 8; ++jj) {
               const int j = o * 8 + jj;
-              const float val = HAS_BETA ? fmaf(v[j], alpha, sm->beta[acc][ew][(c - c0) * 32 + j]) : v[j] * alpha;
+              const float val = I8 ? 0.f : HAS_BETA ? fmaf(v[j], alpha, sm->beta[acc][ew][(c - c0) * 32 + j]) : v[j] * alpha;
               const int rank = __popc(bits & ((1u << j) - 1u));
               const uint32_t ok = (((bits >> j) & 1u) != 0u && base + rank < cap_here) ? 1u : 0u;
               const uint64_t key = make_key(val, (uint32_t)(nc + j));
@@ -1478,6 +1495,22 @@ int32_t make_map_narrow(Ctx* ctx, const __half* base, int64_t rows, int32_t dim1
   return VSK_OK;
 }
 
+// int8 matrix [rows][stride bytes], `cols` of them valid: box = 128 columns x box_rows, 128-byte swizzle; columns past
+// `cols` and rows past `rows` read as zero.  stride must be a multiple of 16.
+int32_t make_map_i8(Ctx* ctx, const int8_t* base, int64_t rows, int32_t cols, int32_t stride, int box_rows, CUtensorMap* map) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(ctx, VSK_ERR_EXECUTION_FAILED, "cuTensorMapEncodeTiled is not available from this driver");
+  cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t gstride[1] = {(cuuint64_t)stride};
+  cuuint32_t box[2] = {(cuuint32_t)(2 * TK), (cuuint32_t)box_rows};
+  cuuint32_t estride[2] = {1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t*>(base), gdim, gstride, box, estride,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(ctx, VSK_ERR_EXECUTION_FAILED, "cuTensorMapEncodeTiled (int8) failed with %d", (int)r);
+  return VSK_OK;
+}
+
 template <int METRIC>
 void launch_prep(Ctx* ctx, const float* x, int64_t n, int dim, int dim16, const float* scale, __half* out, float* aux,
                  float* nrm16, float* err16, float* nrm, PrepStats* stats, FoldArgs fold = FoldArgs{0, 0, 0}) {
@@ -1588,12 +1621,14 @@ int32_t tensor_prepare(Index* ix) {
 }
 
 // Launches the scan over tiles (persistent: one CTA per SM, or per tile when there are fewer tiles).
-template <int MODE, int EW>
+template <int MODE, int EW, bool I8 = false>
 int32_t launch_tc_ew(Ctx* ctx, const CUtensorMap& mq, const CUtensorMap& mx, const TcArgs& a, bool has_beta) {
   static bool attr_done[2][2] = {};
   const bool has_mask = MODE != SCAN_ARGMIN && a.row_masks != nullptr && a.q_masks != nullptr;
   void (*kern)(CUtensorMap, CUtensorMap, TcArgs);
-  if constexpr (MODE == SCAN_ARGMIN) {
+  if constexpr (I8) {
+    kern = tc_scan_kernel<MODE, false, false, EW, true>;
+  } else if constexpr (MODE == SCAN_ARGMIN) {
     kern = has_beta ? tc_scan_kernel<MODE, true, false, EW> : tc_scan_kernel<MODE, false, false, EW>;
   } else {
     kern = has_mask ? (has_beta ? tc_scan_kernel<MODE, true, true, EW> : tc_scan_kernel<MODE, false, true, EW>)
@@ -1945,7 +1980,11 @@ int32_t launch_assign_scan(Ctx* ctx, const CUtensorMap& mx, const CUtensorMap& m
 
 }  // namespace
 
-void tensor_invalidate(Index* ix) { ix->n16 = -1; }
+void tensor_invalidate(Index* ix) {
+  ix->n16 = -1;
+  ix->n8 = -1;
+  ix->i8_rest = 0;
+}
 int32_t tensor_prepare_index(Index* ix) { return tensor_prepare(ix); }
 
 // ---- query operands of a flat search ------------------------------------------------------------------
@@ -3042,6 +3081,307 @@ int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const
     return fail(ctx, VSK_ERR_TIMEOUT, "tensor-core scan: a bounded pipeline wait ran out (role %d)", herr);
   for (int64_t i = 0; i < nq; ++i)
     if (hflags[i]) flagged->push_back((int32_t)i);
+  *handled = true;
+  return VSK_OK;
+}
+
+// ---- int8 codes against int8 queries (dotProduct) -----------------------------------------------------------
+// sum_i q_i x^_i = sum_i q~_i c_i - K with q~ = q / scale, c the codes and K = sum_i q_i offset_i / scale_i.  With q~ rounded
+// to 8 bits (one scale s per query) the contraction runs on the codes as they are stored, at twice the fp16 rate, half
+// the operand bytes and no operand copy of the rows, and its accumulators are exact integers.  What is lost is the
+// query's rounding, |e| C at most (C = largest norm of a code row): too wide for the certificate of the fp16 path,
+// which compares the k-th value with one a few keys further down, so the thresholds are exact instead (every listed row
+// is re-scored after each chunk), as in the list scan: a row is listed iff  A = sum_i q8_i c_i  reaches
+//   s (K - T - |e| C - rounding),   T the k-th exact value so far.
+// 10 000 queries x 6.25 million rows x 384, k = 10: 40.6 ms on the fp16 path, 27.8 ms here.
+struct I8Query {
+  float inv_step;    // s: q8 = round(s q~)
+  float slack;       // |e| C plus the fp32 roundings of the exact values, in true units
+  double offset;     // K
+};
+
+// One warp per query.  A query that is not finite gets an infinite slack: its list overflows and it is re-run.
+__global__ void i8_query_kernel(const float* __restrict__ q, int64_t nq, int dim, int stride, const float* __restrict__ scale,
+                                const float* __restrict__ offset, float max_code_norm, float max_xnorm, int8_t* __restrict__ out,
+                                I8Query* __restrict__ info) {
+  const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= nq) return;
+  const int lane = threadIdx.x & 31;
+  const float* p = q + row * dim;
+  float amax = 0.f, q2 = 0.f, t2 = 0.f;
+  double k = 0.0;
+  bool finite = true;
+  for (int i = lane; i < dim; i += 32) {
+    const float v = __ldg(p + i), sc = __ldg(scale + i), t = __fdiv_rn(v, sc);
+    finite = finite && isfinite(t) && isfinite(v);
+    amax = fmaxf(amax, fabsf(t));
+    q2 = fmaf(v, v, q2);
+    t2 = fmaf(t, t, t2);
+    k += (double)v * (double)__ldg(offset + i) / (double)sc;
+  }
+  finite = __all_sync(0xffffffffu, finite);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    q2 += __shfl_xor_sync(0xffffffffu, q2, o);
+    t2 += __shfl_xor_sync(0xffffffffu, t2, o);
+    k += __shfl_xor_sync(0xffffffffu, k, o);
+  }
+  const bool usable = finite && amax > 1e-30f && amax < 1e30f;
+  const float s = usable ? 127.0f / amax : 1.0f;
+  float e2 = 0.f;
+  for (int i = lane; i < stride; i += 32) {
+    int c = 0;
+    if (usable && i < dim) {
+      const float t = __fdiv_rn(__ldg(p + i), __ldg(scale + i));
+      c = max(-127, min(127, __float2int_rn(t * s)));
+      const float e = fmaf((float)c, -amax * (1.0f / 127.0f), t);
+      e2 = fmaf(e, e, e2);
+    }
+    out[row * stride + i] = (int8_t)c;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) e2 += __shfl_xor_sync(0xffffffffu, e2, o);
+  if (lane == 0) {
+    const float qn = sqrtf(q2), tn = sqrtf(t2);
+    I8Query r;
+    r.inv_step = s;
+    r.offset = k;
+    // the step and q~ are rounded to 2^-22 at worst; an exact value is a sum of dim products of q with x^ = (c - offset)
+    // / scale, whose roundings are below (dim + 8) 2^-23 |q| |x^|
+    r.slack = (sqrtf(e2) * 1.0001f + 1e-6f * tn) * max_code_norm + 1.2e-7f * (float)(dim + 8) * qn * max_xnorm;
+    if (!finite) r.slack = CUDART_INF_F;
+    else if (!usable) r.slack = tn * max_code_norm * 1.0001f + 1.2e-7f * (float)(dim + 8) * qn * max_xnorm;   // q8 = 0
+    info[row] = r;
+  }
+}
+
+// The accumulator a row must reach, from the query's exact threshold (values are -(q.x^)).
+__global__ void i8_bar_kernel(const float* __restrict__ thr_exact, const I8Query* __restrict__ info, int64_t nq,
+                              int32_t* __restrict__ bar) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nq) return;
+  const I8Query r = info[i];
+  const double at = floor((double)r.inv_step * (r.offset - (double)thr_exact[i] - (double)r.slack)) - 1.0;
+  // not a number or below every accumulator: every row is listed (and the list overflows)
+  bar[i] = !(at > -2147483647.0) ? INT_MIN : at > 2147483646.0 ? INT_MAX : (int32_t)at;
+}
+
+// Largest norm of a code row and of its decoded row (the stored codes themselves are the operand).
+__global__ void i8_row_stats_kernel(const int8_t* __restrict__ codes, int64_t n, int dim, const float* __restrict__ scale,
+                                    const float* __restrict__ offset, PrepStats* stats) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  float cmax = 0.f, xmax = 0.f;
+  for (int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < n; row += warps) {
+    const int8_t* p = codes + row * dim;
+    float c2 = 0.f, x2 = 0.f;
+    for (int i = lane; i < dim; i += 32) {
+      const float c = (float)__ldg(p + i), xh = __fdiv_rn(__fsub_rn(c, __ldg(offset + i)), __ldg(scale + i));
+      c2 = fmaf(c, c, c2);
+      x2 = fmaf(xh, xh, x2);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      c2 += __shfl_xor_sync(0xffffffffu, c2, o);
+      x2 += __shfl_xor_sync(0xffffffffu, x2, o);
+    }
+    cmax = fmaxf(cmax, c2);
+    xmax = !(x2 <= xmax) ? x2 : xmax;   // a decoded value that is not a number stays one
+  }
+  if (lane == 0) {
+    const float up = 1.0f + 1e-5f;
+    atomicMax(&stats->max_norm16, __float_as_uint(sqrtf(cmax) * up));
+    atomicMax(&stats->max_norm, __float_as_uint(fabsf(sqrtf(xmax) * up)));
+  }
+}
+
+__global__ void i8_pad_rows_kernel(const int8_t* __restrict__ codes, int64_t n, int dim, int stride, int8_t* __restrict__ out) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n * stride) return;
+  const int64_t r = i / stride;
+  const int c = (int)(i - r * stride);
+  out[i] = c < dim ? __ldg(codes + r * dim + c) : (int8_t)0;
+}
+
+// Once per index state: the norms of the error bound, and a copy with rows padded to 16 bytes (TMA strides) where the
+// dimension is not a multiple of 16.
+static int32_t i8_prepare(Index* ix) {
+  Ctx* ctx = ix->ctx;
+  if (ix->n8 == ix->n) return VSK_OK;
+  dev_free(ix->rows8);
+  ix->rows8 = nullptr;
+  ix->stride8 = (int32_t)(ceil_div(ix->dim, 16) * 16);
+  if (ix->stride8 != ix->dim) {
+    VSK_TRY(dev_alloc(ctx, (void**)&ix->rows8, (size_t)ix->n * ix->stride8));
+    i8_pad_rows_kernel<<<(unsigned)ceil_div(ix->n * ix->stride8, 256), 256, 0, ctx->stream>>>(ix->codes, ix->n, ix->dim, ix->stride8, ix->rows8);
+    ctx->stats.kernel_launches++;
+  }
+  void* p;
+  VSK_TRY(scratch(ctx, SLOT_TC_A, sizeof(PrepStats), &p));
+  VSK_CUDA(ctx, cudaMemsetAsync(p, 0, sizeof(PrepStats), ctx->stream));
+  i8_row_stats_kernel<<<(unsigned)std::min<int64_t>(ceil_div(ix->n, 8), 148 * 8), 256, 0, ctx->stream>>>(
+      ix->codes, ix->n, ix->dim, ix->sq_scale, ix->sq_offset, (PrepStats*)p);
+  ctx->stats.kernel_launches++;
+  VSK_CUDA(ctx, cudaGetLastError());
+  PrepStats h;
+  VSK_CUDA(ctx, cudaMemcpyAsync(&h, p, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
+  VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  memcpy(&ix->max_code_norm, &h.max_norm16, 4);
+  memcpy(&ix->max_xnorm8, &h.max_norm, 4);
+  ix->n8 = ix->n;
+  ix->i8_rest = 0;
+  return VSK_OK;
+}
+
+constexpr int kI8Rest = 15;   // batches an index leaves to the fp16 path after one that did not fit this one
+
+bool i8_search_applicable(const Index* ix, int32_t k) {
+  // 127 * 128 * dim below 2^31: no accumulator can overflow
+  return ix->kind == INDEX_FLAT_I8 && ix->metric == VSK_METRIC_DOT_PRODUCT && ix->ctx->search_path == VSK_PATH_TENSOR_RERANK &&
+         k <= kCandCap / 4 && ix->dim <= 12 * 1024 && ix->n >= kI8MinRows;
+}
+
+int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_dist, int64_t* out_ids, bool* handled) {
+  VSK_TRACE("vsk:i8_scan");
+  Ctx* ctx = ix->ctx;
+  *handled = false;
+  if (ix->i8_rest > 0) {
+    --ix->i8_rest;
+    return VSK_OK;
+  }
+  VSK_TRY(i8_prepare(ix));
+  const float limit = 1e30f;
+  if (!(ix->max_code_norm < limit) || !(ix->max_xnorm8 < limit)) return VSK_OK;
+  const int dim = ix->dim, stride = ix->stride8;
+  const int64_t n = ix->n;
+  void* p;
+  VSK_TRY(scratch(ctx, SLOT_Q16, (size_t)nq * stride, &p));
+  int8_t* q8 = (int8_t*)p;
+  VSK_TRY(scratch(ctx, SLOT_QAUX, (size_t)nq * (sizeof(I8Query) + 4), &p));
+  I8Query* info = (I8Query*)p;
+  int32_t* bar = (int32_t*)(info + nq);
+  VSK_TRY(scratch(ctx, SLOT_TC_B, 64, &p));
+  VSK_CUDA(ctx, cudaMemsetAsync(p, 0, 64, ctx->stream));
+  const float* alpha = (const float*)p + 2;
+  int32_t* err = (int32_t*)p + 3;
+  unsigned long long* rr_total = (unsigned long long*)((char*)p + 16);
+  i8_query_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, ctx->stream>>>(q, nq, dim, stride, ix->sq_scale, ix->sq_offset, ix->max_code_norm,
+                                                                      ix->max_xnorm8, q8, info);
+  ctx->stats.kernel_launches++;
+  CUtensorMap mq, mx;
+  VSK_TRY(make_map_i8(ctx, q8, nq, dim, stride, TM, &mq));
+  VSK_TRY(make_map_i8(ctx, ix->rows8 ? ix->rows8 : ix->codes, n, dim, stride, TN, &mx));
+  CandLists cand;
+  VSK_TRY(cand_lists(ctx, nq, &cand));
+  VSK_TRY(launch_init_cand(ctx, cand, nq));
+  TcArgs a{};
+  a.nq = nq;
+  a.kblocks = (int32_t)ceil_div(dim, 2 * TK);
+  a.k16_last = (int32_t)(ceil_div(dim, 32) - 4 * (a.kblocks - 1));
+  a.mode = SCAN_THRESHOLD;
+  a.alpha = alpha;
+  a.cand = cand;
+  a.cand.thr = (float*)bar;
+  a.cap = kCandCap;
+  a.err = err;
+  // the first rows by the fp32 scan: exact values, and a threshold to start from
+  int64_t seen = std::min<int64_t>(n, schedule_dense_rows(ctx, k));
+  ExactScanArgs ea{};
+  ea.metric = ix->metric;
+  ea.mode = SCAN_DENSE;
+  ea.q = q;
+  ea.x_codes = ix->codes;
+  ea.sq_scale = ix->sq_scale;
+  ea.sq_offset = ix->sq_offset;
+  ea.dim = dim;
+  ea.nq = nq;
+  ea.row_end = seen;
+  ea.bm_hint = nq <= 32 ? 32 : nq <= 64 ? 64 : 0;
+  ea.cand = cand;
+  VSK_TRY(launch_exact_scan(ctx, ea));
+  SelectArgs sel{};
+  sel.cand = cand;
+  sel.nq = nq;
+  sel.keep = k;
+  sel.k = k;
+  sel.dense_count = (int32_t)seen;
+  sel.max_count = (int32_t)seen;
+  VSK_TRY(launch_select(ctx, sel));
+  sel.dense_count = -1;
+  sel.max_count = kCandCap;
+  PinnedBuf& hb = ctx->host_flags[ctx->lane];
+  VSK_TRY(pinned_reserve(ctx, &hb, (size_t)nq * 4 + 16));
+  char* hbuf = (char*)hb.p;
+  const int32_t* hflags = (const int32_t*)(hbuf + 16);
+  auto count_flagged = [&] {
+    int64_t bad = 0;
+    for (int64_t i = 0; i < nq; ++i) bad += hflags[i] != 0;
+    return bad;
+  };
+  const size_t qsm = (size_t)dim * sizeof(float);
+  const int64_t growth = nq <= 2048 ? std::max(16, ctx->tuning.chunk_growth) : std::max(1, ctx->tuning.chunk_growth);
+  bool looked = nq < 256;   // a small batch is cheap to scan twice: no look between its chunks
+  while (seen < n) {
+    // half of the plain schedule's chunk: the bar admits about twice the rows the exact threshold would
+    int64_t chunk = std::min(schedule_chunk(seen, k, 0) / 2, std::max<int64_t>(1024, growth * seen));
+    chunk = std::max<int64_t>(TN, chunk / TN * TN);
+    chunk = std::min(chunk, n - seen);
+    if (!looked && 16 * seen >= n) {
+      // most of the work is still ahead: where many lists have overflowed already (norms far apart, so that |e| C is wide
+      // against the spread of the values), the fp16 path takes the batch
+      VSK_CUDA(ctx, cudaMemcpyAsync(hbuf + 16, cand.flags, (size_t)nq * 4, cudaMemcpyDeviceToHost, ctx->stream));
+      VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+      if (64 * count_flagged() > nq) {
+        ix->i8_rest = kI8Rest;
+        return VSK_OK;
+      }
+      looked = true;
+    }
+    i8_bar_kernel<<<(unsigned)ceil_div(nq, 256), 256, 0, ctx->stream>>>(cand.thr, info, nq, bar);
+    ctx->stats.kernel_launches++;
+    a.row_begin = seen;
+    a.row_end = seen + chunk;
+    if (tc_epilogue_warps(a.kblocks) == 16) VSK_TRY((launch_tc_ew<SCAN_THRESHOLD, 16, true>(ctx, mq, mx, a, false)));
+    else VSK_TRY((launch_tc_ew<SCAN_THRESHOLD, 8, true>(ctx, mq, mx, a, false)));
+    rerank_i8_kernel<VSK_METRIC_DOT_PRODUCT><<<(unsigned)nq, 256, qsm, ctx->stream>>>(q, ix->codes, dim, ix->sq_scale, ix->sq_offset, cand, rr_total);
+    ctx->stats.kernel_launches++;
+    VSK_CUDA(ctx, cudaGetLastError());
+    tl_mark(ctx, "rerank");
+    VSK_TRY(launch_select(ctx, sel));
+    seen += chunk;
+  }
+  SelectArgs fin{};
+  fin.cand = cand;
+  fin.nq = nq;
+  fin.dense_count = -1;
+  fin.keep = k;
+  fin.out_dist = out_dist;
+  fin.out_ids = out_ids;
+  fin.k = k;
+  fin.metric = ix->metric;
+  fin.id_base = ix->id_base;
+  fin.max_count = k;
+  VSK_TRY(launch_select(ctx, fin));
+  VSK_CUDA(ctx, cudaMemcpyAsync(hbuf, err, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  VSK_CUDA(ctx, cudaMemcpyAsync(hbuf + 8, rr_total, 8, cudaMemcpyDeviceToHost, ctx->stream));
+  VSK_CUDA(ctx, cudaMemcpyAsync(hbuf + 16, cand.flags, (size_t)nq * 4, cudaMemcpyDeviceToHost, ctx->stream));
+  VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  int32_t herr;
+  unsigned long long hrr;
+  memcpy(&herr, hbuf, 4);
+  memcpy(&hrr, hbuf + 8, 8);
+  ctx->stats.reranked_rows += (int64_t)hrr;
+  if (herr != 0)
+    return fail(ctx, VSK_ERR_TIMEOUT, "tensor-core scan: a bounded pipeline wait ran out (role %d)", herr);
+  std::vector<int32_t> bad;
+  for (int64_t i = 0; i < nq; ++i)
+    if (hflags[i]) bad.push_back((int32_t)i);
+  if (bad.size() > 1 && 64 * (int64_t)bad.size() > nq) {
+    ix->i8_rest = kI8Rest;
+    return VSK_OK;
+  }
+  if (!bad.empty()) VSK_TRY(fp32_search_subset(ix, q, bad, k, nullptr, nullptr, out_dist, out_ids));
   *handled = true;
   return VSK_OK;
 }

@@ -44,7 +44,11 @@ constexpr int64_t kPqTensorMinQueries = 64, kPqTensorMinRows = 16384;
 bool pq_tensor_applicable(const Index* ix, int64_t nq, int32_t k);
 int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const float* tables, float* out_dist,
                          int64_t* out_ids, std::vector<int32_t>* flagged, bool* handled);
-// Drops the fp16 operand copy after rows were added; makes it (once per index state).
+// A batch of dot products over int8 codes as an integer contraction.  *handled = false: the fp16 path takes the batch.
+constexpr int64_t kI8MinRows = 16384;
+bool i8_search_applicable(const Index* ix, int32_t k);
+int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_dist, int64_t* out_ids, bool* handled);
+// Drops the operand copies after rows were added; makes it (once per index state).
 void tensor_invalidate(Index* ix);
 int32_t tensor_prepare_index(Index* ix);
 
