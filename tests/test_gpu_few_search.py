@@ -1,0 +1,106 @@
+"""The one-launch search of a few queries (scan, per-CTA lists, merge by the last CTA): parity with the oracle at the edges
+of its rounds, lists and merge."""
+import numpy as np
+import pytest
+
+import oracle
+from parity import assert_topk_parity
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def vsk():
+    import vectorstorekit_b200 as v
+    return v
+
+
+@pytest.fixture(scope="module")
+def dev(vsk):
+    return vsk.CUDAAcceleratorStrategy(0).initialize()
+
+
+METRICS = {"euclidean": oracle.EUCLIDEAN, "cosine": oracle.COSINE, "dotProduct": oracle.DOT, "manhattan": oracle.MANHATTAN}
+
+
+def _index(vsk, dev, metric, x, masks=None):
+    ix = vsk.FlatIndex(dev, x.shape[1], vsk.DistanceMetric(metric))
+    ix.add(x, masks)
+    return ix
+
+
+# fewer rows than k, one warp step, one CTA, partial rounds, several rounds per CTA; 1, 2, 4 and 8 staged queries;
+# widths with 16-byte loads and without, around one and two steps of a warp; k up to the path's limit
+@pytest.mark.parametrize("metric", list(METRICS))
+@pytest.mark.parametrize("shape", [(1, 8, 1, 3), (15, 128, 1, 10), (33, 5, 2, 33), (1_000, 131, 3, 128), (10_000, 128, 1, 10),
+                                   (70_001, 96, 1, 100), (200_000, 33, 8, 128), (30_001, 260, 5, 1), (9_999, 1_536, 8, 7)])
+def test_few_queries(vsk, dev, cpu_oracle, metric, shape):
+    n, d, nq, k = shape
+    rng = np.random.default_rng(n + d)
+    x = rng.standard_normal((n, d)).astype(np.float32)
+    q = rng.standard_normal((nq, d)).astype(np.float32)
+    ix = _index(vsk, dev, metric, x)
+    ix2 = _index(vsk, dev, metric, x, np.full(n, 3, np.uint64))
+    rd, ri = cpu_oracle.flat_search(METRICS[metric], q, x, min(k, n))
+    for got in (ix.batchSearch(q, min(k, n)), ix2.batchSearch(q, min(k, n), np.full(nq, 2, np.uint64))):
+        assert_topk_parity(got[0], got[1], rd, ri)
+    if k > n:
+        d_, i_ = ix.batchSearch(q, k)
+        assert np.all(i_[:, n:] == -1) and np.all(np.isinf(d_[:, n:]))
+
+
+@pytest.mark.parametrize("order", ["ascending", "descending", "blocks"])
+def test_order_of_rows_and_ties(vsk, dev, cpu_oracle, order):
+    """Rows sorted by distance (every later row is listed, or none is), the nearest rows all in one CTA's share, and bulk
+    ties: the result is the first k by (distance, id)."""
+    n, d, k = 60_000, 16, 128
+    t = np.repeat(np.arange(n // 50, dtype=np.float32), 50)      # 50 rows tie at every distance
+    if order == "descending":
+        t = t[::-1].copy()
+    if order == "blocks":
+        t = np.roll(t, 1_234)
+    x = np.zeros((n, d), np.float32)
+    x[:, 3] = t
+    ix = _index(vsk, dev, "euclidean", x)
+    q = np.zeros((2, d), np.float32)
+    q[1, 3] = 700.0
+    for m in (1, 2):
+        d_, i_ = ix.batchSearch(q[:m], k)
+        rd, ri = cpu_oracle.flat_search(oracle.EUCLIDEAN, q[:m], x, k)
+        assert np.array_equal(i_, ri) and np.array_equal(d_, rd)
+
+
+def test_filters_few_rows_pass(vsk, dev, cpu_oracle):
+    rng = np.random.default_rng(4)
+    n, d = 40_000, 64
+    x = rng.standard_normal((n, d)).astype(np.float32)
+    masks = np.zeros(n, np.uint64)
+    masks[rng.choice(n, 25, replace=False)] = 1
+    masks[7::1000] |= np.uint64(2)
+    q = rng.standard_normal((4, d)).astype(np.float32)
+    qm = np.array([1, 2, 4, 3], np.uint64)
+    d_, i_ = _index(vsk, dev, "manhattan", x, masks).batchSearch(q, 50, qm)
+    for r in range(4):
+        rows = np.nonzero(masks & qm[r])[0]
+        assert np.all(i_[r, len(rows):] == -1)
+        if len(rows):
+            m = min(50, len(rows))
+            rd, ri = cpu_oracle.flat_search(oracle.MANHATTAN, q[r:r + 1], x[rows], m)
+            assert_topk_parity(d_[r:r + 1, :m], i_[r:r + 1, :m], rd, rows[ri])
+
+
+def test_repeated_calls_leave_the_tickets_at_zero(vsk, dev, cpu_oracle):
+    """Back-to-back calls of different grids on one context, a probe of inverted lists among them."""
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal((20_000, 32)).astype(np.float32)
+    big, small = _index(vsk, dev, "euclidean", x), _index(vsk, dev, "dotProduct", x[:100])
+    ivf = vsk.IVFIndex(dev, 32, 64, 64, maxIterations=2)
+    ivf.train(x[:4_096], x[:64])
+    ivf.insert(x)
+    for r in range(6):
+        q = rng.standard_normal((1 + 2 * (r % 2), 32)).astype(np.float32)
+        rd, ri = cpu_oracle.flat_search(oracle.EUCLIDEAN, q, x, 20)
+        assert_topk_parity(*big.batchSearch(q, 20), rd, ri)
+        assert_topk_parity(*ivf.batchSearch(q, 20), rd, ri)      # every list is probed: the flat result
+        rd, ri = cpu_oracle.flat_search(oracle.DOT, q, x[:100], 5)
+        assert_topk_parity(*small.batchSearch(q, 5), rd, ri)

@@ -479,6 +479,7 @@ static int32_t filtered_grouped_search(Index* ix, const float* q, int64_t nq, in
 }
 
 constexpr int64_t kQueryBatch = 16384;  // queries per pass: bounds the candidate workspace at 512 MB
+constexpr int64_t kFewMaxElems = 128ll << 20;   // unfiltered few-query batches up to this many row elements read the fp32 rows
 
 static int32_t flat_search_dev(Index* ix, const float* q, int64_t nq, int32_t k, const uint64_t* qmasks,
                                float* out_dist, int64_t* out_ids) {
@@ -494,6 +495,28 @@ static int32_t flat_search_dev(Index* ix, const float* q, int64_t nq, int32_t k,
     const int64_t bn = std::min(kQueryBatch, nq - b);
     const float* qb = q + b * ix->dim;
     const uint64_t* mb = qmasks ? qmasks + b : nullptr;
+    const bool tensor_metric = ctx->search_path == VSK_PATH_TENSOR_RERANK && ix->metric != VSK_METRIC_MANHATTAN;
+    if (bn <= kStreamScanMaxQueries && (!tensor_metric || mb || ix->n * ix->dim <= kFewMaxElems)) {
+      FewArgs f{};
+      f.metric = ix->metric;
+      f.q = qb;
+      f.x = ix->rows;
+      f.dim = ix->dim;
+      f.nq = bn;
+      f.n = ix->n;
+      f.k = k;
+      f.xnorm = ix->row_norm;
+      f.row_masks = (mb && ix->has_masks) ? ix->masks : nullptr;
+      f.q_masks = f.row_masks ? mb : nullptr;
+      f.id_base = ix->id_base;
+      f.final_sqrt = ix->metric == VSK_METRIC_EUCLIDEAN;
+      f.out_dist = out_dist + b * k;
+      f.out_ids = out_ids + b * k;
+      if (few_search_applies(ctx, f)) {
+        VSK_TRY(few_search(ctx, f));
+        continue;
+      }
+    }
     float* qnorm = nullptr;
     if (ix->metric == VSK_METRIC_COSINE) {
       void* p;
@@ -504,8 +527,7 @@ static int32_t flat_search_dev(Index* ix, const float* q, int64_t nq, int32_t k,
     // Euclidean, cosine and dot-product batches take the tensor path, filtered or not (the filter is applied to the
     // hits in the contraction's epilogue).  A batch of a few queries is bound by the bytes it reads, not by the
     // contraction: the fp32 streaming scan reads each eligible fp32 row once.
-    const bool tensor = ctx->search_path == VSK_PATH_TENSOR_RERANK && ix->metric != VSK_METRIC_MANHATTAN &&
-                        !(mb && bn <= kStreamScanMaxQueries);
+    const bool tensor = tensor_metric && !(mb && bn <= kStreamScanMaxQueries);
     bool grouped = false;
     if (mb && ix->has_masks)
       VSK_TRY(filtered_grouped_search(ix, qb, bn, k, qnorm, mb, out_dist + b * k, out_ids + b * k, &grouped,
@@ -686,6 +708,7 @@ int32_t vsk_close(vsk_ctx* c) {
   cudaStreamSynchronize(ctx->stream_aux);
   comm_release(ctx);
   for (auto& p : ctx->scratch) dev_free(p);
+  for (auto& p : ctx->few_tickets) dev_free(p);
   for (auto& b : ctx->host_flags)
     if (b.p) cudaFreeHost(b.p);
   for (auto& e : ctx->prof_events) cudaEventDestroy(e);

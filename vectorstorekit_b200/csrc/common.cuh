@@ -157,6 +157,7 @@ struct Ctx {
   size_t scratch_bytes[2 * 64] = {};
   ShardPending pending[2];
   PinnedBuf host_flags[2];   // per lane: the flag words a finished half-search hands to the host
+  unsigned* few_tickets[2] = {};   // per lane: the few-query search's tickets (few_search.cu)
   Comm* comm = nullptr;
   Worker* worker = nullptr;
   // optional event log (vsk_timeline): one event after each marked launch, on the stream it went to
@@ -214,7 +215,7 @@ enum Slot : int {
   SLOT_IVF_PROBE_D, SLOT_IVF_PROBE_I, SLOT_IVF_KEYS, SLOT_IVF_ORDER, SLOT_IVF_PAIR_OFF, SLOT_IVF_ITEM_CNT,
   SLOT_IVF_ITEM_OFF, SLOT_IVF_SUBSET, SLOT_IVF_STAGES, SLOT_KM_NSEG, SLOT_KM_SEGOFF, SLOT_KM_PARTIAL, SLOT_FILTER_PERM, SLOT_FILTER_ROWS, SLOT_FILTER_COUNT, SLOT_SQ_A, SLOT_SQ_B, SLOT_TC_A, SLOT_TC_B, SLOT_TC_C, SLOT_TC_D,
   SLOT_PQ_TABLES, SLOT_SH_D, SLOT_SH_I, SLOT_SH_SEND, SLOT_SH_RECV, SLOT_SH_BOUND, SLOT_SH_MERGED, SLOT_SH_ALL,
-  SLOT_PQ_ROWS,
+  SLOT_PQ_ROWS, SLOT_FEW,
   SLOT_COUNT
 };
 static_assert(SLOT_COUNT <= 64, "grow Ctx::scratch");
@@ -329,6 +330,32 @@ constexpr int kStreamScanMaxSegQueries = 16;   // with per-query row lists (one 
                                                // list-major tiles, which read a list once for all its queries, win
 bool stream_scan_applies(const Ctx* ctx, const ExactScanArgs& a);
 int32_t launch_stream_scan(Ctx* ctx, const ExactScanArgs& a);
+// ---- few_search.cu ---------------------------------------------------------------------------
+// Top-k of a few queries over fp32 rows in one launch (two for 2 - 8 queries): scan, selection, final order.
+constexpr int kFewMaxK = 128;
+struct FewArgs {
+  int32_t metric;
+  const float* q;             // [nq][dim]
+  const float* x;             // [n][dim]
+  int32_t dim;
+  int64_t nq, n;              // with probes: n is the expected number of rows per query (sizes the launch only)
+  int32_t k;
+  const float* xnorm;         // |x| (cosine)
+  const uint64_t* row_masks;  // or null
+  const uint64_t* q_masks;    // or null
+  const int32_t* id_remap;    // or null: a row's id
+  int64_t id_base;
+  int final_sqrt;
+  float* out_dist;            // [nq][k]
+  int64_t* out_ids;
+  // the probed lists of an IVF index, per query (euclidean): list l holds rows [list_offsets[l], list_offsets[l + 1])
+  const int64_t* probes;      // [nq][nprobe], or null
+  int32_t nprobe, nlist;
+  const int64_t* list_offsets;
+  int64_t nan_rows;           // set by few_search
+};
+bool few_search_applies(const Ctx* ctx, const FewArgs& a);
+int32_t few_search(Ctx* ctx, const FewArgs& a);
 int32_t launch_row_norms(Ctx* ctx, const float* x, int64_t n, int32_t dim, int squared, float* out);
 
 // ---- group.cu ----------------------------------------------------------------------------

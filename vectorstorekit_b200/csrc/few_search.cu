@@ -1,0 +1,387 @@
+// Top-k of a few queries in one launch: scan, selection and final order.
+//
+// A call with one query over a small store is bound by launches, not by bytes: 10 000 rows of 128 floats cross HBM in
+// 0.8 us, and the chunked schedule spends a dozen launches on them (109 us for the whole call; 59 us this way).  Here every
+// CTA streams its share of the rows (the inner loop of stream_scan.cu: each row read once, 16-byte loads), keeps its k
+// best keys per query in shared memory - appends below a threshold, a block-wide selection when the list fills up - and
+// writes them out; the last CTA to finish merges the lists.  The merge needs few of the G k keys written: the k-th
+// smallest of the CTAs' best keys bounds the result (k rows lie at or below it), so only CTAs whose best key is within
+// it - k of them - are read.  Values are the same direct fp32 formulas, ties go by id, and the row masks are applied
+// before a key is listed.
+//
+// SEG: every query walks the rows of its own probed lists of an IVF index (one grid row per query), found from the probe
+// list and the list offsets on the device: no row list is written and the host is not asked in between (one query, 10 of
+// 1 024 lists over 1 million rows: 171 -> 96 us).
+#include <math_constants.h>
+
+#include <algorithm>
+
+#include "block_select.cuh"
+#include "common.cuh"
+#include "stream_rows.cuh"
+
+namespace vsk {
+namespace {
+
+constexpr int FEW_THREADS = 256;
+constexpr int FEW_WARPS = FEW_THREADS / 32;
+constexpr int FEW_ROWS = 2;        // rows per warp step (as in stream_scan.cu)
+constexpr int FEW_LIST = 1024;     // keys per query a CTA holds
+constexpr int FEW_ROUND = 512;     // rows per round at most: a round's keys fit behind FEW_LIST - FEW_ROUND listed ones
+constexpr int FEW_MAX_CTAS = 1024; // lists per query the merge looks at (the selection holds 8 keys per thread)
+static_assert(FEW_LIST - FEW_ROUND >= kFewMaxK && FEW_MAX_CTAS <= FEW_THREADS * SEL_ITEMS, "few-query list sizes");
+
+struct FewKernelArgs {
+  FewArgs a;
+  int32_t round;        // rows per CTA and round, a multiple of FEW_WARPS * FEW_ROWS
+  uint64_t* part;       // [nq][grid][k] each CTA's best keys (unordered) ...
+  uint64_t* part_min;   // [nq][grid] ... the smallest of them (all ones: none)
+  int32_t* part_n;      // [nq][grid] ... and how many
+  unsigned* ticket;     // [nq] CTAs of the query that have finished; left at zero
+};
+
+struct FewScratch {     // the selection's words
+  int hist[256];
+  int bin, less, in_bin, out;
+};
+
+// Shortens list[0..cnt) to its k smallest keys (cnt > k) and returns the largest of them; every thread takes part.
+__device__ __forceinline__ uint64_t few_compact(uint64_t* list, int cnt, int k, FewScratch& s) {
+  uint64_t key[SEL_ITEMS];
+#pragma unroll
+  for (int i = 0; i < SEL_ITEMS; ++i) {
+    const int at = threadIdx.x + i * FEW_THREADS;
+    key[i] = at < cnt ? list[at] : kEmptyKey;
+  }
+  if (threadIdx.x == 0) s.out = 0;
+  __syncthreads();
+  const uint64_t pivot = block_radix_select(key, k, s.hist, &s.bin, &s.less, &s.in_bin);
+#pragma unroll
+  for (int i = 0; i < SEL_ITEMS; ++i)
+    if (key[i] <= pivot && key[i] != kEmptyKey) list[atomicAdd(&s.out, 1)] = key[i];
+  __syncthreads();
+  return pivot;
+}
+
+// Merges the lists of one query and writes its result.  `list` has room for FEW_LIST keys, `cand` for FEW_MAX_CTAS list numbers.
+__device__ __forceinline__ void few_merge(const FewKernelArgs& ka, int64_t pos, int lists, uint64_t* list, unsigned short* cand,
+                                          FewScratch& s) {
+  __shared__ int n_cand, n_list, n_have;
+  const FewArgs& a = ka.a;
+  const int k = a.k;
+  const uint64_t* mins = ka.part_min + pos * lists;
+  uint64_t key[SEL_ITEMS];
+  if (threadIdx.x == 0) { n_cand = 0; n_list = 0; n_have = 0; }
+  __syncthreads();
+  int have = 0;
+#pragma unroll
+  for (int i = 0; i < SEL_ITEMS; ++i) {
+    const int at = threadIdx.x + i * FEW_THREADS;
+    key[i] = at < lists ? __ldcg(mins + at) : kEmptyKey;
+    have += key[i] != kEmptyKey;
+  }
+  if (have) atomicAdd(&n_have, have);
+  __syncthreads();
+  // at least k rows lie at or below the k-th smallest best key
+  uint64_t bound = kEmptyKey - 1;
+  if (n_have >= k) bound = block_radix_select(key, k, s.hist, &s.bin, &s.less, &s.in_bin);
+#pragma unroll
+  for (int i = 0; i < SEL_ITEMS; ++i)
+    if (key[i] <= bound && key[i] != kEmptyKey) cand[atomicAdd(&n_cand, 1)] = (unsigned short)(threadIdx.x + i * FEW_THREADS);
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nc = n_cand;
+  int cnt = 0;
+  const int batch = (FEW_LIST - k) / k;   // lists that fit behind the keys already kept
+  for (int c0 = 0; c0 < nc; c0 += batch) {
+    for (int c = c0 + warp; c < min(nc, c0 + batch); c += FEW_WARPS) {
+      const int64_t l = pos * lists + cand[c];
+      const int n = __ldcg(ka.part_n + l);
+      for (int i = lane; i < n; i += 32) {
+        const uint64_t v = __ldcg(ka.part + l * k + i);
+        if (v <= bound) list[atomicAdd(&n_list, 1)] = v;
+      }
+    }
+    __syncthreads();
+    cnt = n_list;
+    if (cnt > k) {
+      const uint64_t pivot = few_compact(list, cnt, k, s);
+      bound = min(bound, pivot);
+      cnt = s.out;
+      if (threadIdx.x == 0) n_list = cnt;
+    }
+    __syncthreads();
+  }
+  const int P = next_pow2(cnt);
+  for (int i = cnt + threadIdx.x; i < P; i += FEW_THREADS) list[i] = kEmptyKey;
+  __syncthreads();
+  bitonic_sort(list, P);
+  for (int j = threadIdx.x; j < k; j += FEW_THREADS) {
+    float d = CUDART_INF_F;
+    int64_t id = -1;
+    if (j < cnt) {
+      d = ordered_to_float((uint32_t)(list[j] >> 32));
+      if (a.final_sqrt) d = sqrtf(d);
+      id = (int64_t)(uint32_t)list[j] + a.id_base;
+    }
+    a.out_dist[pos * k + j] = d;
+    a.out_ids[pos * k + j] = id;
+  }
+}
+
+template <int METRIC, int NQ, bool VEC, bool SEG>
+__global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(FewKernelArgs ka) {
+  static_assert(!SEG || NQ == 1, "per-query lists are scanned one query per grid row");
+  const FewArgs& a = ka.a;
+  extern __shared__ __align__(16) uint8_t smem[];
+  // [NQ][FEW_LIST] keys, then [NQ][dim] queries, then (SEG) [nprobe + 1] first positions and [nprobe] first rows of the lists
+  uint64_t* lists = reinterpret_cast<uint64_t*>(smem);
+  float* sq = reinterpret_cast<float*>(smem + (size_t)NQ * FEW_LIST * 8);
+  int64_t* seg_pos = reinterpret_cast<int64_t*>(smem + (size_t)NQ * FEW_LIST * 8 + ((size_t)NQ * a.dim * 4 + 7) / 8 * 8);
+  int64_t* seg_row = seg_pos + (SEG ? a.nprobe + 1 : 0);
+  __shared__ FewScratch fs;
+  __shared__ uint64_t s_thr[NQ], s_qm[NQ], s_any;
+  __shared__ float s_qn[NQ];
+  __shared__ int s_cnt[NQ];
+  __shared__ unsigned s_last;
+  const int dim = a.dim, k = a.k;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int qb = SEG ? (int)blockIdx.y : 0;
+  const int nq_here = SEG ? 1 : (int)a.nq;
+  for (int i = threadIdx.x; i < NQ * dim; i += FEW_THREADS) sq[i] = i < nq_here * dim ? a.q[(int64_t)qb * dim + i] : 0.f;
+  if (threadIdx.x < NQ) {
+    s_thr[threadIdx.x] = kEmptyKey - 1;
+    s_cnt[threadIdx.x] = 0;
+    s_qm[threadIdx.x] = (int)threadIdx.x < nq_here ? (a.q_masks ? a.q_masks[qb + threadIdx.x] : ~0ull) : 0ull;
+  }
+  if (SEG && warp == 0) {
+    // first position of every probed list (an out-of-range probe is an empty list)
+    int64_t run = 0;
+    for (int p0 = 0; p0 < a.nprobe; p0 += 32) {
+      const int p = p0 + lane;
+      int64_t beg = 0, len = 0;
+      if (p < a.nprobe) {
+        const int64_t l = a.probes[(int64_t)qb * a.nprobe + p];
+        if (l >= 0 && l < a.nlist) {
+          beg = a.list_offsets[l];
+          len = a.list_offsets[l + 1] - beg;
+        }
+      }
+      int64_t incl = len;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int64_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      if (p < a.nprobe) {
+        seg_pos[p] = run + incl - len;
+        seg_row[p] = beg;
+      }
+      run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) seg_pos[a.nprobe] = run;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint64_t any = 0;
+    for (int i = 0; i < NQ; ++i) any |= s_qm[i];
+    s_any = any;
+  }
+  if (METRIC == VSK_METRIC_COSINE)
+    for (int i = warp; i < NQ; i += FEW_WARPS) {   // |q|, summed as the row norms are
+      float ss = 0.f;
+      for (int c = lane; c < dim; c += 32) ss = fmaf(sq[i * dim + c], sq[i * dim + c], ss);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (lane == 0) s_qn[i] = sqrtf(ss);
+    }
+  __syncthreads();
+  const uint64_t any_mask = s_any;
+  const int64_t n = SEG ? seg_pos[a.nprobe] : a.n;
+
+  constexpr int V = FEW_ROWS * NQ;
+  constexpr int OWNER_SHIFT = 5 - Log2<V>::value;
+  const int64_t stride = (int64_t)gridDim.x * ka.round;
+  for (int64_t r0 = (int64_t)blockIdx.x * ka.round; r0 < n; r0 += stride) {
+    const int64_t r1 = min(n, r0 + ka.round);
+    for (int64_t n0 = r0 + warp * FEW_ROWS; n0 < r1; n0 += FEW_WARPS * FEW_ROWS) {
+      bool live[FEW_ROWS];
+      uint32_t rid[FEW_ROWS];
+      uint64_t rmask[FEW_ROWS];
+#pragma unroll
+      for (int r = 0; r < FEW_ROWS; ++r) {
+        const int64_t at = n0 + r;
+        const bool has = at < r1;
+        rid[r] = has ? (uint32_t)at : 0u;
+        if (SEG && has) {
+          int lo = 0, hi = a.nprobe;   // the last list that starts at or before this position (empty lists are passed over)
+          while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (seg_pos[mid] <= at) lo = mid; else hi = mid;
+          }
+          rid[r] = (uint32_t)(seg_row[lo] + (at - seg_pos[lo]));
+        }
+        rmask[r] = (a.row_masks && has) ? __ldg(a.row_masks + rid[r]) : ~0ull;
+        live[r] = has && (rmask[r] & any_mask) != 0;   // a row no query may see is not read
+      }
+      float acc[V];
+#pragma unroll
+      for (int j = 0; j < V; ++j) acc[j] = 0.f;
+      stream_accumulate<METRIC, NQ, VEC, FEW_ROWS>(acc, a.x, dim, sq, rid, live, lane);
+      warp_reduce_scatter<V>(acc, lane);
+      if ((lane & ((1 << OWNER_SHIFT) - 1)) == 0) {
+        const int j = lane >> OWNER_SHIFT;
+        const int r = j / NQ, i = j - r * NQ;
+        bool liver = live[0];
+        uint32_t ridr = rid[0];
+        uint64_t rmaskr = rmask[0];
+#pragma unroll
+        for (int t = 1; t < FEW_ROWS; ++t)
+          if (r == t) { liver = live[t]; ridr = rid[t]; rmaskr = rmask[t]; }
+        if (liver && i < nq_here && (rmaskr & s_qm[i]) != 0) {
+          float v = acc[0];
+          if (METRIC == VSK_METRIC_COSINE) v = 1.0f - v / (s_qn[i] * __ldg(a.xnorm + ridr) + 1e-8f);
+          else if (METRIC == VSK_METRIC_DOT_PRODUCT) v = -v;
+          const uint32_t id = a.id_remap ? (uint32_t)__ldg(a.id_remap + ridr) : ridr;
+          const uint64_t key = make_key(v, id);
+          // a value that is not a number is listed among the first rows only, as the chunked schedule does
+          if (key <= s_thr[i] && (!isnan(v) || n0 + r < a.nan_rows)) lists[i * FEW_LIST + atomicAdd(&s_cnt[i], 1)] = key;
+        }
+      }
+    }
+    __syncthreads();
+    const bool last = r0 + stride >= n;
+#pragma unroll 1
+    for (int i = 0; i < nq_here; ++i) {
+      const int cnt = s_cnt[i];
+      if (cnt > (last ? k : FEW_LIST - FEW_ROUND)) {
+        const uint64_t pivot = few_compact(lists + (size_t)i * FEW_LIST, cnt, k, fs);
+        if (threadIdx.x == 0) {
+          s_cnt[i] = fs.out;
+          s_thr[i] = pivot;
+        }
+      }
+    }
+    __syncthreads();
+  }
+  // ---- this CTA's lists, and the merge by the last one to arrive ----
+#pragma unroll 1
+  for (int i = 0; i < nq_here; ++i) {
+    const int64_t l = (int64_t)(qb + i) * gridDim.x + blockIdx.x;
+    const uint64_t* list = lists + (size_t)i * FEW_LIST;
+    const int cnt = s_cnt[i];
+    for (int j = threadIdx.x; j < cnt; j += FEW_THREADS) ka.part[l * k + j] = list[j];
+    if (warp == 0) {
+      uint64_t best = kEmptyKey;
+      for (int j = lane; j < cnt; j += 32) best = min(best, list[j]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
+      if (lane == 0) {
+        ka.part_min[l] = best;
+        ka.part_n[l] = cnt;
+      }
+    }
+  }
+  if (NQ > 1) return;   // several queries: few_merge_kernel merges them side by side
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(ka.ticket + qb, 1u);
+  __syncthreads();
+  if (s_last != gridDim.x - 1) return;
+  __threadfence();
+  if (threadIdx.x == 0) ka.ticket[qb] = 0u;
+  // the query's staging area is free now: list numbers go there (the launch makes it large enough)
+  few_merge(ka, qb, (int)gridDim.x, lists, reinterpret_cast<unsigned short*>(smem + (size_t)NQ * FEW_LIST * 8), fs);
+}
+
+__global__ void __launch_bounds__(FEW_THREADS) few_merge_kernel(FewKernelArgs ka, int lists) {
+  __shared__ uint64_t list[FEW_LIST];
+  __shared__ unsigned short cand[FEW_MAX_CTAS];
+  __shared__ FewScratch fs;
+  few_merge(ka, blockIdx.x, lists, list, cand, fs);
+}
+
+template <int NQ>
+size_t few_smem(const FewArgs& a) {
+  size_t b = ((size_t)NQ * a.dim * 4 + 7) / 8 * 8;
+  if (a.probes) b += (size_t)(2 * a.nprobe + 1) * 8;
+  b = std::max<size_t>(b, FEW_MAX_CTAS * sizeof(unsigned short));   // the merge's list numbers go here
+  return (size_t)NQ * FEW_LIST * 8 + b;
+}
+constexpr size_t kFewMaxSmem = 110 * 1024;   // two CTAs per SM
+
+template <int METRIC, int NQ, bool VEC, bool SEG>
+int32_t few_launch(Ctx* ctx, FewKernelArgs ka) {
+  const FewArgs& a = ka.a;
+  auto kern = few_topk_kernel<METRIC, NQ, VEC, SEG>;
+  const size_t smem = few_smem<NQ>(a);
+  if (smem > 48 * 1024) VSK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int sms = ctx->prop.multiProcessorCount;
+  const int per_sm = std::max(1, std::min(NQ > 4 ? 2 : 3, (int)(220 * 1024 / (smem + 3072))));
+  // at least two warp steps of rows per CTA; per-query lists share the machine
+  const int64_t rows = std::max<int64_t>(a.n, 1);   // SEG: an estimate, the kernel takes the lists' true lengths
+  const int64_t nseg = SEG ? a.nq : 1;
+  constexpr int kStep = FEW_WARPS * FEW_ROWS;
+  const int64_t grid = std::min({ceil_div(rows, 2 * kStep), std::max<int64_t>(1, (int64_t)sms * per_sm / nseg), (int64_t)FEW_MAX_CTAS});
+  // rounds of whole warp steps, such that the last one is spread evenly
+  const int64_t share = ceil_div(rows, grid);
+  ka.round = (int32_t)std::min<int64_t>(FEW_ROUND, ceil_div(ceil_div(share, ceil_div(share, (int64_t)FEW_ROUND)), kStep) * kStep);
+  void* p;
+  const size_t lists = (size_t)a.nq * grid;
+  VSK_TRY(scratch(ctx, SLOT_FEW, lists * ((size_t)a.k * 8 + 8 + 4), &p));
+  ka.part = (uint64_t*)p;
+  ka.part_min = ka.part + lists * a.k;
+  ka.part_n = (int32_t*)(ka.part_min + lists);
+  prof_begin(ctx);
+  kern<<<dim3((unsigned)grid, (unsigned)nseg), FEW_THREADS, smem, ctx->stream>>>(ka);
+  prof_end(ctx);
+  ctx->stats.kernel_launches++;
+  if (NQ > 1) {
+    few_merge_kernel<<<(unsigned)a.nq, FEW_THREADS, 0, ctx->stream>>>(ka, (int)grid);
+    ctx->stats.kernel_launches++;
+  }
+  VSK_CUDA(ctx, cudaGetLastError());
+  return VSK_OK;
+}
+
+template <int METRIC>
+int32_t few_metric(Ctx* ctx, const FewKernelArgs& ka, bool vec) {
+  const FewArgs& a = ka.a;
+  if (a.nq <= 1) return vec ? few_launch<METRIC, 1, true, false>(ctx, ka) : few_launch<METRIC, 1, false, false>(ctx, ka);
+  if (a.nq <= 2) return vec ? few_launch<METRIC, 2, true, false>(ctx, ka) : few_launch<METRIC, 2, false, false>(ctx, ka);
+  if (a.nq <= 4) return vec ? few_launch<METRIC, 4, true, false>(ctx, ka) : few_launch<METRIC, 4, false, false>(ctx, ka);
+  return vec ? few_launch<METRIC, 8, true, false>(ctx, ka) : few_launch<METRIC, 8, false, false>(ctx, ka);
+}
+
+}  // namespace
+
+bool few_search_applies(const Ctx* ctx, const FewArgs& a) {
+  if (!ctx->tuning.stream_scan || a.k < 1 || a.k > kFewMaxK || a.nq < 1 || a.dim < 1) return false;
+  if (a.probes) return a.metric == VSK_METRIC_EUCLIDEAN && a.nq <= kStreamScanMaxSegQueries && few_smem<1>(a) <= kFewMaxSmem;
+  if (a.nq > kStreamScanMaxQueries) return false;
+  return (a.nq <= 1 ? few_smem<1>(a) : a.nq <= 2 ? few_smem<2>(a) : a.nq <= 4 ? few_smem<4>(a) : few_smem<8>(a)) <= kFewMaxSmem;
+}
+
+int32_t few_search(Ctx* ctx, const FewArgs& a) {
+  VSK_TRACE("vsk:few_search");
+  FewKernelArgs ka{};
+  ka.a = a;
+  ka.a.nan_rows = schedule_dense_rows(ctx, a.k);
+  unsigned*& tickets = ctx->few_tickets[ctx->lane];
+  if (!tickets) {   // zeroed once: the last CTA of a query leaves its ticket at zero
+    VSK_TRY(dev_alloc(ctx, (void**)&tickets, kStreamScanMaxSegQueries * sizeof(unsigned)));
+    VSK_CUDA(ctx, cudaMemsetAsync(tickets, 0, kStreamScanMaxSegQueries * sizeof(unsigned), ctx->stream));
+  }
+  ka.ticket = tickets;
+  const bool vec = a.dim % 4 == 0 && (reinterpret_cast<uintptr_t>(a.x) & 15) == 0;
+  if (a.probes)
+    return vec ? few_launch<VSK_METRIC_EUCLIDEAN, 1, true, true>(ctx, ka) : few_launch<VSK_METRIC_EUCLIDEAN, 1, false, true>(ctx, ka);
+  switch (a.metric) {
+    case VSK_METRIC_EUCLIDEAN: return few_metric<VSK_METRIC_EUCLIDEAN>(ctx, ka, vec);
+    case VSK_METRIC_COSINE: return few_metric<VSK_METRIC_COSINE>(ctx, ka, vec);
+    case VSK_METRIC_DOT_PRODUCT: return few_metric<VSK_METRIC_DOT_PRODUCT>(ctx, ka, vec);
+    case VSK_METRIC_MANHATTAN: return few_metric<VSK_METRIC_MANHATTAN>(ctx, ka, vec);
+    default: return fail(ctx, VSK_ERR_UNSUPPORTED_OPERATION, "metric %d is not supported", a.metric);
+  }
+}
+
+}  // namespace vsk

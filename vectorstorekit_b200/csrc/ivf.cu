@@ -662,6 +662,17 @@ int32_t ivf_search_dev(Index* ix, const float* q, int64_t nq, int32_t k, int32_t
     VSK_TRY(scratch(ctx, SLOT_IVF_PROBE_D, (size_t)bn * nprobe * 4, &pd));
     VSK_TRY(scratch(ctx, SLOT_IVF_PROBE_I, (size_t)bn * nprobe * 8, &pi));
     const bool tensor = ctx->search_path == VSK_PATH_TENSOR_RERANK && ivf_tensor_applicable(ix, bn, nprobe, k);
+    auto few_centroids = [&](int64_t queries) {
+      FewArgs f{};
+      f.metric = VSK_METRIC_EUCLIDEAN;
+      f.x = ix->centroids;
+      f.dim = ix->dim;
+      f.nq = queries;
+      f.n = ix->nlist;
+      f.k = nprobe;
+      f.final_sqrt = 1;
+      return f;
+    };
     if (probe_all) {
       ivf_probe_all_kernel<<<(unsigned)ceil_div(bn * (int64_t)nprobe, 256), 256, 0, ctx->stream>>>((int64_t*)pi, bn, nprobe);
       ctx->stats.kernel_launches++;
@@ -686,6 +697,16 @@ int32_t ivf_search_dev(Index* ix, const float* q, int64_t nq, int32_t k, int32_t
         ix->coarse = co;
       }
       VSK_TRY(tensor_search(ix->coarse, qb, bn, nprobe, nullptr, nullptr, (float*)pd, (int64_t*)pi));
+    } else if (const FewArgs f = few_centroids(bn <= kStreamScanMaxSegQueries ? std::min<int64_t>(bn, kStreamScanMaxQueries) : bn);
+               few_search_applies(ctx, f)) {
+      for (int64_t i = 0; i < bn; i += kStreamScanMaxQueries) {   // one launch for up to eight queries
+        FewArgs g = f;
+        g.q = qb + i * ix->dim;
+        g.nq = std::min<int64_t>(kStreamScanMaxQueries, bn - i);
+        g.out_dist = (float*)pd + i * nprobe;
+        g.out_ids = (int64_t*)pi + i * nprobe;
+        VSK_TRY(few_search(ctx, g));
+      }
     } else {
       ExactScanArgs c{};
       c.metric = VSK_METRIC_EUCLIDEAN;
@@ -710,6 +731,30 @@ int32_t ivf_search_dev(Index* ix, const float* q, int64_t nq, int32_t k, int32_t
       continue;
     }
     if (bn <= kStreamScanMaxSegQueries) {
+      // the probed lists, walked on the device query by query; longer probe lists or results: the chunked schedule
+      FewArgs f{};
+      f.metric = VSK_METRIC_EUCLIDEAN;
+      f.q = qb;
+      f.x = ix->rows;
+      f.dim = ix->dim;
+      f.nq = bn;
+      f.n = ceil_div(ix->n * nprobe, ix->nlist);
+      f.k = k;
+      f.row_masks = (mb && ix->has_masks) ? ix->masks : nullptr;
+      f.q_masks = f.row_masks ? mb : nullptr;
+      f.id_remap = ix->list_rows;
+      f.id_base = ix->id_base;
+      f.final_sqrt = 1;
+      f.out_dist = out_dist + b * k;
+      f.out_ids = out_ids + b * k;
+      f.probes = (const int64_t*)pi;
+      f.nprobe = nprobe;
+      f.nlist = ix->nlist;
+      f.list_offsets = ix->list_offsets;
+      if (few_search_applies(ctx, f)) {
+        VSK_TRY(few_search(ctx, f));
+        continue;
+      }
       bool few = false;
       VSK_TRY(ivf_search_few(ctx, ix, qb, bn, (const int64_t*)pi, nprobe, k, mb, out_dist + b * k, out_ids + b * k, &few));
       if (few) continue;

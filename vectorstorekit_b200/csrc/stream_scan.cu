@@ -16,37 +16,13 @@
 // own dimensions first and the lanes are added afterwards, so a value can differ from the tile's
 // (dimension-order) sum in the last bits.
 #include "common.cuh"
-#include "tile_core.cuh"
+#include "stream_rows.cuh"
 
 namespace vsk {
 namespace {
 
 constexpr int SS_THREADS = 256;
 // Rows per warp step (template parameter): a staged query value is used for all of them.
-
-// v[0..V) per lane -> the total over the warp of v[j] on the lanes with (lane >> (5 - log2 V)) == j, in v[0].
-// Each stage halves the values a lane still carries: a lane keeps the half its lane bit selects and hands the
-// other half to its partner, so V values cost V - 1 + (5 - log2 V) shuffles instead of 5 V.
-template <int V>
-__device__ __forceinline__ void warp_reduce_scatter(float (&v)[V], int lane) {
-  int off = 16;
-#pragma unroll
-  for (int c = V; c > 1; c >>= 1) {
-    const int h = c >> 1;
-    const bool upper = (lane & off) != 0;
-#pragma unroll
-    for (int j = 0; j < h; ++j) {
-      const float keep = upper ? v[j + h] : v[j];
-      const float send = upper ? v[j] : v[j + h];
-      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-    off >>= 1;
-  }
-  for (; off > 0; off >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
-}
-
-template <int V> struct Log2 { static constexpr int value = 1 + Log2<V / 2>::value; };
-template <> struct Log2<1> { static constexpr int value = 0; };
 
 // SEG: every query scans its own slice of the row list (NQ = 1; blockIdx.y is the query's position).
 template <int METRIC, int MODE, int NQ, bool VEC, bool SEG, int SS_ROWS>
@@ -112,61 +88,7 @@ __global__ void __launch_bounds__(SS_THREADS, NQ > 4 ? 3 : 4) stream_scan_kernel
     float acc[V];
 #pragma unroll
     for (int j = 0; j < V; ++j) acc[j] = 0.f;
-    if (VEC) {
-      const int nv = dim >> 2;
-      const float4* p[SS_ROWS];
-#pragma unroll
-      for (int r = 0; r < SS_ROWS; ++r) p[r] = reinterpret_cast<const float4*>(a.x + (int64_t)rid[r] * dim);
-      const float4* sq4 = reinterpret_cast<const float4*>(sq);
-      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int c = lane; c < nv; c += 64) {
-        // four 16-byte loads in flight per lane before the first is used
-        const int c2 = c + 32;
-        const bool two = c2 < nv;
-        float4 x[SS_ROWS][2];
-#pragma unroll
-        for (int r = 0; r < SS_ROWS; ++r) {
-          x[r][0] = live[r] ? __ldg(p[r] + c) : zero;
-          x[r][1] = (live[r] && two) ? __ldg(p[r] + c2) : zero;
-        }
-#pragma unroll
-        for (int i = 0; i < NQ; ++i) {
-          const float4 q = sq4[i * nv + c];
-#pragma unroll
-          for (int r = 0; r < SS_ROWS; ++r) {
-            tile::accum<METRIC>(acc[r * NQ + i], q.x, x[r][0].x);
-            tile::accum<METRIC>(acc[r * NQ + i], q.y, x[r][0].y);
-            tile::accum<METRIC>(acc[r * NQ + i], q.z, x[r][0].z);
-            tile::accum<METRIC>(acc[r * NQ + i], q.w, x[r][0].w);
-          }
-        }
-        if (two) {
-#pragma unroll
-          for (int i = 0; i < NQ; ++i) {
-            const float4 q = sq4[i * nv + c2];
-#pragma unroll
-            for (int r = 0; r < SS_ROWS; ++r) {
-              tile::accum<METRIC>(acc[r * NQ + i], q.x, x[r][1].x);
-              tile::accum<METRIC>(acc[r * NQ + i], q.y, x[r][1].y);
-              tile::accum<METRIC>(acc[r * NQ + i], q.z, x[r][1].z);
-              tile::accum<METRIC>(acc[r * NQ + i], q.w, x[r][1].w);
-            }
-          }
-        }
-      }
-    } else {
-      for (int k = lane; k < dim; k += 32) {
-        float x[SS_ROWS];
-#pragma unroll
-        for (int r = 0; r < SS_ROWS; ++r) x[r] = live[r] ? __ldg(a.x + (int64_t)rid[r] * dim + k) : 0.f;
-#pragma unroll
-        for (int i = 0; i < NQ; ++i) {
-          const float q = sq[i * dim + k];
-#pragma unroll
-          for (int r = 0; r < SS_ROWS; ++r) tile::accum<METRIC>(acc[r * NQ + i], q, x[r]);
-        }
-      }
-    }
+    stream_accumulate<METRIC, NQ, VEC, SS_ROWS>(acc, a.x, dim, sq, rid, live, lane);
     warp_reduce_scatter<V>(acc, lane);
     // the lane that owns pair j = lane >> OWNER_SHIFT finishes it
     if ((lane & ((1 << OWNER_SHIFT) - 1)) != 0) continue;
