@@ -355,7 +355,8 @@ int32_t few_metric(Ctx* ctx, const FewKernelArgs& ka, bool vec) {
 }  // namespace
 
 bool few_search_applies(const Ctx* ctx, const FewArgs& a) {
-  if (!ctx->tuning.stream_scan || a.k < 1 || a.k > kFewMaxK || a.nq < 1 || a.dim < 1) return false;
+  // (the fp32 search path is the chunked schedule by definition)
+  if (ctx->search_path != VSK_PATH_TENSOR_RERANK || !ctx->tuning.stream_scan || a.k < 1 || a.k > kFewMaxK || a.nq < 1 || a.dim < 1) return false;
   if (a.probes) return a.metric == VSK_METRIC_EUCLIDEAN && a.nq <= kStreamScanMaxSegQueries && few_smem<1>(a) <= kFewMaxSmem;
   if (a.nq > kStreamScanMaxQueries) return false;
   return (a.nq <= 1 ? few_smem<1>(a) : a.nq <= 2 ? few_smem<2>(a) : a.nq <= 4 ? few_smem<4>(a) : few_smem<8>(a)) <= kFewMaxSmem;
