@@ -1,0 +1,87 @@
+"""Manhattan batches through the byte filter (vabsdiff4 sums bound the fp32 distances, listed rows are re-scored): the rows
+the CPU oracle finds, for partial tiles, widths around the 16-byte pieces and 64-byte chunks, filters and hostile data."""
+import numpy as np
+import pytest
+
+import oracle
+from parity import assert_topk_parity
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def vsk():
+    import vectorstorekit_b200 as v
+    return v
+
+
+@pytest.fixture(scope="module")
+def dev(vsk):
+    return vsk.CUDAAcceleratorStrategy(0).initialize()
+
+
+def _index(vsk, dev, x, masks=None):
+    ix = vsk.FlatIndex(dev, x.shape[1], vsk.DistanceMetric.manhattan)
+    ix.add(x, masks)
+    return ix
+
+
+# every query tile (32, 64, 128), the smallest batch and index, partial query and row tiles, one and several chunks of
+# bytes, widths that are not multiples of 4 or 16, k up to the path's limit
+@pytest.mark.parametrize("shape", [(16_384, 256, 32, 50), (16_385, 64, 33, 1), (20_001, 65, 64, 10), (17_001, 5, 130, 10),
+                                   (30_000, 100, 128, 100), (18_000, 512, 250, 37), (40_000, 16, 96, 1024), (50_001, 250, 40, 10)])
+def test_byte_filter_finds_the_oracles_rows(vsk, dev, cpu_oracle, shape):
+    n, d, nq, k = shape
+    rng = np.random.default_rng(n + d)
+    x = (rng.uniform(-1, 1, (n, d)) + rng.normal(0, 3, d)).astype(np.float32)       # a centre of its own per dimension
+    q = (x[rng.integers(0, n, nq)] + rng.normal(0, 0.5, (nq, d))).astype(np.float32)
+    q[0] += 5.0                                                                       # outside the rows' range
+    ix = _index(vsk, dev, x)
+    before = dev.stats()["reranked_rows"]
+    got = ix.batchSearch(q, k)
+    assert dev.stats()["reranked_rows"] > before
+    assert_topk_parity(*got, *cpu_oracle.flat_search(oracle.MANHATTAN, q, x, k))
+    ix.add(x[:100] + 40.0)                                                            # a wider range: the grid is made again
+    assert_topk_parity(*ix.batchSearch(q, k), *cpu_oracle.flat_search(oracle.MANHATTAN, q, np.concatenate([x, x[:100] + 40.0]), k))
+
+
+@pytest.mark.parametrize("masks", ["few", "many"])
+def test_filters(vsk, dev, cpu_oracle, masks):
+    """Few distinct masks: a row list per group of queries; many: one pass with the masks tested on listed rows."""
+    rng = np.random.default_rng(9)
+    n, d, nq = 60_000, 32, 300
+    x = rng.uniform(-1, 1, (n, d)).astype(np.float32)
+    q = rng.uniform(-1, 1, (nq, d)).astype(np.float32)
+    rm = rng.integers(0, 2 ** 64, n, dtype=np.uint64)
+    if masks == "few":
+        qm = np.uint64(1) << rng.integers(0, 4, nq).astype(np.uint64)
+    else:
+        qm = rng.integers(1, 2 ** 64, nq, dtype=np.uint64)
+        qm[:5] = 1 << 7
+    got = _index(vsk, dev, x, rm).batchSearch(q, 20, qm)
+    assert_topk_parity(*got, *cpu_oracle.flat_search(oracle.MANHATTAN, q, x, 20, rm, qm))
+
+
+def test_outliers_ties_and_non_finite_values(vsk, dev, cpu_oracle):
+    rng = np.random.default_rng(10)
+    n, d, nq = 30_000, 24, 64
+    x = rng.uniform(-1, 1, (n, d)).astype(np.float32)
+    q = rng.uniform(-1, 1, (nq, d)).astype(np.float32)
+    wide = x.copy()
+    wide[123] = 1e6                                       # the step is wider than every distance: all lists overflow
+    ix = _index(vsk, dev, wide)
+    for _ in range(2):
+        assert_topk_parity(*ix.batchSearch(q, 10), *cpu_oracle.flat_search(oracle.MANHATTAN, q, wide, 10))
+    same = np.repeat(x[:3], n // 3, axis=0)               # thousands of rows at every distance
+    assert_topk_parity(*_index(vsk, dev, same).batchSearch(q, 10), *cpu_oracle.flat_search(oracle.MANHATTAN, q, same, 10))
+    const = np.full((n, d), 0.25, np.float32)             # no range at all
+    assert_topk_parity(*_index(vsk, dev, const).batchSearch(q, 10), *cpu_oracle.flat_search(oracle.MANHATTAN, q, const, 10))
+    bad = q.copy()
+    bad[5, 3], bad[40, 0] = np.nan, np.inf
+    keep = [i for i in range(nq) if i not in (5, 40)]
+    d_, i_ = _index(vsk, dev, x).batchSearch(bad, 10)
+    rd, ri = cpu_oracle.flat_search(oracle.MANHATTAN, q, x, 10)
+    assert_topk_parity(d_[keep], i_[keep], rd[keep], ri[keep])
+    inf = x.copy()
+    inf[7, 2] = np.inf                                    # no grid: the fp32 scan
+    assert_topk_parity(*_index(vsk, dev, inf).batchSearch(q, 10), *cpu_oracle.flat_search(oracle.MANHATTAN, q, inf, 10))

@@ -327,6 +327,11 @@ static int32_t fp32_search(Index* ix, const float* q, int64_t nq, const int32_t*
   a.xnorm = ix->row_norm;
   a.row_masks = (qmasks && ix->has_masks) ? ix->masks : nullptr;
   a.q_masks = a.row_masks ? qmasks : nullptr;
+  if (level == 0 && l1_applicable(ix, ix->n, nq, k)) {
+    bool handled = false;
+    VSK_TRY(l1_topk(ix, a, ix->n, nq, sub_dev, k, out_dist, out_ids, &handled));
+    if (handled) return VSK_OK;
+  }
   return fp32_topk(ix->ctx, a, ix->n, nq, sub_dev, k, ix->id_base, out_dist, out_ids, level);
 }
 
@@ -472,6 +477,11 @@ static int32_t filtered_grouped_search(Index* ix, const float* q, int64_t nq, in
     a.dim = ix->dim;
     a.qnorm = qnorm;
     a.xnorm = ix->row_norm;
+    if (l1_applicable(ix, cnt, e - b, k)) {
+      bool handled = false;
+      VSK_TRY(l1_topk(ix, a, cnt, e - b, qpos, k, out_dist, out_ids, &handled));
+      if (handled) continue;
+    }
     VSK_TRY(fp32_topk(ctx, a, cnt, e - b, qpos, k, ix->id_base, out_dist, out_ids, 0));
   }
   VSK_CUDA(ctx, cudaGetLastError());
@@ -957,6 +967,8 @@ int32_t vsk_index_destroy(vsk_index* i) {
   dev_free(ix->pq_codebooks);
   dev_free(ix->pq_codes);
   dev_free(ix->rows8);
+  dev_free(ix->rows_u8);
+  dev_free(ix->l1_lo);
   dev_free(ix->pq_cb16);
   dev_free(ix->pq_cw2);
   if (ix->coarse) {   // shares the centroids: only its derived buffers are its own

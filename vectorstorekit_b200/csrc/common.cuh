@@ -271,6 +271,14 @@ struct Index {
   int64_t n8 = -1;             // rows the two norms cover
   int i8_rest = 0;             // batches still to be left to the fp16 path
   float max_code_norm = 0.f, max_xnorm8 = 0.f;   // largest norm of a code row / of a decoded row
+  // byte copy of the rows for Manhattan batches (l1_scan.cu): x ~ l1_lo[d] + l1_step * u
+  uint8_t* rows_u8 = nullptr;  // [n][stride_u8]
+  int32_t stride_u8 = 0;
+  int64_t n_u8 = -1;           // rows the copy covers
+  bool l1_ok = false;          // ... and whether it is usable
+  int l1_rest = 0;             // batches still to be left to the fp32 scan
+  float* l1_lo = nullptr;      // [dim]
+  float l1_step = 1.f, l1_mag = 0.f, l1_ex = 0.f;   // grid step, largest |x|, largest L1 distance of a row to its bytes
   // ivf
   int32_t nlist = 0;
   float* centroids = nullptr;      // [nlist][dim]

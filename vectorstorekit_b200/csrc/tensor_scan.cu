@@ -1984,6 +1984,7 @@ void tensor_invalidate(Index* ix) {
   ix->n16 = -1;
   ix->n8 = -1;
   ix->i8_rest = 0;
+  ix->n_u8 = -1;
 }
 int32_t tensor_prepare_index(Index* ix) { return tensor_prepare(ix); }
 
