@@ -634,7 +634,7 @@ struct AsArgs {
   int32_t* log_count;         // [gridDim.x] entries written (capped); a CTA that ran out of room raises err = 9
   int64_t log_cap;            // entries per CTA = log_total / gridDim.x (set at launch)
   int64_t log_total;
-  unsigned long long* best;   // [n] SCAN_ARGMIN: smallest (value, centroid) key, pre-set to all ones
+  unsigned* best_value;       // [n] SCAN_ARGMIN: smallest value (float_to_ordered), pre-set to all ones
   int32_t* err;
   uint32_t wait_limit;
 };
@@ -983,38 +983,29 @@ assign_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
           }
           continue;
         }
-        float bv = CUDART_INF_F;   // SCAN_ARGMIN: this thread's best over its columns of the block
-        int bj = 0;
-#pragma unroll 1
-        for (int c = c0; c < c0 + GROUPS; ++c) {
-          float v[32];
-          tc_ld32(trow + (uint32_t)(c * 32), v);
-          const int left = a.k - (col_base + c * 32);   // valid centroids from this group's first column on
-          if (left <= 0) continue;
-          // alpha < 0: the smallest value of the group is alpha times its largest accumulator - one max per value;
-          // the column is looked for only when the group beats the best so far (ever more rarely as groups go by)
-          float amax = -CUDART_INF_F;
-          if (left >= 32) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) amax = fmaxf(amax, v[j]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) amax = j < left ? fmaxf(amax, v[j]) : amax;
-          }
-          const float gmin = amax * alpha;
-          if (gmin < bv) {   // strict '<': an earlier (lower) centroid keeps a tie
-            bv = gmin;
-            int jj = 31;
-#pragma unroll
-            for (int j = 31; j >= 0; --j) jj = (j < left && v[j] == amax) ? j : jj;   // the lowest column holding the max
-            bj = c * 32 + jj;
-          }
-        }
-        if (qok && bv < CUDART_INF_F)
-          atomicMin(a.best + q, (unsigned long long)make_key(bv, (uint32_t)(col_base + bj)));
+        // SCAN_ARGMIN: only the value is wanted (it becomes the row's threshold, and the pass that uses the threshold lists
+        // the centroids), so it costs half an instruction per column, the accumulator goes back before the values are
+        // looked at as above, and a warp's rows are one 128-byte atomic.  With the column and a 64-bit key per row the pass
+        // took 21.7 ms over 10 million rows x 128 and 4 096 centroids, twice the threshold pass.
+        float v0[32], v1[32];
+        tc_ld32_issue(trow + (uint32_t)(c0 * 32), v0);
+        tc_ld32_issue(trow + (uint32_t)((c0 + 1) * 32), v1);
+        tc_ld_wait();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm->tmem_empty[acc]);
+        const int left = a.k - (col_base + c0 * 32);   // valid centroids from this warp's first column on
+        if (left < 64) {   // the last block only
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            v0[j] = j < left ? v0[j] : -CUDART_INF_F;
+            v1[j] = j + 32 < left ? v1[j] : -CUDART_INF_F;
+          }
+        }
+        // alpha < 0: the smallest value is alpha times the largest accumulator
+        const float amax = fmaxf(max3(max8<0>(v0), max8<8>(v0), fmaxf(max8<16>(v0), max8<24>(v0))),
+                                 max3(max8<0>(v1), max8<8>(v1), fmaxf(max8<16>(v1), max8<24>(v1))));
+        if (qok && left > 0 && amax > -CUDART_INF_F) atomicMin(a.best_value + q, float_to_ordered(amax * alpha));
       }
     }
   }
@@ -1708,6 +1699,14 @@ __global__ void assign_threshold_kernel(const unsigned long long* __restrict__ b
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
   thr[r] = ordered_to_float((uint32_t)(best[r] >> 32)) + 2.0f * eps[r];
+  count[r] = 0;
+}
+// ... from the stationary kernel's values
+__global__ void assign_value_threshold_kernel(const unsigned* __restrict__ best, const float* __restrict__ eps, int64_t n,
+                                              float* __restrict__ thr, int32_t* __restrict__ count) {
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n) return;
+  thr[r] = ordered_to_float(best[r]) + 2.0f * eps[r];
   count[r] = 0;
 }
 
@@ -3484,7 +3483,7 @@ int32_t tensor_assign(Ctx* ctx, TensorAssign* ta, const float* rows, const float
     sa.log = reinterpret_cast<uint2*>(ta->keys);
     sa.log_total = n * (int64_t)kAssignLogPerRow;
     sa.log_count = ta->count;
-    sa.best = ta->best;
+    sa.best_value = reinterpret_cast<unsigned*>(ta->best);
     sa.err = (int32_t*)(sm + 5);
     // The centroids of the previous call and how far each has moved since: rows whose centroid has hardly moved take
     // their threshold from the triangle inequality instead of a read of the row (assign_prev_threshold_kernel).
@@ -3513,9 +3512,9 @@ int32_t tensor_assign(Ctx* ctx, TensorAssign* ta, const float* rows, const float
         launch_prev_threshold(ctx, rows, n, dim, centroids, assign, eps, ta->thr, ta->count, with_bound ? dist : nullptr,
                               ta->shift, st + 2 * n, 0.02f);
       } else {
-        VSK_CUDA(ctx, cudaMemsetAsync(ta->best, 0xff, (size_t)n * sizeof(unsigned long long), ctx->stream));
+        VSK_CUDA(ctx, cudaMemsetAsync(sa.best_value, 0xff, (size_t)n * sizeof(unsigned), ctx->stream));
         VSK_TRY(launch_assign_scan<SCAN_ARGMIN>(ctx, mr, mc, mrn, mcn, sa));
-        assign_threshold_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, ctx->stream>>>(ta->best, eps, n, ta->thr, ta->count);
+        assign_value_threshold_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, ctx->stream>>>(sa.best_value, eps, n, ta->thr, ta->count);
       }
       VSK_CUDA(ctx, cudaMemsetAsync(ta->best, 0xff, (size_t)n * sizeof(unsigned long long), ctx->stream));
       tl_mark(ctx, "assign_thresholds");
