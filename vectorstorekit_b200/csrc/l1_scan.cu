@@ -381,6 +381,7 @@ int32_t l1_topk(Index* ix, const ExactScanArgs& proto, int64_t n, int64_t nq, co
   VSK_TRY(launch_select(ctx, sel));
   sel.dense_count = -1;
   sel.max_count = kCandCap;
+  sel.by_length = 1;
   L1Args a{};
   a.q8 = q8;
   a.x8 = ix->rows_u8;

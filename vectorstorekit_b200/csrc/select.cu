@@ -31,6 +31,8 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 10 : 2) select_kernel(SelectAr
     c = a.dense_count;
   } else {
     const int raw = a.cand.count[q];
+    if (a.by_length == 2 && raw > CAPACITY) return;                  // the wide launch's
+    if (a.by_length == 3 && raw <= 128 * SEL_ITEMS) return;          // the narrow launch has taken it
     c = min(raw, CAPACITY);
     if (raw > CAPACITY && threadIdx.x == 0) atomicOr(&a.cand.flags[q], 1);
   }
@@ -352,6 +354,10 @@ int32_t launch_merge_keys(Ctx* ctx, const uint64_t* in, int32_t g, int64_t strid
   return VSK_OK;
 }
 
+// Compactions whose lists may be long but rarely are (by_length): 10 000 lists of a few hundred keys take the 512-thread
+// kernel 141 us and the 128-thread one 50; a pass over lists that are another launch's costs a few microseconds.
+constexpr int64_t kSelectByLengthMin = 1024;
+
 int32_t launch_select(Ctx* ctx, const SelectArgs& a) {
   if (a.nq <= 0) return VSK_OK;
   // lists known to hold at most 1024 keys take the 128-thread variant (four times as many CTAs per SM);
@@ -368,7 +374,14 @@ int32_t launch_select(Ctx* ctx, const SelectArgs& a) {
     prefer_shared_carveout(merge_keys_kernel<SEL_THREADS>);
     carveout_done = true;
   }
-  if (small) {
+  if (a.by_length == 1 && !small && a.dense_count < 0 && a.nq >= kSelectByLengthMin) {
+    SelectArgs one = a;
+    one.by_length = 2;   // first: what it shortens is short for the wide launch's test too
+    select_kernel<128><<<(unsigned)a.nq, 128, 0, ctx->stream>>>(one);
+    one.by_length = 3;
+    select_kernel<SEL_THREADS><<<(unsigned)a.nq, SEL_THREADS, 0, ctx->stream>>>(one);
+    ctx->stats.kernel_launches++;
+  } else if (small) {
     const size_t smem = a.out_ids ? 128 * SEL_ITEMS * sizeof(uint64_t) : 0;
     select_kernel<128><<<(unsigned)a.nq, 128, smem, ctx->stream>>>(a);
   } else {

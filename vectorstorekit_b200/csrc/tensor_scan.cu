@@ -2720,6 +2720,7 @@ int32_t ivf_tensor_search(Index* ix, const float* q, int64_t nq, const int64_t* 
     rerank_kernel<VSK_METRIC_EUCLIDEAN><<<(unsigned)nq, 256, qsm, ctx->stream>>>(q, ix->rows, dim, nullptr, nullptr, cand, rr_total);
     ctx->stats.kernel_launches++;
     sel.max_count = stage == 0 ? pilot_keep : kCandCap;
+    sel.by_length = stage == 0 ? 0 : 1;
     VSK_TRY(launch_select(ctx, sel));
     if (stage == 0) {
       // was the coarse pre-selection safe?  (also refreshes the coarse thresholds, which the next launch recomputes)
@@ -3010,6 +3011,7 @@ int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const
   VSK_TRY(launch_select(ctx, sel));
   sel.dense_count = -1;
   sel.max_count = kCandCap;
+  sel.by_length = 1;
   const int64_t growth = nq <= 2048 ? std::max(16, ctx->tuning.chunk_growth) : std::max(1, ctx->tuning.chunk_growth);
   PinnedBuf& hb = ctx->host_flags[ctx->lane];
   VSK_TRY(pinned_reserve(ctx, &hb, (size_t)nq * 4 + 16));
@@ -3310,6 +3312,7 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
   VSK_TRY(launch_select(ctx, sel));
   sel.dense_count = -1;
   sel.max_count = kCandCap;
+  sel.by_length = 1;
   PinnedBuf& hb = ctx->host_flags[ctx->lane];
   VSK_TRY(pinned_reserve(ctx, &hb, (size_t)nq * 4 + 16));
   char* hbuf = (char*)hb.p;
