@@ -1024,6 +1024,374 @@ assign_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   }
 }
 
+// ---- row lists of a batch with a STATIONARY query block ---------------------------------------------------------
+// The searches whose listed rows are re-scored after every chunk need one bit per (query, row) from the contraction: can the
+// row still be among the query's best?  With a short inner dimension the general kernel is paced by its operands: a
+// 128 x 256 tile of 144 fp16 columns fetches 144 KB for 1 152 cycles of MMAs through a ring that holds one tile and a half
+// (10 000 queries x 10 million decoded rows: 38 ms, 1.8 us per tile).  Here, as in assign_scan_kernel, a block of 256
+// queries stays in shared memory and 128-row tiles stream past it, a whole tile per ring stage (36 KB, four of them).
+// The queries' thresholds ride inside the contraction as well, subtracted in columns (fp16) or in a K step (int8) of their
+// own, so that "listed" is the sign of the accumulator: one instruction looks at three values, whatever their columns.
+//   order     rows are walked in windows that stay in L2; inside a window every CTA takes an equal stretch of the
+//             (query block, row tile) sequence, so it changes its block once or twice per window and no CTA is left over
+//   fp16      fold columns: eight hold the row term (pieces p0 x2, p1 x2, p2 x4 of R / 16, queries: 8u x4, 4u x4), eight
+//             the threshold (rows: the constant kLsBarConst, queries: pieces of minus the bar)
+//   int8      a K32 step of a constant tile (all kLsBarByte) against the queries' 32 threshold bytes
+// warp 0 TMA producer, warp 1 MMA issuer, 16 epilogue warps: a row per lane, 64 queries per warp.  A listed row goes to the
+// CTA's stretch of a log, its slot from a shared-memory counter, and ls_scatter_kernel moves the log to the candidate lists:
+// with an atomic on the list itself a warp sat out the round trip to L2, most tiles held such a warp, and the launch was no
+// faster than the general kernel (1.8 us per tile).  A full log falls back to that atomic.  The query operand is padded to
+// whole blocks with queries whose threshold nothing reaches, so the epilogue knows nothing of the last block's end (a test
+// there made its CTAs twice as slow as the rest).  Every wait is bounded.
+constexpr int LS_RING_BYTES = 224 * 1024;
+constexpr int LS_MAX_STAGES = 8;
+constexpr float kLsBarConst = 32768.f;
+constexpr int kLsBarByte = 127;
+
+struct LsSmem {
+  uint8_t ring[LS_RING_BYTES];   // [resident query block][constant tile (int8)][stages x 128-row tiles]
+  uint64_t full[LS_MAX_STAGES];
+  uint64_t empty[LS_MAX_STAGES];
+  uint64_t q_full, q_empty;
+  uint64_t tmem_full[2];
+  uint64_t tmem_empty[2];
+  uint64_t drain;
+  uint32_t tmem_base;
+  volatile int abort_flag;
+  int log_n;                     // rows this CTA has listed so far
+};
+constexpr size_t kLsSmemBytes = sizeof(LsSmem) + 1024;
+
+struct LsArgs {
+  int64_t rows;               // rows of the row operand
+  int64_t nq;
+  int64_t row_id0;            // id of operand row 0
+  int32_t kblocks;            // 128-byte K blocks, the fold block included
+  int32_t k16_last;           // 32-byte K steps of the last block that hold operand columns
+  int32_t window;             // row tiles per window
+  uint2* log;                 // [gridDim.x][log_cap] {row id, query}
+  int32_t* log_count;         // [gridDim.x]
+  int64_t log_cap;
+  CandLists cand;
+  int32_t* err;
+  uint32_t wait_limit;
+};
+
+// Bytes of the resident block and of a row tile; false when two whole-tile stages do not fit beside the block.
+struct LsLayout {
+  int nfull, res_bytes, const_off, bar_off, tile_bytes, stages;
+  bool narrow;
+};
+__host__ __device__ inline LsLayout ls_layout(int kblocks, int k16_last, bool i8) {
+  LsLayout l;
+  l.narrow = !i8 && k16_last == 1 && kblocks >= 2;   // the fold columns begin a block of their own: a 16-column tile
+  l.nfull = l.narrow ? kblocks - 1 : kblocks;
+  int at = l.nfull * B_BYTES + (l.narrow ? B_NARROW_BYTES : 0);
+  l.bar_off = at;
+  if (i8) at += B_NARROW_BYTES;
+  l.const_off = at;
+  if (i8) at += A_NARROW_BYTES;
+  l.res_bytes = at;
+  l.tile_bytes = l.nfull * A_BYTES + (l.narrow ? A_NARROW_BYTES : 0);
+  l.stages = (LS_RING_BYTES - at) / l.tile_bytes;
+  if (l.stages > LS_MAX_STAGES) l.stages = LS_MAX_STAGES;
+  return l;
+}
+
+// The stretches of (query block, row tile) pairs a CTA takes, one after the other.
+struct LsWalk {
+  int64_t ntiles, w0;      // row tiles in all; first tile of the current window
+  int nb, window;
+  int64_t pos, end;        // the CTA's part of the window's sequence (block-major)
+  int wt;                  // tiles of the window
+  __device__ __forceinline__ void start(int64_t nt, int blocks, int win) {
+    ntiles = nt;
+    nb = blocks;
+    window = win;
+    w0 = -win;
+    pos = end = 0;
+  }
+  // next stretch: block b, tiles [t, t + count)
+  __device__ __forceinline__ bool next(int& b, int64_t& t, int& count) {
+    while (pos >= end) {
+      w0 += window;
+      if (w0 >= ntiles) return false;
+      wt = (int)min((int64_t)window, ntiles - w0);
+      const int64_t all = (int64_t)wt * nb;
+      pos = all * blockIdx.x / gridDim.x;
+      end = all * (blockIdx.x + 1) / gridDim.x;
+    }
+    b = (int)(pos / wt);
+    const int in = (int)(pos - (int64_t)b * wt);
+    count = (int)min((int64_t)(wt - in), end - pos);
+    t = w0 + in;
+    pos += count;
+    return true;
+  }
+};
+
+template <bool I8>
+__global__ void __launch_bounds__(AS_THREADS, 1)
+list_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_q,
+                 const __grid_constant__ CUtensorMap map_xn, const __grid_constant__ CUtensorMap map_qn, LsArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  LsSmem* sm = reinterpret_cast<LsSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t wait_limit = a.wait_limit ? a.wait_limit : WAIT_LIMIT;
+  const LsLayout l = ls_layout(a.kblocks, a.k16_last, I8);
+  constexpr int KCOLS = I8 ? 2 * TK : TK;
+  const int nb = (int)((a.nq + TN - 1) / TN);
+  const int64_t ntiles = (a.rows + TM - 1) / TM;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < LS_MAX_STAGES; ++s) {
+      mbar_init(&sm->full[s], 1);
+      mbar_init(&sm->empty[s], 1);
+    }
+    mbar_init(&sm->q_full, 1);
+    mbar_init(&sm->q_empty, 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&sm->tmem_full[b], 1);
+      mbar_init(&sm->tmem_empty[b], AS_EW);
+    }
+    mbar_init(&sm->drain, 1);
+    sm->abort_flag = 0;
+    sm->log_n = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (I8) {   // the constant tile: the same byte everywhere, so its swizzle does not matter
+    for (int i = threadIdx.x; i < A_NARROW_BYTES / 4; i += AS_THREADS)
+      reinterpret_cast<uint32_t*>(sm->ring + l.const_off)[i] = 0x01010101u * (uint32_t)kLsBarByte;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm->tmem_base)),
+                 "r"(TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = sm->tmem_base;
+  uint8_t* ring = sm->ring + l.res_bytes;
+
+  if (warp == 0) {
+    // ---------------- TMA producer ----------------
+    if (lane == 0) {
+      int s = 0;
+      uint32_t ph = 0, qph = 0, issued = 0, issued_ph = 0, q_last = 0;
+      bool ok = true, q_issued = false;
+      LsWalk w;
+      w.start(ntiles, nb, a.window);
+      int b, count;
+      int64_t t;
+      while (ok && w.next(b, t, count)) {
+        // the block may be replaced once every MMA that read the previous one has retired
+        if (!mbar_wait(&sm->q_empty, qph ^ 1, &sm->abort_flag, a.err, 5, wait_limit)) break;
+        mbar_expect_tx(&sm->q_full, (uint32_t)(l.res_bytes - (I8 ? A_NARROW_BYTES : 0)));
+        for (int kb = 0; kb < l.nfull; ++kb) tma_load_2d(sm->ring + kb * B_BYTES, &map_q, &sm->q_full, kb * KCOLS, b * TN);
+        if (l.narrow) tma_load_2d(sm->ring + l.nfull * B_BYTES, &map_qn, &sm->q_full, l.nfull * KCOLS, b * TN);
+        if (I8) tma_load_2d(sm->ring + l.bar_off, &map_qn, &sm->q_full, 0, b * TN);
+        q_issued = true;
+        q_last = qph;
+        qph ^= 1;
+        for (int i = 0; i < count; ++i, ++t) {
+          if (!mbar_wait(&sm->empty[s], ph ^ 1, &sm->abort_flag, a.err, 1, wait_limit)) { ok = false; break; }
+          uint8_t* st = ring + s * l.tile_bytes;
+          mbar_expect_tx(&sm->full[s], (uint32_t)l.tile_bytes);
+          for (int kb = 0; kb < l.nfull; ++kb) tma_load_2d(st + kb * A_BYTES, &map_x, &sm->full[s], kb * KCOLS, (int32_t)(t * TM));
+          if (l.narrow) tma_load_2d(st + l.nfull * A_BYTES, &map_xn, &sm->full[s], l.nfull * KCOLS, (int32_t)(t * TM));
+          issued |= 1u << s;
+          issued_ph = (issued_ph & ~(1u << s)) | (ph << s);
+          if (++s == l.stages) { s = 0; ph ^= 1; }
+        }
+      }
+      // copies still in flight must land before the CTA's shared memory is released
+      if (q_issued)
+        for (uint32_t it = 0; it < wait_limit; ++it) {
+          if (mbar_try_wait(&sm->q_full, q_last)) break;
+          __nanosleep(64);
+        }
+      for (int i = 0; i < l.stages; ++i)
+        if (issued & (1u << i))
+          for (uint32_t it = 0; it < wait_limit; ++it) {
+            if (mbar_try_wait(&sm->full[i], (issued_ph >> i) & 1)) break;
+            __nanosleep(64);
+          }
+    }
+  } else if (warp == 1) {
+    // ---------------- MMA issuer (see assign_scan_kernel for why it looks ahead) ----------------
+    if (lane == 0) {
+      const uint32_t a_lo0 = desc_lo(smem_u32(ring)), stage_lo = (uint32_t)l.tile_bytes >> 4;
+      const uint32_t b_lo0 = desc_lo(smem_u32(sm->ring)), bn_lo = desc_lo(smem_u32(sm->ring + l.nfull * B_BYTES));
+      const uint32_t bar_lo = desc_lo(smem_u32(sm->ring + l.bar_off)), const_lo = desc_lo(smem_u32(sm->ring + l.const_off));
+      const uint32_t full0 = smem_u32(&sm->full[0]), empty0 = smem_u32(&sm->empty[0]);
+      const uint32_t tfull0 = smem_u32(&sm->tmem_full[0]), tempty0 = smem_u32(&sm->tmem_empty[0]);
+      const int last_nk4 = l.narrow ? 4 : a.k16_last;
+      uint32_t s = 0, ph = 0, qph = 0, acc = 0, aph = 0;
+      bool ok = true, pre_acc = false, pre_stage = false;
+      LsWalk w;
+      w.start(ntiles, nb, a.window);
+      int b, count;
+      int64_t t;
+      while (ok && w.next(b, t, count)) {
+        if (!mbar_wait(&sm->q_full, qph, &sm->abort_flag, a.err, 6, wait_limit)) break;
+        qph ^= 1;
+        for (int left = count; left > 0; --left) {
+          if (!pre_acc && !mbar_wait(&sm->tmem_empty[acc], aph ^ 1, &sm->abort_flag, a.err, 2, wait_limit)) { ok = false; break; }
+          if (!pre_stage && !mbar_wait(&sm->full[s], ph, &sm->abort_flag, a.err, 3, wait_limit)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t tmem_d = tmem_base + acc * (uint32_t)TN;
+          const uint32_t a_lo = a_lo0 + s * stage_lo;
+          const uint32_t ns = s + 1 == (uint32_t)l.stages ? 0u : s + 1;
+          const uint32_t nph = s + 1 == (uint32_t)l.stages ? ph ^ 1u : ph;
+          const uint32_t naph = acc ? aph ^ 1u : aph;
+          const bool more = left > 1;
+          pre_acc = false;
+          pre_stage = false;
+          if (I8)   // first, as it needs nothing of the row tile
+            tc_mma_i8(tmem_d, desc_pack(const_lo, kDescHiNarrow), desc_pack(bar_lo, kDescHiNarrow), kIdescI8, 0u);
+          for (int kb = 0; kb < l.nfull; ++kb) {
+            if (kb == l.nfull - 1 && more) {
+              pre_stage = mbar_test_wait_a(full0 + ns * 8u, nph);
+              pre_acc = mbar_test_wait_a(tempty0 + (acc ^ 1u) * 8u, naph ^ 1u);
+            }
+            const int nk4 = kb == l.nfull - 1 ? last_nk4 : TK / 16;
+#pragma unroll
+            for (int k4 = 0; k4 < TK / 16; ++k4)
+              if (k4 < nk4) {
+                const uint64_t ad = desc_pack(a_lo + (uint32_t)(kb * (A_BYTES >> 4) + k4 * 2), kDescHi);
+                const uint64_t bd = desc_pack(b_lo0 + (uint32_t)(kb * (B_BYTES >> 4) + k4 * 2), kDescHi);
+                if (I8) tc_mma_i8(tmem_d, ad, bd, kIdescI8, 1u);
+                else tc_mma(tmem_d, ad, bd, kIdesc, (kb | k4) ? 1u : 0u);
+              }
+          }
+          if (l.narrow) {
+            // a second look for what the first one came too early for
+            if (more && !pre_stage) pre_stage = mbar_test_wait_a(full0 + ns * 8u, nph);
+            if (more && !pre_acc) pre_acc = mbar_test_wait_a(tempty0 + (acc ^ 1u) * 8u, naph ^ 1u);
+            tc_mma(tmem_d, desc_pack(a_lo + (uint32_t)(l.nfull * (A_BYTES >> 4)), kDescHiNarrow), desc_pack(bn_lo, kDescHiNarrow), kIdesc, 1u);
+          }
+          tc_commit_a(empty0 + s * 8u);
+          tc_commit_a(tfull0 + acc * 8u);
+          s = ns;
+          ph = nph;
+          aph = naph;
+          acc ^= 1u;
+        }
+        if (ok) tc_commit(&sm->q_empty);
+      }
+      // all issued MMAs must retire before tensor memory is freed
+      tc_commit(&sm->drain);
+      for (uint32_t it = 0; it < wait_limit; ++it) {
+        if (mbar_try_wait(&sm->drain, 0)) break;
+        __nanosleep(64);
+      }
+    }
+  } else {
+    // ---------------- epilogue: one row per lane, 64 queries per warp ----------------
+    const int quarter = warp & 3, part = (warp - 2) >> 2;
+    const int et = quarter * 32 + lane;
+    bool ok = true;
+    uint32_t acc = 0, aph = 0;
+    LsWalk w;
+    w.start(ntiles, nb, a.window);
+    int b, count;
+    int64_t t;
+    uint2* my_log = a.log + (int64_t)blockIdx.x * a.log_cap;
+    while (ok && w.next(b, t, count)) {
+      const int64_t col0 = (int64_t)b * TN + part * 64;
+      for (int i = 0; i < count; ++i, ++t) {
+        bool got = mbar_wait(&sm->tmem_full[acc], aph, &sm->abort_flag, a.err, 4, wait_limit);
+        got = __all_sync(0xffffffffu, got);
+        if (!got) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t trow = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * (uint32_t)TN + (uint32_t)(part * 64);
+        float v0[32], v1[32];
+        tc_ld32_issue(trow, v0);
+        tc_ld32_issue(trow + 32u, v1);
+        tc_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm->tmem_empty[acc]);   // the accumulator goes back before the values are looked at
+        aph = acc ? aph ^ 1u : aph;
+        acc ^= 1u;
+        const int64_t row = t * TM + et;
+        // the sign bits of eight values at a time: clear in the AND of the values' words iff one is not negative
+        uint32_t neg[8];
+#pragma unroll
+        for (int o = 0; o < 4; ++o) {
+          neg[o] = 0xffffffffu;
+          neg[o + 4] = 0xffffffffu;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            neg[o] &= __float_as_uint(v0[8 * o + j]);
+            neg[o + 4] &= __float_as_uint(v1[8 * o + j]);
+          }
+        }
+        const uint32_t all = neg[0] & neg[1] & neg[2] & neg[3] & neg[4] & neg[5] & neg[6] & neg[7];
+        const bool mine = (int)all >= 0 && row < a.rows;
+        if (!__any_sync(0xffffffffu, mine)) continue;
+        if (!mine) continue;
+        const uint32_t id = (uint32_t)(a.row_id0 + row);
+        auto append = [&](uint32_t bits, int64_t first) {
+          while (bits) {
+            const int j = __ffs((int)bits) - 1;
+            bits &= bits - 1u;
+            const int64_t q = first + j;
+            const int at = atomicAdd(&sm->log_n, 1);
+            if (at < a.log_cap) {
+              my_log[at] = make_uint2(id, (uint32_t)q);
+            } else {
+              const int slot = atomicAdd(&a.cand.count[q], 1);
+              if (slot < kCandCap) a.cand.keys[q * kCandCap + slot] = make_key(0.f, id);
+            }
+          }
+        };
+#pragma unroll
+        for (int o = 0; o < 4; ++o) {
+          if ((int)neg[o] >= 0) {
+            uint32_t bits = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) bits |= (__float_as_uint(v0[8 * o + j]) >> 31) << j;
+            append(bits ^ 0xffu, col0 + 8 * o);
+          }
+        }
+#pragma unroll
+        for (int o = 0; o < 4; ++o) {
+          if ((int)neg[o + 4] >= 0) {
+            uint32_t bits = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) bits |= (__float_as_uint(v1[8 * o + j]) >> 31) << j;
+            append(bits ^ 0xffu, col0 + 32 + 8 * o);
+          }
+        }
+      }
+    }
+  }
+
+  // ---------------- teardown ----------------
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x == 0) a.log_count[blockIdx.x] = (int32_t)min((int64_t)sm->log_n, a.log_cap);
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+  }
+}
+
+// The logs of the CTAs (blockIdx.y) to the candidate lists; a key's value is formed by the re-scoring.
+__global__ void __launch_bounds__(256) ls_scatter_kernel(const uint2* __restrict__ log, const int32_t* __restrict__ log_count, int64_t log_cap,
+                                                         CandLists cand) {
+  const int cnt = log_count[blockIdx.y];
+  const uint2* mine = log + (int64_t)blockIdx.y * log_cap;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < cnt; e += gridDim.x * blockDim.x) {
+    const uint2 h = mine[e];
+    const int slot = atomicAdd(&cand.count[h.y], 1);
+    if (slot < kCandCap) cand.keys[(int64_t)h.y * kCandCap + slot] = make_key(0.f, h.x);
+  }
+}
+
 // One warp per logged hit: the exact squared distance of the row to the listed centroid, direct fp32 formula, merged
 // into best[row] - smallest (value, centroid), the reference's strict '<' scan (KMeansClustering.swift:283-288).
 template <bool VEC>
@@ -1499,6 +1867,21 @@ int32_t make_map_i8(Ctx* ctx, const int8_t* base, int64_t rows, int32_t cols, in
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(ctx, VSK_ERR_EXECUTION_FAILED, "cuTensorMapEncodeTiled (int8) failed with %d", (int)r);
+  return VSK_OK;
+}
+
+// bytes [rows][32], whole rows: box = 32 bytes x box_rows, 32-byte swizzle
+int32_t make_map_bytes(Ctx* ctx, const int8_t* base, int64_t rows, int box_rows, CUtensorMap* map) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(ctx, VSK_ERR_EXECUTION_FAILED, "cuTensorMapEncodeTiled is not available from this driver");
+  cuuint64_t gdim[2] = {32, (cuuint64_t)rows};
+  cuuint64_t gstride[1] = {32};
+  cuuint32_t box[2] = {32u, (cuuint32_t)box_rows};
+  cuuint32_t estride[2] = {1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t*>(base), gdim, gstride, box, estride,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(ctx, VSK_ERR_EXECUTION_FAILED, "cuTensorMapEncodeTiled (bytes) failed with %d", (int)r);
   return VSK_OK;
 }
 
@@ -1994,6 +2377,7 @@ struct QueryOperands {
   __half* q16 = nullptr;
   float* eps = nullptr;
   float* alpha = nullptr;
+  float* scale = nullptr;   // device scalar s_q
   int32_t* err = nullptr;
   unsigned long long* rr_total = nullptr;
 };
@@ -2024,8 +2408,10 @@ int32_t prepare_query_operands(Index* ix, const float* q, int64_t nq, QueryOpera
   const int metric = ix->metric;
   const int dim = ix->dim, dim16 = ix->dim16;
   void* p;
-  VSK_TRY(scratch(ctx, SLOT_Q16, (size_t)nq * dim16 * sizeof(__half), &p));
+  const int64_t nq_pad = ix->kind == INDEX_PQ ? ceil_div(nq, TN) * TN : nq;   // (list_scan_kernel's whole blocks)
+  VSK_TRY(scratch(ctx, SLOT_Q16, (size_t)nq_pad * dim16 * sizeof(__half), &p));
   __half* q16 = (__half*)p;
+  if (nq_pad > nq) VSK_CUDA(ctx, cudaMemsetAsync(q16 + nq * dim16, 0, (size_t)(nq_pad - nq) * dim16 * sizeof(__half), ctx->stream));
   VSK_TRY(scratch(ctx, SLOT_QAUX, (size_t)nq * 4 * sizeof(float) + 64, &p));
   float* qn16 = (float*)p;
   float* qe16 = qn16 + nq;
@@ -2060,7 +2446,9 @@ int32_t prepare_query_operands(Index* ix, const float* q, int64_t nq, QueryOpera
   }
   const bool fold = ix->fold16;
   const FoldArgs qfold{fold ? 2 : 0, fold_col0(ix->dim), ix->fold_exp};
-  choose_scale_kernel<<<1, 1, 0, ctx->stream>>>(q_absmax, cosine ? 1 : 0, q_scale, fold ? 1 : 0, ix->fold_exp);
+  // (a product-quantised index may put twice the constants into the fold columns, list_scan_kernel)
+  choose_scale_kernel<<<1, 1, 0, ctx->stream>>>(q_absmax, cosine ? 1 : 0, q_scale, fold ? 1 : 0,
+                                                ix->fold_exp - (ix->kind == INDEX_PQ ? 1 : 0));
   ctx->stats.kernel_launches++;
   BoundConsts bc{ix->scale16, ix->max_xnorm16, ix->max_xerr16, ix->max_xnorm, ix->min_xnorm_nz, dim16, fold ? ix->fold_bmax : 0.f};
   const unsigned bgrid = (unsigned)ceil_div(nq, 256);
@@ -2091,6 +2479,7 @@ int32_t prepare_query_operands(Index* ix, const float* q, int64_t nq, QueryOpera
   out->q16 = q16;
   out->eps = eps;
   out->alpha = alpha;
+  out->scale = q_scale;
   out->err = err;
   out->rr_total = rr_total;
   return VSK_OK;
@@ -2763,6 +3152,91 @@ int32_t ivf_tensor_search(Index* ix, const float* q, int64_t nq, const int64_t* 
   return VSK_OK;
 }
 
+constexpr int64_t kLsWindowBytes = 40ll << 20;   // rows a window of list_scan_kernel keeps in L2
+
+template <bool I8>
+static int32_t launch_list_scan(Ctx* ctx, const CUtensorMap& mx, const CUtensorMap& mq, const CUtensorMap& mxn, const CUtensorMap& mqn,
+                                LsArgs a, int64_t row_bytes) {
+  static bool attr_done = false;
+  if (!attr_done) {
+    VSK_CUDA(ctx, cudaFuncSetAttribute(list_scan_kernel<I8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLsSmemBytes));
+    attr_done = true;
+  }
+  const int64_t tiles = ceil_div(a.nq, TN) * ceil_div(a.rows, TM);
+  if (tiles <= 0) return VSK_OK;
+  a.window = (int32_t)std::max<int64_t>(1, kLsWindowBytes / (row_bytes * TM));
+  a.wait_limit = ctx->tuning.wait_limit_log2 > 0 ? (1u << std::min(ctx->tuning.wait_limit_log2, 30)) : 0u;
+  const unsigned grid = (unsigned)std::min<int64_t>(tiles, ctx->prop.multiProcessorCount);
+  // room for 256 rows per query (a chunk lists a few times k); what does not fit is appended by the scan itself
+  const int64_t total = std::max<int64_t>(1 << 16, std::min<int64_t>(a.nq * 256, 8 << 20));
+  void* p;
+  VSK_TRY(scratch(ctx, SLOT_LS_LOG, (size_t)total * sizeof(uint2) + (size_t)grid * sizeof(int32_t), &p));
+  a.log = (uint2*)p;
+  a.log_count = (int32_t*)(a.log + total);
+  a.log_cap = total / grid;
+  prof_begin(ctx);
+  list_scan_kernel<I8><<<grid, AS_THREADS, kLsSmemBytes, ctx->stream>>>(mx, mq, mxn, mqn, a);
+  prof_end(ctx);
+  tl_mark(ctx, "list_scan");
+  ls_scatter_kernel<<<dim3(8, grid), 256, 0, ctx->stream>>>(a.log, a.log_count, a.log_cap, a.cand);
+  ctx->stats.kernel_launches += 2;
+  ctx->stats.tensor_tiles += tiles;
+  VSK_CUDA(ctx, cudaGetLastError());
+  return VSK_OK;
+}
+
+// Fold columns of the query operand for list_scan_kernel, once per chunk: the row term's constants (8u x4, 4u x4) and the
+// pieces of minus the bar.  A row is listed iff  acc = s_q s_x (q.x - |x|^2 / 2)  reaches  bar = -thr s_q s_x / 2, lowered by
+// the fp32 accumulation error of its own products.  A bar the columns cannot hold from below flags the query.
+__global__ void ls_fold_queries_kernel(const float* __restrict__ thr, int64_t nq, int64_t nq_pad, const float* scale_q, float scale_x, int fold_exp,
+                                       int dim16, int col0, __half* __restrict__ q16, int32_t* __restrict__ flags) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nq_pad) return;
+  const float s = *scale_q, u = i < nq ? ldexpf(s, -fold_exp) : 0.f;
+  float R = i < nq ? -0.5f * thr[i] * s * scale_x : 1e9f;   // the bar
+  R = R - fabsf(R) * ((float)dim16 * 2.3841858e-7f + 1e-6f) - 1e-30f;
+  constexpr float kTop = 2.0f * kLsBarConst * 60000.f;
+  if (!(R >= -kTop)) {                                 // (also what is not a number)
+    R = -kTop;
+    atomicOr(&flags[i], 2);
+  }
+  R = fminf(R, kTop);
+  const float inv = 1.0f / (2.0f * kLsBarConst);       // minus the bar = 2 c p0 + 2 c p1 + 4 c p2
+  const __half p0 = __float2half_rn(-R * inv);
+  const float r1 = -R - 2.0f * kLsBarConst * __half2float(p0);
+  const __half p1 = __float2half_rn(r1 * inv);
+  const __half p2 = __float2half_ru((r1 - 2.0f * kLsBarConst * __half2float(p1)) * (0.5f * inv));   // never below: the bar is not raised
+  __align__(16) __half h[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j)
+    h[j] = j < 8 ? __float2half_rn(j < 4 ? 8.0f * u : 4.0f * u) : j < 10 ? p0 : j < 12 ? p1 : p2;
+  uint4* dst = reinterpret_cast<uint4*>(q16 + i * dim16 + col0);
+  dst[0] = *reinterpret_cast<const uint4*>(&h[0]);
+  dst[1] = *reinterpret_cast<const uint4*>(&h[8]);
+}
+
+// The same for int8 operands: 32 bytes b per query with 127 sum(b) >= -bar, the bar rounded down to a step of 127.
+__global__ void ls_bar_bytes_kernel(const int32_t* __restrict__ bar, int64_t nq, int64_t nq_pad, int8_t* __restrict__ out,
+                                    int32_t* __restrict__ flags) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nq_pad) return;
+  const int64_t want = i < nq ? -(int64_t)bar[i] : -100000;
+  int64_t total = want >= 0 ? (want + kLsBarByte - 1) / kLsBarByte : -((-want) / kLsBarByte);   // rounded up
+  if (total > 32 * 127) {   // more rows would have to be listed than the bytes can ask for
+    total = 32 * 127;
+    atomicOr(&flags[i], 2);
+  }
+  total = max(total, (int64_t)-32 * 128);
+  const int base = (int)(total >= 0 ? total / 32 : -((-total + 31) / 32));
+  const int rest = (int)(total - (int64_t)base * 32);   // 0 .. 31 of the bytes are one larger
+  __align__(16) int8_t h[32];
+#pragma unroll
+  for (int j = 0; j < 32; ++j) h[j] = (int8_t)(base + (j < rest ? 1 : 0));
+  uint4* dst = reinterpret_cast<uint4*>(out + i * 32);
+  dst[0] = *reinterpret_cast<const uint4*>(&h[0]);
+  dst[1] = *reinterpret_cast<const uint4*>(&h[16]);
+}
+
 // ---- product-quantised rows on the tensor cores -------------------------------------------------------------
 // The asymmetric distance of a code row is the squared distance between the query and the row the code decodes to,
 // so a batch of queries over m-byte codes is the same contraction as over fp32 rows.  The table scan (pq.cu) does m
@@ -2818,7 +3292,11 @@ __global__ void __launch_bounds__(256) pq_decode16_kernel(const uint8_t* __restr
       const __half p1 = __float2half_rn(r1 * 0.0625f);
       const __half p2 = __float2half_rn((r1 - 16.0f * __half2float(p1)) * 0.0625f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) h[j] = __hneg(c == col0 ? (j < 4 ? p0 : p1) : p2);
+      for (int j = 0; j < 8; ++j) {
+        // fold 2: list_scan_kernel's columns (the row term in eight of them, the constant of the thresholds in the rest)
+        if (fold == 2) h[j] = c == col0 ? __hneg(j < 2 ? p0 : j < 4 ? p1 : p2) : __float2half_rn(kLsBarConst);
+        else h[j] = __hneg(c == col0 ? (j < 4 ? p0 : p1) : p2);
+      }
     } else if (DS > 0 && c + 8 <= dim) {
       constexpr int W = DS > 0 ? (DS < 8 ? DS : 8) : 1;   // halves taken from one codeword
 #pragma unroll
@@ -2971,6 +3449,9 @@ int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const
   const int m = ix->pq_m, ksub = ix->pq_ksub, dim = ix->dim, dim16 = ix->dim16, ds = dim / m;
   const int64_t n = ix->n;
   const bool fold = ix->fold16;
+  // a short contraction with the folded row term: queries resident, rows streamed, thresholds folded in too
+  const int k16_last = k16_last_of(fold ? fold_col0(dim) + kFoldCols : dim, dim16);
+  const bool list = fold && dim16 / TK <= AS_MAX_KB && ls_layout(dim16 / TK, k16_last, false).stages >= 2;
   void* p;
   // the decoded block; without room for it the table scan takes the batch
   const int64_t block = std::min(ceil_div(n, TN) * TN, std::max<int64_t>(TN, kPqBlockBytes / ((int64_t)dim16 * 2) / TN * TN));
@@ -2980,8 +3461,9 @@ int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const
   QueryOperands qo;
   VSK_TRY(prepare_query_operands(ix, q, nq, &qo));
   const float* qnorm = qo.eps + nq;   // |q| as the operand preparation measured it
-  CUtensorMap mq, mx;
-  VSK_TRY(make_map(ctx, qo.q16, nq, dim16, TM, &mq));
+  CUtensorMap mq, mx, mqn, mxn;
+  VSK_TRY(make_map(ctx, qo.q16, list ? ceil_div(nq, TN) * TN : nq, dim16, list ? TN : TM, &mq));
+  VSK_TRY(make_map_narrow(ctx, qo.q16, ceil_div(nq, TN) * TN, dim16, TN, &mqn));
   CandLists cand;
   VSK_TRY(cand_lists(ctx, nq, &cand));
   VSK_TRY(launch_init_cand(ctx, cand, nq));
@@ -2991,7 +3473,7 @@ int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const
   TcArgs a{};
   a.nq = nq;
   a.kblocks = dim16 / TK;
-  a.k16_last = k16_last_of(fold ? fold_col0(dim) + kFoldCols : dim, dim16);
+  a.k16_last = k16_last;
   a.mode = SCAN_THRESHOLD;
   a.alpha = qo.alpha;
   a.beta = fold ? nullptr : aux;
@@ -3036,7 +3518,7 @@ int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const
     const size_t dsm = (size_t)PQ_DEC_ROWS * m;
 #define VSK_PQ_DEC(DS_)                                                                                                          \
     pq_decode16_kernel<DS_><<<dgrid, 256, dsm, ctx->stream>>>(ix->pq_codes + seen * m, chunk, dim, dim16, m, ksub, ds, ix->pq_cb16, \
-                                                              ix->pq_cw2, ix->scale16, fold ? 1 : 0, fold_col0(dim), ix->fold_exp,  \
+                                                              ix->pq_cw2, ix->scale16, list ? 2 : fold ? 1 : 0, fold_col0(dim), ix->fold_exp,  \
                                                               rows16, fold ? nullptr : aux)
     if (ds == 8) VSK_PQ_DEC(8);
     else if (ds % 8 == 0) VSK_PQ_DEC(16);
@@ -3044,14 +3526,32 @@ int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const
     else if (ds == 2) VSK_PQ_DEC(2);
     else VSK_PQ_DEC(0);
 #undef VSK_PQ_DEC
+    tl_mark(ctx, "pq_decode");
     pq_coarse_threshold_kernel<<<(unsigned)ceil_div(nq, 256), 256, 0, ctx->stream>>>(
         cand.thr, qnorm, qo.eps, nq, (float)(m + ds + 8), (float)(ceil_div(dim, 32) + 16), cand_coarse.thr);
     ctx->stats.kernel_launches += 2;
     VSK_CUDA(ctx, cudaGetLastError());
-    VSK_TRY(make_map(ctx, rows16, chunk, dim16, TN, &mx));
-    a.row_begin = 0;
-    a.row_end = chunk;
-    VSK_TRY(launch_tc<SCAN_THRESHOLD>(ctx, mq, mx, a, !fold));
+    if (list) {
+      VSK_TRY(make_map(ctx, rows16, chunk, dim16, TM, &mx));
+      VSK_TRY(make_map_narrow(ctx, rows16, chunk, dim16, TM, &mxn));
+      const int64_t nq_pad = ceil_div(nq, TN) * TN;
+      ls_fold_queries_kernel<<<(unsigned)(nq_pad / 256), 256, 0, ctx->stream>>>(cand_coarse.thr, nq, nq_pad, qo.scale, ix->scale16, ix->fold_exp,
+                                                                                   dim16, fold_col0(dim), qo.q16, cand.flags);
+      ctx->stats.kernel_launches++;
+      LsArgs la{};
+      la.rows = chunk;
+      la.nq = nq;
+      la.kblocks = dim16 / TK;
+      la.k16_last = k16_last;
+      la.cand = cand;
+      la.err = qo.err;
+      VSK_TRY(launch_list_scan<false>(ctx, mx, mq, mxn, mqn, la, (int64_t)dim16 * 2));
+    } else {
+      VSK_TRY(make_map(ctx, rows16, chunk, dim16, TN, &mx));
+      a.row_begin = 0;
+      a.row_end = chunk;
+      VSK_TRY(launch_tc<SCAN_THRESHOLD>(ctx, mq, mx, a, !fold));
+    }
     pq_rescore_kernel<<<(unsigned)nq, 128, 0, ctx->stream>>>(tables, ix->pq_codes, m, ksub, seen, (int)std::min<int64_t>(k, seen), cand, qo.rr_total);
     ctx->stats.kernel_launches++;
     VSK_CUDA(ctx, cudaGetLastError());
@@ -3258,11 +3758,18 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
   const int dim = ix->dim, stride = ix->stride8;
   const int64_t n = ix->n;
   void* p;
-  VSK_TRY(scratch(ctx, SLOT_Q16, (size_t)nq * stride, &p));
+  const int64_t nq_pad = ceil_div(nq, TN) * TN;   // (list_scan_kernel's whole blocks)
+  VSK_TRY(scratch(ctx, SLOT_Q16, (size_t)nq_pad * stride, &p));
   int8_t* q8 = (int8_t*)p;
+  VSK_CUDA(ctx, cudaMemsetAsync(q8 + nq * stride, 0, (size_t)(nq_pad - nq) * stride, ctx->stream));
   VSK_TRY(scratch(ctx, SLOT_QAUX, (size_t)nq * (sizeof(I8Query) + 4), &p));
   I8Query* info = (I8Query*)p;
   int32_t* bar = (int32_t*)(info + nq);
+  // up to three K blocks: queries resident, rows streamed, the bars folded in
+  const int32_t kblocks = (int32_t)ceil_div(dim, 2 * TK), k_last = (int32_t)(ceil_div(dim, 32) - 4 * (kblocks - 1));
+  const bool list = ls_layout(kblocks, k_last, true).stages >= 2;
+  VSK_TRY(scratch(ctx, SLOT_TC_C, (size_t)nq_pad * 32, &p));
+  int8_t* bar8 = (int8_t*)p;
   VSK_TRY(scratch(ctx, SLOT_TC_B, 64, &p));
   VSK_CUDA(ctx, cudaMemsetAsync(p, 0, 64, ctx->stream));
   const float* alpha = (const float*)p + 2;
@@ -3271,16 +3778,18 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
   i8_query_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, ctx->stream>>>(q, nq, dim, stride, ix->sq_scale, ix->sq_offset, ix->max_code_norm,
                                                                       ix->max_xnorm8, q8, info);
   ctx->stats.kernel_launches++;
-  CUtensorMap mq, mx;
-  VSK_TRY(make_map_i8(ctx, q8, nq, dim, stride, TM, &mq));
-  VSK_TRY(make_map_i8(ctx, ix->rows8 ? ix->rows8 : ix->codes, n, dim, stride, TN, &mx));
+  CUtensorMap mq, mx, mb;
+  const int8_t* rows8 = ix->rows8 ? ix->rows8 : ix->codes;
+  VSK_TRY(make_map_i8(ctx, q8, list ? nq_pad : nq, dim, stride, list ? TN : TM, &mq));
+  VSK_TRY(make_map_i8(ctx, rows8, n, dim, stride, list ? TM : TN, &mx));
+  VSK_TRY(make_map_bytes(ctx, bar8, nq_pad, TN, &mb));
   CandLists cand;
   VSK_TRY(cand_lists(ctx, nq, &cand));
   VSK_TRY(launch_init_cand(ctx, cand, nq));
   TcArgs a{};
   a.nq = nq;
-  a.kblocks = (int32_t)ceil_div(dim, 2 * TK);
-  a.k16_last = (int32_t)(ceil_div(dim, 32) - 4 * (a.kblocks - 1));
+  a.kblocks = kblocks;
+  a.k16_last = k_last;
   a.mode = SCAN_THRESHOLD;
   a.alpha = alpha;
   a.cand = cand;
@@ -3345,7 +3854,20 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
     ctx->stats.kernel_launches++;
     a.row_begin = seen;
     a.row_end = seen + chunk;
-    if (tc_epilogue_warps(a.kblocks) == 16) VSK_TRY((launch_tc_ew<SCAN_THRESHOLD, 16, true>(ctx, mq, mx, a, false)));
+    if (list) {
+      ls_bar_bytes_kernel<<<(unsigned)(nq_pad / 256), 256, 0, ctx->stream>>>(bar, nq, nq_pad, bar8, cand.flags);
+      ctx->stats.kernel_launches++;
+      VSK_TRY(make_map_i8(ctx, rows8 + seen * stride, chunk, dim, stride, TM, &mx));
+      LsArgs la{};
+      la.rows = chunk;
+      la.nq = nq;
+      la.row_id0 = seen;
+      la.kblocks = kblocks;
+      la.k16_last = k_last;
+      la.cand = cand;
+      la.err = err;
+      VSK_TRY(launch_list_scan<true>(ctx, mx, mq, mx, mb, la, stride));
+    } else if (tc_epilogue_warps(a.kblocks) == 16) VSK_TRY((launch_tc_ew<SCAN_THRESHOLD, 16, true>(ctx, mq, mx, a, false)));
     else VSK_TRY((launch_tc_ew<SCAN_THRESHOLD, 8, true>(ctx, mq, mx, a, false)));
     rerank_i8_kernel<VSK_METRIC_DOT_PRODUCT><<<(unsigned)nq, 256, qsm, ctx->stream>>>(q, ix->codes, dim, ix->sq_scale, ix->sq_offset, cand, rr_total);
     ctx->stats.kernel_launches++;
