@@ -104,3 +104,30 @@ def test_repeated_calls_leave_the_tickets_at_zero(vsk, dev, cpu_oracle):
         assert_topk_parity(*ivf.batchSearch(q, 20), rd, ri)      # every list is probed: the flat result
         rd, ri = cpu_oracle.flat_search(oracle.DOT, q, x[:100], 5)
         assert_topk_parity(*small.batchSearch(q, 5), rd, ri)
+
+
+@pytest.fixture(scope="module")
+def large():
+    """Rows beyond the line from which the fp16 copy is read; row 7 twice, and a nearest row 1 500 times for one query."""
+    rng = np.random.default_rng(6)
+    x = rng.standard_normal((110_000, 1_300), dtype=np.float32)
+    x[90_000] = x[7]
+    q = rng.standard_normal((6, 1_300), dtype=np.float32)
+    q[1] = x[7] + 0.01
+    q[4] = x[500] * 1.1
+    x[60_000:61_500] = x[500]
+    return x, q
+
+
+@pytest.mark.parametrize("metric", ["euclidean", "cosine", "dotProduct"])
+@pytest.mark.parametrize("nq,k", [(1, 10), (3, 100), (6, 128)])
+def test_large_store_reads_the_fp16_copy(vsk, dev, cpu_oracle, large, metric, nq, k):
+    x, q = large
+    ix = _index(vsk, dev, metric, x)
+    before = dev.stats()
+    got = ix.batchSearch(q[:nq], k)
+    after = dev.stats()
+    assert after["tensor_tiles"] == before["tensor_tiles"]
+    assert (after["fallback_queries"] > before["fallback_queries"]) == (nq > 4)    # 1 500 equal rows fill one query's list
+    assert_topk_parity(*got, *cpu_oracle.flat_search(METRICS[metric], q[:nq], x, k))
+    ix.close()

@@ -506,7 +506,7 @@ static int32_t flat_search_dev(Index* ix, const float* q, int64_t nq, int32_t k,
     const float* qb = q + b * ix->dim;
     const uint64_t* mb = qmasks ? qmasks + b : nullptr;
     const bool tensor_metric = ctx->search_path == VSK_PATH_TENSOR_RERANK && ix->metric != VSK_METRIC_MANHATTAN;
-    if (bn <= kStreamScanMaxQueries && (!tensor_metric || mb || ix->n * ix->dim <= kFewMaxElems)) {
+    if (bn <= kStreamScanMaxQueries) {
       FewArgs f{};
       f.metric = ix->metric;
       f.q = qb;
@@ -523,8 +523,10 @@ static int32_t flat_search_dev(Index* ix, const float* q, int64_t nq, int32_t k,
       f.out_dist = out_dist + b * k;
       f.out_ids = out_ids + b * k;
       if (few_search_applies(ctx, f)) {
-        VSK_TRY(few_search(ctx, f));
-        continue;
+        bool handled = false;
+        if (tensor_metric && !mb && ix->n * ix->dim > kFewMaxElems) VSK_TRY(few_search_half(ix, f, &handled));
+        else VSK_TRY(few_search(ctx, f));
+        if (handled || !tensor_metric || mb || ix->n * ix->dim <= kFewMaxElems) continue;
       }
     }
     float* qnorm = nullptr;

@@ -364,6 +364,9 @@ struct FewArgs {
 };
 bool few_search_applies(const Ctx* ctx, const FewArgs& a);
 int32_t few_search(Ctx* ctx, const FewArgs& a);
+// ... over the fp16 operand copy of a flat index, re-scored against the fp32 rows (drains the stream).  *handled = false:
+// the batch does not fit this form.
+int32_t few_search_half(Index* ix, const FewArgs& a, bool* handled);
 int32_t launch_row_norms(Ctx* ctx, const float* x, int64_t n, int32_t dim, int squared, float* out);
 
 // ---- group.cu ----------------------------------------------------------------------------

@@ -19,6 +19,7 @@
 #include "block_select.cuh"
 #include "common.cuh"
 #include "stream_rows.cuh"
+#include "tensor_scan.cuh"
 
 namespace vsk {
 namespace {
@@ -293,6 +294,287 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(F
   few_merge(ka, qb, (int)gridDim.x, lists, reinterpret_cast<unsigned short*>(smem + (size_t)NQ * FEW_LIST * 8), fs);
 }
 
+// ---- the same over the fp16 operand copy ----------------------------------------------------------------------------
+// A large store is bound by the bytes of its rows: one query over 1 million x 768 reads 3 GB of fp32 rows, or 1.5 GB of the
+// fp16 copy the tensor path keeps (that path padded the query to a tile of 128 and reached 3.4 TB/s: 490 us).  The queries
+// stay in fp32, so a coarse value is off by no more than |q| E_x and its own summation (eps).  Every CTA keeps its
+// k + kFewMargin best coarse keys; the last step lists every row within 2 eps of the k-th best, re-scores those with the
+// direct formulas and orders them.  A query for which that list or one CTA's share of it does not fit is flagged and run
+// over the fp32 rows.
+constexpr int kFewMargin = 64;
+constexpr int FEWH_ROWS = 4;   // rows per warp step: four 16-byte loads in flight per lane
+
+struct FewHalf {
+  const __half* x16;      // [n][dim16], s x (cosine: s x / |x|)
+  const float* aux;       // |x|^2 (euclidean)
+  int32_t dim16;
+  float inv_scale;        // 1 / s
+  float err, norm;        // largest |s x - x16| / s and |x16| / s of a row
+  float max_norm, min_norm_nz;
+  int32_t* flags;         // [nq], set to 0 or 1
+};
+
+// |coarse - exact| for every row, in coarse units (bound_kernel's terms with an unrounded query)
+template <int METRIC>
+__device__ __forceinline__ float few_eps(const FewHalf& h, int dim, float qn) {
+  const float q = METRIC == VSK_METRIC_COSINE ? 1.0f : qn;
+  float e = q * h.err + 1.2e-7f * (float)(dim + 16) * q * h.norm;
+  if (METRIC == VSK_METRIC_EUCLIDEAN) {
+    e = 2.0f * e + 2.4e-7f * (float)(dim + 16) * h.max_norm * h.max_norm +
+        1.2e-7f * (h.max_norm * h.max_norm + 2.0f * qn * h.max_norm) + 1.2e-7f * (float)(dim + 16) * qn * h.max_norm + 1.2e-7f * (float)(dim / 32 + 8) * qn * qn;
+  } else if (METRIC == VSK_METRIC_COSINE) {
+    const float den = qn * h.min_norm_nz;
+    e += den > 0.f ? 1e-8f / (den + 1e-8f) + 4.8e-7f : 4.8e-7f;
+  }
+  return e * 1.0001f + 1e-30f;
+}
+
+template <int METRIC, int NQ>
+__global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_coarse_kernel(FewKernelArgs ka, FewHalf h) {
+  const FewArgs& a = ka.a;
+  extern __shared__ __align__(16) uint8_t smem[];
+  uint64_t* lists = reinterpret_cast<uint64_t*>(smem);                       // [NQ][FEW_LIST]
+  float4* sq = reinterpret_cast<float4*>(smem + (size_t)NQ * FEW_LIST * 8);  // [NQ][2][dim16 / 8]: halves of 8 dimensions
+  __shared__ FewScratch fs;
+  __shared__ uint64_t s_thr[NQ];
+  __shared__ float s_qn[NQ];
+  __shared__ int s_cnt[NQ];
+  const int dim = a.dim, keep = a.k + kFewMargin, nv = h.dim16 >> 3;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nq = (int)a.nq;
+  if (threadIdx.x < NQ) {
+    s_thr[threadIdx.x] = kEmptyKey - 1;
+    s_cnt[threadIdx.x] = 0;
+  }
+  for (int i = warp; i < NQ; i += FEW_WARPS) {
+    float ss = 0.f;
+    for (int c = lane; c < dim; c += 32) {
+      const float v = i < nq ? __ldg(a.q + (int64_t)i * dim + c) : 0.f;
+      ss = fmaf(v, v, ss);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float qn = sqrtf(ss), f = METRIC == VSK_METRIC_COSINE ? (qn > 0.f ? 1.0f / qn : 0.f) : 1.0f;
+    if (lane == 0) s_qn[i] = qn;
+    for (int c = lane; c < h.dim16; c += 32) {
+      const float v = (i < nq && c < dim) ? __ldg(a.q + (int64_t)i * dim + c) * f : 0.f;
+      reinterpret_cast<float*>(sq)[((i * 2 + ((c >> 2) & 1)) * nv + (c >> 3)) * 4 + (c & 3)] = v;
+    }
+  }
+  __syncthreads();
+  constexpr int V = FEWH_ROWS * NQ;
+  constexpr int OWNER_SHIFT = 5 - Log2<V>::value;
+  const float alpha = (METRIC == VSK_METRIC_EUCLIDEAN ? -2.0f : -1.0f) * h.inv_scale;
+  const int64_t n = a.n, stride = (int64_t)gridDim.x * ka.round;
+  for (int64_t r0 = (int64_t)blockIdx.x * ka.round; r0 < n; r0 += stride) {
+    const int64_t r1 = min(n, r0 + ka.round);
+    for (int64_t n0 = r0 + warp * FEWH_ROWS; n0 < r1; n0 += FEW_WARPS * FEWH_ROWS) {
+      float acc[V];
+#pragma unroll
+      for (int j = 0; j < V; ++j) acc[j] = 0.f;
+      const uint4* p[FEWH_ROWS];
+#pragma unroll
+      for (int r = 0; r < FEWH_ROWS; ++r) p[r] = reinterpret_cast<const uint4*>(h.x16 + min(n0 + r, n - 1) * h.dim16);
+      for (int c = lane; c < nv; c += 32) {
+        uint4 x[FEWH_ROWS];
+#pragma unroll
+        for (int r = 0; r < FEWH_ROWS; ++r) x[r] = __ldg(p[r] + c);
+        float2 f[FEWH_ROWS][4];
+#pragma unroll
+        for (int r = 0; r < FEWH_ROWS; ++r) {
+          f[r][0] = __half22float2(*reinterpret_cast<const __half2*>(&x[r].x));
+          f[r][1] = __half22float2(*reinterpret_cast<const __half2*>(&x[r].y));
+          f[r][2] = __half22float2(*reinterpret_cast<const __half2*>(&x[r].z));
+          f[r][3] = __half22float2(*reinterpret_cast<const __half2*>(&x[r].w));
+        }
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) {
+          const float4 lo = sq[(i * 2) * nv + c], hi = sq[(i * 2 + 1) * nv + c];
+#pragma unroll
+          for (int r = 0; r < FEWH_ROWS; ++r) {
+            float& s = acc[r * NQ + i];
+            s = fmaf(lo.x, f[r][0].x, s); s = fmaf(lo.y, f[r][0].y, s); s = fmaf(lo.z, f[r][1].x, s); s = fmaf(lo.w, f[r][1].y, s);
+            s = fmaf(hi.x, f[r][2].x, s); s = fmaf(hi.y, f[r][2].y, s); s = fmaf(hi.z, f[r][3].x, s); s = fmaf(hi.w, f[r][3].y, s);
+          }
+        }
+      }
+      warp_reduce_scatter<V>(acc, lane);
+      if ((lane & ((1 << OWNER_SHIFT) - 1)) == 0) {
+        const int j = lane >> OWNER_SHIFT;
+        const int r = j / NQ, i = j - r * NQ;
+        if (n0 + r < r1 && i < nq) {
+          float v = acc[0] * alpha;
+          if (METRIC == VSK_METRIC_EUCLIDEAN) v += __ldg(h.aux + n0 + r);
+          const uint64_t key = make_key(v, (uint32_t)(n0 + r));
+          if (key <= s_thr[i]) lists[i * FEW_LIST + atomicAdd(&s_cnt[i], 1)] = key;
+        }
+      }
+    }
+    __syncthreads();
+    const bool last = r0 + stride >= n;
+#pragma unroll 1
+    for (int i = 0; i < nq; ++i) {
+      const int cnt = s_cnt[i];
+      if (cnt > (last ? keep : FEW_LIST - FEW_ROUND)) {
+        const uint64_t pivot = few_compact(lists + (size_t)i * FEW_LIST, cnt, keep, fs);
+        if (threadIdx.x == 0) {
+          s_cnt[i] = fs.out;
+          s_thr[i] = pivot;
+        }
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll 1
+  for (int i = 0; i < nq; ++i) {
+    const int64_t l = (int64_t)i * gridDim.x + blockIdx.x;
+    const uint64_t* list = lists + (size_t)i * FEW_LIST;
+    const int cnt = s_cnt[i];
+    for (int j = threadIdx.x; j < cnt; j += FEW_THREADS) ka.part[l * keep + j] = list[j];
+    if (warp == 0) {
+      uint64_t best = kEmptyKey;
+      for (int j = lane; j < cnt; j += 32) best = min(best, list[j]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
+      if (lane == 0) {
+        ka.part_min[l] = best;
+        ka.part_n[l] = cnt;
+      }
+    }
+  }
+}
+
+// One CTA per query: the rows within 2 eps of the k-th best coarse value, re-scored with the direct formulas and ordered.
+template <int METRIC>
+__global__ void __launch_bounds__(FEW_THREADS) few_refine_kernel(FewKernelArgs ka, FewHalf h, int lists) {
+  __shared__ uint64_t list[FEW_LIST];
+  __shared__ unsigned short cand[FEW_MAX_CTAS];
+  __shared__ FewScratch fs;
+  __shared__ int n_cand, n_list, n_have, s_bad;
+  __shared__ float s_qn;
+  const FewArgs& a = ka.a;
+  const int k = a.k, keep = k + kFewMargin, dim = a.dim;
+  const int64_t pos = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const float* q = a.q + pos * dim;
+  if (threadIdx.x == 0) { n_cand = 0; n_list = 0; n_have = 0; s_bad = 0; }
+  if (warp == 0) {
+    float ss = 0.f;
+    for (int c = lane; c < dim; c += 32) ss = fmaf(__ldg(q + c), __ldg(q + c), ss);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (lane == 0) s_qn = sqrtf(ss);
+  }
+  __syncthreads();
+  const float qn = s_qn, band = 2.0f * few_eps<METRIC>(h, dim, qn);
+  uint64_t key[SEL_ITEMS];
+  int have = 0;
+#pragma unroll
+  for (int i = 0; i < SEL_ITEMS; ++i) {
+    const int at = threadIdx.x + i * FEW_THREADS;
+    key[i] = at < lists ? __ldcg(ka.part_min + pos * lists + at) : kEmptyKey;
+    have += key[i] != kEmptyKey;
+  }
+  if (have) atomicAdd(&n_have, have);
+  __syncthreads();
+  // rows at or below `value` + band; what is not a number leaves every row in
+  auto widened = [&](uint64_t kth) {
+    const float b = ordered_to_float((uint32_t)(kth >> 32)) + band;
+    return b < CUDART_INF_F ? ((uint64_t)float_to_ordered(b) << 32) | 0xffffffffull : kEmptyKey - 1;
+  };
+  uint64_t bound = kEmptyKey - 1;
+  if (n_have >= k) bound = widened(block_radix_select(key, k, fs.hist, &fs.bin, &fs.less, &fs.in_bin));
+#pragma unroll
+  for (int i = 0; i < SEL_ITEMS; ++i)
+    if (key[i] <= bound && key[i] != kEmptyKey) cand[atomicAdd(&n_cand, 1)] = (unsigned short)(threadIdx.x + i * FEW_THREADS);
+  __syncthreads();
+  const int nc = n_cand;
+  for (int c = warp; c < nc; c += FEW_WARPS) {
+    const int64_t l = pos * lists + cand[c];
+    const int m = __ldcg(ka.part_n + l);
+    bool all = m >= keep;   // a shortened list whose every key is within the bound may have dropped such a row
+    for (int i = lane; i < m; i += 32) {
+      const uint64_t v = __ldcg(ka.part + l * keep + i);
+      if (v <= bound) {
+        const int at = atomicAdd(&n_list, 1);
+        if (at < FEW_LIST) list[at] = v;
+      } else {
+        all = false;
+      }
+    }
+    if (__all_sync(0xffffffffu, all) && lane == 0) s_bad = 1;
+  }
+  __syncthreads();
+  int cnt = n_list;
+  if (cnt > FEW_LIST || s_bad != 0 || !(band < CUDART_INF_F)) {
+    if (threadIdx.x == 0) h.flags[pos] = 1;
+    return;
+  }
+  if (cnt > k) {   // the k-th best of all, then only what is within the band of it
+#pragma unroll
+    for (int i = 0; i < SEL_ITEMS; ++i) {
+      const int at = threadIdx.x + i * FEW_THREADS;
+      key[i] = at < cnt ? list[at] : kEmptyKey;
+    }
+    if (threadIdx.x == 0) fs.out = 0;
+    __syncthreads();
+    bound = widened(block_radix_select(key, k, fs.hist, &fs.bin, &fs.less, &fs.in_bin));
+#pragma unroll
+    for (int i = 0; i < SEL_ITEMS; ++i)
+      if (key[i] <= bound && key[i] != kEmptyKey) list[atomicAdd(&fs.out, 1)] = key[i];
+    __syncthreads();
+    cnt = fs.out;
+  }
+  // exact values, summed as the tensor path's re-scoring sums them: four rows per warp step
+  constexpr int RR = 4;
+  for (int c0 = warp * RR; c0 < cnt; c0 += FEW_WARPS * RR) {
+    uint32_t id[RR];
+    float s[RR];
+#pragma unroll
+    for (int r = 0; r < RR; ++r) {
+      id[r] = (uint32_t)list[min(c0 + r, cnt - 1)];
+      s[r] = 0.f;
+    }
+    for (int i = lane; i < dim; i += 32) {
+      const float qv = __ldg(q + i);
+#pragma unroll
+      for (int r = 0; r < RR; ++r) {
+        const float xv = __ldg(a.x + (int64_t)id[r] * dim + i);
+        tile::accum<METRIC>(s[r], qv, xv);
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < RR; ++r) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
+      if (lane == 0 && c0 + r < cnt) {
+        float v = s[r];
+        if (METRIC == VSK_METRIC_COSINE) v = 1.0f - v / (qn * __ldg(a.xnorm + id[r]) + 1e-8f);
+        else if (METRIC == VSK_METRIC_DOT_PRODUCT) v = -v;
+        list[c0 + r] = make_key(v, id[r]);
+      }
+    }
+  }
+  __syncthreads();
+  const int P = next_pow2(cnt);
+  for (int i = cnt + threadIdx.x; i < P; i += FEW_THREADS) list[i] = kEmptyKey;
+  __syncthreads();
+  bitonic_sort(list, P);
+  for (int j = threadIdx.x; j < k; j += FEW_THREADS) {
+    float d = CUDART_INF_F;
+    int64_t id = -1;
+    if (j < cnt) {
+      d = ordered_to_float((uint32_t)(list[j] >> 32));
+      if (METRIC == VSK_METRIC_EUCLIDEAN) d = sqrtf(d);
+      id = (int64_t)(uint32_t)list[j] + a.id_base;
+    }
+    a.out_dist[pos * k + j] = d;
+    a.out_ids[pos * k + j] = id;
+  }
+  if (threadIdx.x == 0) h.flags[pos] = 0;
+}
+
 __global__ void __launch_bounds__(FEW_THREADS) few_merge_kernel(FewKernelArgs ka, int lists) {
   __shared__ uint64_t list[FEW_LIST];
   __shared__ unsigned short cand[FEW_MAX_CTAS];
@@ -354,6 +636,84 @@ int32_t few_metric(Ctx* ctx, const FewKernelArgs& ka, bool vec) {
 }
 
 }  // namespace
+
+namespace {
+
+template <int METRIC, int NQ>
+int32_t few_half_launch(Ctx* ctx, FewKernelArgs ka, const FewHalf& h) {
+  const FewArgs& a = ka.a;
+  auto kern = few_coarse_kernel<METRIC, NQ>;
+  const size_t smem = (size_t)NQ * (FEW_LIST * 8 + (size_t)h.dim16 * 4);
+  if (smem > 48 * 1024) VSK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int per_sm = std::max(1, std::min(NQ > 4 ? 2 : 3, (int)(220 * 1024 / (smem + 3072))));
+  constexpr int kStep = FEW_WARPS * FEWH_ROWS;
+  const int64_t grid = std::min<int64_t>(ceil_div(a.n, kStep), (int64_t)ctx->prop.multiProcessorCount * per_sm);
+  const int64_t share = ceil_div(a.n, grid);
+  ka.round = (int32_t)std::min<int64_t>(FEW_ROUND, ceil_div(ceil_div(share, ceil_div(share, (int64_t)FEW_ROUND)), kStep) * kStep);
+  void* p;
+  const size_t lists = (size_t)a.nq * grid, keep = (size_t)a.k + kFewMargin;
+  VSK_TRY(scratch(ctx, SLOT_FEW, lists * (keep * 8 + 8 + 4), &p));
+  ka.part = (uint64_t*)p;
+  ka.part_min = ka.part + lists * keep;
+  ka.part_n = (int32_t*)(ka.part_min + lists);
+  prof_begin(ctx);
+  kern<<<(unsigned)grid, FEW_THREADS, smem, ctx->stream>>>(ka, h);
+  prof_end(ctx);
+  few_refine_kernel<METRIC><<<(unsigned)a.nq, FEW_THREADS, 0, ctx->stream>>>(ka, h, (int)grid);
+  ctx->stats.kernel_launches += 2;
+  VSK_CUDA(ctx, cudaGetLastError());
+  return VSK_OK;
+}
+
+template <int METRIC>
+int32_t few_half_metric(Ctx* ctx, const FewKernelArgs& ka, const FewHalf& h) {
+  if (ka.a.nq <= 1) return few_half_launch<METRIC, 1>(ctx, ka, h);
+  if (ka.a.nq <= 2) return few_half_launch<METRIC, 2>(ctx, ka, h);
+  if (ka.a.nq <= 4) return few_half_launch<METRIC, 4>(ctx, ka, h);
+  return few_half_launch<METRIC, 8>(ctx, ka, h);
+}
+
+}  // namespace
+
+int32_t few_search_half(Index* ix, const FewArgs& a, bool* handled) {
+  VSK_TRACE("vsk:few_search_half");
+  Ctx* ctx = ix->ctx;
+  *handled = false;
+  const size_t staged = a.nq <= 1 ? 1 : a.nq <= 2 ? 2 : a.nq <= 4 ? 4 : 8;
+  if (ctx->search_path != VSK_PATH_TENSOR_RERANK || !ctx->tuning.stream_scan || a.k < 1 || a.k > kFewMaxK || a.nq < 1 ||
+      a.nq > kStreamScanMaxQueries || a.row_masks || staged * (FEW_LIST * 8 + (size_t)(a.dim + 80) * 4) > kFewMaxSmem)
+    return VSK_OK;
+  VSK_TRY(tensor_prepare_index(ix));
+  FewHalf h{};
+  h.x16 = ix->rows16;
+  h.aux = ix->row_aux;
+  h.dim16 = ix->dim16;
+  h.inv_scale = 1.0f / ix->scale16;
+  h.err = ix->max_xerr16 * h.inv_scale;
+  h.norm = ix->max_xnorm16 * h.inv_scale;
+  h.max_norm = ix->max_xnorm;
+  h.min_norm_nz = ix->min_xnorm_nz;
+  void* p;
+  VSK_TRY(scratch(ctx, SLOT_CAND_FLAGS, (size_t)a.nq * sizeof(int32_t), &p));
+  h.flags = (int32_t*)p;
+  PinnedBuf& hb = ctx->host_flags[ctx->lane];
+  VSK_TRY(pinned_reserve(ctx, &hb, (size_t)a.nq * 4));
+  FewKernelArgs ka{};
+  ka.a = a;
+  switch (a.metric) {
+    case VSK_METRIC_EUCLIDEAN: VSK_TRY(few_half_metric<VSK_METRIC_EUCLIDEAN>(ctx, ka, h)); break;
+    case VSK_METRIC_COSINE: VSK_TRY(few_half_metric<VSK_METRIC_COSINE>(ctx, ka, h)); break;
+    default: VSK_TRY(few_half_metric<VSK_METRIC_DOT_PRODUCT>(ctx, ka, h)); break;
+  }
+  VSK_CUDA(ctx, cudaMemcpyAsync(hb.p, h.flags, (size_t)a.nq * 4, cudaMemcpyDeviceToHost, ctx->stream));
+  VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  int64_t bad = 0;
+  for (int64_t i = 0; i < a.nq; ++i) bad += ((const int32_t*)hb.p)[i] != 0;
+  *handled = true;
+  if (bad == 0) return VSK_OK;
+  ctx->stats.fallback_queries += bad;
+  return few_search(ctx, a);   // the fp32 rows: all of these few queries again
+}
 
 bool few_search_applies(const Ctx* ctx, const FewArgs& a) {
   // (the fp32 search path is the chunked schedule by definition)
