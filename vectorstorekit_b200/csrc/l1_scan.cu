@@ -78,15 +78,21 @@ __global__ void __launch_bounds__(L1_THREADS, 2) l1_scan_kernel(L1Args a) {
   }
   __syncthreads();
   const int nsteps = a.stride >> 4, nchunks = (nsteps + 3) >> 2;
+  // a thread copies the same 16-byte piece of every 64th row
+  const int frow = threadIdx.x >> 2, part = threadIdx.x & 3;
+  const uint8_t* fq[(BM + 63) / 64];
+#pragma unroll
+  for (int i = 0; i < (BM + 63) / 64; ++i) fq[i] = a.q8 + min(m0 + frow + 64 * i, a.nq - 1) * a.stride + part * 16;
+  const uint8_t* fx = a.x8 + part * 16;
   auto fetch = [&](int c) {
-    uint8_t* st = sm + (c % L1_STAGES) * T::STAGE;
-    const int parts = min(4, nsteps - 4 * c);   // 16-byte pieces of a row in this chunk
-    for (int p = threadIdx.x; p < (BM + T::BN) * 4; p += L1_THREADS) {
-      const int r = p >> 2, part = p & 3;
-      if (part < parts) {
-        const uint8_t* src = r < BM ? a.q8 + min(m0 + r, a.nq - 1) * a.stride : a.x8 + (int64_t)s_row[r - BM] * a.stride;
-        cp16(st + r * L1_PITCH + part * 16, src + c * L1_CHUNK + part * 16);
-      }
+    uint8_t* st = sm + (c % L1_STAGES) * T::STAGE + frow * L1_PITCH + part * 16;
+    if (part < nsteps - 4 * c) {   // (the last chunk may hold fewer than four pieces)
+#pragma unroll
+      for (int i = 0; i < (BM + 63) / 64; ++i)
+        if (BM >= 64 || frow < BM) cp16(st + i * 64 * L1_PITCH, fq[i] + c * L1_CHUNK);
+#pragma unroll
+      for (int i = 0; i < T::BN / 64; ++i)
+        cp16(st + (BM + i * 64) * L1_PITCH, fx + (int64_t)s_row[frow + i * 64] * a.stride + c * L1_CHUNK);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
