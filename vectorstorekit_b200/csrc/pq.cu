@@ -120,15 +120,26 @@ __global__ void __launch_bounds__(256) pq_encode_fast_kernel(const float* __rest
   const float cmax = sqrtf(top) * 1.00001f;
   constexpr int R = 2;
   const int64_t r0 = (int64_t)blockIdx.x * (blockDim.x * R) + threadIdx.x;
-  float v[R][DS], best[R], second[R];
+  const bool wide = (dim & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  __align__(16) float v[R][DS];
+  float best[R], second[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int64_t row = min(r0 + (int64_t)r * blockDim.x, n - 1);
+    const float* seg = x + row * dim + (int64_t)s * DS;
+    if (wide) {   // (lanes read rows dim floats apart: a 16-byte load costs what a 4-byte one does)
 #pragma unroll
-    for (int i = 0; i < DS; ++i) v[r][i] = -2.0f * __ldg(x + row * dim + (int64_t)s * DS + i);
+      for (int i = 0; i < DS; i += 4) *reinterpret_cast<float4*>(&v[r][i]) = __ldg(reinterpret_cast<const float4*>(seg + i));
+    } else {
+#pragma unroll
+      for (int i = 0; i < DS; ++i) v[r][i] = __ldg(seg + i);
+    }
+#pragma unroll
+    for (int i = 0; i < DS; ++i) v[r][i] *= -2.0f;
     best[r] = CUDART_INF_F;
     second[r] = CUDART_INF_F;
   }
+#pragma unroll 4
   for (int c = 0; c < ksub; ++c) {
     float w[DS];
 #pragma unroll
