@@ -82,6 +82,54 @@ int32_t pinned_reserve(Ctx* ctx, PinnedBuf* b, size_t bytes) {
   return VSK_OK;
 }
 
+constexpr size_t kStagedIn = 64 << 10, kStagedOut = 12 << 10;   // bytes a staged call may bring and take (1 024 results)
+
+int32_t host_call_begin(Ctx* ctx, const float* q, int64_t nq, int32_t dim, const uint64_t* qmasks, int32_t k, HostCall* c) {
+  void* p;
+  const size_t qb = (size_t)nq * dim * 4, mb = qmasks ? (size_t)nq * 8 : 0, ob = (size_t)nq * k * 12;
+  VSK_TRY(scratch(ctx, SLOT_Q, qb, &p));
+  c->q = (float*)p;
+  if (qmasks) {
+    VSK_TRY(scratch(ctx, SLOT_QMASK, mb, &p));
+    c->masks = (uint64_t*)p;
+  }
+  const float* src = q;
+  const uint64_t* msrc = qmasks;
+  c->staged = qb + mb <= kStagedIn && ob <= kStagedOut;
+  if (c->staged) {
+    VSK_TRY(pinned_reserve(ctx, &ctx->host_io, kStagedIn + kStagedOut));
+    char* h = (char*)ctx->host_io.p;   // results first (8-byte aligned ids, then distances), then masks and queries
+    c->ids = (int64_t*)h;
+    c->dist = (float*)(h + (size_t)nq * k * 8);
+    if (qmasks) memcpy(h + kStagedOut, qmasks, mb);
+    memcpy(h + kStagedOut + mb, q, qb);
+    msrc = (const uint64_t*)(h + kStagedOut);
+    src = (const float*)(h + kStagedOut + mb);
+  } else {
+    VSK_TRY(scratch(ctx, SLOT_OUT_D, (size_t)nq * k * 4, &p));
+    c->dist = (float*)p;
+    VSK_TRY(scratch(ctx, SLOT_OUT_I, (size_t)nq * k * 8, &p));
+    c->ids = (int64_t*)p;
+  }
+  VSK_CUDA(ctx, cudaMemcpyAsync(c->q, src, qb, cudaMemcpyHostToDevice, ctx->stream));
+  if (qmasks) VSK_CUDA(ctx, cudaMemcpyAsync(c->masks, msrc, mb, cudaMemcpyHostToDevice, ctx->stream));
+  return VSK_OK;
+}
+
+int32_t host_call_end(Ctx* ctx, const HostCall& c, int64_t nq, int32_t dim, int32_t k, float* out_dist, int64_t* out_ids) {
+  if (c.staged) {
+    memcpy(out_dist, c.dist, (size_t)nq * k * 4);
+    memcpy(out_ids, c.ids, (size_t)nq * k * 8);
+  } else {
+    VSK_CUDA(ctx, cudaMemcpyAsync(out_dist, c.dist, (size_t)nq * k * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    VSK_CUDA(ctx, cudaMemcpyAsync(out_ids, c.ids, (size_t)nq * k * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  }
+  ctx->stats.h2d_bytes += nq * dim * 4 + (c.masks ? nq * 8 : 0);
+  ctx->stats.d2h_bytes += nq * k * 12;
+  return VSK_OK;
+}
+
 int32_t scratch(Ctx* ctx, int slot, size_t bytes, void** out) {
   slot += ctx->lane * 64;   // each lane has its own set of buffers
   if (ctx->scratch_bytes[slot] < bytes) {
@@ -723,6 +771,7 @@ int32_t vsk_close(vsk_ctx* c) {
   for (auto& p : ctx->few_tickets) dev_free(p);
   for (auto& b : ctx->host_flags)
     if (b.p) cudaFreeHost(b.p);
+  if (ctx->host_io.p) cudaFreeHost(ctx->host_io.p);
   for (auto& e : ctx->prof_events) cudaEventDestroy(e);
   for (auto& m : ctx->marks) cudaEventDestroy(m.ev);
   if (ctx->tl_origin) cudaEventDestroy(ctx->tl_origin);
@@ -1106,21 +1155,10 @@ int32_t vsk_search(vsk_index* i, const float* q, int64_t nq, int32_t k, const ui
   if (nq <= 0) return fail(ctx, VSK_ERR_EMPTY_INPUT, "no queries");
   if (k <= 0) return fail(ctx, VSK_ERR_INVALID_INPUT, "k must be positive");
   if (!q || !out_dist || !out_ids) return fail(ctx, VSK_ERR_INVALID_INPUT, "null pointer");
-  void *dq, *dd, *di, *dm = nullptr;
-  VSK_TRY(scratch(ctx, SLOT_Q, (size_t)nq * ix->dim * 4, &dq));
-  VSK_TRY(scratch(ctx, SLOT_OUT_D, (size_t)nq * k * 4, &dd));
-  VSK_TRY(scratch(ctx, SLOT_OUT_I, (size_t)nq * k * 8, &di));
-  VSK_CUDA(ctx, cudaMemcpyAsync(dq, q, (size_t)nq * ix->dim * 4, cudaMemcpyHostToDevice, ctx->stream));
-  if (qmasks) {
-    VSK_TRY(scratch(ctx, SLOT_QMASK, (size_t)nq * 8, &dm));
-    VSK_CUDA(ctx, cudaMemcpyAsync(dm, qmasks, (size_t)nq * 8, cudaMemcpyHostToDevice, ctx->stream));
-  }
-  VSK_TRY(vsk_search_dev(i, (const float*)dq, nq, k, (const uint64_t*)dm, (float*)dd, (int64_t*)di));
-  VSK_CUDA(ctx, cudaMemcpyAsync(out_dist, dd, (size_t)nq * k * 4, cudaMemcpyDeviceToHost, ctx->stream));
-  VSK_CUDA(ctx, cudaMemcpyAsync(out_ids, di, (size_t)nq * k * 8, cudaMemcpyDeviceToHost, ctx->stream));
-  VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  ctx->stats.h2d_bytes += nq * ix->dim * 4 + (qmasks ? nq * 8 : 0);
-  ctx->stats.d2h_bytes += nq * k * 12;
+  HostCall c;
+  VSK_TRY(host_call_begin(ctx, q, nq, ix->dim, qmasks, k, &c));
+  VSK_TRY(vsk_search_dev(i, c.q, nq, k, c.masks, c.dist, c.ids));
+  VSK_TRY(host_call_end(ctx, c, nq, ix->dim, k, out_dist, out_ids));
   return VSK_OK;
 }
 

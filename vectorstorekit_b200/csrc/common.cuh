@@ -156,6 +156,7 @@ struct Ctx {
   void* scratch[2 * 64] = {};
   size_t scratch_bytes[2 * 64] = {};
   ShardPending pending[2];
+  PinnedBuf host_io;         // staging of small host-pointer calls (HostCall)
   PinnedBuf host_flags[2];   // per lane: the flag words a finished half-search hands to the host
   unsigned* few_tickets[2] = {};   // per lane: the few-query search's tickets (few_search.cu)
   Comm* comm = nullptr;
@@ -207,6 +208,21 @@ struct LaneGuard {
 int32_t lanes_fork(Ctx* ctx);
 int32_t lanes_join(Ctx* ctx);
 int32_t pinned_reserve(Ctx* ctx, PinnedBuf* b, size_t bytes);
+
+// Buffers of a host-pointer search: device copies of the queries and masks, and where the results go.  A small call is
+// staged in pinned memory: the queries leave for the device without the driver's own staging, the last kernel writes its
+// few results straight into the pinned buffer (which the device can address), and the one wait at the end of the search is
+// the only one - two copies back, each waited for, cost more than a search over a small store.
+struct HostCall {
+  float* q = nullptr;
+  uint64_t* masks = nullptr;
+  float* dist = nullptr;      // device addresses for the search's results
+  int64_t* ids = nullptr;
+  bool staged = false;
+};
+int32_t host_call_begin(Ctx* ctx, const float* q, int64_t nq, int32_t dim, const uint64_t* qmasks, int32_t k, HostCall* c);
+// after the search has drained its stream
+int32_t host_call_end(Ctx* ctx, const HostCall& c, int64_t nq, int32_t dim, int32_t k, float* out_dist, int64_t* out_ids);
 
 enum Slot : int {
   SLOT_Q = 0, SLOT_OUT_D, SLOT_OUT_I, SLOT_QMASK, SLOT_CAND_KEYS, SLOT_CAND_COUNT, SLOT_CAND_THR,

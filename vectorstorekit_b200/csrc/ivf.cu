@@ -915,22 +915,10 @@ int32_t vsk_ivf_search_filtered(vsk_index* i, const float* q, int64_t nq, int32_
   if (nq <= 0) return fail(ctx, VSK_ERR_EMPTY_INPUT, "no queries");
   if (k <= 0) return fail(ctx, VSK_ERR_INVALID_INPUT, "k must be positive");
   if (!q || !out_dist || !out_ids) return fail(ctx, VSK_ERR_INVALID_INPUT, "null pointer");
-  void *dq, *dd, *di, *dm = nullptr;
-  VSK_TRY(scratch(ctx, SLOT_Q, (size_t)nq * ix->dim * 4, &dq));
-  VSK_TRY(scratch(ctx, SLOT_OUT_D, (size_t)nq * k * 4, &dd));
-  VSK_TRY(scratch(ctx, SLOT_OUT_I, (size_t)nq * k * 8, &di));
-  VSK_CUDA(ctx, cudaMemcpyAsync(dq, q, (size_t)nq * ix->dim * 4, cudaMemcpyHostToDevice, ctx->stream));
-  if (qmasks) {
-    VSK_TRY(scratch(ctx, SLOT_QMASK, (size_t)nq * 8, &dm));
-    VSK_CUDA(ctx, cudaMemcpyAsync(dm, qmasks, (size_t)nq * 8, cudaMemcpyHostToDevice, ctx->stream));
-    ctx->stats.h2d_bytes += nq * 8;
-  }
-  VSK_TRY(ivf_search_dev(ix, (const float*)dq, nq, k, nprobe, (const uint64_t*)dm, (float*)dd, (int64_t*)di));
-  VSK_CUDA(ctx, cudaMemcpyAsync(out_dist, dd, (size_t)nq * k * 4, cudaMemcpyDeviceToHost, ctx->stream));
-  VSK_CUDA(ctx, cudaMemcpyAsync(out_ids, di, (size_t)nq * k * 8, cudaMemcpyDeviceToHost, ctx->stream));
-  VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  ctx->stats.h2d_bytes += nq * ix->dim * 4;
-  ctx->stats.d2h_bytes += nq * k * 12;
+  HostCall c;
+  VSK_TRY(host_call_begin(ctx, q, nq, ix->dim, qmasks, k, &c));
+  VSK_TRY(ivf_search_dev(ix, c.q, nq, k, nprobe, c.masks, c.dist, c.ids));
+  VSK_TRY(host_call_end(ctx, c, nq, ix->dim, k, out_dist, out_ids));
   return VSK_OK;
 }
 
