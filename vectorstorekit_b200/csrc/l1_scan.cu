@@ -158,8 +158,9 @@ __global__ void __launch_bounds__(L1_THREADS, 2) l1_scan_kernel(L1Args a) {
 }
 
 // Exact values (sum |q - x| in fp32, in dimension order: the fp32 tile's value bit for bit) for the rows listed since the
-// last compaction - the keys of value zero, as the scan leaves them; a kept row at distance zero is formed again.  One CTA
-// per query, a thread per row with four 16-byte loads in flight (VEC) or sixteen scalar ones.
+// last compaction - the keys of value zero, as the scan leaves them; a kept row at distance zero is formed again.  A thread
+// per row with four 16-byte loads in flight (VEC) or sixteen scalar ones; a small group of queries takes several CTAs per
+// query (blockIdx.y), as the gathers are bound by their latency (156 queries: 64 us a launch with one).
 constexpr int L1_RS_THREADS = 128;
 template <bool VEC>
 __global__ void __launch_bounds__(L1_RS_THREADS) l1_rescore_kernel(const float* __restrict__ q, const float* __restrict__ x, int dim,
@@ -170,9 +171,9 @@ __global__ void __launch_bounds__(L1_RS_THREADS) l1_rescore_kernel(const float* 
   const int cnt = min(cand.count[pos], kCandCap);
   uint64_t* keys = cand.keys + pos * kCandCap;
   for (int i = threadIdx.x; i < dim; i += L1_RS_THREADS) qs[i] = __ldg(q + qi * dim + i);
-  if (threadIdx.x == 0) atomicAdd(total, (unsigned long long)cnt);
+  if (threadIdx.x == 0 && blockIdx.y == 0) atomicAdd(total, (unsigned long long)cnt);
   __syncthreads();
-  for (int c = threadIdx.x; c < cnt; c += L1_RS_THREADS) {
+  for (int c = blockIdx.y * L1_RS_THREADS + threadIdx.x; c < cnt; c += gridDim.y * L1_RS_THREADS) {
     const uint64_t key = keys[c];
     if ((uint32_t)(key >> 32) != 0x80000000u) continue;
     const float* p = x + (int64_t)(uint32_t)key * dim;
@@ -416,8 +417,9 @@ int32_t l1_topk(Index* ix, const ExactScanArgs& proto, int64_t n, int64_t nq, co
     if (bm == 128) VSK_TRY(l1_launch<128>(ctx, a));
     else if (bm == 64) VSK_TRY(l1_launch<64>(ctx, a));
     else VSK_TRY(l1_launch<32>(ctx, a));
-    if (vec) l1_rescore_kernel<true><<<(unsigned)nq, L1_RS_THREADS, qsm, ctx->stream>>>(proto.q, ix->rows, dim, sub_dev, cand, total);
-    else l1_rescore_kernel<false><<<(unsigned)nq, L1_RS_THREADS, qsm, ctx->stream>>>(proto.q, ix->rows, dim, sub_dev, cand, total);
+    const dim3 rgrid((unsigned)nq, (unsigned)std::max<int64_t>(1, std::min<int64_t>(8, 8 * ctx->prop.multiProcessorCount / nq)));
+    if (vec) l1_rescore_kernel<true><<<rgrid, L1_RS_THREADS, qsm, ctx->stream>>>(proto.q, ix->rows, dim, sub_dev, cand, total);
+    else l1_rescore_kernel<false><<<rgrid, L1_RS_THREADS, qsm, ctx->stream>>>(proto.q, ix->rows, dim, sub_dev, cand, total);
     ctx->stats.kernel_launches++;
     VSK_CUDA(ctx, cudaGetLastError());
     tl_mark(ctx, "l1_rescore");
