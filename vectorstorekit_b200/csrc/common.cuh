@@ -376,6 +376,7 @@ struct FewArgs {
   const int64_t* probes;      // [nq][nprobe], or null
   int32_t nprobe, nlist;
   const int64_t* list_offsets;
+  const int32_t* q_subset;    // or null: queries to run, by number (with probes only); inputs and outputs are the batch's
   int64_t nan_rows;           // set by few_search
 };
 bool few_search_applies(const Ctx* ctx, const FewArgs& a);

@@ -64,8 +64,8 @@ __device__ __forceinline__ uint64_t few_compact(uint64_t* list, int cnt, int k, 
   return pivot;
 }
 
-// Merges the lists of one query and writes its result.  `list` has room for FEW_LIST keys, `cand` for FEW_MAX_CTAS list numbers.
-__device__ __forceinline__ void few_merge(const FewKernelArgs& ka, int64_t pos, int lists, uint64_t* list, unsigned short* cand,
+// Merges the lists of the launch's query `pos` and writes the result of query `out`.  `list` has room for FEW_LIST keys, `cand` for FEW_MAX_CTAS list numbers.
+__device__ __forceinline__ void few_merge(const FewKernelArgs& ka, int64_t pos, int64_t out, int lists, uint64_t* list, unsigned short* cand,
                                           FewScratch& s) {
   __shared__ int n_cand, n_list, n_have;
   const FewArgs& a = ka.a;
@@ -124,8 +124,8 @@ __device__ __forceinline__ void few_merge(const FewKernelArgs& ka, int64_t pos, 
       if (a.final_sqrt) d = sqrtf(d);
       id = (int64_t)(uint32_t)list[j] + a.id_base;
     }
-    a.out_dist[pos * k + j] = d;
-    a.out_ids[pos * k + j] = id;
+    a.out_dist[out * k + j] = d;
+    a.out_ids[out * k + j] = id;
   }
 }
 
@@ -146,7 +146,8 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(F
   __shared__ unsigned s_last;
   const int dim = a.dim, k = a.k;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qb = SEG ? (int)blockIdx.y : 0;
+  const int qp = SEG ? (int)blockIdx.y : 0;                         // position in this launch
+  const int qb = (SEG && a.q_subset) ? a.q_subset[qp] : qp;         // first query of this CTA
   const int nq_here = SEG ? 1 : (int)a.nq;
   for (int i = threadIdx.x; i < NQ * dim; i += FEW_THREADS) sq[i] = i < nq_here * dim ? a.q[(int64_t)qb * dim + i] : 0.f;
   if (threadIdx.x < NQ) {
@@ -202,6 +203,7 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(F
   constexpr int V = FEW_ROWS * NQ;
   constexpr int OWNER_SHIFT = 5 - Log2<V>::value;
   const int64_t stride = (int64_t)gridDim.x * ka.round;
+  int cur = 0;   // SEG: the list of the current position
   for (int64_t r0 = (int64_t)blockIdx.x * ka.round; r0 < n; r0 += stride) {
     const int64_t r1 = min(n, r0 + ka.round);
     for (int64_t n0 = r0 + warp * FEW_ROWS; n0 < r1; n0 += FEW_WARPS * FEW_ROWS) {
@@ -213,13 +215,9 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(F
         const int64_t at = n0 + r;
         const bool has = at < r1;
         rid[r] = has ? (uint32_t)at : 0u;
-        if (SEG && has) {
-          int lo = 0, hi = a.nprobe;   // the last list that starts at or before this position (empty lists are passed over)
-          while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (seg_pos[mid] <= at) lo = mid; else hi = mid;
-          }
-          rid[r] = (uint32_t)(seg_row[lo] + (at - seg_pos[lo]));
+        if (SEG && has) {   // positions only grow: the warp's current list serves until the next one starts
+          while (cur + 1 < a.nprobe && seg_pos[cur + 1] <= at) ++cur;
+          rid[r] = (uint32_t)(seg_row[cur] + (at - seg_pos[cur]));
         }
         rmask[r] = (a.row_masks && has) ? __ldg(a.row_masks + rid[r]) : ~0ull;
         live[r] = has && (rmask[r] & any_mask) != 0;   // a row no query may see is not read
@@ -242,10 +240,13 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(F
           float v = acc[0];
           if (METRIC == VSK_METRIC_COSINE) v = 1.0f - v / (s_qn[i] * __ldg(a.xnorm + ridr) + 1e-8f);
           else if (METRIC == VSK_METRIC_DOT_PRODUCT) v = -v;
-          const uint32_t id = a.id_remap ? (uint32_t)__ldg(a.id_remap + ridr) : ridr;
-          const uint64_t key = make_key(v, id);
-          // a value that is not a number is listed among the first rows only, as the chunked schedule does
-          if (key <= s_thr[i] && (!isnan(v) || n0 + r < a.nan_rows)) lists[i * FEW_LIST + atomicAdd(&s_cnt[i], 1)] = key;
+          // (the id is looked up only for a value that can be listed: the load would be on every step's path)
+          if (float_to_ordered(v) <= (uint32_t)(s_thr[i] >> 32)) {
+            const uint32_t id = a.id_remap ? (uint32_t)__ldg(a.id_remap + ridr) : ridr;
+            const uint64_t key = make_key(v, id);
+            // a value that is not a number is listed among the first rows only, as the chunked schedule does
+            if (key <= s_thr[i] && (!isnan(v) || n0 + r < a.nan_rows)) lists[i * FEW_LIST + atomicAdd(&s_cnt[i], 1)] = key;
+          }
         }
       }
     }
@@ -267,7 +268,7 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(F
   // ---- this CTA's lists, and the merge by the last one to arrive ----
 #pragma unroll 1
   for (int i = 0; i < nq_here; ++i) {
-    const int64_t l = (int64_t)(qb + i) * gridDim.x + blockIdx.x;
+    const int64_t l = (int64_t)(qp + i) * gridDim.x + blockIdx.x;
     const uint64_t* list = lists + (size_t)i * FEW_LIST;
     const int cnt = s_cnt[i];
     for (int j = threadIdx.x; j < cnt; j += FEW_THREADS) ka.part[l * k + j] = list[j];
@@ -285,13 +286,13 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(F
   if (NQ > 1) return;   // several queries: few_merge_kernel merges them side by side
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(ka.ticket + qb, 1u);
+  if (threadIdx.x == 0) s_last = atomicAdd(ka.ticket + qp, 1u);
   __syncthreads();
   if (s_last != gridDim.x - 1) return;
   __threadfence();
-  if (threadIdx.x == 0) ka.ticket[qb] = 0u;
+  if (threadIdx.x == 0) ka.ticket[qp] = 0u;
   // the query's staging area is free now: list numbers go there (the launch makes it large enough)
-  few_merge(ka, qb, (int)gridDim.x, lists, reinterpret_cast<unsigned short*>(smem + (size_t)NQ * FEW_LIST * 8), fs);
+  few_merge(ka, qp, qb, (int)gridDim.x, lists, reinterpret_cast<unsigned short*>(smem + (size_t)NQ * FEW_LIST * 8), fs);
 }
 
 // ---- the same over the fp16 operand copy ----------------------------------------------------------------------------
@@ -579,7 +580,7 @@ __global__ void __launch_bounds__(FEW_THREADS) few_merge_kernel(FewKernelArgs ka
   __shared__ uint64_t list[FEW_LIST];
   __shared__ unsigned short cand[FEW_MAX_CTAS];
   __shared__ FewScratch fs;
-  few_merge(ka, blockIdx.x, lists, list, cand, fs);
+  few_merge(ka, blockIdx.x, blockIdx.x, lists, list, cand, fs);
 }
 
 template <int NQ>
@@ -589,7 +590,10 @@ size_t few_smem(const FewArgs& a) {
   b = std::max<size_t>(b, FEW_MAX_CTAS * sizeof(unsigned short));   // the merge's list numbers go here
   return (size_t)NQ * FEW_LIST * 8 + b;
 }
-constexpr int kFewShortRow = 32;   // three or more queries over rows this short: the chunked schedule
+// Three or more queries over rows this short keep to the chunked schedule, whose overflow count (vsk_stats.fallback_queries)
+// is part of what callers see there.  It is not the faster one: three queries over 40 000 x 32 take it 104 us, over 40 000 x
+// 36 one launch takes 46.
+constexpr int kFewShortRow = 32;
 constexpr size_t kFewMaxSmem = 110 * 1024;   // two CTAs per SM
 
 template <int METRIC, int NQ, bool VEC, bool SEG>

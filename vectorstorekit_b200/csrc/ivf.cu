@@ -715,29 +715,13 @@ int32_t ivf_search_dev(Index* ix, const float* q, int64_t nq, int32_t k, int32_t
       c.dim = ix->dim;
       VSK_TRY(fp32_topk(ctx, c, ix->nlist, bn, nullptr, nprobe, 0, (float*)pd, (int64_t*)pi, 0));
     }
-    if (tensor) {
-      // coarse scan of the probed lists on the tensor cores + exact rerank; what it cannot certify is re-run below
-      std::vector<int32_t> redo;
-      VSK_TRY(ivf_tensor_search(ix, qb, bn, (const int64_t*)pi, nprobe, k, mb, out_dist + b * k, out_ids + b * k, &redo));
-      if (!redo.empty()) {
-        void* p;
-        VSK_TRY(scratch(ctx, SLOT_MISC4, redo.size() * 4, &p));
-        VSK_CUDA(ctx, cudaMemcpyAsync(p, redo.data(), redo.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-        VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        ctx->stats.fallback_queries += (int64_t)redo.size();
-        VSK_TRY(ivf_search_positions(ctx, ix, qb, (int64_t)redo.size(), (const int32_t*)p, (const int64_t*)pi, nprobe, k, mb,
-                                     out_dist + b * k, out_ids + b * k, false));
-      }
-      continue;
-    }
-    if (bn <= kStreamScanMaxSegQueries) {
-      // the probed lists, walked on the device query by query; longer probe lists or results: the chunked schedule
+    auto few_lists = [&](int64_t queries) {
       FewArgs f{};
       f.metric = VSK_METRIC_EUCLIDEAN;
       f.q = qb;
       f.x = ix->rows;
       f.dim = ix->dim;
-      f.nq = bn;
+      f.nq = queries;
       f.n = ceil_div(ix->n * nprobe, ix->nlist);
       f.k = k;
       f.row_masks = (mb && ix->has_masks) ? ix->masks : nullptr;
@@ -751,6 +735,39 @@ int32_t ivf_search_dev(Index* ix, const float* q, int64_t nq, int32_t k, int32_t
       f.nprobe = nprobe;
       f.nlist = ix->nlist;
       f.list_offsets = ix->list_offsets;
+      return f;
+    };
+    if (tensor) {
+      // coarse scan of the probed lists on the tensor cores + exact rerank; what it cannot certify is re-run below
+      std::vector<int32_t> redo;
+      VSK_TRY(ivf_tensor_search(ix, qb, bn, (const int64_t*)pi, nprobe, k, mb, out_dist + b * k, out_ids + b * k, &redo));
+      if (!redo.empty()) {
+        void* p;
+        VSK_TRY(scratch(ctx, SLOT_MISC4, redo.size() * 4, &p));
+        VSK_CUDA(ctx, cudaMemcpyAsync(p, redo.data(), redo.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+        VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        ctx->stats.fallback_queries += (int64_t)redo.size();
+        // A few of them: their lists walked query by query.  Two re-runs of a batch over 10 million rows took the list tiles
+        // and their chunk schedule 24 ms; for hundreds the tiles, which read a list once for all its queries, are faster (270
+        // re-runs over lists of 100 000 rows x 89: 12 ms against 27).
+        const FewArgs f = few_lists(kStreamScanMaxSegQueries);
+        if (redo.size() <= 64 && few_search_applies(ctx, f)) {
+          for (size_t i = 0; i < redo.size(); i += kStreamScanMaxSegQueries) {
+            FewArgs g = f;
+            g.nq = (int64_t)std::min<size_t>(kStreamScanMaxSegQueries, redo.size() - i);
+            g.q_subset = (const int32_t*)p + i;
+            VSK_TRY(few_search(ctx, g));
+          }
+          continue;
+        }
+        VSK_TRY(ivf_search_positions(ctx, ix, qb, (int64_t)redo.size(), (const int32_t*)p, (const int64_t*)pi, nprobe, k, mb,
+                                     out_dist + b * k, out_ids + b * k, false));
+      }
+      continue;
+    }
+    if (bn <= kStreamScanMaxSegQueries) {
+      // the probed lists, walked on the device query by query; longer probe lists or results: the chunked schedule
+      const FewArgs f = few_lists(bn);
       if (few_search_applies(ctx, f)) {
         VSK_TRY(few_search(ctx, f));
         continue;
