@@ -8,6 +8,9 @@
 //   table      t[s][c] = squared L2 between the query's segment s and codeword c       (:205-233)
 //   distance   sqrt(sum over s, in order, of t[s][code[s]])       (ProductQuantizerTypes.swift:14-20)
 //
+// From 64 queries on, a search decodes code rows and contracts them on the tensor cores, and forms the table sums only for the
+// rows that can be among the best (pq_tensor_search, tensor_scan.cu); the scan here serves the rest.
+//
 // Every sum is formed with separately rounded multiplies and adds in the reference's order, so codes and
 // distances equal the CPU restatement bit for bit.  The scan is byte work: per (row, query) m table look-ups in
 // shared memory and m adds.  A CTA keeps the tables of TQ queries in shared memory, interleaved by query
