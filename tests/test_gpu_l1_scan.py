@@ -85,3 +85,29 @@ def test_outliers_ties_and_non_finite_values(vsk, dev, cpu_oracle):
     inf = x.copy()
     inf[7, 2] = np.inf                                    # no grid: the fp32 scan
     assert_topk_parity(*_index(vsk, dev, inf).batchSearch(q, 10), *cpu_oracle.flat_search(oracle.MANHATTAN, q, inf, 10))
+
+
+def test_a_row_that_is_not_a_number_among_many(vsk, dev, cpu_oracle):
+    """A warp of the byte conversion takes several rows (more than 18 944 in all), so the NaN row must outlast the rows after
+    it.  Query 0's filter passes four rows and the NaN row only: the fp32 scan does not list that row, and neither may this."""
+    rng = np.random.default_rng(31)
+    n, d, nq, bad = 60_000, 24, 64, 20_000
+    x = rng.uniform(-1, 1, (n, d)).astype(np.float32)
+    x[bad, 5] = np.nan
+    q = rng.uniform(-1, 1, (nq, d)).astype(np.float32)
+    rm = rng.integers(1, 2 ** 62, n, dtype=np.uint64)
+    qm = rng.integers(1, 2 ** 62, nq, dtype=np.uint64)          # every query a mask of its own: one pass, not grouped
+    qm[0] = np.uint64(1) << np.uint64(63)
+    rm[[100, 30_000, 45_000, 59_999, bad]] |= qm[0]
+    ix = _index(vsk, dev, x, rm)
+    got = ix.batchSearch(q, 10, qm)
+    plain = ix.batchSearch(q, 10)
+    dev.set_search_path(1)
+    try:
+        ref, ref_plain = ix.batchSearch(q, 10, qm), ix.batchSearch(q, 10)
+    finally:
+        dev.set_search_path(0)
+        ix.close()
+    assert sorted(ref[1][0].tolist()) == [-1] * 6 + [100, 30_000, 45_000, 59_999]
+    assert np.array_equal(got[1], ref[1]) and np.array_equal(got[0], ref[0])
+    assert np.array_equal(plain[1], ref_plain[1]) and np.array_equal(plain[0], ref_plain[0])

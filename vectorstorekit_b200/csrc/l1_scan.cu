@@ -259,7 +259,7 @@ __global__ void l1_bytes_kernel(const float* __restrict__ x, int64_t n, int dim,
     }
     e = e * (1.0f + 1e-5f) + 2.4e-7f * (float)dim * (big + mag);
     if (err && lane == 0) err[row] = e;
-    worst = !(e <= worst) ? e : worst;   // what is not a number stays
+    if (isnan(e) || e > worst) worst = e;   // what is not a number stays: nothing compares greater than it
   }
   if (err_max && lane == 0) atomicMax(err_max, __float_as_uint(fabsf(worst)));
 }

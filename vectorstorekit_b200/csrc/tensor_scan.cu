@@ -3694,7 +3694,7 @@ __global__ void i8_row_stats_kernel(const int8_t* __restrict__ codes, int64_t n,
       x2 += __shfl_xor_sync(0xffffffffu, x2, o);
     }
     cmax = fmaxf(cmax, c2);
-    xmax = !(x2 <= xmax) ? x2 : xmax;   // a decoded value that is not a number stays one
+    if (isnan(x2) || x2 > xmax) xmax = x2;   // a decoded value that is not a number stays: nothing compares greater
   }
   if (lane == 0) {
     const float up = 1.0f + 1e-5f;
