@@ -71,3 +71,66 @@ def test_lists_that_overflow_go_to_the_other_paths(vsk, dev, cpu_oracle):
     keep = [i for i in range(300) if i not in (7, 9)]
     rd, ri = cpu_oracle.sq8_search(oracle.DOT, q[keep], codes, scale, offset, 20)
     assert_topk_parity(d_[keep], i_[keep], rd, ri)
+
+
+def _marks(dev, call):
+    """(what the call returned, the names of the launches it logged)"""
+    dev.timeline(True)
+    dev.timeline_read()
+    got = call()
+    names = [what for _, what, _ in dev.timeline_read()]
+    dev.timeline(False)
+    return got, names
+
+
+# resident query block (up to three K blocks) and the general kernel beyond it; the integer path answers by itself
+@pytest.mark.parametrize("shape", [(20_000, 64, 100, 10), (20_000, 384, 300, 10), (17_000, 513, 70, 10), (16_385, 129, 1, 10)])
+def test_the_integer_contraction_answers_ordinary_batches(vsk, dev, cpu_oracle, shape):
+    n, d, nq, k = shape
+    rng = np.random.default_rng(n + d)
+    ix, codes, scale, offset = _quantised(vsk, dev, rng.standard_normal((n, d)).astype(np.float32))
+    q = rng.standard_normal((nq, d)).astype(np.float32)
+    before = dev.stats()["fallback_queries"]
+    (got, names) = _marks(dev, lambda: ix.batchSearch(q, k))
+    assert "query_operands" not in names                          # (the fp16 path's first launch)
+    assert ("list_scan" in names) == (d <= 384) and ("scan" in names) == (d > 384)
+    assert dev.stats()["fallback_queries"] == before
+    assert_topk_parity(*got, *cpu_oracle.sq8_search(oracle.DOT, q, codes, scale, offset, k))
+
+
+def test_a_few_degenerate_queries_decide_for_themselves_only(vsk, dev, cpu_oracle):
+    """Zero vectors tie with every row and non-finite ones have no 8-bit form: they are re-run one by one, their batch keeps its
+    results and the batches after it their path."""
+    rng = np.random.default_rng(21)
+    ix, codes, scale, offset = _quantised(vsk, dev, rng.standard_normal((20_000, 64)).astype(np.float32))
+    q = rng.standard_normal((100, 64)).astype(np.float32)
+    rd, ri = cpu_oracle.sq8_search(oracle.DOT, q, codes, scale, offset, 10)
+    bad = q.copy()
+    bad[3], bad[50] = 0.0, 0.0
+    bad[60, 1], bad[61, 2] = np.nan, np.inf
+    keep = [i for i in range(100) if i not in (3, 50, 60, 61)]
+    before = dev.stats()["fallback_queries"]
+    (d_, i_), names = _marks(dev, lambda: ix.batchSearch(bad, 10))
+    assert "list_scan" in names and "query_operands" not in names
+    assert 4 <= dev.stats()["fallback_queries"] - before < 50     # (a zero query ties again in its re-run, which counts too)
+    assert_topk_parity(d_[keep], i_[keep], rd[keep], ri[keep])
+    assert np.all(d_[[3, 50]] == 0.0) and i_[3].tolist() == i_[50].tolist() == list(range(10))
+    got, names = _marks(dev, lambda: ix.batchSearch(q, 10))
+    assert "list_scan" in names and "query_operands" not in names
+    assert_topk_parity(*got, rd, ri)
+
+
+def test_small_batches_that_overflow_rest_together(vsk, dev, cpu_oracle):
+    """No single small batch is evidence; a hundred and more of their queries are."""
+    rng = np.random.default_rng(22)
+    n, d = 30_000, 48
+    base = rng.standard_normal(d).astype(np.float32)
+    x = np.linspace(0.01, 1.0, n, dtype=np.float32)[:, None] * base + 1e-3 * rng.standard_normal((n, d)).astype(np.float32)
+    ix, codes, scale, offset = _quantised(vsk, dev, x)
+    rests = []
+    for r in range(8):
+        q = (base + 0.1 * rng.standard_normal((40, d))).astype(np.float32)
+        got, names = _marks(dev, lambda: ix.batchSearch(q, 20))
+        rests.append("list_scan" not in names)
+        assert_topk_parity(*got, *cpu_oracle.sq8_search(oracle.DOT, q, codes, scale, offset, 20))
+    assert not rests[0] and all(rests[4:])

@@ -93,8 +93,32 @@ struct CandLists {
   uint64_t* keys = nullptr;   // [nq][kCandCap]
   int32_t* count = nullptr;   // [nq] appended so far (may exceed cap: overflow)
   float* thr = nullptr;       // [nq] rows with value <= thr are appended
-  int32_t* flags = nullptr;   // [nq] bit0: list overflowed; bit1: certificate failed
+  int32_t* flags = nullptr;   // [nq] bit0: list overflowed; bit1: certificate failed; bit2 (kFlagDegenerate)
   int64_t nq = 0;
+};
+
+// The query has no form on the path that was asked (a zero vector, values that are not finite): it is re-run by itself and says
+// nothing about the path.
+constexpr int32_t kFlagDegenerate = 4;
+
+// Whether an index leaves batches to the path behind a filter path whose lists overflow too often to pay.  Queries are
+// evidence, not calls: nothing is decided before 128 of them have been seen, over as many batches as that takes.
+struct PathRest {
+  int left = 0;                 // batches still to be left to the other path
+  int64_t seen = 0, bad = 0;    // queries since the last decision, and those of them whose list overflowed
+  bool resting() {
+    if (left == 0) return false;
+    --left;
+    return true;
+  }
+  // more than one in `one_in` overflowed: the next fifteen batches rest
+  void note(int64_t queries, int64_t overflowed, int one_in) {
+    seen += queries;
+    bad += overflowed;
+    if (seen < 128) return;
+    if (bad * one_in > seen) left = 15;
+    seen = bad = 0;
+  }
 };
 
 enum ScanMode : int { SCAN_DENSE = 0, SCAN_THRESHOLD = 1, SCAN_MATRIX = 2, SCAN_ARGMIN = 3 };
@@ -285,7 +309,7 @@ struct Index {
   int8_t* rows8 = nullptr;     // [n][stride8] padded copy where dim is not a multiple of 16, else null: the codes serve
   int32_t stride8 = 0;
   int64_t n8 = -1;             // rows the two norms cover
-  int i8_rest = 0;             // batches still to be left to the fp16 path
+  PathRest i8_rest;            // ... from the integer contraction, for the fp16 path
   float max_code_norm = 0.f, max_xnorm8 = 0.f;   // largest norm of a code row / of a decoded row
   // byte copy of the rows for Manhattan batches (l1_scan.cu): x ~ l1_lo[d] + l1_step * u
   uint8_t* rows_u8 = nullptr;  // [n][stride_u8]

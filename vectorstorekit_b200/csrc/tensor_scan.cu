@@ -2365,7 +2365,7 @@ int32_t launch_assign_scan(Ctx* ctx, const CUtensorMap& mx, const CUtensorMap& m
 void tensor_invalidate(Index* ix) {
   ix->n16 = -1;
   ix->n8 = -1;
-  ix->i8_rest = 0;
+  ix->i8_rest = PathRest{};
   ix->n_u8 = -1;
 }
 int32_t tensor_prepare_index(Index* ix) { return tensor_prepare(ix); }
@@ -3607,10 +3607,11 @@ struct I8Query {
   double offset;     // K
 };
 
-// One warp per query.  A query that is not finite gets an infinite slack: its list overflows and it is re-run.
+// One warp per query.  A query that is not finite or all but zero has no 8-bit form (every row would be listed): it is flagged, its
+// bar is out of reach, and it is re-run by itself.
 __global__ void i8_query_kernel(const float* __restrict__ q, int64_t nq, int dim, int stride, const float* __restrict__ scale,
                                 const float* __restrict__ offset, float max_code_norm, float max_xnorm, int8_t* __restrict__ out,
-                                I8Query* __restrict__ info) {
+                                I8Query* __restrict__ info, int32_t* __restrict__ flags) {
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= nq) return;
   const int lane = threadIdx.x & 31;
@@ -3657,8 +3658,10 @@ __global__ void i8_query_kernel(const float* __restrict__ q, int64_t nq, int dim
     // the step and q~ are rounded to 2^-22 at worst; an exact value is a sum of dim products of q with x^ = (c - offset)
     // / scale, whose roundings are below (dim + 8) 2^-23 |q| |x^|
     r.slack = (sqrtf(e2) * 1.0001f + 1e-6f * tn) * max_code_norm + 1.2e-7f * (float)(dim + 8) * qn * max_xnorm;
-    if (!finite) r.slack = CUDART_INF_F;
-    else if (!usable) r.slack = tn * max_code_norm * 1.0001f + 1.2e-7f * (float)(dim + 8) * qn * max_xnorm;   // q8 = 0
+    if (!usable) {
+      r.slack = -CUDART_INF_F;
+      flags[row] = kFlagDegenerate;   // (the flags have just been cleared)
+    }
     info[row] = r;
   }
 }
@@ -3671,7 +3674,7 @@ __global__ void i8_bar_kernel(const float* __restrict__ thr_exact, const I8Query
   const I8Query r = info[i];
   const double at = floor((double)r.inv_step * (r.offset - (double)thr_exact[i] - (double)r.slack)) - 1.0;
   // not a number or below every accumulator: every row is listed (and the list overflows)
-  bar[i] = !(at > -2147483647.0) ? INT_MIN : at > 2147483646.0 ? INT_MAX : (int32_t)at;
+  bar[i] = r.slack == -CUDART_INF_F ? INT_MAX : !(at > -2147483647.0) ? INT_MIN : at > 2147483646.0 ? INT_MAX : (int32_t)at;
 }
 
 // Largest norm of a code row and of its decoded row (the stored codes themselves are the operand).
@@ -3737,11 +3740,10 @@ static int32_t i8_prepare(Index* ix) {
   memcpy(&ix->max_code_norm, &h.max_norm16, 4);
   memcpy(&ix->max_xnorm8, &h.max_norm, 4);
   ix->n8 = ix->n;
-  ix->i8_rest = 0;
   return VSK_OK;
 }
 
-constexpr int kI8Rest = 15;   // batches an index leaves to the fp16 path after one that did not fit this one
+constexpr int kI8RestOneIn = 64;   // more than one query in so many that overflows costs what the integer contraction gains
 
 bool i8_search_applicable(const Index* ix, int32_t k) {
   // 127 * 128 * dim below 2^31: no accumulator can overflow
@@ -3753,10 +3755,7 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
   VSK_TRACE("vsk:i8_scan");
   Ctx* ctx = ix->ctx;
   *handled = false;
-  if (ix->i8_rest > 0) {
-    --ix->i8_rest;
-    return VSK_OK;
-  }
+  if (ix->i8_rest.resting()) return VSK_OK;
   VSK_TRY(i8_prepare(ix));
   const float limit = 1e30f;
   if (!(ix->max_code_norm < limit) || !(ix->max_xnorm8 < limit)) return VSK_OK;
@@ -3780,9 +3779,6 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
   const float* alpha = (const float*)p + 2;
   int32_t* err = (int32_t*)p + 3;
   unsigned long long* rr_total = (unsigned long long*)((char*)p + 16);
-  i8_query_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, ctx->stream>>>(q, nq, dim, stride, ix->sq_scale, ix->sq_offset, ix->max_code_norm,
-                                                                      ix->max_xnorm8, q8, info);
-  ctx->stats.kernel_launches++;
   CUtensorMap mq, mx, mb;
   const int8_t* rows8 = ix->rows8 ? ix->rows8 : ix->codes;
   VSK_TRY(make_map_i8(ctx, q8, list ? nq_pad : nq, dim, stride, list ? TN : TM, &mq));
@@ -3791,6 +3787,9 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
   CandLists cand;
   VSK_TRY(cand_lists(ctx, nq, &cand));
   VSK_TRY(launch_init_cand(ctx, cand, nq));
+  i8_query_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, ctx->stream>>>(q, nq, dim, stride, ix->sq_scale, ix->sq_offset, ix->max_code_norm,
+                                                                      ix->max_xnorm8, q8, info, cand.flags);
+  ctx->stats.kernel_launches++;
   TcArgs a{};
   a.nq = nq;
   a.kblocks = kblocks;
@@ -3831,9 +3830,9 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
   VSK_TRY(pinned_reserve(ctx, &hb, (size_t)nq * 4 + 16));
   char* hbuf = (char*)hb.p;
   const int32_t* hflags = (const int32_t*)(hbuf + 16);
-  auto count_flagged = [&] {
+  auto count_overflowed = [&] {
     int64_t bad = 0;
-    for (int64_t i = 0; i < nq; ++i) bad += hflags[i] != 0;
+    for (int64_t i = 0; i < nq; ++i) bad += hflags[i] != 0 && !(hflags[i] & kFlagDegenerate);
     return bad;
   };
   const size_t qsm = (size_t)dim * sizeof(float);
@@ -3849,8 +3848,9 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
       // against the spread of the values), the fp16 path takes the batch
       VSK_CUDA(ctx, cudaMemcpyAsync(hbuf + 16, cand.flags, (size_t)nq * 4, cudaMemcpyDeviceToHost, ctx->stream));
       VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-      if (64 * count_flagged() > nq) {
-        ix->i8_rest = kI8Rest;
+      const int64_t over = count_overflowed();
+      if (kI8RestOneIn * over > nq) {
+        ix->i8_rest.note(nq, over, kI8RestOneIn);
         return VSK_OK;
       }
       looked = true;
@@ -3907,10 +3907,10 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
   std::vector<int32_t> bad;
   for (int64_t i = 0; i < nq; ++i)
     if (hflags[i]) bad.push_back((int32_t)i);
-  if (bad.size() > 1 && 64 * (int64_t)bad.size() > nq) {
-    ix->i8_rest = kI8Rest;
-    return VSK_OK;
-  }
+  // a few queries are re-run by themselves, whatever share of the batch they are; many send the batch to the fp16 path
+  const int64_t over = count_overflowed();
+  ix->i8_rest.note(nq, over, kI8RestOneIn);
+  if (over > 8 && kI8RestOneIn * over > nq) return VSK_OK;
   if (!bad.empty()) VSK_TRY(fp32_search_subset(ix, q, bad, k, nullptr, nullptr, out_dist, out_ids));
   *handled = true;
   return VSK_OK;
