@@ -111,3 +111,38 @@ def test_a_row_that_is_not_a_number_among_many(vsk, dev, cpu_oracle):
     assert sorted(ref[1][0].tolist()) == [-1] * 6 + [100, 30_000, 45_000, 59_999]
     assert np.array_equal(got[1], ref[1]) and np.array_equal(got[0], ref[0])
     assert np.array_equal(plain[1], ref_plain[1]) and np.array_equal(plain[0], ref_plain[0])
+
+
+def _marks(dev, call):
+    """(what the call returned, the names of the launches it logged)"""
+    dev.timeline(True)
+    dev.timeline_read()
+    got = call()
+    names = [what for _, what, _ in dev.timeline_read()]
+    dev.timeline(False)
+    return got, names
+
+
+def test_one_filter_group_that_overflows_does_not_shut_out_the_others(vsk, dev):
+    rng = np.random.default_rng(32)
+    groups, n, d, per = 5, 100_000, 128, 400
+    x = rng.uniform(-1, 1, (n, d)).astype(np.float32)
+    rm = np.uint64(1) << (np.arange(n) % groups).astype(np.uint64)
+    q = rng.uniform(-1, 1, (groups * per, d)).astype(np.float32)
+    qm = np.uint64(1) << (np.arange(groups * per) // per).astype(np.uint64)
+    late = np.arange(n - 75_000, n)
+    x[late[rm[late] == 1]] = 0.01                                # 15 000 equal rows, nearest to all of group 0's queries
+    q[: per // 2] = 0.0
+    q[5, 3] = np.nan                                             # no evidence of anything
+    ix = _index(vsk, dev, x, rm)
+    dev.set_search_path(1)
+    ref = ix.batchSearch(q, 10, qm)
+    dev.set_search_path(0)
+    for _ in range(3):
+        before = dev.stats()["fallback_queries"]
+        got, names = _marks(dev, lambda: ix.batchSearch(q, 10, qm))
+        assert dev.stats()["fallback_queries"] - before >= per
+        assert names.count("l1_dense") == groups                 # all groups took the byte filter, on every call
+        keep = np.arange(len(q)) != 5
+        assert np.array_equal(got[1][keep], ref[1][keep]) and np.array_equal(got[0][keep], ref[0][keep])
+    ix.close()

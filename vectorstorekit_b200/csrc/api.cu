@@ -359,7 +359,7 @@ int32_t fp32_topk(Ctx* ctx, const ExactScanArgs& proto, int64_t n, int64_t nq, c
 
 static int32_t fp32_search(Index* ix, const float* q, int64_t nq, const int32_t* sub_dev, int32_t k,
                            const float* qnorm, const uint64_t* qmasks, float* out_dist, int64_t* out_ids,
-                           int level) {
+                           int level, L1Call* l1) {
   ExactScanArgs a{};
   a.metric = ix->metric;
   a.q = q;
@@ -375,9 +375,9 @@ static int32_t fp32_search(Index* ix, const float* q, int64_t nq, const int32_t*
   a.xnorm = ix->row_norm;
   a.row_masks = (qmasks && ix->has_masks) ? ix->masks : nullptr;
   a.q_masks = a.row_masks ? qmasks : nullptr;
-  if (level == 0 && l1_applicable(ix, ix->n, nq, k)) {
+  if (l1 && level == 0 && l1_applicable(ix, ix->n, nq, k)) {
     bool handled = false;
-    VSK_TRY(l1_topk(ix, a, ix->n, nq, sub_dev, k, out_dist, out_ids, &handled));
+    VSK_TRY(l1_topk(ix, a, ix->n, nq, sub_dev, k, out_dist, out_ids, l1, &handled));
     if (handled) return VSK_OK;
   }
   return fp32_topk(ix->ctx, a, ix->n, nq, sub_dev, k, ix->id_base, out_dist, out_ids, level);
@@ -448,7 +448,7 @@ static int pick_query_tile(int64_t g) {
 // fp32 tile's rate) and this path is taken only when the filters leave less than that share of the (query, row)
 // pairs eligible - then scanning only eligible rows wins all the same.
 static int32_t filtered_grouped_search(Index* ix, const float* q, int64_t nq, int32_t k, const float* qnorm,
-                                       const uint64_t* qmasks, float* out_dist, int64_t* out_ids, bool* handled,
+                                       const uint64_t* qmasks, float* out_dist, int64_t* out_ids, L1Call* l1, bool* handled,
                                        double max_fraction = -1.0) {
   Ctx* ctx = ix->ctx;
   *handled = false;
@@ -527,7 +527,7 @@ static int32_t filtered_grouped_search(Index* ix, const float* q, int64_t nq, in
     a.xnorm = ix->row_norm;
     if (l1_applicable(ix, cnt, e - b, k)) {
       bool handled = false;
-      VSK_TRY(l1_topk(ix, a, cnt, e - b, qpos, k, out_dist, out_ids, &handled));
+      VSK_TRY(l1_topk(ix, a, cnt, e - b, qpos, k, out_dist, out_ids, l1, &handled));
       if (handled) continue;
     }
     VSK_TRY(fp32_topk(ctx, a, cnt, e - b, qpos, k, ix->id_base, out_dist, out_ids, 0));
@@ -589,16 +589,18 @@ static int32_t flat_search_dev(Index* ix, const float* q, int64_t nq, int32_t k,
     // contraction: the fp32 streaming scan reads each eligible fp32 row once.
     const bool tensor = tensor_metric && !(mb && bn <= kStreamScanMaxQueries);
     bool grouped = false;
+    L1Call l1;
     if (mb && ix->has_masks)
-      VSK_TRY(filtered_grouped_search(ix, qb, bn, k, qnorm, mb, out_dist + b * k, out_ids + b * k, &grouped,
+      VSK_TRY(filtered_grouped_search(ix, qb, bn, k, qnorm, mb, out_dist + b * k, out_ids + b * k, &l1, &grouped,
                                       tensor ? 0.03 : -1.0));
     if (grouped) {
       // done: every group of equal masks was scanned against its own eligible rows
     } else if (tensor) {
       VSK_TRY(tensor_search(ix, qb, bn, k, qnorm, mb, out_dist + b * k, out_ids + b * k));
     } else {
-      VSK_TRY(fp32_search(ix, qb, bn, nullptr, k, qnorm, mb, out_dist + b * k, out_ids + b * k, 0));
+      VSK_TRY(fp32_search(ix, qb, bn, nullptr, k, qnorm, mb, out_dist + b * k, out_ids + b * k, 0, &l1));
     }
+    if (l1.seen > 0) ix->l1_rest.note(l1.seen, l1.bad, kL1RestOneIn);   // the grid is too coarse for these rows
   }
   VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return VSK_OK;
@@ -614,7 +616,7 @@ int32_t fp32_search_subset(Index* ix, const float* q, const std::vector<int32_t>
   VSK_CUDA(ctx, cudaMemcpyAsync(p, subset.data(), subset.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
   VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   ctx->stats.fallback_queries += (int64_t)subset.size();
-  return fp32_search(ix, q, (int64_t)subset.size(), (const int32_t*)p, k, qnorm, qmasks, out_dist, out_ids, 0);
+  return fp32_search(ix, q, (int64_t)subset.size(), (const int32_t*)p, k, qnorm, qmasks, out_dist, out_ids, 0, nullptr);
 }
 
 int32_t flat_reserve(Index* ix, int64_t need) {

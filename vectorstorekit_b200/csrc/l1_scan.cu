@@ -31,7 +31,6 @@ constexpr int L1_THREADS = 256;
 constexpr int L1_CHUNK = 64;        // bytes of a row per stage
 constexpr int L1_PITCH = L1_CHUNK + 16;
 constexpr int L1_STAGES = 2;
-constexpr int kL1Rest = 15;         // batches an index leaves to the fp32 scan after one whose lists overflowed
 
 struct L1Args {
   const uint8_t* q8;          // [nq][stride] by list position
@@ -197,11 +196,16 @@ __global__ void __launch_bounds__(L1_RS_THREADS) l1_rescore_kernel(const float* 
 }
 
 // Largest byte sum at which a row can still be at or below the query's exact threshold; the fp32 sums compared are off by
-// (dim + 8) 2^-23 of their size at most.
+// (dim + 8) 2^-23 of their size at most.  A query that is not finite lists nothing and is re-run by itself.
 __global__ void l1_bar_kernel(const float* __restrict__ thr, const float* __restrict__ eq, int64_t nq, float ex, float step, int dim,
-                              int32_t* __restrict__ bar) {
+                              int32_t* __restrict__ bar, int32_t* __restrict__ flags) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nq) return;
+  if (!(eq[i] < CUDART_INF_F)) {
+    atomicOr(&flags[i], kFlagDegenerate);
+    bar[i] = -1;
+    return;
+  }
   const double t = thr[i];
   const double at = (t * (1.0 + 1.2e-7 * (dim + 8)) + (double)eq[i] + (double)ex) / (double)step + 1.0;
   bar[i] = at < 2147483000.0 ? (int32_t)at : INT_MAX;   // (also for what is not a number: every row is listed)
@@ -298,7 +302,6 @@ int32_t l1_prepare(Index* ix) {
     mag = std::max(mag, std::max(std::fabs(a), std::fabs(b)));
   }
   ix->n_u8 = ix->n;   // looked at, usable or not
-  ix->l1_rest = 0;
   if (!finite || !(mag < 1e30f)) return VSK_OK;
   const float step = range > 1e-30f ? range / 255.0f : 1.0f;
   if (dev_alloc(ctx, (void**)&ix->rows_u8, (size_t)ix->n * ix->stride_u8) != VSK_OK) return VSK_OK;   // no room: the fp32 scan
@@ -342,14 +345,15 @@ bool l1_applicable(const Index* ix, int64_t n, int64_t nq, int32_t k) {
 }
 
 int32_t l1_topk(Index* ix, const ExactScanArgs& proto, int64_t n, int64_t nq, const int32_t* sub_dev, int32_t k, float* out_dist,
-                int64_t* out_ids, bool* handled) {
+                int64_t* out_ids, L1Call* call, bool* handled) {
   VSK_TRACE("vsk:l1_scan");
   Ctx* ctx = ix->ctx;
   *handled = false;
-  if (ix->l1_rest > 0) {
-    --ix->l1_rest;
-    return VSK_OK;
+  if (!call->asked) {
+    call->asked = true;
+    call->allowed = !ix->l1_rest.resting();
   }
+  if (!call->allowed) return VSK_OK;
   VSK_TRY(l1_prepare(ix));
   if (!ix->l1_ok) return VSK_OK;
   const int dim = ix->dim, stride = ix->stride_u8;
@@ -410,7 +414,7 @@ int32_t l1_topk(Index* ix, const ExactScanArgs& proto, int64_t n, int64_t nq, co
     // most seven times what has been seen: a listed row costs a gather
     int64_t chunk = std::min(schedule_chunk(seen, k, 0) / 4, 7 * seen);
     chunk = std::min(std::max<int64_t>(chunk, 1024), n - seen);
-    l1_bar_kernel<<<(unsigned)ceil_div(nq, 256), 256, 0, ctx->stream>>>(cand.thr, eq, nq, ix->l1_ex, ix->l1_step, dim, bar);
+    l1_bar_kernel<<<(unsigned)ceil_div(nq, 256), 256, 0, ctx->stream>>>(cand.thr, eq, nq, ix->l1_ex, ix->l1_step, dim, bar, cand.flags);
     ctx->stats.kernel_launches++;
     a.row_begin = seen;
     a.row_end = seen + chunk;
@@ -450,11 +454,13 @@ int32_t l1_topk(Index* ix, const ExactScanArgs& proto, int64_t n, int64_t nq, co
   memcpy(&hrr, hb.p, 8);
   ctx->stats.reranked_rows += (int64_t)hrr;
   std::vector<int32_t> bad;
-  for (int64_t i = 0; i < nq; ++i)
+  for (int64_t i = 0; i < nq; ++i) {
     if (hflags[i]) bad.push_back(sub_dev ? hsub[i] : (int32_t)i);
+    call->bad += hflags[i] != 0 && !(hflags[i] & kFlagDegenerate);
+  }
+  call->seen += nq;
   *handled = true;
   if (bad.empty()) return VSK_OK;
-  if (4 * (int64_t)bad.size() > nq) ix->l1_rest = kL1Rest;   // the grid is too coarse for these rows
   VSK_TRY(scratch(ctx, SLOT_SUBSET, bad.size() * sizeof(int32_t), &p));
   VSK_CUDA(ctx, cudaMemcpyAsync(p, bad.data(), bad.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
   VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -51,9 +51,15 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
 // Manhattan batches through the byte filter (l1_scan.cu); `proto` as for fp32_topk, its rows those of the index.
 // *handled = false: the fp32 scan takes the batch.
 constexpr int64_t kL1MinQueries = 32, kL1MinRows = 16384;
+// One search call: its filter groups are decided, and counted as evidence (Index::l1_rest), together.
+struct L1Call {
+  bool asked = false, allowed = false;
+  int64_t seen = 0, bad = 0;   // queries that took the filter, and those of them whose list overflowed
+};
+constexpr int kL1RestOneIn = 4;
 bool l1_applicable(const Index* ix, int64_t n, int64_t nq, int32_t k);
 int32_t l1_topk(Index* ix, const ExactScanArgs& proto, int64_t n, int64_t nq, const int32_t* sub_dev, int32_t k, float* out_dist,
-                int64_t* out_ids, bool* handled);
+                int64_t* out_ids, L1Call* call, bool* handled);
 // Candidate lists for nq queries in the current lane's scratch.
 int32_t cand_lists(Ctx* ctx, int64_t nq, CandLists* cand);
 // Drops the operand copies after rows were added; makes it (once per index state).
