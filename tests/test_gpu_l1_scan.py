@@ -146,3 +146,35 @@ def test_one_filter_group_that_overflows_does_not_shut_out_the_others(vsk, dev):
         keep = np.arange(len(q)) != 5
         assert np.array_equal(got[1][keep], ref[1][keep]) and np.array_equal(got[0][keep], ref[0][keep])
     ix.close()
+
+
+def test_only_rows_that_are_re_scored_are_counted(vsk, dev):
+    """The k rows kept from chunk to chunk carry their exact values already."""
+    rng = np.random.default_rng(33)
+    n, d, nq, k = 40_000, 32, 64, 1_000
+    ix = _index(vsk, dev, rng.uniform(-1, 1, (n, d)).astype(np.float32))
+    q = rng.uniform(-1, 1, (nq, d)).astype(np.float32)
+    before = dev.stats()
+    _, names = _marks(dev, lambda: ix.batchSearch(q, k))
+    after = dev.stats()
+    counted, chunks = after["reranked_rows"] - before["reranked_rows"], names.count("l1_scan")
+    assert chunks > 1 and after["fallback_queries"] == before["fallback_queries"]
+    # a chunk adds 0.65 of the rows seen before it, and so lists about 0.65 k rows a query: less than the k it finds kept
+    assert 0 < counted < nq * k * chunks
+    ix.close()
+
+
+def test_the_widest_rows_of_the_path(vsk, dev):
+    """A query of 12 288 dimensions fills the 48 KB of the re-scoring kernel."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(35)
+    x = torch.empty((16_384, 12_288), device="cuda").uniform_(-1.0, 1.0, generator=gen)
+    q = torch.empty((32, 12_288), device="cuda").uniform_(-1.0, 1.0, generator=gen)
+    ix = _index(vsk, dev, x)
+    (gd, gi), names = _marks(dev, lambda: ix.batchSearch(q, 10))
+    assert "l1_rescore" in names
+    dev.set_search_path(1)
+    rd, ri = ix.batchSearch(q, 10)
+    dev.set_search_path(0)
+    assert torch.equal(gi, ri) and torch.equal(gd, rd)
+    ix.close()

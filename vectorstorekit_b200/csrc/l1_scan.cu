@@ -170,8 +170,8 @@ __global__ void __launch_bounds__(L1_RS_THREADS) l1_rescore_kernel(const float* 
   const int cnt = min(cand.count[pos], kCandCap);
   uint64_t* keys = cand.keys + pos * kCandCap;
   for (int i = threadIdx.x; i < dim; i += L1_RS_THREADS) qs[i] = __ldg(q + qi * dim + i);
-  if (threadIdx.x == 0 && blockIdx.y == 0) atomicAdd(total, (unsigned long long)cnt);
   __syncthreads();
+  int formed = 0;
   for (int c = blockIdx.y * L1_RS_THREADS + threadIdx.x; c < cnt; c += gridDim.y * L1_RS_THREADS) {
     const uint64_t key = keys[c];
     if ((uint32_t)(key >> 32) != 0x80000000u) continue;
@@ -192,7 +192,17 @@ __global__ void __launch_bounds__(L1_RS_THREADS) l1_rescore_kernel(const float* 
     }
     for (; d < dim; ++d) s += fabsf(qs[d] - __ldg(p + d));
     keys[c] = make_key(s, (uint32_t)key);
+    ++formed;
   }
+  // rows formed by this CTA, one atomic per CTA (the query is done with, its first word takes the sum: with a static word beside
+  // it the widest rows would no longer fit into 48 KB)
+  int* sum = reinterpret_cast<int*>(qs);
+  __syncthreads();
+  if (threadIdx.x == 0) *sum = 0;
+  __syncthreads();
+  if (formed) atomicAdd(sum, formed);
+  __syncthreads();
+  if (threadIdx.x == 0 && *sum) atomicAdd(total, (unsigned long long)*sum);
 }
 
 // Largest byte sum at which a row can still be at or below the query's exact threshold; the fp32 sums compared are off by
