@@ -178,3 +178,31 @@ def test_the_widest_rows_of_the_path(vsk, dev):
     dev.set_search_path(0)
     assert torch.equal(gi, ri) and torch.equal(gd, rd)
     ix.close()
+
+
+def test_the_byte_copy_is_made_when_it_pays(vsk, dev):
+    """Adding and searching in turn keeps to the fp32 tile for batches that would not pay for the copy; so do batches that are
+    too small to gain from a copy that exists.  Batches on rows that stay as they are pay for it together."""
+    rng = np.random.default_rng(34)
+    n, d, k = 100_000, 256, 10
+    x = rng.uniform(-1, 1, (n, d)).astype(np.float32)
+    q = rng.uniform(-1, 1, (800, d)).astype(np.float32)
+    ix = _index(vsk, dev, x)
+
+    def filtered(nq):
+        dev.set_search_path(1)
+        ref = ix.batchSearch(q[:nq], k)
+        dev.set_search_path(0)
+        got, names = _marks(dev, lambda: ix.batchSearch(q[:nq], k))
+        assert np.array_equal(got[1], ref[1]) and np.array_equal(got[0], ref[0])
+        return "l1_scan" in names
+
+    assert filtered(32)                                          # the first batch makes the copy
+    assert not filtered(32) and filtered(64)                     # 0.8e9 and 1.6e9 steps
+    for nq in (64, 256, 64, 256):
+        ix.add(x[:50] * 0.9)
+        assert not filtered(nq)
+    assert [filtered(64) for _ in range(6)] == [False] * 4 + [True] * 2   # 256 + 5 x 64 queries: 1.48e10 steps
+    ix.add(x[:50] * 0.9)
+    assert filtered(800)
+    ix.close()

@@ -590,6 +590,7 @@ static int32_t flat_search_dev(Index* ix, const float* q, int64_t nq, int32_t k,
     const bool tensor = tensor_metric && !(mb && bn <= kStreamScanMaxQueries);
     bool grouped = false;
     L1Call l1;
+    l1.queries = bn;
     if (mb && ix->has_masks)
       VSK_TRY(filtered_grouped_search(ix, qb, bn, k, qnorm, mb, out_dist + b * k, out_ids + b * k, &l1, &grouped,
                                       tensor ? 0.03 : -1.0));

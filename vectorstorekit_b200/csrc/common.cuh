@@ -316,6 +316,7 @@ struct Index {
   int32_t stride_u8 = 0;
   int64_t n_u8 = -1;           // rows the copy covers
   bool l1_ok = false;          // ... and whether it is usable
+  double l1_work = 0.0;        // query x row x dimension steps the fp32 tile has done for want of the copy
   PathRest l1_rest;            // ... from the byte filter, for the fp32 scan
   float* l1_lo = nullptr;      // [dim]
   float l1_step = 1.f, l1_mag = 0.f, l1_ex = 0.f;   // grid step, largest |x|, largest L1 distance of a row to its bytes

@@ -2367,6 +2367,7 @@ void tensor_invalidate(Index* ix) {
   ix->n8 = -1;
   ix->i8_rest = PathRest{};
   ix->n_u8 = -1;
+  ix->l1_work = 0.0;
   ix->l1_rest = PathRest{};
 }
 int32_t tensor_prepare_index(Index* ix) { return tensor_prepare(ix); }

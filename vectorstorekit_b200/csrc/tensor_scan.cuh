@@ -54,6 +54,7 @@ constexpr int64_t kL1MinQueries = 32, kL1MinRows = 16384;
 // One search call: its filter groups are decided, and counted as evidence (Index::l1_rest), together.
 struct L1Call {
   bool asked = false, allowed = false;
+  int64_t queries = 0;         // of the call that no group has taken yet
   int64_t seen = 0, bad = 0;   // queries that took the filter, and those of them whose list overflowed
 };
 constexpr int kL1RestOneIn = 4;
