@@ -108,3 +108,61 @@ def test_non_finite_queries_do_not_disturb_the_others(vsk, dev, cpu_oracle):
     assert dev.stats()["tensor_tiles"] == before
     rd, ri = cpu_oracle.pq_search(q, codes, cb2, 10)
     assert np.array_equal(ids, ri) and np.array_equal(dist, rd)
+
+
+def _marks(dev, call):
+    """(what the call returned, the names of the launches it logged)"""
+    dev.timeline(True)
+    dev.timeline_read()
+    got = call()
+    names = [what for _, what, _ in dev.timeline_read()]
+    dev.timeline(False)
+    return got, names
+
+
+def test_ordinary_batches_are_answered_by_the_contraction(vsk, dev, cpu_oracle):
+    """Not by the table scan behind it: no query is handed back."""
+    for m, ds in ((16, 8), (10, 32)):                             # queries resident, and the general kernel
+        rng = np.random.default_rng(m)
+        q, cb, x = _clustered(rng, 30_000, 100, m, 256, ds)
+        codes = cpu_oracle.pq_encode(x, cb)
+        ix = _index(vsk, dev, cb, codes)
+        before = dev.stats()["fallback_queries"]
+        (dist, ids), names = _marks(dev, lambda: ix.batchSearch(q, 10))
+        assert ("list_scan" if m == 16 else "scan") in names
+        assert dev.stats()["fallback_queries"] == before
+        rd, ri = cpu_oracle.pq_search(q, codes, cb, 10)
+        assert np.array_equal(ids, ri) and np.array_equal(dist, rd)
+
+
+def test_an_index_of_bulk_ties_rests_from_the_contraction(vsk, dev, cpu_oracle):
+    rng = np.random.default_rng(16)
+    n, m, ds = 60_000, 2, 4
+    cb = rng.standard_normal((m, 16, ds)).astype(np.float32)
+    q = rng.standard_normal((150, m * ds)).astype(np.float32)
+    codes = rng.integers(0, 3, (n, m)).astype(np.uint8)          # 9 distinct rows
+    ix = _index(vsk, dev, cb, codes)
+    rd, ri = cpu_oracle.pq_search(q, codes, cb, 100)
+    decoded = []
+    for _ in range(17):
+        (dist, ids), names = _marks(dev, lambda: ix.batchSearch(q, 100))
+        decoded.append("pq_decode" in names)
+        assert np.array_equal(ids, ri) and np.array_equal(dist, rd)
+    assert decoded == [True] + [False] * 15 + [True]
+
+
+def test_entries_of_nearly_equal_size(vsk, dev, cpu_oracle):
+    """Vectors in the positive quadrant: the thresholds lie near half the largest squared norm, the far end of what the operand
+    columns hold.  The contraction still answers."""
+    rng = np.random.default_rng(17)
+    m, ds, n, nq = 16, 8, 30_000, 100
+    x = rng.uniform(0.5, 1.0, (n, m * ds)).astype(np.float32)
+    q = rng.uniform(0.5, 1.0, (nq, m * ds)).astype(np.float32)
+    cb = np.ascontiguousarray(np.stack([x[rng.choice(n, 256, replace=False)][:, s * ds:(s + 1) * ds] for s in range(m)]))
+    codes = cpu_oracle.pq_encode(x, cb)
+    ix = _index(vsk, dev, cb, codes)
+    before = dev.stats()["fallback_queries"]
+    dist, ids = ix.batchSearch(q, 10)
+    rd, ri = cpu_oracle.pq_search(q, codes, cb, 10)
+    assert np.array_equal(ids, ri) and np.array_equal(dist, rd)
+    assert dev.stats()["fallback_queries"] == before

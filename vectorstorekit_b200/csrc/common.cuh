@@ -335,6 +335,7 @@ struct Index {
   uint8_t* pq_codes = nullptr;     // [capacity][pq_m]
   __half* pq_cb16 = nullptr;       // codebooks as fp16 operand values (made at the first tensor-path search) ...
   float* pq_cw2 = nullptr;         // [pq_m][pq_ksub] ... and the codewords' squared norms
+  PathRest pq_rest;                // batches left to the table scan after some whose lists overflowed
   int pq_operands = 0;             // 0: not made yet, 1: usable, -1: this codebook has no usable fp16 form
 };
 

@@ -487,6 +487,7 @@ int32_t pq_adopt_rows(Index* ix, int64_t n) {
   if (n > ix->capacity) return fail(ix->ctx, VSK_ERR_INVALID_BUFFER_SIZE, "more rows than reserved");
   VSK_TRY(pq_check_codes(ix, 0, n));
   ix->n = n;
+  ix->pq_rest = PathRest{};
   return VSK_OK;
 }
 
@@ -705,6 +706,7 @@ static int32_t pq_add(vsk_index* i, const uint8_t* codes, int64_t n, bool on_dev
   VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   VSK_TRY(pq_check_codes(ix, ix->n, n));   // rejected rows are not counted in
   ix->n += n;
+  ix->pq_rest = PathRest{};
   return VSK_OK;
 }
 

@@ -3335,11 +3335,12 @@ __global__ void __launch_bounds__(256) pq_decode16_kernel(const uint8_t* __restr
 // terms, and eps covers the coarse value against |x^|^2 - 2 q.x^ itself.
 __global__ void pq_coarse_threshold_kernel(const float* __restrict__ thr_exact, const float* __restrict__ qnorm,
                                            const float* __restrict__ eps, int64_t nq, float sum_terms, float norm_terms,
-                                           float* __restrict__ thr_coarse) {
+                                           float* __restrict__ thr_coarse, int32_t* __restrict__ flags) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nq) return;
   const float t = thr_exact[i];
   float tc = CUDART_INF_F;
+  if (!(t < CUDART_INF_F)) atomicOr(&flags[i], kFlagDegenerate);   // (the first rows gave it k values: it is not finite)
   if (!(t == CUDART_INF_F)) {
     const float t2 = t * t, qn2 = qnorm[i] * qnorm[i];
     tc = (t2 - qn2) + eps[i] + 1.2e-7f * (sum_terms * t2 + norm_terms * qn2);
@@ -3452,7 +3453,7 @@ int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const
   *handled = false;
   flagged->clear();
   VSK_TRY(pq_tensor_prepare(ix));
-  if (ix->pq_operands < 0) return VSK_OK;
+  if (ix->pq_operands < 0 || ix->pq_rest.resting()) return VSK_OK;
   const int m = ix->pq_m, ksub = ix->pq_ksub, dim = ix->dim, dim16 = ix->dim16, ds = dim / m;
   const int64_t n = ix->n;
   const bool fold = ix->fold16;
@@ -3506,6 +3507,11 @@ int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const
   VSK_TRY(pinned_reserve(ctx, &hb, (size_t)nq * 4 + 16));
   char* hbuf = (char*)hb.p;
   const int32_t* hflags = (const int32_t*)(hbuf + 16);
+  auto count_overflowed = [&] {
+    int64_t bad = 0;
+    for (int64_t i = 0; i < nq; ++i) bad += hflags[i] != 0 && !(hflags[i] & kFlagDegenerate);
+    return bad;
+  };
   bool looked = false;
   while (seen < n) {
     int64_t chunk = std::min(schedule_chunk(seen, k, 0), std::max<int64_t>(1024, growth * seen));
@@ -3516,9 +3522,11 @@ int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const
       // table scan, which can pass over a tied row, takes the whole batch.
       VSK_CUDA(ctx, cudaMemcpyAsync(hbuf + 16, cand.flags, (size_t)nq * 4, cudaMemcpyDeviceToHost, ctx->stream));
       VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-      int64_t bad = 0;
-      for (int64_t i = 0; i < nq; ++i) bad += hflags[i] != 0;
-      if (4 * bad > nq) return VSK_OK;
+      const int64_t over = count_overflowed();
+      if (kPqRestOneIn * over > nq) {
+        ix->pq_rest.note(nq, over, kPqRestOneIn);
+        return VSK_OK;
+      }
       looked = true;
     }
     const unsigned dgrid = (unsigned)ceil_div(chunk, PQ_DEC_ROWS);
@@ -3535,7 +3543,8 @@ int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const
 #undef VSK_PQ_DEC
     tl_mark(ctx, "pq_decode");
     pq_coarse_threshold_kernel<<<(unsigned)ceil_div(nq, 256), 256, 0, ctx->stream>>>(
-        cand.thr, qnorm, qo.eps, nq, (float)(m + ds + 8), (float)(ceil_div(dim, 32) + 16), cand_coarse.thr);
+        cand.thr, qnorm, qo.eps, nq, (float)(m + ds + 8), (float)(ceil_div(dim, 32) + 16), cand_coarse.thr,
+        cand.flags);
     ctx->stats.kernel_launches += 2;
     VSK_CUDA(ctx, cudaGetLastError());
     if (list) {
@@ -3590,6 +3599,7 @@ int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const
     return fail(ctx, VSK_ERR_TIMEOUT, "tensor-core scan: a bounded pipeline wait ran out (role %d)", herr);
   for (int64_t i = 0; i < nq; ++i)
     if (hflags[i]) flagged->push_back((int32_t)i);
+  ix->pq_rest.note(nq, count_overflowed(), kPqRestOneIn);
   *handled = true;
   return VSK_OK;
 }

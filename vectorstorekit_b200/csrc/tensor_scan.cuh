@@ -41,6 +41,7 @@ int32_t ivf_tensor_search(Index* ix, const float* q, int64_t nq, const int64_t* 
 // scan's bit for bit.  *handled = false (nothing written): the table scan takes the batch.  Queries whose list
 // overflowed are returned in `flagged` for the table scan.
 constexpr int64_t kPqTensorMinQueries = 64, kPqTensorMinRows = 16384;
+constexpr int kPqRestOneIn = 4;   // rows that tie in bulk: more than one query in so many that overflows
 bool pq_tensor_applicable(const Index* ix, int64_t nq, int32_t k);
 int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const float* tables, float* out_dist,
                          int64_t* out_ids, std::vector<int32_t>* flagged, bool* handled);
