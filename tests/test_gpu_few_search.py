@@ -131,3 +131,41 @@ def test_large_store_reads_the_fp16_copy(vsk, dev, cpu_oracle, large, metric, nq
     assert (after["fallback_queries"] > before["fallback_queries"]) == (nq > 4)    # 1 500 equal rows fill one query's list
     assert_topk_parity(*got, *cpu_oracle.flat_search(METRICS[metric], q[:nq], x, k))
     ix.close()
+
+
+# batches on the list tiles of which a few queries overflow: the last step walks the lists of those alone, by number
+@pytest.mark.parametrize("d,nbad", [(16, 1), (16, 17), (40, 3), (40, 64), (40, 65)])
+def test_overflowed_queries_of_an_inverted_file_batch(vsk, dev, cpu_oracle, d, nbad):
+    rng = np.random.default_rng(d + nbad)
+    n, nlist, nq, k = 120_000, 8, 300, 10
+    centres = 4.0 * rng.standard_normal((nlist, d)).astype(np.float32)
+    x = (centres[rng.integers(0, nlist, n)] + rng.standard_normal((n, d))).astype(np.float32)
+    x[60_000:66_000] = centres[0] + 0.3                           # 6 000 equal rows
+    q = (centres[rng.integers(1, nlist, nq)] + rng.standard_normal((nq, d))).astype(np.float32)
+    hit = rng.choice(nq, nbad, replace=False)
+    q[hit] = centres[0] + 0.3 + 1e-3 * rng.standard_normal((nbad, d)).astype(np.float32)
+    ivf = vsk.IVFIndex(dev, d, nlist, 2, maxIterations=4, tolerance=-1.0)
+    ivf.train(x[:20_000], centres.copy())
+    ivf.insert(x)
+    before = dev.stats()
+    got = ivf.batchSearch(q, k)
+    after = dev.stats()
+    assert after["tensor_tiles"] > before["tensor_tiles"]
+    # (the list tiles, which take more than 64 of them, overflow once more and count it)
+    again = after["fallback_queries"] - before["fallback_queries"]
+    assert again == nbad if nbad <= 64 else again >= nbad
+    assert_topk_parity(*got, *cpu_oracle.ivf_search(q, x, ivf.centroids, ivf.assignments(), 2, k))
+    ivf.close()
+
+
+def test_probes_of_short_rows_take_one_launch(vsk, dev, cpu_oracle):
+    """Up to sixteen queries over rows of at most 32 dimensions: the probe selection, and the walk of re-run queries, have no
+    reason to keep to the chunked schedule (the lists themselves do, and count what overflows there)."""
+    rng = np.random.default_rng(9)
+    x = rng.standard_normal((30_000, 24)).astype(np.float32)
+    ivf = vsk.IVFIndex(dev, 24, 64, 64, maxIterations=2)
+    ivf.train(x[:4_096], x[:64])
+    ivf.insert(x)
+    for nq in (3, 8, 16):
+        q = rng.standard_normal((nq, 24)).astype(np.float32)
+        assert_topk_parity(*ivf.batchSearch(q, 20), *cpu_oracle.flat_search(oracle.EUCLIDEAN, q, x, 20))

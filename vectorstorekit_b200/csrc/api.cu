@@ -570,7 +570,7 @@ static int32_t flat_search_dev(Index* ix, const float* q, int64_t nq, int32_t k,
       f.final_sqrt = ix->metric == VSK_METRIC_EUCLIDEAN;
       f.out_dist = out_dist + b * k;
       f.out_ids = out_ids + b * k;
-      if (few_search_applies(ctx, f)) {
+      if (!few_keeps_schedule(bn, ix->dim) && few_search_applies(ctx, f)) {
         bool handled = false;
         if (tensor_metric && !mb && ix->n * ix->dim > kFewMaxElems) VSK_TRY(few_search_half(ix, f, &handled));
         else VSK_TRY(few_search(ctx, f));

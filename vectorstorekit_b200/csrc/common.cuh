@@ -406,6 +406,11 @@ struct FewArgs {
   int64_t nan_rows;           // set by few_search
 };
 bool few_search_applies(const Ctx* ctx, const FewArgs& a);
+// A flat or inverted-file search of three or more queries over rows this short keeps to the chunked schedule, whose overflow
+// count (vsk_stats.fallback_queries) is part of what its callers see.  It is not the faster one: three queries over 40 000 x 32
+// take it 104 us, over 40 000 x 36 one launch takes 46.  Steps inside a search (probe selection, the walk of re-run queries)
+// have no such count and take the one launch.
+inline bool few_keeps_schedule(int64_t nq, int32_t dim) { return nq > 2 && dim <= 32; }
 int32_t few_search(Ctx* ctx, const FewArgs& a);
 // ... over the fp16 operand copy of a flat index, re-scored against the fp32 rows (drains the stream).  *handled = false:
 // the batch does not fit this form.

@@ -590,10 +590,6 @@ size_t few_smem(const FewArgs& a) {
   b = std::max<size_t>(b, FEW_MAX_CTAS * sizeof(unsigned short));   // the merge's list numbers go here
   return (size_t)NQ * FEW_LIST * 8 + b;
 }
-// Three or more queries over rows this short keep to the chunked schedule, whose overflow count (vsk_stats.fallback_queries)
-// is part of what callers see there.  It is not the faster one: three queries over 40 000 x 32 take it 104 us, over 40 000 x
-// 36 one launch takes 46.
-constexpr int kFewShortRow = 32;
 constexpr size_t kFewMaxSmem = 110 * 1024;   // two CTAs per SM
 
 template <int METRIC, int NQ, bool VEC, bool SEG>
@@ -722,7 +718,6 @@ int32_t few_search_half(Index* ix, const FewArgs& a, bool* handled) {
 bool few_search_applies(const Ctx* ctx, const FewArgs& a) {
   // (the fp32 search path is the chunked schedule by definition)
   if (ctx->search_path != VSK_PATH_TENSOR_RERANK || !ctx->tuning.stream_scan || a.k < 1 || a.k > kFewMaxK || a.nq < 1 || a.dim < 1) return false;
-  if (a.nq > 2 && a.dim <= kFewShortRow) return false;
   if (a.probes) return a.metric == VSK_METRIC_EUCLIDEAN && a.nq <= kStreamScanMaxSegQueries && few_smem<1>(a) <= kFewMaxSmem;
   if (a.nq > kStreamScanMaxQueries) return false;
   return (a.nq <= 1 ? few_smem<1>(a) : a.nq <= 2 ? few_smem<2>(a) : a.nq <= 4 ? few_smem<4>(a) : few_smem<8>(a)) <= kFewMaxSmem;

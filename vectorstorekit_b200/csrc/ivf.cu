@@ -768,7 +768,7 @@ int32_t ivf_search_dev(Index* ix, const float* q, int64_t nq, int32_t k, int32_t
     if (bn <= kStreamScanMaxSegQueries) {
       // the probed lists, walked on the device query by query; longer probe lists or results: the chunked schedule
       const FewArgs f = few_lists(bn);
-      if (few_search_applies(ctx, f)) {
+      if (!few_keeps_schedule(bn, ix->dim) && few_search_applies(ctx, f)) {
         VSK_TRY(few_search(ctx, f));
         continue;
       }
