@@ -166,3 +166,30 @@ def test_entries_of_nearly_equal_size(vsk, dev, cpu_oracle):
     rd, ri = cpu_oracle.pq_search(q, codes, cb, 10)
     assert np.array_equal(ids, ri) and np.array_equal(dist, rd)
     assert dev.stats()["fallback_queries"] == before
+
+
+# segment lengths with the short form; codebooks of a size that fills no warp; rows far from the origin, rows far from every
+# codeword, rows at equal distances from two codewords, and rows that are not finite
+@pytest.mark.parametrize("ds,ksub", [(4, 256), (8, 256), (16, 256), (8, 33), (16, 2)])
+@pytest.mark.parametrize("offset", [0.0, 10.0, 1e4])
+def test_encoding_equals_the_exact_sums(vsk, dev, cpu_oracle, ds, ksub, offset):
+    rng = np.random.default_rng(ds + ksub)
+    m, n = 3, 5_003
+    x = (rng.standard_normal((n, m * ds)) + offset * rng.standard_normal(m * ds)).astype(np.float32)
+    cb = np.ascontiguousarray(np.stack([x[rng.choice(n, ksub, replace=False)][:, s * ds:(s + 1) * ds] for s in range(m)]))
+    cb[:, ksub - 1] = cb[:, 0]                                    # equal codewords: the lower code
+    x[11] *= 1e3
+    x[12] *= 1e18                                                 # squares that overflow
+    x[13, 1], x[14, 2] = np.nan, np.inf
+    x[15] = 0.5 * (np.concatenate(list(cb[:, 0])) + np.concatenate(list(cb[:, 1])))
+    assert np.array_equal(_encode(dev, cb, x), cpu_oracle.pq_encode(x, cb))
+
+
+def _encode(dev, cb, x):
+    """vsk_pq_encode with a codebook size that need not be a power of two."""
+    import ctypes as C
+    m, ksub, ds = cb.shape
+    codes = np.empty((x.shape[0], m), np.uint8)
+    dev.check(dev._lib.vsk_pq_encode(dev._h, cb.ctypes.data_as(C.c_void_p), m * ds, m, ksub, x.ctypes.data_as(C.c_void_p),
+                                     x.shape[0], codes.ctypes.data_as(C.c_void_p)))
+    return codes

@@ -90,21 +90,65 @@ __global__ void __launch_bounds__(PQ_THREADS) pq_encode_kernel(const float* __re
   codes[r * m + s] = (uint8_t)bc;
 }
 
+// The code of one (row, segment) by the exact sums, over codewords first, first + step, ...: smallest value, lowest code.
+template <int DS>
+__device__ __forceinline__ void pq_exact_code(const float* __restrict__ seg, const float* __restrict__ cb, int ksub, int first, int step,
+                                              bool wide, float& low, int& code) {
+  __align__(16) float x[DS];
+#pragma unroll
+  for (int i = 0; i < DS; ++i) x[i] = __ldg(seg + i);
+  low = CUDART_INF_F;
+  code = 0;
+#pragma unroll 1
+  for (int c = first; c < ksub; c += step) {
+    __align__(16) float w[DS];
+    if (wide) {
+#pragma unroll
+      for (int i = 0; i < DS; i += 4) *reinterpret_cast<float4*>(&w[i]) = __ldg(reinterpret_cast<const float4*>(cb + c * DS + i));
+    } else {
+#pragma unroll
+      for (int i = 0; i < DS; ++i) w[i] = __ldg(cb + c * DS + i);
+    }
+    float d = 0.f;
+#pragma unroll
+    for (int i = 0; i < DS; ++i) d = sqdiff_accum(d, x[i], w[i]);
+    if (d < low) { low = d; code = c; }
+  }
+}
+
 // The same codes for the usual segment lengths at half the instructions.  The exact sum costs three per dimension (its
 // operations are rounded one by one), the form |c|^2 - 2 x.c one; the exact sums decide only where the two smallest values
-// of that form lie closer together than both forms' roundings:
-//   |v + |x|^2 - D| <= E = 2 (DS + 4) 2^-24 (|x| + |c|)^2,   v: the short form, D: the exact sum as the encoder forms it.
-// The code rides in the value's eight low mantissa bits (2^-15 of it, added to the band).  A thread takes two rows, so that a
-// codeword read from shared memory (a broadcast) serves both.  1 million x 128, 16 segments of 256 codewords: 3.96 ms for
-// the kernel above.
+// of that form lie closer together than both forms' roundings.  Rows and codewords are taken relative to the segment's mean
+// codeword there, so that the roundings follow the spread of the data and not its distance from the origin:
+//   |v + |x|^2 - D| <= E = (3 DS + 8) 2^-24 (|x| + |c|)^2,   v: the short form, D: the exact sum as the encoder forms it
+// (2 DS of it the short form's, DS + 2 the exact sum's, 2 from rounding x and c to the mean).  The code rides in the value's
+// eight low mantissa bits (2^-15 of it, added to the band).  A thread takes two rows, so that a codeword read from shared
+// memory (a broadcast) serves both.  The few undecided (row, segment) pairs of a warp are decided one after the other by the
+// whole warp, a codeword per lane: left to their threads, one of them cost the warp all 256 codewords.
+// 1 million x 128, 16 segments of 256 codewords: 3.96 ms for the kernel above, 2.33 here; with a mean of ten standard
+// deviations in every dimension too (6.00 with the origin as the reference point and undecided pairs left to their threads).
+constexpr int kPqOpenOwn = 16;   // more undecided pairs than this in a warp: every thread its own (256 steps, against 8 and an exchange per pair)
 template <int DS>
 __global__ void __launch_bounds__(256) pq_encode_fast_kernel(const float* __restrict__ x, int64_t n, int dim, int m, int ksub,
                                                              const float* __restrict__ cb, uint8_t* __restrict__ codes) {
-  extern __shared__ __align__(16) float cbs[];   // [ksub][DS], then [ksub] squared norms
-  __shared__ float s_top[8];
+  extern __shared__ __align__(16) float cbs[];   // [ksub][DS] less the mean, then [ksub] squared norms
+  __shared__ float s_top[8], s_mean[DS];
   float* norms = cbs + ksub * DS;
-  const int s = blockIdx.y;
-  for (int i = threadIdx.x; i < ksub * DS; i += blockDim.x) cbs[i] = cb[(int64_t)s * ksub * DS + i];
+  const int s = blockIdx.y, lane = threadIdx.x & 31;
+  const float* cb_seg = cb + (int64_t)s * ksub * DS;
+  for (int i = threadIdx.x; i < ksub * DS; i += blockDim.x) cbs[i] = cb_seg[i];
+  if (threadIdx.x < DS) s_mean[threadIdx.x] = 0.f;
+  __syncthreads();
+  {
+    // (the order of the sum varies; any reference point gives the same codes)
+    float t = 0.f;
+    for (int i = threadIdx.x; i < ksub * DS; i += blockDim.x) t += cbs[i];   // 256 is a multiple of DS: one dimension per thread
+#pragma unroll
+    for (int o = 16; o >= DS; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane < DS) atomicAdd(&s_mean[lane], t / (float)ksub);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < ksub * DS; i += blockDim.x) cbs[i] -= s_mean[i % DS];
   __syncthreads();
   float top = 0.f;
   for (int c = threadIdx.x; c < ksub; c += blockDim.x) {
@@ -116,7 +160,7 @@ __global__ void __launch_bounds__(256) pq_encode_fast_kernel(const float* __rest
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-  if ((threadIdx.x & 31) == 0) s_top[threadIdx.x >> 5] = top;
+  if (lane == 0) s_top[threadIdx.x >> 5] = top;
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < 8; ++w) top = fmaxf(top, s_top[w]);
@@ -124,6 +168,7 @@ __global__ void __launch_bounds__(256) pq_encode_fast_kernel(const float* __rest
   constexpr int R = 2;
   const int64_t r0 = (int64_t)blockIdx.x * (blockDim.x * R) + threadIdx.x;
   const bool wide = (dim & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  const bool cb_wide = (reinterpret_cast<uintptr_t>(cb) & 15) == 0;
   __align__(16) float v[R][DS];
   float best[R], second[R];
 #pragma unroll
@@ -138,7 +183,7 @@ __global__ void __launch_bounds__(256) pq_encode_fast_kernel(const float* __rest
       for (int i = 0; i < DS; ++i) v[r][i] = __ldg(seg + i);
     }
 #pragma unroll
-    for (int i = 0; i < DS; ++i) v[r][i] *= -2.0f;
+    for (int i = 0; i < DS; ++i) v[r][i] = (v[r][i] - s_mean[i]) * -2.0f;
     best[r] = CUDART_INF_F;
     second[r] = CUDART_INF_F;
   }
@@ -161,26 +206,33 @@ __global__ void __launch_bounds__(256) pq_encode_fast_kernel(const float* __rest
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int64_t row = r0 + (int64_t)r * blockDim.x;
-    if (row >= n) continue;
     float x2 = 0.f;
 #pragma unroll
     for (int i = 0; i < DS; ++i) x2 = fmaf(v[r][i], v[r][i], x2);
     const float a = 0.5f * sqrtf(x2) * 1.00001f + cmax;
     // twice both bounds; the packed bits move either value by 2^-15 of its size, |v| <= (|x| + |c|)^2
-    const float band = (4.0f * (float)(DS + 4) * 5.9604645e-8f + 6.2e-5f) * a * a + 1e-37f;
+    const float band = (2.0f * (float)(3 * DS + 8) * 5.9604645e-8f + 6.2e-5f) * a * a + 1e-37f;
     int bc = (int)(__float_as_uint(best[r]) & 0xffu);
-    if (!(second[r] - best[r] > band)) {   // (also whatever is not a number)
-      float low = CUDART_INF_F;
-      bc = 0;
-#pragma unroll 1
-      for (int c = 0; c < ksub; ++c) {
-        float d = 0.f;
-#pragma unroll
-        for (int i = 0; i < DS; ++i) d = sqdiff_accum(d, __ldg(x + row * dim + (int64_t)s * DS + i), cbs[c * DS + i]);
-        if (d < low) { low = d; bc = c; }
-      }
+    const bool open = row < n && !(second[r] - best[r] > band);   // (also whatever is not a number)
+    unsigned todo = __ballot_sync(0xffffffffu, open);
+    float low;
+    if (__popc(todo) > kPqOpenOwn) {
+      if (open) pq_exact_code<DS>(x + row * dim + (int64_t)s * DS, cb_seg, ksub, 0, 1, cb_wide, low, bc);
+      todo = 0u;
     }
-    codes[row * m + s] = (uint8_t)bc;
+    for (; todo; todo &= todo - 1u) {
+      const int src = __ffs((int)todo) - 1;
+      int code;
+      pq_exact_code<DS>(x + (row - lane + src) * dim + (int64_t)s * DS, cb_seg, ksub, lane, 32, cb_wide, low, code);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float l2 = __shfl_xor_sync(0xffffffffu, low, o);
+        const int c2 = __shfl_xor_sync(0xffffffffu, code, o);
+        if (l2 < low || (l2 == low && c2 < code)) { low = l2; code = c2; }
+      }
+      if (lane == src) bc = code;
+    }
+    if (row < n) codes[row * m + s] = (uint8_t)bc;
   }
 }
 
