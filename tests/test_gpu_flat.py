@@ -611,3 +611,20 @@ def test_ring_stage_granularity_does_not_change_results(vsk, cpu_oracle, d):
         ix.close()
     finally:
         dev.close()
+
+
+@pytest.mark.parametrize("n,nq,k", [(18_000, 64, 100), (17_500, 200, 50), (1_100, 64, 24), (296_500, 40, 37), (18_000, 64, 1_000)])
+def test_no_small_last_chunk_in_a_small_batch(vsk, dev, cpu_oracle, n, nq, k):
+    """Row counts whose longest chunks (sixteen times the rows seen) leave a small remainder: its threshold would lie next to the
+    final one, and the certificate of most queries over embeddings of many dimensions would fail."""
+    rng = np.random.default_rng(n + k)
+    d = 768 if n < 100_000 else 320
+    x = rng.standard_normal((n, d), dtype=np.float32)
+    x /= np.linalg.norm(x, axis=1, keepdims=True)
+    q = rng.standard_normal((nq, d), dtype=np.float32)
+    before = dev.stats()["fallback_queries"]
+    ix = _flat(vsk, dev, "cosine", x)
+    got = ix.batchSearch(q, k)
+    ix.close()
+    assert dev.stats()["fallback_queries"] - before <= nq // 20
+    assert_topk_parity(*got, *cpu_oracle.flat_search(oracle.COSINE, q, x, k))

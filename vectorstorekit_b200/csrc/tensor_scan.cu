@@ -2515,12 +2515,7 @@ int32_t tensor_search_begin(Index* ix, const float* q, int64_t nq, int32_t k, co
   VSK_TRY(tensor_prepare(ix));
   const int metric = ix->metric;
   const int dim16 = ix->dim16;
-  // The certificate needs the keep-th coarse value to lie 2 eps above the k-th.  A small batch can afford the longer lists
-  // that make it hold for nearly every query (777 queries, k = 37, 300 000 x 333: 12 - 23 of them were re-run with k + 8,
-  // a third of the call); for a large one the extra hits cost more than the rare re-run, and so they do for a small k
-  // (1 000 queries, k = 10: 204 us with k + 8, 225 with k + 32).
-  const int32_t margin = std::max(8, nq <= 2048 ? k / 2 : k / 8);
-  const int32_t keep = std::min<int32_t>(kCandCap / 2, k + margin);
+  const int32_t keep = std::min<int32_t>(kCandCap / 2, k + std::max(8, k / 8));
   QueryOperands qo;
   VSK_TRY(prepare_query_operands(ix, q, nq, &qo));
   const bool fold = ix->fold16;
@@ -2588,6 +2583,12 @@ int32_t tensor_search_begin(Index* ix, const float* q, int64_t nq, int32_t k, co
     chunk = std::min<int64_t>(chunk, std::max<int64_t>(growth >= 100 ? room : 1024, growth * seen));
     chunk = std::max<int64_t>(TN, chunk / TN * TN);   // whole row tiles
     chunk = std::min(chunk, n - seen);
+    // The certificate compares the k-th value with the threshold of the last chunk, the keep-th value of the rows before it: were
+    // that chunk a small remainder, the two would lie next to each other.  The last two chunks are of one ratio then.
+    // 300 000 x 768, cosine, 1 000 queries, k = 100 (1 024, 16 384, 278 528 and 4 064 rows): 564 queries re-run, 8 290 us,
+    // now none and 690 (lists of 3 k / 2 keys: 710, but 1 million x 128, dot product, 2 000 queries: 1 350 for 1 236).
+    if (const int64_t rest = n - seen - chunk; rest > 0 && 2 * rest < seen + chunk)
+      chunk = std::min(chunk, ceil_div((int64_t)std::sqrt((double)seen * (double)n) - seen, TN) * TN);
     a.row_begin = seen;
     a.row_end = seen + chunk;
     VSK_TRY(launch_tc<SCAN_THRESHOLD>(ctx, mq, mx, a, has_beta));
