@@ -447,7 +447,7 @@ struct SelectArgs {
   const float* cert_eps;    // non-null: last compaction of a coarse scan (see select.cu); uses k
   int32_t max_count;        // > 0: no list of this launch is expected to hold more keys (picks the kernel width)
   int by_length;            // 1: the lists' lengths are only known on the device, most are short (launch_select: a launch per
-                            //   width, each taking the lists of its own lengths); 2, 3: one of those launches
+                            //   width, each taking the lists of its own lengths)
   // Row-sharded search (the two halves of a shard's search, see tensor_scan.cuh):
   float* bound_out;         // non-null: measure only.  Writes the bound_rank-th smallest value of the list plus
   int32_t bound_rank;       //   bound_eps[q] (+inf when the list is shorter) and leaves the list as it is.

@@ -18,7 +18,8 @@ constexpr int SEL_THREADS = 512;   // widest variant: 512 threads x 8 keys = the
 // NT threads handle a list of at most NT * 8 keys.  The host picks NT from an upper bound on the list
 // lengths of the launch (SelectArgs::max_count); a list that is longer all the same is flagged like an
 // overflowed list and its query is re-run.
-template <int NT>
+// SHARE: the launch is one of two over the same lists (SelectArgs::by_length) and takes those of its own lengths.
+template <int NT, bool SHARE = false>
 __global__ void __launch_bounds__(NT, NT == 128 ? 10 : 2) select_kernel(SelectArgs a) {
   extern __shared__ __align__(16) uint64_t s[];
   constexpr int CAPACITY = NT * SEL_ITEMS;
@@ -31,8 +32,8 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 10 : 2) select_kernel(SelectAr
     c = a.dense_count;
   } else {
     const int raw = a.cand.count[q];
-    if (a.by_length == 2 && raw > CAPACITY) return;                  // the wide launch's
-    if (a.by_length == 3 && raw <= 128 * SEL_ITEMS) return;          // the narrow launch has taken it
+    if (SHARE && NT == 128 && raw > CAPACITY) return;                // the wide launch's
+    if (SHARE && NT != 128 && raw <= 128 * SEL_ITEMS) return;        // the narrow launch has taken it
     c = min(raw, CAPACITY);
     if (raw > CAPACITY && threadIdx.x == 0) atomicOr(&a.cand.flags[q], 1);
   }
@@ -367,6 +368,8 @@ int32_t launch_select(Ctx* ctx, const SelectArgs& a) {
   if (!carveout_done) {
     prefer_shared_carveout(select_kernel<128>);
     prefer_shared_carveout(select_kernel<SEL_THREADS>);
+    prefer_shared_carveout(select_kernel<128, true>);
+    prefer_shared_carveout(select_kernel<SEL_THREADS, true>);
     prefer_shared_carveout(init_cand_kernel);
     prefer_shared_carveout(pack_keys_kernel);
     prefer_shared_carveout(unpack_keys_kernel);
@@ -375,11 +378,9 @@ int32_t launch_select(Ctx* ctx, const SelectArgs& a) {
     carveout_done = true;
   }
   if (a.by_length == 1 && !small && a.dense_count < 0 && a.nq >= kSelectByLengthMin) {
-    SelectArgs one = a;
-    one.by_length = 2;   // first: what it shortens is short for the wide launch's test too
-    select_kernel<128><<<(unsigned)a.nq, 128, 0, ctx->stream>>>(one);
-    one.by_length = 3;
-    select_kernel<SEL_THREADS><<<(unsigned)a.nq, SEL_THREADS, 0, ctx->stream>>>(one);
+    // the narrow one first: what it shortens is short for the wide launch's test too
+    select_kernel<128, true><<<(unsigned)a.nq, 128, 0, ctx->stream>>>(a);
+    select_kernel<SEL_THREADS, true><<<(unsigned)a.nq, SEL_THREADS, 0, ctx->stream>>>(a);
     ctx->stats.kernel_launches++;
   } else if (small) {
     const size_t smem = a.out_ids ? 128 * SEL_ITEMS * sizeof(uint64_t) : 0;
