@@ -143,3 +143,12 @@ def test_cpp_host_mirror_compiles_and_refuses_without_gpu(lib, tmp_path):
     out = subprocess.run([exe], capture_output=True, text=True)
     assert out.returncode == 0, out
     assert out.stdout.strip() == ("ok" if torch.cuda.is_available() else "no-device")
+
+
+def test_launch_attributes_are_not_kept_per_process():
+    """A kernel's attributes belong to one device: a flag that lives as long as the process would leave a second device opened
+    in it without them (no second device is at hand to launch on)."""
+    import glob
+    for path in glob.glob(os.path.join(ROOT, "vectorstorekit_b200", "csrc", "*.cu*")):
+        for line in open(path):
+            assert not re.search(r"static bool \w*(attr|carveout)", line), f"{os.path.basename(path)}: {line.strip()}"

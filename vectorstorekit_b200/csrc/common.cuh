@@ -182,6 +182,8 @@ struct Ctx {
   ShardPending pending[2];
   PinnedBuf host_io;         // staging of small host-pointer calls (HostCall)
   PinnedBuf host_flags[2];   // per lane: the flag words a finished half-search hands to the host
+  std::vector<const void*> configured;   // kernels that have their shared memory on this device (opt_in_shared) ...
+  std::vector<const void*> carved;       // ... and first ones of groups with the carve-out (prefer_shared_carveout)
   unsigned* few_tickets[2] = {};   // per lane: the few-query search's tickets (few_search.cu)
   Comm* comm = nullptr;
   Worker* worker = nullptr;
@@ -210,10 +212,25 @@ void tl_mark(Ctx* ctx, const char* name);
 // carve-out, the configuration the contraction kernel runs under: an SM does not switch its L1 / shared-memory split
 // while it holds a CTA, so a kernel that preferred another split could not join the contraction's CTAs on an SM and
 // the two lanes of a context would take turns instead of overlapping.
-template <typename K>
-inline void prefer_shared_carveout(K kernel) {
-  cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+// (once per context: an attribute belongs to the device's copy of the kernel)
+template <typename... K>
+inline void prefer_shared_carveout(Ctx* ctx, K... kernels) {
+  const void* all[] = {(const void*)kernels...};
+  for (const void* k : ctx->carved)
+    if (k == all[0]) return;
+  for (const void* k : all) cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   cudaGetLastError();
+  ctx->carved.push_back(all[0]);
+}
+
+// More than 48 KB of dynamic shared memory for a kernel, always the same number of bytes: once per context.
+template <typename K>
+inline cudaError_t opt_in_shared(Ctx* ctx, K kernel, size_t bytes) {
+  for (const void* k : ctx->configured)
+    if (k == (const void*)kernel) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) ctx->configured.push_back((const void*)kernel);
+  return e;
 }
 
 // Issues on lane `lane` until it goes out of scope.

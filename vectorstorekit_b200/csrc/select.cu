@@ -364,19 +364,8 @@ int32_t launch_select(Ctx* ctx, const SelectArgs& a) {
   // lists known to hold at most 1024 keys take the 128-thread variant (four times as many CTAs per SM);
   // only the final ordering sorts in shared memory
   const bool small = a.max_count > 0 && a.max_count <= 128 * SEL_ITEMS && (a.dense_count < 0 || a.dense_count <= 128 * SEL_ITEMS);
-  static bool carveout_done = false;
-  if (!carveout_done) {
-    prefer_shared_carveout(select_kernel<128>);
-    prefer_shared_carveout(select_kernel<SEL_THREADS>);
-    prefer_shared_carveout(select_kernel<128, true>);
-    prefer_shared_carveout(select_kernel<SEL_THREADS, true>);
-    prefer_shared_carveout(init_cand_kernel);
-    prefer_shared_carveout(pack_keys_kernel);
-    prefer_shared_carveout(unpack_keys_kernel);
-    prefer_shared_carveout(merge_keys_kernel<128>);
-    prefer_shared_carveout(merge_keys_kernel<SEL_THREADS>);
-    carveout_done = true;
-  }
+  prefer_shared_carveout(ctx, select_kernel<128>, select_kernel<SEL_THREADS>, select_kernel<128, true>, select_kernel<SEL_THREADS, true>,
+                         init_cand_kernel, pack_keys_kernel, unpack_keys_kernel, merge_keys_kernel<128>, merge_keys_kernel<SEL_THREADS>);
   if (a.by_length == 1 && !small && a.dense_count < 0 && a.nq >= kSelectByLengthMin) {
     // the narrow one first: what it shortens is short for the wide launch's test too
     select_kernel<128, true><<<(unsigned)a.nq, 128, 0, ctx->stream>>>(a);

@@ -1997,7 +1997,6 @@ int32_t tensor_prepare(Index* ix) {
 // Launches the scan over tiles (persistent: one CTA per SM, or per tile when there are fewer tiles).
 template <int MODE, int EW, bool I8 = false>
 int32_t launch_tc_ew(Ctx* ctx, const CUtensorMap& mq, const CUtensorMap& mx, const TcArgs& a, bool has_beta) {
-  static bool attr_done[2][2] = {};
   const bool has_mask = MODE != SCAN_ARGMIN && a.row_masks != nullptr && a.q_masks != nullptr;
   void (*kern)(CUtensorMap, CUtensorMap, TcArgs);
   if constexpr (I8) {
@@ -2009,10 +2008,7 @@ int32_t launch_tc_ew(Ctx* ctx, const CUtensorMap& mq, const CUtensorMap& mx, con
                     : (has_beta ? tc_scan_kernel<MODE, true, false, EW> : tc_scan_kernel<MODE, false, false, EW>);
   }
   constexpr size_t smem = tc_smem_bytes<EW>();
-  if (!attr_done[has_beta][has_mask]) {
-    VSK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_done[has_beta][has_mask] = true;
-  }
+  VSK_CUDA(ctx, opt_in_shared(ctx, kern, smem));
   const int64_t tiles = a.tiles ? a.num_tiles : ceil_div(a.nq, TM) * ceil_div(a.row_end - a.row_begin, TN);
   if (tiles <= 0) return VSK_OK;
   const int sms = ctx->prop.multiProcessorCount;
@@ -2330,11 +2326,7 @@ __global__ void assign_fill_fold_kernel(__half* __restrict__ rows16, int64_t n, 
 template <int MODE>
 int32_t launch_assign_scan(Ctx* ctx, const CUtensorMap& mx, const CUtensorMap& mc, const CUtensorMap& mxn, const CUtensorMap& mcn,
                            AsArgs a, unsigned* grid_out = nullptr, int64_t* log_cap_out = nullptr) {
-  static bool attr_done = false;
-  if (!attr_done) {
-    VSK_CUDA(ctx, cudaFuncSetAttribute(assign_scan_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAsSmemBytes));
-    attr_done = true;
-  }
+  VSK_CUDA(ctx, opt_in_shared(ctx, assign_scan_kernel<MODE>, kAsSmemBytes));
   const int sms = ctx->prop.multiProcessorCount;
   const int nb = (int)ceil_div(a.k, TN);
   const int64_t qtiles = ceil_div(a.n, TM);
@@ -2387,26 +2379,11 @@ struct QueryOperands {
 int32_t prepare_query_operands(Index* ix, const float* q, int64_t nq, QueryOperands* out) {
   VSK_TRACE("vsk:query_operands");
   Ctx* ctx = ix->ctx;
-  static bool carveout_done = false;
-  if (!carveout_done) {
-    prefer_shared_carveout(absmax_kernel);
-    prefer_shared_carveout(choose_scale_kernel);
-    prefer_shared_carveout(scale_queries_kernel);
-    prefer_shared_carveout(prep_rows_kernel<VSK_METRIC_EUCLIDEAN>);
-    prefer_shared_carveout(prep_rows_kernel<VSK_METRIC_COSINE>);
-    prefer_shared_carveout(prep_rows_kernel<VSK_METRIC_DOT_PRODUCT>);
-    prefer_shared_carveout(bound_kernel<VSK_METRIC_EUCLIDEAN>);
-    prefer_shared_carveout(bound_kernel<VSK_METRIC_COSINE>);
-    prefer_shared_carveout(bound_kernel<VSK_METRIC_DOT_PRODUCT>);
-    prefer_shared_carveout(bound_i8_kernel<VSK_METRIC_EUCLIDEAN>);
-    prefer_shared_carveout(bound_i8_kernel<VSK_METRIC_DOT_PRODUCT>);
-    prefer_shared_carveout(rerank_kernel<VSK_METRIC_EUCLIDEAN>);
-    prefer_shared_carveout(rerank_kernel<VSK_METRIC_COSINE>);
-    prefer_shared_carveout(rerank_kernel<VSK_METRIC_DOT_PRODUCT>);
-    prefer_shared_carveout(rerank_i8_kernel<VSK_METRIC_EUCLIDEAN>);
-    prefer_shared_carveout(rerank_i8_kernel<VSK_METRIC_DOT_PRODUCT>);
-    carveout_done = true;
-  }
+  prefer_shared_carveout(ctx, absmax_kernel, choose_scale_kernel, scale_queries_kernel, prep_rows_kernel<VSK_METRIC_EUCLIDEAN>,
+                         prep_rows_kernel<VSK_METRIC_COSINE>, prep_rows_kernel<VSK_METRIC_DOT_PRODUCT>, bound_kernel<VSK_METRIC_EUCLIDEAN>,
+                         bound_kernel<VSK_METRIC_COSINE>, bound_kernel<VSK_METRIC_DOT_PRODUCT>, bound_i8_kernel<VSK_METRIC_EUCLIDEAN>,
+                         bound_i8_kernel<VSK_METRIC_DOT_PRODUCT>, rerank_kernel<VSK_METRIC_EUCLIDEAN>, rerank_kernel<VSK_METRIC_COSINE>,
+                         rerank_kernel<VSK_METRIC_DOT_PRODUCT>, rerank_i8_kernel<VSK_METRIC_EUCLIDEAN>, rerank_i8_kernel<VSK_METRIC_DOT_PRODUCT>);
   const int metric = ix->metric;
   const int dim = ix->dim, dim16 = ix->dim16;
   void* p;
@@ -3165,11 +3142,7 @@ constexpr int64_t kLsWindowBytes = 40ll << 20;   // rows a window of list_scan_k
 template <bool I8>
 static int32_t launch_list_scan(Ctx* ctx, const CUtensorMap& mx, const CUtensorMap& mq, const CUtensorMap& mxn, const CUtensorMap& mqn,
                                 LsArgs a, int64_t row_bytes) {
-  static bool attr_done = false;
-  if (!attr_done) {
-    VSK_CUDA(ctx, cudaFuncSetAttribute(list_scan_kernel<I8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLsSmemBytes));
-    attr_done = true;
-  }
+  VSK_CUDA(ctx, opt_in_shared(ctx, list_scan_kernel<I8>, kLsSmemBytes));
   const int64_t tiles = ceil_div(a.nq, TN) * ceil_div(a.rows, TM);
   if (tiles <= 0) return VSK_OK;
   a.window = (int32_t)std::max<int64_t>(1, kLsWindowBytes / (row_bytes * TM));
