@@ -16,7 +16,8 @@ CHECKED = os.environ.get("VSK_CHECKED", "0") not in ("", "0")
 
 SUITES = ["tests/test_gpu_checked.py", "tests/test_gpu_odd_shapes.py", "tests/test_gpu_flat.py",
           "tests/test_gpu_stream_scan.py", "tests/test_gpu_filters.py", "tests/test_gpu_ivf_sq8.py",
-          "tests/test_gpu_pq.py", "tests/test_gpu_image.py", "tests/test_gpu_store.py"]
+          "tests/test_gpu_pq.py", "tests/test_gpu_image.py", "tests/test_gpu_store.py", "tests/test_gpu_few_search.py",
+          "tests/test_gpu_l1_scan.py", "tests/test_gpu_i8_scan.py", "tests/test_gpu_pq_tensor.py"]
 
 
 @pytest.mark.skipif(CHECKED, reason="this is the child process")

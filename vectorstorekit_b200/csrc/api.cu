@@ -69,6 +69,7 @@ int32_t pinned_reserve(Ctx* ctx, PinnedBuf* b, size_t bytes) {
   // the old buffer may still be the target of a copy in flight
   VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream_main));
   VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream_aux));
+  chk_remove(b->p);
   if (b->p) cudaFreeHost(b->p);
   b->p = nullptr;
   b->bytes = 0;
@@ -79,6 +80,7 @@ int32_t pinned_reserve(Ctx* ctx, PinnedBuf* b, size_t bytes) {
     return fail(ctx, VSK_ERR_OUT_OF_MEMORY, "pinned host memory: %zu bytes not available", want);
   }
   b->bytes = want;
+  chk_add(b->p, want);   // kernels write a staged call's results there
   return VSK_OK;
 }
 
@@ -773,7 +775,11 @@ int32_t vsk_close(vsk_ctx* c) {
   for (auto& p : ctx->scratch) dev_free(p);
   for (auto& p : ctx->few_tickets) dev_free(p);
   for (auto& b : ctx->host_flags)
-    if (b.p) cudaFreeHost(b.p);
+    if (b.p) {
+      chk_remove(b.p);
+      cudaFreeHost(b.p);
+    }
+  chk_remove(ctx->host_io.p);
   if (ctx->host_io.p) cudaFreeHost(ctx->host_io.p);
   for (auto& e : ctx->prof_events) cudaEventDestroy(e);
   for (auto& m : ctx->marks) cudaEventDestroy(m.ev);

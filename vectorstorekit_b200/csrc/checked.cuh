@@ -1,8 +1,10 @@
 // Device side of the CHECKED build (-DVSK_CHECKED): the range test of the kernels' global accesses.
 //
 // Works at source level: in a checked build the names __ldg and atomicAdd / Min / Max / Or / CAS stand for the templates
-// below, which pass the address through vsk_chk_access first, and VSK_CHK(p) does the same for a plain load or store
-// (it is p itself in a normal build).  The function and the pointer to the range table are `static`: every module
+// below, which pass the address through vsk_chk_access first, and VSK_CHK(p) / VSK_CHK_W(p) do the same for a plain load /
+// store (they are p itself in a normal build): `*VSK_CHK_W(out + i) = v;`.  The kernels of the few-query search, the Manhattan byte
+// filter, the row lists, the int8 and product-quantised paths carry them at every global access but TMA's, whose tensor maps
+// bound it.  Older kernels are tested at their read-only loads and atomics.  The function and the pointer to the range table are `static`: every module
 // carries its own copy (the library is built without relocatable device code), and every module registers a setter
 // with the host side (checked.cu) so that vsk_open can hand all of them the same table.
 #pragma once
@@ -104,6 +106,8 @@ static __device__ __forceinline__ T atomic_cas(T* p, C c, V v) {
 #define atomicOr(...) ::vsk::chk::atomic_or(__VA_ARGS__)
 #define atomicCAS(...) ::vsk::chk::atomic_cas(__VA_ARGS__)
 #define VSK_CHK(p) (::vsk::chk::at(p))
+#define VSK_CHK_W(p) (::vsk::chk::at(p, 0x100u))
 #else
 #define VSK_CHK(p) (p)
+#define VSK_CHK_W(p) (p)
 #endif  // VSK_CHECKED

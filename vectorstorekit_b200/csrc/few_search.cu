@@ -64,6 +64,46 @@ __device__ __forceinline__ uint64_t few_compact(uint64_t* list, int cnt, int k, 
   return pivot;
 }
 
+// After a round of rows: lists that a further round could overfill are shortened to their `keep` smallest keys and tighten their
+// query's threshold; after the last round every list is.
+__device__ __forceinline__ void few_end_round(uint64_t* lists, int nq, int keep, bool last, int* s_cnt, uint64_t* s_thr, FewScratch& s) {
+  __syncthreads();
+#pragma unroll 1
+  for (int i = 0; i < nq; ++i) {
+    const int cnt = s_cnt[i];
+    if (cnt > (last ? keep : FEW_LIST - FEW_ROUND)) {
+      const uint64_t pivot = few_compact(lists + (size_t)i * FEW_LIST, cnt, keep, s);
+      if (threadIdx.x == 0) {
+        s_cnt[i] = s.out;
+        s_thr[i] = pivot;
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// Writes this CTA's lists of queries [pos, pos + nq) with their lengths and smallest keys.
+__device__ __forceinline__ void few_write_lists(const FewKernelArgs& ka, const uint64_t* lists, int pos, int nq, int keep, const int* s_cnt) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int i = 0; i < nq; ++i) {
+    const int64_t l = (int64_t)(pos + i) * gridDim.x + blockIdx.x;
+    const uint64_t* list = lists + (size_t)i * FEW_LIST;
+    const int cnt = s_cnt[i];
+    for (int j = threadIdx.x; j < cnt; j += FEW_THREADS) *VSK_CHK_W(ka.part + l * keep + j) = list[j];
+    if (warp == 0) {
+      uint64_t best = kEmptyKey;
+      for (int j = lane; j < cnt; j += 32) best = min(best, list[j]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
+      if (lane == 0) {
+        *VSK_CHK_W(ka.part_min + l) = best;
+        *VSK_CHK_W(ka.part_n + l) = cnt;
+      }
+    }
+  }
+}
+
 // Merges the lists of the launch's query `pos` and writes the result of query `out`.  `list` has room for FEW_LIST keys, `cand` for FEW_MAX_CTAS list numbers.
 __device__ __forceinline__ void few_merge(const FewKernelArgs& ka, int64_t pos, int64_t out, int lists, uint64_t* list, unsigned short* cand,
                                           FewScratch& s) {
@@ -78,7 +118,7 @@ __device__ __forceinline__ void few_merge(const FewKernelArgs& ka, int64_t pos, 
 #pragma unroll
   for (int i = 0; i < SEL_ITEMS; ++i) {
     const int at = threadIdx.x + i * FEW_THREADS;
-    key[i] = at < lists ? __ldcg(mins + at) : kEmptyKey;
+    key[i] = at < lists ? __ldcg(VSK_CHK(mins + at)) : kEmptyKey;
     have += key[i] != kEmptyKey;
   }
   if (have) atomicAdd(&n_have, have);
@@ -96,9 +136,9 @@ __device__ __forceinline__ void few_merge(const FewKernelArgs& ka, int64_t pos, 
   for (int c0 = 0; c0 < nc; c0 += batch) {
     for (int c = c0 + warp; c < min(nc, c0 + batch); c += FEW_WARPS) {
       const int64_t l = pos * lists + cand[c];
-      const int n = __ldcg(ka.part_n + l);
+      const int n = __ldcg(VSK_CHK(ka.part_n + l));
       for (int i = lane; i < n; i += 32) {
-        const uint64_t v = __ldcg(ka.part + l * k + i);
+        const uint64_t v = __ldcg(VSK_CHK(ka.part + l * k + i));
         if (v <= bound) list[atomicAdd(&n_list, 1)] = v;
       }
     }
@@ -124,8 +164,8 @@ __device__ __forceinline__ void few_merge(const FewKernelArgs& ka, int64_t pos, 
       if (a.final_sqrt) d = sqrtf(d);
       id = (int64_t)(uint32_t)list[j] + a.id_base;
     }
-    a.out_dist[out * k + j] = d;
-    a.out_ids[out * k + j] = id;
+    *VSK_CHK_W(a.out_dist + out * k + j) = d;
+    *VSK_CHK_W(a.out_ids + out * k + j) = id;
   }
 }
 
@@ -147,13 +187,13 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(F
   const int dim = a.dim, k = a.k;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int qp = SEG ? (int)blockIdx.y : 0;                         // position in this launch
-  const int qb = (SEG && a.q_subset) ? a.q_subset[qp] : qp;         // first query of this CTA
+  const int qb = (SEG && a.q_subset) ? *VSK_CHK(a.q_subset + qp) : qp;         // first query of this CTA
   const int nq_here = SEG ? 1 : (int)a.nq;
-  for (int i = threadIdx.x; i < NQ * dim; i += FEW_THREADS) sq[i] = i < nq_here * dim ? a.q[(int64_t)qb * dim + i] : 0.f;
+  for (int i = threadIdx.x; i < NQ * dim; i += FEW_THREADS) sq[i] = i < nq_here * dim ? *VSK_CHK(a.q + (int64_t)qb * dim + i) : 0.f;
   if (threadIdx.x < NQ) {
     s_thr[threadIdx.x] = kEmptyKey - 1;
     s_cnt[threadIdx.x] = 0;
-    s_qm[threadIdx.x] = (int)threadIdx.x < nq_here ? (a.q_masks ? a.q_masks[qb + threadIdx.x] : ~0ull) : 0ull;
+    s_qm[threadIdx.x] = (int)threadIdx.x < nq_here ? (a.q_masks ? *VSK_CHK(a.q_masks + qb + threadIdx.x) : ~0ull) : 0ull;
   }
   if (SEG && warp == 0) {
     // first position of every probed list (an out-of-range probe is an empty list)
@@ -162,10 +202,10 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(F
       const int p = p0 + lane;
       int64_t beg = 0, len = 0;
       if (p < a.nprobe) {
-        const int64_t l = a.probes[(int64_t)qb * a.nprobe + p];
+        const int64_t l = *VSK_CHK(a.probes + (int64_t)qb * a.nprobe + p);
         if (l >= 0 && l < a.nlist) {
-          beg = a.list_offsets[l];
-          len = a.list_offsets[l + 1] - beg;
+          beg = *VSK_CHK(a.list_offsets + l);
+          len = *VSK_CHK(a.list_offsets + l + 1) - beg;
         }
       }
       int64_t incl = len;
@@ -250,39 +290,10 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(F
         }
       }
     }
-    __syncthreads();
-    const bool last = r0 + stride >= n;
-#pragma unroll 1
-    for (int i = 0; i < nq_here; ++i) {
-      const int cnt = s_cnt[i];
-      if (cnt > (last ? k : FEW_LIST - FEW_ROUND)) {
-        const uint64_t pivot = few_compact(lists + (size_t)i * FEW_LIST, cnt, k, fs);
-        if (threadIdx.x == 0) {
-          s_cnt[i] = fs.out;
-          s_thr[i] = pivot;
-        }
-      }
-    }
-    __syncthreads();
+    few_end_round(lists, nq_here, k, r0 + stride >= n, s_cnt, s_thr, fs);
   }
   // ---- this CTA's lists, and the merge by the last one to arrive ----
-#pragma unroll 1
-  for (int i = 0; i < nq_here; ++i) {
-    const int64_t l = (int64_t)(qp + i) * gridDim.x + blockIdx.x;
-    const uint64_t* list = lists + (size_t)i * FEW_LIST;
-    const int cnt = s_cnt[i];
-    for (int j = threadIdx.x; j < cnt; j += FEW_THREADS) ka.part[l * k + j] = list[j];
-    if (warp == 0) {
-      uint64_t best = kEmptyKey;
-      for (int j = lane; j < cnt; j += 32) best = min(best, list[j]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-      if (lane == 0) {
-        ka.part_min[l] = best;
-        ka.part_n[l] = cnt;
-      }
-    }
-  }
+  few_write_lists(ka, lists, qp, nq_here, k, s_cnt);
   if (NQ > 1) return;   // several queries: few_merge_kernel merges them side by side
   __threadfence();
   __syncthreads();
@@ -290,7 +301,7 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(F
   __syncthreads();
   if (s_last != gridDim.x - 1) return;
   __threadfence();
-  if (threadIdx.x == 0) ka.ticket[qp] = 0u;
+  if (threadIdx.x == 0) *VSK_CHK_W(ka.ticket + qp) = 0u;
   // the query's staging area is free now: list numbers go there (the launch makes it large enough)
   few_merge(ka, qp, qb, (int)gridDim.x, lists, reinterpret_cast<unsigned short*>(smem + (size_t)NQ * FEW_LIST * 8), fs);
 }
@@ -411,38 +422,9 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_coarse_kernel
         }
       }
     }
-    __syncthreads();
-    const bool last = r0 + stride >= n;
-#pragma unroll 1
-    for (int i = 0; i < nq; ++i) {
-      const int cnt = s_cnt[i];
-      if (cnt > (last ? keep : FEW_LIST - FEW_ROUND)) {
-        const uint64_t pivot = few_compact(lists + (size_t)i * FEW_LIST, cnt, keep, fs);
-        if (threadIdx.x == 0) {
-          s_cnt[i] = fs.out;
-          s_thr[i] = pivot;
-        }
-      }
-    }
-    __syncthreads();
+    few_end_round(lists, nq, keep, r0 + stride >= n, s_cnt, s_thr, fs);
   }
-#pragma unroll 1
-  for (int i = 0; i < nq; ++i) {
-    const int64_t l = (int64_t)i * gridDim.x + blockIdx.x;
-    const uint64_t* list = lists + (size_t)i * FEW_LIST;
-    const int cnt = s_cnt[i];
-    for (int j = threadIdx.x; j < cnt; j += FEW_THREADS) ka.part[l * keep + j] = list[j];
-    if (warp == 0) {
-      uint64_t best = kEmptyKey;
-      for (int j = lane; j < cnt; j += 32) best = min(best, list[j]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-      if (lane == 0) {
-        ka.part_min[l] = best;
-        ka.part_n[l] = cnt;
-      }
-    }
-  }
+  few_write_lists(ka, lists, 0, nq, keep, s_cnt);
 }
 
 // One CTA per query: the rows within 2 eps of the k-th best coarse value, re-scored with the direct formulas and ordered.
@@ -473,7 +455,7 @@ __global__ void __launch_bounds__(FEW_THREADS) few_refine_kernel(FewKernelArgs k
 #pragma unroll
   for (int i = 0; i < SEL_ITEMS; ++i) {
     const int at = threadIdx.x + i * FEW_THREADS;
-    key[i] = at < lists ? __ldcg(ka.part_min + pos * lists + at) : kEmptyKey;
+    key[i] = at < lists ? __ldcg(VSK_CHK(ka.part_min + pos * lists + at)) : kEmptyKey;
     have += key[i] != kEmptyKey;
   }
   if (have) atomicAdd(&n_have, have);
@@ -492,10 +474,10 @@ __global__ void __launch_bounds__(FEW_THREADS) few_refine_kernel(FewKernelArgs k
   const int nc = n_cand;
   for (int c = warp; c < nc; c += FEW_WARPS) {
     const int64_t l = pos * lists + cand[c];
-    const int m = __ldcg(ka.part_n + l);
+    const int m = __ldcg(VSK_CHK(ka.part_n + l));
     bool all = m >= keep;   // a shortened list whose every key is within the bound may have dropped such a row
     for (int i = lane; i < m; i += 32) {
-      const uint64_t v = __ldcg(ka.part + l * keep + i);
+      const uint64_t v = __ldcg(VSK_CHK(ka.part + l * keep + i));
       if (v <= bound) {
         const int at = atomicAdd(&n_list, 1);
         if (at < FEW_LIST) list[at] = v;
@@ -508,7 +490,7 @@ __global__ void __launch_bounds__(FEW_THREADS) few_refine_kernel(FewKernelArgs k
   __syncthreads();
   int cnt = n_list;
   if (cnt > FEW_LIST || s_bad != 0 || !(band < CUDART_INF_F)) {
-    if (threadIdx.x == 0) h.flags[pos] = 1;
+    if (threadIdx.x == 0) *VSK_CHK_W(h.flags + pos) = 1;
     return;
   }
   if (cnt > k) {   // the k-th best of all, then only what is within the band of it
@@ -570,10 +552,10 @@ __global__ void __launch_bounds__(FEW_THREADS) few_refine_kernel(FewKernelArgs k
       if (METRIC == VSK_METRIC_EUCLIDEAN) d = sqrtf(d);
       id = (int64_t)(uint32_t)list[j] + a.id_base;
     }
-    a.out_dist[pos * k + j] = d;
-    a.out_ids[pos * k + j] = id;
+    *VSK_CHK_W(a.out_dist + pos * k + j) = d;
+    *VSK_CHK_W(a.out_ids + pos * k + j) = id;
   }
-  if (threadIdx.x == 0) h.flags[pos] = 0;
+  if (threadIdx.x == 0) *VSK_CHK_W(h.flags + pos) = 0;
 }
 
 __global__ void __launch_bounds__(FEW_THREADS) few_merge_kernel(FewKernelArgs ka, int lists) {

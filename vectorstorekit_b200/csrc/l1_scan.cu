@@ -50,7 +50,7 @@ __device__ __forceinline__ void sad4(uint32_t& acc, uint32_t a, uint32_t b) {
   asm("vabsdiff4.u32.u32.u32.add %0, %1, %2, %0;" : "+r"(acc) : "r"(a), "r"(b));
 }
 __device__ __forceinline__ void cp16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(VSK_CHK(reinterpret_cast<const uint4*>(src))) : "memory");
 }
 
 template <int BM> struct L1Tile {
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(L1_THREADS, 2) l1_scan_kernel(L1Args a) {
       const int32_t row = s_row[at];
       if (a.row_masks && (__ldg(a.row_masks + row) & qm) == 0ull) continue;
       const int pos = atomicAdd(&a.cand.count[m], 1);
-      if (pos < kCandCap) a.cand.keys[m * kCandCap + pos] = make_key(0.f, (uint32_t)row);
+      if (pos < kCandCap) *VSK_CHK_W(a.cand.keys + m * kCandCap + pos) = make_key(0.f, (uint32_t)row);
     }
   }
 }
@@ -167,13 +167,13 @@ __global__ void __launch_bounds__(L1_RS_THREADS) l1_rescore_kernel(const float* 
                                                                    unsigned long long* total) {
   extern __shared__ __align__(16) float qs[];
   const int64_t pos = blockIdx.x, qi = q_subset ? (int64_t)__ldg(q_subset + pos) : pos;
-  const int cnt = min(cand.count[pos], kCandCap);
+  const int cnt = min(*VSK_CHK(cand.count + pos), kCandCap);
   uint64_t* keys = cand.keys + pos * kCandCap;
   for (int i = threadIdx.x; i < dim; i += L1_RS_THREADS) qs[i] = __ldg(q + qi * dim + i);
   __syncthreads();
   int formed = 0;
   for (int c = blockIdx.y * L1_RS_THREADS + threadIdx.x; c < cnt; c += gridDim.y * L1_RS_THREADS) {
-    const uint64_t key = keys[c];
+    const uint64_t key = *VSK_CHK(keys + c);
     if ((uint32_t)(key >> 32) != 0x80000000u) continue;
     const float* p = x + (int64_t)(uint32_t)key * dim;
     float s = 0.f;
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(L1_RS_THREADS) l1_rescore_kernel(const float* 
       for (int u = 0; u < 16; ++u) s += fabsf(qs[d + u] - v[u]);
     }
     for (; d < dim; ++d) s += fabsf(qs[d] - __ldg(p + d));
-    keys[c] = make_key(s, (uint32_t)key);
+    *VSK_CHK_W(keys + c) = make_key(s, (uint32_t)key);
     ++formed;
   }
   // rows formed by this CTA, one atomic per CTA (the query is done with, its first word takes the sum: with a static word beside
@@ -211,14 +211,14 @@ __global__ void l1_bar_kernel(const float* __restrict__ thr, const float* __rest
                               int32_t* __restrict__ bar, int32_t* __restrict__ flags) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nq) return;
-  if (!(eq[i] < CUDART_INF_F)) {
+  if (!(*VSK_CHK(eq + i) < CUDART_INF_F)) {
     atomicOr(&flags[i], kFlagDegenerate);
-    bar[i] = -1;
+    *VSK_CHK_W(bar + i) = -1;
     return;
   }
-  const double t = thr[i];
+  const double t = *VSK_CHK(thr + i);
   const double at = (t * (1.0 + 1.2e-7 * (dim + 8)) + (double)eq[i] + (double)ex) / (double)step + 1.0;
-  bar[i] = at < 2147483000.0 ? (int32_t)at : INT_MAX;   // (also for what is not a number: every row is listed)
+  *VSK_CHK_W(bar + i) = at < 2147483000.0 ? (int32_t)at : INT_MAX;   // (also for what is not a number: every row is listed)
 }
 
 // lowest and highest value of every dimension
@@ -264,7 +264,7 @@ __global__ void l1_bytes_kernel(const float* __restrict__ x, int64_t n, int dim,
           word |= (uint32_t)u << (8 * b);
         }
       }
-      reinterpret_cast<uint32_t*>(out + row * stride)[w] = word;
+      *VSK_CHK_W(reinterpret_cast<uint32_t*>(out + row * stride) + w) = word;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -272,7 +272,7 @@ __global__ void l1_bytes_kernel(const float* __restrict__ x, int64_t n, int dim,
       big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
     }
     e = e * (1.0f + 1e-5f) + 2.4e-7f * (float)dim * (big + mag);
-    if (err && lane == 0) err[row] = e;
+    if (err && lane == 0) *VSK_CHK_W(err + row) = e;
     if (isnan(e) || e > worst) worst = e;   // what is not a number stays: nothing compares greater than it
   }
   if (err_max && lane == 0) atomicMax(err_max, __float_as_uint(fabsf(worst)));

@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256) pq_encode_fast_kernel(const float* __rest
   float* norms = cbs + ksub * DS;
   const int s = blockIdx.y, lane = threadIdx.x & 31;
   const float* cb_seg = cb + (int64_t)s * ksub * DS;
-  for (int i = threadIdx.x; i < ksub * DS; i += blockDim.x) cbs[i] = cb_seg[i];
+  for (int i = threadIdx.x; i < ksub * DS; i += blockDim.x) cbs[i] = *VSK_CHK(cb_seg + i);
   if (threadIdx.x < DS) s_mean[threadIdx.x] = 0.f;
   __syncthreads();
   {
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(256) pq_encode_fast_kernel(const float* __rest
       }
       if (lane == src) bc = code;
     }
-    if (row < n) codes[row * m + s] = (uint8_t)bc;
+    if (row < n) *VSK_CHK_W(codes + row * m + s) = (uint8_t)bc;
   }
 }
 

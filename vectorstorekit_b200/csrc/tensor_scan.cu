@@ -1341,10 +1341,10 @@ list_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             const int64_t q = first + j;
             const int at = atomicAdd(&sm->log_n, 1);
             if (at < a.log_cap) {
-              my_log[at] = make_uint2(id, (uint32_t)q);
+              *VSK_CHK_W(my_log + at) = make_uint2(id, (uint32_t)q);
             } else {
               const int slot = atomicAdd(&a.cand.count[q], 1);
-              if (slot < kCandCap) a.cand.keys[q * kCandCap + slot] = make_key(0.f, id);
+              if (slot < kCandCap) *VSK_CHK_W(a.cand.keys + q * kCandCap + slot) = make_key(0.f, id);
             }
           }
         };
@@ -1373,7 +1373,7 @@ list_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   // ---------------- teardown ----------------
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0) a.log_count[blockIdx.x] = (int32_t)min((int64_t)sm->log_n, a.log_cap);
+  if (threadIdx.x == 0) *VSK_CHK_W(a.log_count + blockIdx.x) = (int32_t)min((int64_t)sm->log_n, a.log_cap);
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
@@ -1383,12 +1383,12 @@ list_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 // The logs of the CTAs (blockIdx.y) to the candidate lists; a key's value is formed by the re-scoring.
 __global__ void __launch_bounds__(256) ls_scatter_kernel(const uint2* __restrict__ log, const int32_t* __restrict__ log_count, int64_t log_cap,
                                                          CandLists cand) {
-  const int cnt = log_count[blockIdx.y];
+  const int cnt = *VSK_CHK(log_count + blockIdx.y);
   const uint2* mine = log + (int64_t)blockIdx.y * log_cap;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < cnt; e += gridDim.x * blockDim.x) {
-    const uint2 h = mine[e];
+    const uint2 h = *VSK_CHK(mine + e);
     const int slot = atomicAdd(&cand.count[h.y], 1);
-    if (slot < kCandCap) cand.keys[(int64_t)h.y * kCandCap + slot] = make_key(0.f, h.x);
+    if (slot < kCandCap) *VSK_CHK_W(cand.keys + (int64_t)h.y * kCandCap + slot) = make_key(0.f, h.x);
   }
 }
 
@@ -2915,7 +2915,7 @@ __global__ void ivf_coarse_threshold_kernel(const float* __restrict__ thr_exact,
     const float qn2 = qnorm[i] * qnorm[i];
     tc = (t - qn2) + eps[i] + 2e-6f * (qn2 + max_xnorm * max_xnorm + t);
   }
-  thr_coarse[i] = tc;
+  *VSK_CHK_W(thr_coarse + i) = tc;
   if (dropped && dropped[i] <= tc) atomicOr(&flags[i], 2);
 }
 
@@ -3174,7 +3174,7 @@ __global__ void ls_fold_queries_kernel(const float* __restrict__ thr, int64_t nq
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nq_pad) return;
   const float s = *scale_q, u = i < nq ? ldexpf(s, -fold_exp) : 0.f;
-  float R = i < nq ? -0.5f * thr[i] * s * scale_x : 1e9f;   // the bar
+  float R = i < nq ? -0.5f * *VSK_CHK(thr + i) * s * scale_x : 1e9f;   // the bar
   R = R - fabsf(R) * ((float)dim16 * 2.3841858e-7f + 1e-6f) - 1e-30f;
   constexpr float kTop = 2.0f * kLsBarConst * 60000.f;
   if (!(R >= -kTop)) {                                 // (also what is not a number)
@@ -3192,8 +3192,8 @@ __global__ void ls_fold_queries_kernel(const float* __restrict__ thr, int64_t nq
   for (int j = 0; j < 16; ++j)
     h[j] = j < 8 ? __float2half_rn(j < 4 ? 8.0f * u : 4.0f * u) : j < 10 ? p0 : j < 12 ? p1 : p2;
   uint4* dst = reinterpret_cast<uint4*>(q16 + i * dim16 + col0);
-  dst[0] = *reinterpret_cast<const uint4*>(&h[0]);
-  dst[1] = *reinterpret_cast<const uint4*>(&h[8]);
+  *VSK_CHK_W(dst) = *reinterpret_cast<const uint4*>(&h[0]);
+  *VSK_CHK_W(dst + 1) = *reinterpret_cast<const uint4*>(&h[8]);
 }
 
 // The same for int8 operands: 32 bytes b per query with 127 sum(b) >= -bar, the bar rounded down to a step of 127.
@@ -3201,7 +3201,7 @@ __global__ void ls_bar_bytes_kernel(const int32_t* __restrict__ bar, int64_t nq,
                                     int32_t* __restrict__ flags) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nq_pad) return;
-  const int64_t want = i < nq ? -(int64_t)bar[i] : -100000;
+  const int64_t want = i < nq ? -(int64_t)*VSK_CHK(bar + i) : -100000;
   int64_t total = want >= 0 ? (want + kLsBarByte - 1) / kLsBarByte : -((-want) / kLsBarByte);   // rounded up
   if (total > 32 * 127) {   // more rows would have to be listed than the bytes can ask for
     total = 32 * 127;
@@ -3214,8 +3214,8 @@ __global__ void ls_bar_bytes_kernel(const int32_t* __restrict__ bar, int64_t nq,
 #pragma unroll
   for (int j = 0; j < 32; ++j) h[j] = (int8_t)(base + (j < rest ? 1 : 0));
   uint4* dst = reinterpret_cast<uint4*>(out + i * 32);
-  dst[0] = *reinterpret_cast<const uint4*>(&h[0]);
-  dst[1] = *reinterpret_cast<const uint4*>(&h[16]);
+  *VSK_CHK_W(dst) = *reinterpret_cast<const uint4*>(&h[0]);
+  *VSK_CHK_W(dst + 1) = *reinterpret_cast<const uint4*>(&h[16]);
 }
 
 // ---- product-quantised rows on the tensor cores -------------------------------------------------------------
@@ -3257,7 +3257,7 @@ __global__ void __launch_bounds__(256) pq_decode16_kernel(const uint8_t* __restr
     s += __shfl_xor_sync(0xffffffffu, s, 2);
     if (part == 0 && r < rows) {
       n2[r] = s;
-      if (aux) aux[r0 + r] = s;
+      if (aux) *VSK_CHK_W(aux + r0 + r) = s;
     }
   }
   __syncthreads();
@@ -3287,7 +3287,7 @@ __global__ void __launch_bounds__(256) pq_decode16_kernel(const uint8_t* __restr
         if constexpr (W == 8) *reinterpret_cast<uint4*>(&h[j]) = __ldg(reinterpret_cast<const uint4*>(w));
         else if constexpr (W == 4) *reinterpret_cast<uint2*>(&h[j]) = __ldg(reinterpret_cast<const uint2*>(w));
         else if constexpr (W == 2) *reinterpret_cast<uint32_t*>(&h[j]) = __ldg(reinterpret_cast<const uint32_t*>(w));
-        else h[j] = *w;
+        else h[j] = *VSK_CHK(w);
       }
     } else {
 #pragma unroll
@@ -3295,12 +3295,12 @@ __global__ void __launch_bounds__(256) pq_decode16_kernel(const uint8_t* __restr
         __half v = __float2half_rn(0.f);
         if (c + j < dim) {
           const int g = (c + j) / ds;
-          v = cb16[((int64_t)g * ksub + sc[r * m + g]) * ds + ((c + j) - g * ds)];
+          v = *VSK_CHK(cb16 + ((int64_t)g * ksub + sc[r * m + g]) * ds + ((c + j) - g * ds));
         }
         h[j] = v;
       }
     }
-    *reinterpret_cast<uint4*>(out + (r0 + r) * dim16 + c) = *reinterpret_cast<const uint4*>(h);
+    *VSK_CHK_W(reinterpret_cast<uint4*>(out + (r0 + r) * dim16 + c)) = *reinterpret_cast<const uint4*>(h);
   }
 }
 
@@ -3312,14 +3312,14 @@ __global__ void pq_coarse_threshold_kernel(const float* __restrict__ thr_exact, 
                                            float* __restrict__ thr_coarse, int32_t* __restrict__ flags) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nq) return;
-  const float t = thr_exact[i];
+  const float t = *VSK_CHK(thr_exact + i);
   float tc = CUDART_INF_F;
   if (!(t < CUDART_INF_F)) atomicOr(&flags[i], kFlagDegenerate);   // (the first rows gave it k values: it is not finite)
   if (!(t == CUDART_INF_F)) {
-    const float t2 = t * t, qn2 = qnorm[i] * qnorm[i];
-    tc = (t2 - qn2) + eps[i] + 1.2e-7f * (sum_terms * t2 + norm_terms * qn2);
+    const float qn = *VSK_CHK(qnorm + i), t2 = t * t, qn2 = qn * qn;
+    tc = (t2 - qn2) + *VSK_CHK(eps + i) + 1.2e-7f * (sum_terms * t2 + norm_terms * qn2);
   }
-  thr_coarse[i] = tc;
+  *VSK_CHK_W(thr_coarse + i) = tc;
 }
 
 // Entries [kept, count) of a query's list are rows of the decoded block (numbered from its first row): their coarse
@@ -3329,17 +3329,17 @@ __global__ void __launch_bounds__(128) pq_rescore_kernel(const float* __restrict
                                                          int ksub, int64_t row0, int kept, CandLists cand,
                                                          unsigned long long* total) {
   const int64_t qi = blockIdx.x;
-  const int cnt = min(cand.count[qi], kCandCap);
+  const int cnt = min(*VSK_CHK(cand.count + qi), kCandCap);
   uint64_t* keys = cand.keys + qi * kCandCap;
   const float* tab = tables + qi * m * ksub;
   if (threadIdx.x == 0 && cnt > kept) atomicAdd(total, (unsigned long long)(cnt - kept));
   for (int c = kept + threadIdx.x; c < cnt; c += blockDim.x) {
-    const int64_t row = row0 + (int64_t)(uint32_t)keys[c];
+    const int64_t row = row0 + (int64_t)(uint32_t)*VSK_CHK(keys + c);
     const uint8_t* src = codes + row * m;
     float s = 0.f;
 #pragma unroll 4
     for (int g = 0; g < m; ++g) s = __fadd_rn(s, __ldg(tab + (int64_t)g * ksub + __ldg(src + g)));
-    keys[c] = make_key(__fsqrt_rn(s), (uint32_t)row);
+    *VSK_CHK_W(keys + c) = make_key(__fsqrt_rn(s), (uint32_t)row);
   }
 }
 
@@ -3632,7 +3632,7 @@ __global__ void i8_query_kernel(const float* __restrict__ q, int64_t nq, int dim
       const float e = fmaf((float)c, -amax * (1.0f / 127.0f), t);
       e2 = fmaf(e, e, e2);
     }
-    out[row * stride + i] = (int8_t)c;
+    *VSK_CHK_W(out + row * stride + i) = (int8_t)c;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) e2 += __shfl_xor_sync(0xffffffffu, e2, o);
@@ -3646,9 +3646,9 @@ __global__ void i8_query_kernel(const float* __restrict__ q, int64_t nq, int dim
     r.slack = (sqrtf(e2) * 1.0001f + 1e-6f * tn) * max_code_norm + 1.2e-7f * (float)(dim + 8) * qn * max_xnorm;
     if (!usable) {
       r.slack = -CUDART_INF_F;
-      flags[row] = kFlagDegenerate;   // (the flags have just been cleared)
+      *VSK_CHK_W(flags + row) = kFlagDegenerate;   // (the flags have just been cleared)
     }
-    info[row] = r;
+    *VSK_CHK_W(info + row) = r;
   }
 }
 
@@ -3657,10 +3657,10 @@ __global__ void i8_bar_kernel(const float* __restrict__ thr_exact, const I8Query
                               int32_t* __restrict__ bar) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nq) return;
-  const I8Query r = info[i];
-  const double at = floor((double)r.inv_step * (r.offset - (double)thr_exact[i] - (double)r.slack)) - 1.0;
+  const I8Query r = *VSK_CHK(info + i);
+  const double at = floor((double)r.inv_step * (r.offset - (double)*VSK_CHK(thr_exact + i) - (double)r.slack)) - 1.0;
   // not a number or below every accumulator: every row is listed (and the list overflows)
-  bar[i] = r.slack == -CUDART_INF_F ? INT_MAX : !(at > -2147483647.0) ? INT_MIN : at > 2147483646.0 ? INT_MAX : (int32_t)at;
+  *VSK_CHK_W(bar + i) = r.slack == -CUDART_INF_F ? INT_MAX : !(at > -2147483647.0) ? INT_MIN : at > 2147483646.0 ? INT_MAX : (int32_t)at;
 }
 
 // Largest norm of a code row and of its decoded row (the stored codes themselves are the operand).
@@ -3697,7 +3697,7 @@ __global__ void i8_pad_rows_kernel(const int8_t* __restrict__ codes, int64_t n, 
   if (i >= n * stride) return;
   const int64_t r = i / stride;
   const int c = (int)(i - r * stride);
-  out[i] = c < dim ? __ldg(codes + r * dim + c) : (int8_t)0;
+  *VSK_CHK_W(out + i) = c < dim ? __ldg(codes + r * dim + c) : (int8_t)0;
 }
 
 // Once per index state: the norms of the error bound, and a copy with rows padded to 16 bytes (TMA strides) where the
