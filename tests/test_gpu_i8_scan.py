@@ -134,3 +134,22 @@ def test_small_batches_that_overflow_rest_together(vsk, dev, cpu_oracle):
         rests.append("list_scan" not in names)
         assert_topk_parity(*got, *cpu_oracle.sq8_search(oracle.DOT, q, codes, scale, offset, 20))
     assert not rests[0] and all(rests[4:])
+
+
+def test_a_bounded_wait_of_the_row_lists_runs_out(vsk, cpu_oracle):
+    """One CTA's first row tile is never filled: its waits give up after 2^16 polls, the kernel returns, the call answers Timeout
+    and the context stays usable."""
+    dev = vsk.CUDAAcceleratorStrategy(0).initialize()
+    try:
+        rng = np.random.default_rng(41)
+        ix, codes, scale, offset = _quantised(vsk, dev, rng.standard_normal((40_000, 128)).astype(np.float32))
+        q = rng.standard_normal((300, 128)).astype(np.float32)
+        dev.set_tuning(wait_limit_log2=16, test_stall_scan=1)
+        with pytest.raises(vsk.Timeout):
+            ix.batchSearch(q, 10)
+        assert dev.tuning()["test_stall_scan"] == 0          # one shot, taken by this kernel
+        dev.set_tuning(wait_limit_log2=0)
+        _check(cpu_oracle, ix, codes, scale, offset, q, 10)
+        ix.close()
+    finally:
+        dev.close()

@@ -193,3 +193,23 @@ def _encode(dev, cb, x):
     dev.check(dev._lib.vsk_pq_encode(dev._h, cb.ctypes.data_as(C.c_void_p), m * ds, m, ksub, x.ctypes.data_as(C.c_void_p),
                                      x.shape[0], codes.ctypes.data_as(C.c_void_p)))
     return codes
+
+
+def test_a_bounded_wait_of_the_row_lists_runs_out(vsk, cpu_oracle):
+    dev = vsk.CUDAAcceleratorStrategy(0).initialize()
+    try:
+        rng = np.random.default_rng(42)
+        q, cb, x = _clustered(rng, 40_000, 100, 16, 256, 8)
+        codes = cpu_oracle.pq_encode(x, cb)
+        ix = _index(vsk, dev, cb, codes)
+        dev.set_tuning(wait_limit_log2=16, test_stall_scan=1)
+        with pytest.raises(vsk.Timeout):
+            ix.batchSearch(q, 10)
+        assert dev.tuning()["test_stall_scan"] == 0
+        dev.set_tuning(wait_limit_log2=0)
+        dist, ids = ix.batchSearch(q, 10)
+        rd, ri = cpu_oracle.pq_search(q, codes, cb, 10)
+        assert np.array_equal(ids, ri) and np.array_equal(dist, rd)
+        ix.close()
+    finally:
+        dev.close()

@@ -1075,6 +1075,7 @@ struct LsArgs {
   CandLists cand;
   int32_t* err;
   uint32_t wait_limit;
+  int32_t stall;              // testing only: CTA 0 never fills its first row tile (see TcArgs::stall_kblock)
 };
 
 // Bytes of the resident block and of a row tile; false when two whole-tile stages do not fit beside the block.
@@ -1180,7 +1181,7 @@ list_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     if (lane == 0) {
       int s = 0;
       uint32_t ph = 0, qph = 0, issued = 0, issued_ph = 0, q_last = 0;
-      bool ok = true, q_issued = false;
+      bool ok = true, q_issued = false, stall = a.stall != 0 && blockIdx.x == 0;
       LsWalk w;
       w.start(ntiles, nb, a.window);
       int b, count;
@@ -1198,11 +1199,15 @@ list_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         for (int i = 0; i < count; ++i, ++t) {
           if (!mbar_wait(&sm->empty[s], ph ^ 1, &sm->abort_flag, a.err, 1, wait_limit)) { ok = false; break; }
           uint8_t* st = ring + s * l.tile_bytes;
-          mbar_expect_tx(&sm->full[s], (uint32_t)l.tile_bytes);
-          for (int kb = 0; kb < l.nfull; ++kb) tma_load_2d(st + kb * A_BYTES, &map_x, &sm->full[s], kb * KCOLS, (int32_t)(t * TM));
-          if (l.narrow) tma_load_2d(st + l.nfull * A_BYTES, &map_xn, &sm->full[s], l.nfull * KCOLS, (int32_t)(t * TM));
-          issued |= 1u << s;
-          issued_ph = (issued_ph & ~(1u << s)) | (ph << s);
+          if (stall) {
+            stall = false;   // this stage is never filled, the consumer's bounded wait for it runs out
+          } else {
+            mbar_expect_tx(&sm->full[s], (uint32_t)l.tile_bytes);
+            for (int kb = 0; kb < l.nfull; ++kb) tma_load_2d(st + kb * A_BYTES, &map_x, &sm->full[s], kb * KCOLS, (int32_t)(t * TM));
+            if (l.narrow) tma_load_2d(st + l.nfull * A_BYTES, &map_xn, &sm->full[s], l.nfull * KCOLS, (int32_t)(t * TM));
+            issued |= 1u << s;
+            issued_ph = (issued_ph & ~(1u << s)) | (ph << s);
+          }
           if (++s == l.stages) { s = 0; ph ^= 1; }
         }
       }
@@ -3147,6 +3152,10 @@ static int32_t launch_list_scan(Ctx* ctx, const CUtensorMap& mx, const CUtensorM
   if (tiles <= 0) return VSK_OK;
   a.window = (int32_t)std::max<int64_t>(1, kLsWindowBytes / (row_bytes * TM));
   a.wait_limit = ctx->tuning.wait_limit_log2 > 0 ? (1u << std::min(ctx->tuning.wait_limit_log2, 30)) : 0u;
+  if (ctx->tuning.test_stall_scan > 0) {   // testing only, one shot
+    a.stall = 1;
+    ctx->tuning.test_stall_scan = 0;
+  }
   const unsigned grid = (unsigned)std::min<int64_t>(tiles, ctx->prop.multiProcessorCount);
   // room for 256 rows per query (a chunk lists a few times k); what does not fit is appended by the scan itself
   const int64_t total = std::max<int64_t>(1 << 16, std::min<int64_t>(a.nq * 256, 8 << 20));
