@@ -247,9 +247,13 @@ class Bench:
         self.index.add(self.rows, self.masks)
         self.index.set_id_base(self.lo)
         if wl["metric"] == "manhattan":
-            # FP32 lane-instructions of the eligible pairs: 2 per pair-dimension (subtract; add |.|)
-            self.flops = 2.0 * self.nq * (self.hi - self.lo) * 0.5 * wl["dim"]
-            self.bound = "fp32"
+            pairs = self.nq * (self.hi - self.lo) * 0.5 * wl["dim"]
+            if self.path == "tensor" and self.nq >= 32:
+                # the byte filter: one vabsdiff4 lane-instruction per four dimensions of an eligible pair
+                self.flops, self.bound = 0.25 * pairs, "sad"
+            else:
+                # FP32 lane-instructions of the eligible pairs: 2 per pair-dimension (subtract; add |.|)
+                self.flops, self.bound = 2.0 * pairs, "fp32"
         else:
             # the contraction forms every pair and the filter sits in its epilogue: all pairs are counted, as for the
             # unfiltered workload the step time is compared with
@@ -359,7 +363,7 @@ class Bench:
         self.sq = sq
         self.rows = None
         self.flops = 2.0 * self.nq * n * wl["dim"]
-        self.bound = "tensor"
+        self.bound = "tensor_i8" if wl["metric"] == "dotProduct" and self.path == "tensor" else "tensor"
 
     def _build_pq(self):
         wl, t = self.wl, self.torch
@@ -387,10 +391,13 @@ class Bench:
         n = self.hi - self.lo
         self.extra = {"segments": wl["segments"], "codebook_size": 1 << wl["code_bits"], "train_s": t1 - t0,
                       "encode_rows_per_s": n / (t2 - t1), "code_bytes": n * wl["segments"]}
-        # one table look-up (a 4-byte word of shared memory) and one add per (query, row, segment)
-        self.flops = 1.0 * self.nq * n * wl["segments"]
         self.bytes_per_query = float(n * wl["segments"])
-        self.bound = "smem"
+        if self.path == "tensor" and self.nq >= 64:
+            # the contraction of decoded rows, sixteen columns for the row term and the thresholds
+            self.flops, self.bound = 2.0 * self.nq * n * (wl["dim"] + 16), "tensor"
+        else:
+            # one table look-up (a 4-byte word of shared memory) and one add per (query, row, segment)
+            self.flops, self.bound = 1.0 * self.nq * n * wl["segments"], "smem"
 
     # ---- steps ----
     def local_search(self, queries, k):
@@ -733,9 +740,11 @@ def main():
             "kernel_ms_per_step": scan_ms / prof_steps, "kernel_launches_per_step": scan_n / prof_steps, "traffic": None,
             "timed_steps": prof_steps}
     secs = scan_ms * 1e-3 * args.steps / prof_steps     # the formulas below are written per `args.steps` steps
-    if b.bound == "tensor":
-        roof.update(unit="TFLOP/s", achieved=b.flops * args.steps / secs / 1e12 if secs > 0 else None,
-                    peak=pk["bf16_tflops"], peak_source=pk["source"] + " (cuBLAS bf16, sustained)")
+    if b.bound in ("tensor", "tensor_i8"):
+        i8 = b.bound == "tensor_i8"
+        roof.update(unit="TOP/s" if i8 else "TFLOP/s", achieved=b.flops * args.steps / secs / 1e12 if secs > 0 else None,
+                    peak=pk["bf16_tflops"] * (2 if i8 else 1),
+                    peak_source=pk["source"] + (" (twice cuBLAS bf16, sustained: the int8 rate)" if i8 else " (cuBLAS bf16, sustained)"))
         if wl["kind"] == "ivf":
             # second view: a contraction this short (two or three K blocks) is paced by reading its accumulators out
             # of tensor memory, 4 bytes per (query, row) pair, against the measured tcgen05.ld rate
@@ -762,6 +771,13 @@ def main():
                     algorithmic_codes_gbs=b.bytes_per_query * nq * args.steps / secs / 1e9 if secs > 0 else None,
                     note="one 4-byte table word per (query, row, segment); query-major code bytes are given for "
                          "the HBM view: a query tile re-reads the codes from L2")
+    elif b.bound == "sad":
+        sm = dev.info()["sm_count"]
+        roof.update(unit="T lane-instr/s", achieved=b.flops * args.steps / secs / 1e12 if secs > 0 else None,
+                    peak=dev.measure_peak("fp32_issue") / 2e12,
+                    peak_source="half the FP32 issue rate measured in this run (vabsdiff4 with accumulate: 226 dimensions per clock "
+                                "and SM of 256)",
+                    nominal_peak=sm * 64 * 1.965e9 / 1e12)
     else:
         sm = dev.info()["sm_count"]
         roof.update(unit="T lane-instr/s", achieved=b.flops * args.steps / secs / 1e12 if secs > 0 else None,
@@ -798,7 +814,8 @@ def main():
         "unit": "queries/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": elapsed_ms / args.steps, "wall_ms_per_step": float(wall_t.item()) / args.steps,
         "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
-        "dtype": ("f16 operands, f32 accumulate, f32 rerank" if args.path == "tensor" and b.bound == "tensor" else "f32"),
+        "dtype": {"tensor": "f16 operands, f32 accumulate, f32 rerank", "tensor_i8": "i8 operands, i32 accumulate, f32 rerank",
+                  "sad": "u8 filter, f32 rerank"}.get(b.bound if args.path == "tensor" else "", "f32"),
         "data": "synthetic",
         "config": config_of(wl, world, args.path),
         "workload_detail": b.extra,
