@@ -3178,6 +3178,9 @@ static int32_t launch_list_scan(Ctx* ctx, const CUtensorMap& mx, const CUtensorM
 // Fold columns of the query operand for list_scan_kernel, once per chunk: the row term's constants (8u x4, 4u x4) and the
 // pieces of minus the bar.  A row is listed iff  acc = s_q s_x (q.x - |x|^2 / 2)  reaches  bar = -thr s_q s_x / 2, lowered by
 // the fp32 accumulation error of its own products.  A bar the columns cannot hold from below flags the query.
+// The columns hold |bar| <= kTop = 3.9e9.  With X the bound on the rows' norms, s_q s_x X^2 / 2 is below 2^30 (fold_exp and the
+// query scale, choose_scale_kernel), and so is |bar| / (2 |q| / X + 1): only queries of more than 1.3 X can come near kTop.  A bar above
+// it is clipped, which lists more rows.
 __global__ void ls_fold_queries_kernel(const float* __restrict__ thr, int64_t nq, int64_t nq_pad, const float* scale_q, float scale_x, int fold_exp,
                                        int dim16, int col0, __half* __restrict__ q16, int32_t* __restrict__ flags) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -3206,6 +3209,9 @@ __global__ void ls_fold_queries_kernel(const float* __restrict__ thr, int64_t nq
 }
 
 // The same for int8 operands: 32 bytes b per query with 127 sum(b) >= -bar, the bar rounded down to a step of 127.
+// The bytes hold bars from -516 128 to 520 192; accumulators reach 127 x 127 x 384 = 6.2e6.  Codes and queries
+// that are not far from centred stay within (N(0,1) data, 384 dimensions: 1e5); where the k-th product lies beyond, the clipped
+// bar lists rows that cannot matter, lists may overflow, and the index rests from this path (Index::i8_rest).
 __global__ void ls_bar_bytes_kernel(const int32_t* __restrict__ bar, int64_t nq, int64_t nq_pad, int8_t* __restrict__ out,
                                     int32_t* __restrict__ flags) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -3595,7 +3601,8 @@ int32_t pq_tensor_search(Index* ix, const float* q, int64_t nq, int32_t k, const
 // which compares the k-th value with one a few keys further down, so the thresholds are exact instead (every listed row
 // is re-scored after each chunk), as in the list scan: a row is listed iff  A = sum_i q8_i c_i  reaches
 //   s (K - T - |e| C - rounding),   T the k-th exact value so far.
-// 10 000 queries x 6.25 million rows x 384, k = 10: 40.6 ms on the fp16 path, 27.8 ms here.
+// 10 000 queries x 6.25 million rows x 384, k = 10: 40.6 ms on the fp16 path, 20.0 here (27.8 on the general kernel, which rows of
+// more than three K blocks take).
 struct I8Query {
   float inv_step;    // s: q8 = round(s q~)
   float slack;       // |e| C plus the fp32 roundings of the exact values, in true units
