@@ -34,3 +34,13 @@ def assert_topk_parity(got_d, got_i, ref_d, ref_i, id_tie_rtol=ID_TIE_RTOL, dist
         bad += 0 if ok else 1
     assert bad == 0, f"{bad} id mismatches not explained by ties"
     return int(mism.sum())
+
+
+def logged_launches(dev, call):
+    """(what the call returned, the names of the launches it logged)"""
+    dev.timeline(True)
+    dev.timeline_read()
+    got = call()
+    names = [what for _, what, _ in dev.timeline_read()]
+    dev.timeline(False)
+    return got, names

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import oracle
-from parity import assert_topk_parity
+from parity import assert_topk_parity, logged_launches
 
 pytestmark = pytest.mark.gpu
 
@@ -73,16 +73,6 @@ def test_lists_that_overflow_go_to_the_other_paths(vsk, dev, cpu_oracle):
     assert_topk_parity(d_[keep], i_[keep], rd, ri)
 
 
-def _marks(dev, call):
-    """(what the call returned, the names of the launches it logged)"""
-    dev.timeline(True)
-    dev.timeline_read()
-    got = call()
-    names = [what for _, what, _ in dev.timeline_read()]
-    dev.timeline(False)
-    return got, names
-
-
 # resident query block (up to three K blocks) and the general kernel beyond it; the integer path answers by itself
 @pytest.mark.parametrize("shape", [(20_000, 64, 100, 10), (20_000, 384, 300, 10), (17_000, 513, 70, 10), (16_385, 129, 1, 10)])
 def test_the_integer_contraction_answers_ordinary_batches(vsk, dev, cpu_oracle, shape):
@@ -91,7 +81,7 @@ def test_the_integer_contraction_answers_ordinary_batches(vsk, dev, cpu_oracle, 
     ix, codes, scale, offset = _quantised(vsk, dev, rng.standard_normal((n, d)).astype(np.float32))
     q = rng.standard_normal((nq, d)).astype(np.float32)
     before = dev.stats()["fallback_queries"]
-    (got, names) = _marks(dev, lambda: ix.batchSearch(q, k))
+    (got, names) = logged_launches(dev, lambda: ix.batchSearch(q, k))
     assert "query_operands" not in names                          # (the fp16 path's first launch)
     assert ("list_scan" in names) == (d <= 384) and ("scan" in names) == (d > 384)
     assert dev.stats()["fallback_queries"] == before
@@ -110,12 +100,12 @@ def test_a_few_degenerate_queries_decide_for_themselves_only(vsk, dev, cpu_oracl
     bad[60, 1], bad[61, 2] = np.nan, np.inf
     keep = [i for i in range(100) if i not in (3, 50, 60, 61)]
     before = dev.stats()["fallback_queries"]
-    (d_, i_), names = _marks(dev, lambda: ix.batchSearch(bad, 10))
+    (d_, i_), names = logged_launches(dev, lambda: ix.batchSearch(bad, 10))
     assert "list_scan" in names and "query_operands" not in names
     assert 4 <= dev.stats()["fallback_queries"] - before < 50     # (a zero query ties again in its re-run, which counts too)
     assert_topk_parity(d_[keep], i_[keep], rd[keep], ri[keep])
     assert np.all(d_[[3, 50]] == 0.0) and i_[3].tolist() == i_[50].tolist() == list(range(10))
-    got, names = _marks(dev, lambda: ix.batchSearch(q, 10))
+    got, names = logged_launches(dev, lambda: ix.batchSearch(q, 10))
     assert "list_scan" in names and "query_operands" not in names
     assert_topk_parity(*got, rd, ri)
 
@@ -130,7 +120,7 @@ def test_small_batches_that_overflow_rest_together(vsk, dev, cpu_oracle):
     rests = []
     for r in range(8):
         q = (base + 0.1 * rng.standard_normal((40, d))).astype(np.float32)
-        got, names = _marks(dev, lambda: ix.batchSearch(q, 20))
+        got, names = logged_launches(dev, lambda: ix.batchSearch(q, 20))
         rests.append("list_scan" not in names)
         assert_topk_parity(*got, *cpu_oracle.sq8_search(oracle.DOT, q, codes, scale, offset, 20))
     assert not rests[0] and all(rests[4:])

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import oracle
-from parity import assert_topk_parity
+from parity import assert_topk_parity, logged_launches
 
 pytestmark = pytest.mark.gpu
 
@@ -113,16 +113,6 @@ def test_a_row_that_is_not_a_number_among_many(vsk, dev, cpu_oracle):
     assert np.array_equal(plain[1], ref_plain[1]) and np.array_equal(plain[0], ref_plain[0])
 
 
-def _marks(dev, call):
-    """(what the call returned, the names of the launches it logged)"""
-    dev.timeline(True)
-    dev.timeline_read()
-    got = call()
-    names = [what for _, what, _ in dev.timeline_read()]
-    dev.timeline(False)
-    return got, names
-
-
 def test_one_filter_group_that_overflows_does_not_shut_out_the_others(vsk, dev):
     rng = np.random.default_rng(32)
     groups, n, d, per = 5, 100_000, 128, 400
@@ -140,7 +130,7 @@ def test_one_filter_group_that_overflows_does_not_shut_out_the_others(vsk, dev):
     dev.set_search_path(0)
     for _ in range(3):
         before = dev.stats()["fallback_queries"]
-        got, names = _marks(dev, lambda: ix.batchSearch(q, 10, qm))
+        got, names = logged_launches(dev, lambda: ix.batchSearch(q, 10, qm))
         assert dev.stats()["fallback_queries"] - before >= per
         assert names.count("l1_dense") == groups                 # all groups took the byte filter, on every call
         keep = np.arange(len(q)) != 5
@@ -155,7 +145,7 @@ def test_only_rows_that_are_re_scored_are_counted(vsk, dev):
     ix = _index(vsk, dev, rng.uniform(-1, 1, (n, d)).astype(np.float32))
     q = rng.uniform(-1, 1, (nq, d)).astype(np.float32)
     before = dev.stats()
-    _, names = _marks(dev, lambda: ix.batchSearch(q, k))
+    _, names = logged_launches(dev, lambda: ix.batchSearch(q, k))
     after = dev.stats()
     counted, chunks = after["reranked_rows"] - before["reranked_rows"], names.count("l1_scan")
     assert chunks > 1 and after["fallback_queries"] == before["fallback_queries"]
@@ -171,7 +161,7 @@ def test_the_widest_rows_of_the_path(vsk, dev):
     x = torch.empty((16_384, 12_288), device="cuda").uniform_(-1.0, 1.0, generator=gen)
     q = torch.empty((32, 12_288), device="cuda").uniform_(-1.0, 1.0, generator=gen)
     ix = _index(vsk, dev, x)
-    (gd, gi), names = _marks(dev, lambda: ix.batchSearch(q, 10))
+    (gd, gi), names = logged_launches(dev, lambda: ix.batchSearch(q, 10))
     assert "l1_rescore" in names
     dev.set_search_path(1)
     rd, ri = ix.batchSearch(q, 10)
@@ -193,7 +183,7 @@ def test_the_byte_copy_is_made_when_it_pays(vsk, dev):
         dev.set_search_path(1)
         ref = ix.batchSearch(q[:nq], k)
         dev.set_search_path(0)
-        got, names = _marks(dev, lambda: ix.batchSearch(q[:nq], k))
+        got, names = logged_launches(dev, lambda: ix.batchSearch(q[:nq], k))
         assert np.array_equal(got[1], ref[1]) and np.array_equal(got[0], ref[0])
         return "l1_scan" in names
 

@@ -3,6 +3,8 @@ re-scored from the distance tables): ids and distances equal the CPU oracle's ta
 import numpy as np
 import pytest
 
+from parity import logged_launches
+
 pytestmark = pytest.mark.gpu
 
 
@@ -110,16 +112,6 @@ def test_non_finite_queries_do_not_disturb_the_others(vsk, dev, cpu_oracle):
     assert np.array_equal(ids, ri) and np.array_equal(dist, rd)
 
 
-def _marks(dev, call):
-    """(what the call returned, the names of the launches it logged)"""
-    dev.timeline(True)
-    dev.timeline_read()
-    got = call()
-    names = [what for _, what, _ in dev.timeline_read()]
-    dev.timeline(False)
-    return got, names
-
-
 def test_ordinary_batches_are_answered_by_the_contraction(vsk, dev, cpu_oracle):
     """Not by the table scan behind it: no query is handed back."""
     for m, ds in ((16, 8), (10, 32)):                             # queries resident, and the general kernel
@@ -128,7 +120,7 @@ def test_ordinary_batches_are_answered_by_the_contraction(vsk, dev, cpu_oracle):
         codes = cpu_oracle.pq_encode(x, cb)
         ix = _index(vsk, dev, cb, codes)
         before = dev.stats()["fallback_queries"]
-        (dist, ids), names = _marks(dev, lambda: ix.batchSearch(q, 10))
+        (dist, ids), names = logged_launches(dev, lambda: ix.batchSearch(q, 10))
         assert ("list_scan" if m == 16 else "scan") in names
         assert dev.stats()["fallback_queries"] == before
         rd, ri = cpu_oracle.pq_search(q, codes, cb, 10)
@@ -145,7 +137,7 @@ def test_an_index_of_bulk_ties_rests_from_the_contraction(vsk, dev, cpu_oracle):
     rd, ri = cpu_oracle.pq_search(q, codes, cb, 100)
     decoded = []
     for _ in range(17):
-        (dist, ids), names = _marks(dev, lambda: ix.batchSearch(q, 100))
+        (dist, ids), names = logged_launches(dev, lambda: ix.batchSearch(q, 100))
         decoded.append("pq_decode" in names)
         assert np.array_equal(ids, ri) and np.array_equal(dist, rd)
     assert decoded == [True] + [False] * 15 + [True]
