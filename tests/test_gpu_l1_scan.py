@@ -159,7 +159,7 @@ def test_the_widest_rows_of_the_path(vsk, dev):
     import torch
     gen = torch.Generator(device="cuda").manual_seed(35)
     x = torch.empty((16_384, 12_288), device="cuda").uniform_(-1.0, 1.0, generator=gen)
-    q = torch.empty((32, 12_288), device="cuda").uniform_(-1.0, 1.0, generator=gen)
+    q = torch.empty((192, 12_288), device="cuda").uniform_(-1.0, 1.0, generator=gen)
     ix = _index(vsk, dev, x)
     (gd, gi), names = logged_launches(dev, lambda: ix.batchSearch(q, 10))
     assert "l1_rescore" in names
@@ -172,27 +172,33 @@ def test_the_widest_rows_of_the_path(vsk, dev):
 
 def test_the_byte_copy_is_made_when_it_pays(vsk, dev):
     """Adding and searching in turn keeps to the fp32 tile for batches that would not pay for the copy; so do batches that are
-    too small to gain from a copy that exists.  Batches on rows that stay as they are pay for it together."""
+    too small to gain from a copy that exists, and first batches over many rows.  Batches on rows that stay as they are pay for
+    it together."""
     rng = np.random.default_rng(34)
-    n, d, k = 100_000, 256, 10
+    n, d, k = 60_000, 256, 10
     x = rng.uniform(-1, 1, (n, d)).astype(np.float32)
-    q = rng.uniform(-1, 1, (800, d)).astype(np.float32)
+    q = rng.uniform(-1, 1, (900, d)).astype(np.float32)
     ix = _index(vsk, dev, x)
 
-    def filtered(nq):
+    def filtered(nq, index=None):
+        index = index or ix
         dev.set_search_path(1)
-        ref = ix.batchSearch(q[:nq], k)
+        ref = index.batchSearch(q[:nq], k)
         dev.set_search_path(0)
-        got, names = logged_launches(dev, lambda: ix.batchSearch(q[:nq], k))
+        got, names = logged_launches(dev, lambda: index.batchSearch(q[:nq], k))
         assert np.array_equal(got[1], ref[1]) and np.array_equal(got[0], ref[0])
         return "l1_scan" in names
 
-    assert filtered(32)                                          # the first batch makes the copy
-    assert not filtered(32) and filtered(64)                     # 0.8e9 and 1.6e9 steps
-    for nq in (64, 256, 64, 256):
+    assert filtered(32)                                          # 15 million elements: the first batch makes the copy
+    assert not filtered(32) and filtered(80)                     # 0.5e9 and 1.2e9 steps
+    for nq in (80, 256, 80, 256):
         ix.add(x[:50] * 0.9)
         assert not filtered(nq)
-    assert [filtered(64) for _ in range(6)] == [False] * 4 + [True] * 2   # 256 + 5 x 64 queries: 1.48e10 steps
+    # 1.1e10 steps and 110 per element are 826 queries over these rows
+    assert [filtered(80) for _ in range(10)] == [False] * 7 + [True] * 3
     ix.add(x[:50] * 0.9)
-    assert filtered(800)
+    assert filtered(900)
     ix.close()
+    wide = _index(vsk, dev, np.concatenate([x, x[:10_000] + 0.1]))   # 17.9 million elements, 724 queries
+    assert [filtered(m, wide) for m in (80, 600, 80)] == [False, False, True]
+    wide.close()

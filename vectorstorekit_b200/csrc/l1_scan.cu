@@ -358,16 +358,18 @@ bool l1_applicable(const Index* ix, int64_t n, int64_t nq, int32_t k) {
 //   the copy exists     w >= 1e9.  The filter's launches cost 110 us more than the tile's and save 0.064 ns per 1 000 steps:
 //                       us, tile / filter: 65 536 rows x 128, 64 queries (0.5e9) 163 / 209, 128 (1.1e9) 241 / 234; 16 384 x
 //                       256, 128 (0.5e9) 213 / 241, 512 (2.1e9) 350 / 285; 1 million x 256, 256 (6.6e10) 5 458 / 1 404.
-//   rows were added     the copy has to be made again, 0.7 ms plus 7 ps per element (1 million x 256: 2.5 ms, 262 144 x 256:
-//                       0.9): when the batches since then, this one included, would have saved that, 1.1e10 steps and 110
-//                       per element.  Adding and searching in turn thus stays with the tile unless the batch is large (1
-//                       million x 256, 64 queries: tile 1.35 ms, copy and filter 3 - 10 ms; 256: 5.5 and 3.9 ms).
-//   never made          the first batch makes it, as every operand copy is made: rows that are loaded once are searched often.
+//   no copy of the rows it has to be made, 0.7 ms plus 7 ps per element (1 million x 256: 2.5 ms, 262 144 x 256: 0.9): when the
+//   as they are         batches since rows were last added, this one included, would have saved that, 1.1e10 steps and 110 per
+//                       element.  Adding and searching in turn thus stays with the tile unless the batch is large (1 million x
+//                       256, 64 queries: tile 1.35 ms, copy and filter 3 - 10 ms; 256: 5.5 and 3.9 ms).
+//   never made, small   up to 16 million elements the first batch makes it, at 0.8 ms at most: rows that are loaded once are
+//                       searched often.
+constexpr int64_t kL1SmallElems = 16ll << 20;
 static bool l1_pays(Index* ix, int64_t n, int64_t nq, L1Call* call) {
   const double per_query = (double)n * ix->dim, work = per_query * (double)nq;
   const double ahead = per_query * (double)std::max(nq, call->queries);   // groups to come have about as many rows
   call->queries -= nq;
-  if (ix->l1_lo == nullptr) return true;
+  if (ix->l1_lo == nullptr && ix->n * ix->dim <= kL1SmallElems) return true;
   if (work < 1e9) return false;
   if (ix->n_u8 == ix->n || ix->l1_work + ahead >= 1.1e10 + 110.0 * (double)ix->n * ix->dim) return true;
   ix->l1_work += work;
