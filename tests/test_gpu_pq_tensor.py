@@ -177,6 +177,47 @@ def test_encoding_equals_the_exact_sums(vsk, dev, cpu_oracle, ds, ksub, offset):
     assert np.array_equal(_encode(dev, cb, x), cpu_oracle.pq_encode(x, cb))
 
 
+# The contraction takes 129 or more codewords from 65 536 (row, segment) pairs on (131 072 for two dimensions): whole and ragged
+# row tiles, whole and partial groups of segments.
+@pytest.mark.parametrize("ds,m,ksub,n", [(2, 8, 256, 16_384), (2, 10, 129, 13_185), (4, 8, 256, 8_319), (4, 9, 200, 8_000), (8, 4, 256, 20_001),
+                                         (8, 5, 255, 13_185), (8, 16, 256, 19_072), (16, 2, 256, 32_896), (16, 3, 130, 22_007)])
+def test_encoding_on_the_tensor_cores_equals_the_exact_sums(vsk, dev, cpu_oracle, ds, m, ksub, n):
+    rng = np.random.default_rng(ds * 100 + m)
+    x = (rng.standard_normal((n, m * ds)) + 2.0 * rng.standard_normal(m * ds)).astype(np.float32)
+    cb = np.ascontiguousarray(np.stack([x[rng.choice(n, ksub, replace=False)][:, s * ds:(s + 1) * ds] for s in range(m)]))
+    cb[:, ksub - 1] = cb[:, 3]                                    # equal codewords: the lower code
+    cb[m - 1, 7] *= 40.0                                          # one far out: the others share few operand bits
+    x[5] = np.concatenate(list(cb[:, 3]))
+    x[6] = 0.5 * (np.concatenate(list(cb[:, 0])) + np.concatenate(list(cb[:, 1])))
+    for i in range(100):                                          # between two codewords, in one four or in two
+        a, b = (2 * i) % (ksub - 2), (2 * i + (1 if i % 2 else 17)) % (ksub - 2)
+        x[20 + i] = 0.5 * (np.concatenate(list(cb[:, a])) + np.concatenate(list(cb[:, b])))
+    x[7] *= 1e4                                                   # more than fp16 holds beside the codewords
+    x[8] *= 1e19                                                  # squares that overflow
+    x[9, 1], x[10, 0] = np.nan, np.inf
+    x[n - 1] = x[5]
+    assert np.array_equal(_encode(dev, cb, x), cpu_oracle.pq_encode(x, cb))
+
+
+@pytest.mark.parametrize("what", ["equal", "tiny", "huge", "nan"])
+def test_encoding_with_unusual_codebooks(vsk, dev, cpu_oracle, what):
+    rng = np.random.default_rng(8)
+    m, ksub, ds, n = 5, 256, 8, 13_200
+    x = rng.standard_normal((n, m * ds)).astype(np.float32)
+    cb = rng.standard_normal((m, ksub, ds)).astype(np.float32)
+    if what == "equal":
+        cb[1] = cb[1, 0]
+    elif what == "tiny":
+        cb[1] *= np.float32(1e-41)
+        x[:, ds:2 * ds] *= np.float32(1e-41)
+    elif what == "huge":
+        cb[1] *= np.float32(1e20)
+        x[:, ds:2 * ds] *= np.float32(1e18)
+    else:
+        cb[1, 9, 3], cb[2, 200, 0] = np.nan, np.inf
+    assert np.array_equal(_encode(dev, cb, x), cpu_oracle.pq_encode(x, cb))
+
+
 def _encode(dev, cb, x):
     """vsk_pq_encode with a codebook size that need not be a power of two."""
     import ctypes as C

@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "pq_encode.cuh"
 #include "tensor_scan.cuh"
 
 namespace vsk {
@@ -35,11 +36,6 @@ namespace {
 constexpr int PQ_THREADS = 512;
 constexpr size_t PQ_SMEM_LIMIT = 200 * 1024;
 
-__device__ __forceinline__ float sqdiff_accum(float acc, float a, float b) {
-  const float diff = __fsub_rn(a, b);
-  return __fadd_rn(acc, __fmul_rn(diff, diff));
-}
-
 // tables[q][s][c]; one block per (query, segment), one thread per codeword
 __global__ void __launch_bounds__(256) pq_tables_kernel(const float* __restrict__ q, int dim, int m, int ksub, int ds,
                                                         const float* __restrict__ cb, float* __restrict__ tables) {
@@ -49,7 +45,7 @@ __global__ void __launch_bounds__(256) pq_tables_kernel(const float* __restrict_
   for (int c = threadIdx.x; c < ksub; c += blockDim.x) {
     const float* cw = cb + ((int64_t)s * ksub + c) * ds;
     float sum = 0.f;
-    for (int i = 0; i < ds; ++i) sum = sqdiff_accum(sum, __ldg(seg + i), __ldg(cw + i));
+    for (int i = 0; i < ds; ++i) sum = pq_sqdiff_accum(sum, __ldg(seg + i), __ldg(cw + i));
     tables[(a * m + s) * ksub + c] = sum;
   }
 }
@@ -77,46 +73,21 @@ __global__ void __launch_bounds__(PQ_THREADS) pq_encode_kernel(const float* __re
     for (int c = 0; c < ksub; ++c) {
       float d = 0.f;
 #pragma unroll
-      for (int i = 0; i < DS; ++i) d = sqdiff_accum(d, v[i], cbs[c * DS + i]);
+      for (int i = 0; i < DS; ++i) d = pq_sqdiff_accum(d, v[i], cbs[c * DS + i]);
       if (d < best) { best = d; bc = c; }
     }
   } else {
     for (int c = 0; c < ksub; ++c) {
       float d = 0.f;
-      for (int i = 0; i < ds; ++i) d = sqdiff_accum(d, __ldg(seg + i), cbs[c * ds + i]);
+      for (int i = 0; i < ds; ++i) d = pq_sqdiff_accum(d, __ldg(seg + i), cbs[c * ds + i]);
       if (d < best) { best = d; bc = c; }
     }
   }
   codes[r * m + s] = (uint8_t)bc;
 }
 
-// The code of one (row, segment) by the exact sums, over codewords first, first + step, ...: smallest value, lowest code.
-template <int DS>
-__device__ __forceinline__ void pq_exact_code(const float* __restrict__ seg, const float* __restrict__ cb, int ksub, int first, int step,
-                                              bool wide, float& low, int& code) {
-  __align__(16) float x[DS];
-#pragma unroll
-  for (int i = 0; i < DS; ++i) x[i] = __ldg(seg + i);
-  low = CUDART_INF_F;
-  code = 0;
-#pragma unroll 1
-  for (int c = first; c < ksub; c += step) {
-    __align__(16) float w[DS];
-    if (wide) {
-#pragma unroll
-      for (int i = 0; i < DS; i += 4) *reinterpret_cast<float4*>(&w[i]) = __ldg(reinterpret_cast<const float4*>(cb + c * DS + i));
-    } else {
-#pragma unroll
-      for (int i = 0; i < DS; ++i) w[i] = __ldg(cb + c * DS + i);
-    }
-    float d = 0.f;
-#pragma unroll
-    for (int i = 0; i < DS; ++i) d = sqdiff_accum(d, x[i], w[i]);
-    if (d < low) { low = d; code = c; }
-  }
-}
-
-// The same codes for the usual segment lengths at half the instructions.  The exact sum costs three per dimension (its
+// The same codes for the usual segment lengths at half the instructions, for calls that the tensor cores do not take
+// (pq_encode_tensor_applies: few rows, at most 128 codewords, unaligned rows).  The exact sum costs three per dimension (its
 // operations are rounded one by one), the form |c|^2 - 2 x.c one; the exact sums decide only where the two smallest values
 // of that form lie closer together than both forms' roundings.  Rows and codewords are taken relative to the segment's mean
 // codeword there, so that the roundings follow the spread of the data and not its distance from the origin:
@@ -222,14 +193,7 @@ __global__ void __launch_bounds__(256) pq_encode_fast_kernel(const float* __rest
     }
     for (; todo; todo &= todo - 1u) {
       const int src = __ffs((int)todo) - 1;
-      int code;
-      pq_exact_code<DS>(x + (row - lane + src) * dim + (int64_t)s * DS, cb_seg, ksub, lane, 32, cb_wide, low, code);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float l2 = __shfl_xor_sync(0xffffffffu, low, o);
-        const int c2 = __shfl_xor_sync(0xffffffffu, code, o);
-        if (l2 < low || (l2 == low && c2 < code)) { low = l2; code = c2; }
-      }
+      const int code = pq_exact_code_warp<DS>(x + (row - lane + src) * dim + (int64_t)s * DS, cb_seg, ksub, lane, cb_wide);
       if (lane == src) bc = code;
     }
     if (row < n) *VSK_CHK_W(codes + row * m + s) = (uint8_t)bc;
@@ -407,6 +371,7 @@ int32_t check_shape(Ctx* ctx, int32_t dim, int32_t m, int32_t ksub) {
 
 int32_t encode_dev(Ctx* ctx, const float* cb, int32_t dim, int32_t m, int32_t ksub, const float* x, int64_t n,
                    uint8_t* codes) {
+  if (pq_encode_tensor_applies(x, n, dim, m, ksub)) return pq_encode_tensor(ctx, cb, dim, m, ksub, x, n, codes);
   const int ds = dim / m;
   const size_t smem = (size_t)ksub * ds * sizeof(float);
   if (smem > PQ_SMEM_LIMIT) return fail(ctx, VSK_ERR_INVALID_BUFFER_SIZE, "a segment's codebook (%d x %d floats) does not fit in shared memory", ksub, ds);

@@ -2369,6 +2369,20 @@ void tensor_invalidate(Index* ix) {
 }
 int32_t tensor_prepare_index(Index* ix) { return tensor_prepare(ix); }
 
+int32_t make_map_rows_f32(Ctx* ctx, const float* base, int64_t rows, int32_t dim, int box_cols, int box_rows, CUtensorMap* map) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(ctx, VSK_ERR_EXECUTION_FAILED, "cuTensorMapEncodeTiled is not available from this driver");
+  cuuint64_t gdim[2] = {(cuuint64_t)dim, (cuuint64_t)rows};
+  cuuint64_t gstride[1] = {(cuuint64_t)dim * 4};
+  cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+  cuuint32_t estride[2] = {1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), gdim, gstride, box, estride,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(ctx, VSK_ERR_EXECUTION_FAILED, "cuTensorMapEncodeTiled (fp32 rows) failed with %d", (int)r);
+  return VSK_OK;
+}
+
 // ---- query operands of a flat search ------------------------------------------------------------------
 // fp16 operand rows of the queries, their error bound eps[q], the output coefficient alpha, and the small words a
 // search needs (device error word, re-scored row counter), all in the current lane's scratch.

@@ -1,6 +1,8 @@
 // Entry points of the tensor-core search path (tensor_scan.cu) and of the int8 scan (sq8.cu)
 // used by the C ABI layer, plus the fp32 re-run the tensor path falls back on per query.
 #pragma once
+#include <cuda.h>
+
 #include <vector>
 
 #include "common.cuh"
@@ -67,6 +69,9 @@ int32_t cand_lists(Ctx* ctx, int64_t nq, CandLists* cand);
 // Drops the operand copies after rows were added; makes it (once per index state).
 void tensor_invalidate(Index* ix);
 int32_t tensor_prepare_index(Index* ix);
+// fp32 matrix [rows][dim], dim a multiple of 4 and base of 16 bytes: box = box_cols (32 or 16) columns x box_rows, 128-byte
+// (64-byte) swizzle; columns past `dim` and rows past `rows` read as zero.
+int32_t make_map_rows_f32(Ctx* ctx, const float* base, int64_t rows, int32_t dim, int box_cols, int box_rows, CUtensorMap* map);
 
 // fp32 scan of the listed queries of a batch (api.cu).
 int32_t fp32_search_subset(Index* ix, const float* q, const std::vector<int32_t>& subset, int32_t k,
