@@ -49,6 +49,36 @@ def test_few_queries(vsk, dev, cpu_oracle, metric, shape):
         assert np.all(i_[:, n:] == -1) and np.all(np.isinf(d_[:, n:]))
 
 
+# one query: widths around the short-row forms and around what travels in the launch's arguments; lists handed over whole (96 keys)
+# and shortened; the query on the host and on the device
+@pytest.mark.parametrize("metric", list(METRICS))
+@pytest.mark.parametrize("shape", [(20_003, 128, 96), (20_003, 132, 97), (40_001, 256, 10), (9_001, 260, 128), (3_001, 1_024, 5), (3_001, 1_028, 128),
+                                   (120_001, 4, 128)])
+def test_one_query(vsk, dev, cpu_oracle, metric, shape):
+    import torch
+    n, d, k = shape
+    rng = np.random.default_rng(n + d + k)
+    x = rng.standard_normal((n, d)).astype(np.float32)
+    q = rng.standard_normal((1, d)).astype(np.float32)
+    ix = _index(vsk, dev, metric, x)
+    got = ix.batchSearch(q, k)
+    assert_topk_parity(*got, *cpu_oracle.flat_search(METRICS[metric], q, x, k))
+    on_device = ix.batchSearch(torch.from_numpy(q).cuda(), k)
+    assert np.array_equal(got[0], on_device[0].cpu().numpy()) and np.array_equal(got[1], on_device[1].cpu().numpy())
+
+
+def test_merge_of_lists_within_the_bound(vsk, dev, cpu_oracle):
+    """Rows that all tie at one distance but for a few: every key of every list is within the merge's bound."""
+    x = np.zeros((60_000, 64), np.float32)
+    x[::1_000, 0] = 1.0
+    ix = _index(vsk, dev, "euclidean", x)
+    q = np.zeros((1, 64), np.float32)
+    for k in (1, 50, 128):
+        d_, i_ = ix.batchSearch(q, k)
+        rd, ri = cpu_oracle.flat_search(oracle.EUCLIDEAN, q, x, k)
+        assert np.array_equal(i_, ri) and np.array_equal(d_, rd)
+
+
 @pytest.mark.parametrize("order", ["ascending", "descending", "blocks"])
 def test_order_of_rows_and_ties(vsk, dev, cpu_oracle, order):
     """Rows sorted by distance (every later row is listed, or none is), the nearest rows all in one CTA's share, and bulk

@@ -86,7 +86,9 @@ int32_t pinned_reserve(Ctx* ctx, PinnedBuf* b, size_t bytes) {
 
 constexpr size_t kStagedIn = 64 << 10, kStagedOut = 12 << 10;   // bytes a staged call may bring and take (1 024 results)
 
-int32_t host_call_begin(Ctx* ctx, const float* q, int64_t nq, int32_t dim, const uint64_t* qmasks, int32_t k, HostCall* c) {
+int32_t host_call_begin(Ctx* ctx, const float* q, int64_t nq, int32_t dim, const uint64_t* qmasks, int32_t k, HostCall* c,
+                        bool may_wait) {
+  ctx->host_query.pending = false;
   void* p;
   const size_t qb = (size_t)nq * dim * 4, mb = qmasks ? (size_t)nq * 8 : 0, ob = (size_t)nq * k * 12;
   VSK_TRY(scratch(ctx, SLOT_Q, qb, &p));
@@ -113,8 +115,19 @@ int32_t host_call_begin(Ctx* ctx, const float* q, int64_t nq, int32_t dim, const
     VSK_TRY(scratch(ctx, SLOT_OUT_I, (size_t)nq * k * 8, &p));
     c->ids = (int64_t*)p;
   }
-  VSK_CUDA(ctx, cudaMemcpyAsync(c->q, src, qb, cudaMemcpyHostToDevice, ctx->stream));
+  if (c->staged && may_wait && nq == 1)
+    ctx->host_query = Ctx::HostQuery{c->q, src, qb, true};
+  else
+    VSK_CUDA(ctx, cudaMemcpyAsync(c->q, src, qb, cudaMemcpyHostToDevice, ctx->stream));
   if (qmasks) VSK_CUDA(ctx, cudaMemcpyAsync(c->masks, msrc, mb, cudaMemcpyHostToDevice, ctx->stream));
+  return VSK_OK;
+}
+
+int32_t host_query_upload(Ctx* ctx) {
+  Ctx::HostQuery& h = ctx->host_query;
+  if (!h.pending) return VSK_OK;
+  h.pending = false;
+  VSK_CUDA(ctx, cudaMemcpyAsync(const_cast<float*>(h.dev), h.host, h.bytes, cudaMemcpyHostToDevice, ctx->stream));
   return VSK_OK;
 }
 
@@ -579,6 +592,7 @@ static int32_t flat_search_dev(Index* ix, const float* q, int64_t nq, int32_t k,
         if (handled || !tensor_metric || mb || ix->n * ix->dim <= kFewMaxElems) continue;
       }
     }
+    VSK_TRY(host_query_upload(ctx));
     float* qnorm = nullptr;
     if (ix->metric == VSK_METRIC_COSINE) {
       void* p;
@@ -1165,8 +1179,10 @@ int32_t vsk_search(vsk_index* i, const float* q, int64_t nq, int32_t k, const ui
   if (k <= 0) return fail(ctx, VSK_ERR_INVALID_INPUT, "k must be positive");
   if (!q || !out_dist || !out_ids) return fail(ctx, VSK_ERR_INVALID_INPUT, "null pointer");
   HostCall c;
-  VSK_TRY(host_call_begin(ctx, q, nq, ix->dim, qmasks, k, &c));
-  VSK_TRY(vsk_search_dev(i, c.q, nq, k, c.masks, c.dist, c.ids));
+  VSK_TRY(host_call_begin(ctx, q, nq, ix->dim, qmasks, k, &c, ix->kind == INDEX_FLAT_F32));
+  const int32_t st = vsk_search_dev(i, c.q, nq, k, c.masks, c.dist, c.ids);
+  ctx->host_query.pending = false;
+  VSK_TRY(st);
   VSK_TRY(host_call_end(ctx, c, nq, ix->dim, k, out_dist, out_ids));
   return VSK_OK;
 }

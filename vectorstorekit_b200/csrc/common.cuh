@@ -180,6 +180,14 @@ struct Ctx {
   void* scratch[2 * 64] = {};
   size_t scratch_bytes[2 * 64] = {};
   ShardPending pending[2];
+  // The query of a host-pointer call that is staged in pinned memory and not on the device yet: a kernel may take it in its
+  // arguments, everything else asks for the copy first (host_query_upload).
+  struct HostQuery {
+    const float* dev = nullptr;
+    const float* host = nullptr;
+    size_t bytes = 0;
+    bool pending = false;
+  } host_query;
   PinnedBuf host_io;         // staging of small host-pointer calls (HostCall)
   PinnedBuf host_flags[2];   // per lane: the flag words a finished half-search hands to the host
   std::vector<const void*> configured;   // kernels that have their shared memory on this device (opt_in_shared) ...
@@ -261,7 +269,9 @@ struct HostCall {
   int64_t* ids = nullptr;
   bool staged = false;
 };
-int32_t host_call_begin(Ctx* ctx, const float* q, int64_t nq, int32_t dim, const uint64_t* qmasks, int32_t k, HostCall* c);
+// may_wait: the caller's search paths ask for the copy of a single query themselves
+int32_t host_call_begin(Ctx* ctx, const float* q, int64_t nq, int32_t dim, const uint64_t* qmasks, int32_t k, HostCall* c, bool may_wait = false);
+int32_t host_query_upload(Ctx* ctx);
 // after the search has drained its stream
 int32_t host_call_end(Ctx* ctx, const HostCall& c, int64_t nq, int32_t dim, int32_t k, float* out_dist, int64_t* out_ids);
 

@@ -1,7 +1,7 @@
 // Top-k of a few queries in one launch: scan, selection and final order.
 //
 // A call with one query over a small store is bound by launches, not by bytes: 10 000 rows of 128 floats cross HBM in
-// 0.8 us, and the chunked schedule spends a dozen launches on them (109 us for the whole call; 32 us this way, its query and results staged in pinned memory).  Here every
+// 0.8 us, and the chunked schedule spends a dozen launches on them (109 us for the whole call; 26 us this way, its query in the launch's arguments and its results staged in pinned memory).  Here every
 // CTA streams its share of the rows (the inner loop of stream_scan.cu: each row read once, 16-byte loads), keeps its k
 // best keys per query in shared memory - appends below a threshold, a block-wide selection when the list fills up - and
 // writes them out; the last CTA to finish merges the lists.  The merge needs few of the G k keys written: the k-th
@@ -11,10 +11,12 @@
 //
 // SEG: every query walks the rows of its own probed lists of an IVF index (one grid row per query), found from the probe
 // list and the list offsets on the device: no row list is written and the host is not asked in between (one query, 10 of
-// 1 024 lists over 1 million rows: 143 -> 67 us with the staged call).
+// 1 024 lists over 1 million rows, 60 000 rows in all: 143 us for the chunked schedule, 56 this way; 75 with two rows per step that
+// were waited for, rounds sized by the mean list, an id looked up per listed row and the query copied first).
 #include <math_constants.h>
 
 #include <algorithm>
+#include <cstring>
 
 #include "block_select.cuh"
 #include "common.cuh"
@@ -26,7 +28,8 @@ namespace {
 
 constexpr int FEW_THREADS = 256;
 constexpr int FEW_WARPS = FEW_THREADS / 32;
-constexpr int FEW_ROWS = 2;        // rows per warp step (as in stream_scan.cu)
+constexpr int kFewShort = 96;      // keys a CTA hands over as they are: shortening a list costs more than the merge's test of its keys
+constexpr int kFewRank = 256;      // keys the merge orders by counting the smaller ones (one per thread, no barrier)
 constexpr int FEW_LIST = 1024;     // keys per query a CTA holds
 constexpr int FEW_ROUND = 512;     // rows per round at most: a round's keys fit behind FEW_LIST - FEW_ROUND listed ones
 constexpr int FEW_MAX_CTAS = 1024; // lists per query the merge looks at (the selection holds 8 keys per thread)
@@ -34,12 +37,24 @@ static_assert(FEW_LIST - FEW_ROUND >= kFewMaxK && FEW_MAX_CTAS <= FEW_THREADS * 
 
 struct FewKernelArgs {
   FewArgs a;
-  int32_t round;        // rows per CTA and round, a multiple of FEW_WARPS * FEW_ROWS
-  uint64_t* part;       // [nq][grid][k] each CTA's best keys (unordered) ...
+  int32_t round;        // rows per CTA and round, a multiple of FEW_WARPS * rows per warp step (SEG: the kernel's own)
+  int32_t stride;       // room of a CTA's list of one query in `part`
+  uint64_t* part;       // [nq][grid][stride] each CTA's best keys (unordered) ...
   uint64_t* part_min;   // [nq][grid] ... the smallest of them (all ones: none)
   int32_t* part_n;      // [nq][grid] ... and how many
   unsigned* ticket;     // [nq] CTAs of the query that have finished; left at zero
 };
+
+// A host call's one query, in the launch's arguments: no copy to the device before the launch (1.8 us, and 7.5 more until the
+// kernel behind it began).
+constexpr int kFewInline = 1024;
+template <bool INL> struct FewInline { float q[kFewInline]; };
+template <> struct FewInline<false> {};
+template <bool INL>
+__device__ __forceinline__ float few_query(const FewInline<INL>& iq, const float* q, int64_t i) {
+  if constexpr (INL) return iq.q[i];
+  else return *VSK_CHK(q + i);
+}
 
 struct FewScratch {     // the selection's words
   int hist[256];
@@ -65,13 +80,13 @@ __device__ __forceinline__ uint64_t few_compact(uint64_t* list, int cnt, int k, 
 }
 
 // After a round of rows: lists that a further round could overfill are shortened to their `keep` smallest keys and tighten their
-// query's threshold; after the last round every list is.
-__device__ __forceinline__ void few_end_round(uint64_t* lists, int nq, int keep, bool last, int* s_cnt, uint64_t* s_thr, FewScratch& s) {
+// query's threshold; after the last round those that do not fit `stride` are.
+__device__ __forceinline__ void few_end_round(uint64_t* lists, int nq, int keep, int stride, bool last, int* s_cnt, uint64_t* s_thr, FewScratch& s) {
   __syncthreads();
 #pragma unroll 1
   for (int i = 0; i < nq; ++i) {
     const int cnt = s_cnt[i];
-    if (cnt > (last ? keep : FEW_LIST - FEW_ROUND)) {
+    if (cnt > (last ? stride : FEW_LIST - FEW_ROUND)) {
       const uint64_t pivot = few_compact(lists + (size_t)i * FEW_LIST, cnt, keep, s);
       if (threadIdx.x == 0) {
         s_cnt[i] = s.out;
@@ -83,14 +98,14 @@ __device__ __forceinline__ void few_end_round(uint64_t* lists, int nq, int keep,
 }
 
 // Writes this CTA's lists of queries [pos, pos + nq) with their lengths and smallest keys.
-__device__ __forceinline__ void few_write_lists(const FewKernelArgs& ka, const uint64_t* lists, int pos, int nq, int keep, const int* s_cnt) {
+__device__ __forceinline__ void few_write_lists(const FewKernelArgs& ka, const uint64_t* lists, int pos, int nq, const int* s_cnt) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll 1
   for (int i = 0; i < nq; ++i) {
     const int64_t l = (int64_t)(pos + i) * gridDim.x + blockIdx.x;
     const uint64_t* list = lists + (size_t)i * FEW_LIST;
     const int cnt = s_cnt[i];
-    for (int j = threadIdx.x; j < cnt; j += FEW_THREADS) *VSK_CHK_W(ka.part + l * keep + j) = list[j];
+    for (int j = threadIdx.x; j < cnt; j += FEW_THREADS) *VSK_CHK_W(ka.part + l * ka.stride + j) = list[j];
     if (warp == 0) {
       uint64_t best = kEmptyKey;
       for (int j = lane; j < cnt; j += 32) best = min(best, list[j]);
@@ -102,6 +117,29 @@ __device__ __forceinline__ void few_write_lists(const FewKernelArgs& ka, const u
       }
     }
   }
+}
+
+// The k smallest of list[0..cnt) in order, and their distances and ids out; every thread takes part.
+__device__ __forceinline__ void few_order(uint64_t* list, int cnt, int k, bool root, int64_t id_base, float* out_dist, int64_t* out_ids) {
+  auto put = [&](int j, uint64_t key, bool has) {
+    float d = has ? ordered_to_float((uint32_t)(key >> 32)) : CUDART_INF_F;
+    if (has && root) d = sqrtf(d);
+    *VSK_CHK_W(out_dist + j) = d;
+    *VSK_CHK_W(out_ids + j) = has ? (int64_t)(uint32_t)key + id_base : -1;
+  };
+  if (cnt <= kFewRank) {   // keys are distinct: a key's place is the number of smaller ones
+    const uint64_t mine = (int)threadIdx.x < cnt ? list[threadIdx.x] : kEmptyKey;
+    int below = 0;
+    for (int j = 0; j < cnt; ++j) below += list[j] < mine;
+    if ((int)threadIdx.x < cnt && below < k) put(below, mine, true);
+    for (int j = cnt + threadIdx.x; j < k; j += FEW_THREADS) put(j, 0ull, false);
+    return;
+  }
+  const int P = next_pow2(cnt);
+  for (int i = cnt + threadIdx.x; i < P; i += FEW_THREADS) list[i] = kEmptyKey;
+  __syncthreads();
+  bitonic_sort(list, P);
+  for (int j = threadIdx.x; j < k; j += FEW_THREADS) put(j, j < cnt ? list[j] : 0ull, j < cnt);
 }
 
 // Merges the lists of the launch's query `pos` and writes the result of query `out`.  `list` has room for FEW_LIST keys, `cand` for FEW_MAX_CTAS list numbers.
@@ -132,19 +170,29 @@ __device__ __forceinline__ void few_merge(const FewKernelArgs& ka, int64_t pos, 
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nc = n_cand;
   int cnt = 0;
-  const int batch = (FEW_LIST - k) / k;   // lists that fit behind the keys already kept
+  // All of them at once as a rule - few of their keys are within the bound; lists that hold more than there is room for, a
+  // batch at a time, shortened in between.
+  int batch = max(nc, 1);
   for (int c0 = 0; c0 < nc; c0 += batch) {
     for (int c = c0 + warp; c < min(nc, c0 + batch); c += FEW_WARPS) {
       const int64_t l = pos * lists + cand[c];
       const int n = __ldcg(VSK_CHK(ka.part_n + l));
-      for (int i = lane; i < n; i += 32) {
-        const uint64_t v = __ldcg(VSK_CHK(ka.part + l * k + i));
-        if (v <= bound) list[atomicAdd(&n_list, 1)] = v;
+      for (int i = lane; i < ka.stride; i += 32) {   // (the keys come with their number: what lies behind it is old)
+        const uint64_t v = __ldcg(VSK_CHK(ka.part + l * ka.stride + i));
+        if (i < n && v <= bound) {
+          const int at = atomicAdd(&n_list, 1);
+          if (at < FEW_LIST) list[at] = v;
+        }
       }
     }
     __syncthreads();
     cnt = n_list;
-    if (cnt > k) {
+    __syncthreads();
+    if (cnt > FEW_LIST) {   // (the first attempt only)
+      batch = (FEW_LIST - k) / ka.stride;
+      c0 = -batch;
+      if (threadIdx.x == 0) n_list = 0;
+    } else if (cnt > max(k, kFewRank) || (cnt > k && batch < nc)) {
       const uint64_t pivot = few_compact(list, cnt, k, s);
       bound = min(bound, pivot);
       cnt = s.out;
@@ -152,26 +200,17 @@ __device__ __forceinline__ void few_merge(const FewKernelArgs& ka, int64_t pos, 
     }
     __syncthreads();
   }
-  const int P = next_pow2(cnt);
-  for (int i = cnt + threadIdx.x; i < P; i += FEW_THREADS) list[i] = kEmptyKey;
-  __syncthreads();
-  bitonic_sort(list, P);
-  for (int j = threadIdx.x; j < k; j += FEW_THREADS) {
-    float d = CUDART_INF_F;
-    int64_t id = -1;
-    if (j < cnt) {
-      d = ordered_to_float((uint32_t)(list[j] >> 32));
-      if (a.final_sqrt) d = sqrtf(d);
-      id = (int64_t)(uint32_t)list[j] + a.id_base;
-    }
-    *VSK_CHK_W(a.out_dist + out * k + j) = d;
-    *VSK_CHK_W(a.out_ids + out * k + j) = id;
-  }
+  few_order(list, cnt, k, a.final_sqrt, a.id_base, a.out_dist + out * k, a.out_ids + out * k);
 }
 
-template <int METRIC, int NQ, bool VEC, bool SEG>
-__global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(FewKernelArgs ka) {
+// FEW_ROWS rows per warp step.  CH > 0 (one query, 16-byte loads): rows of at most CH * 128 dimensions, CH loads per row and
+// lane, those of the next step issued before this one is reduced.
+template <int METRIC, int NQ, bool VEC, bool SEG, int FEW_ROWS, int CH, bool INL>
+__global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(const __grid_constant__ FewKernelArgs ka,
+                                                                              const __grid_constant__ FewInline<INL> iq) {
+  static_assert(CH == 0 || (NQ == 1 && VEC), "short rows: one query");
   static_assert(!SEG || NQ == 1, "per-query lists are scanned one query per grid row");
+  static_assert(!INL || NQ == 1, "one query travels in the arguments");
   const FewArgs& a = ka.a;
   extern __shared__ __align__(16) uint8_t smem[];
   // [NQ][FEW_LIST] keys, then [NQ][dim] queries, then (SEG) [nprobe + 1] first positions and [nprobe] first rows of the lists
@@ -189,7 +228,7 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(F
   const int qp = SEG ? (int)blockIdx.y : 0;                         // position in this launch
   const int qb = (SEG && a.q_subset) ? *VSK_CHK(a.q_subset + qp) : qp;         // first query of this CTA
   const int nq_here = SEG ? 1 : (int)a.nq;
-  for (int i = threadIdx.x; i < NQ * dim; i += FEW_THREADS) sq[i] = i < nq_here * dim ? *VSK_CHK(a.q + (int64_t)qb * dim + i) : 0.f;
+  for (int i = threadIdx.x; i < NQ * dim; i += FEW_THREADS) sq[i] = i < nq_here * dim ? few_query<INL>(iq, a.q, (int64_t)qb * dim + i) : 0.f;
   if (threadIdx.x < NQ) {
     s_thr[threadIdx.x] = kEmptyKey - 1;
     s_cnt[threadIdx.x] = 0;
@@ -242,58 +281,137 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(F
 
   constexpr int V = FEW_ROWS * NQ;
   constexpr int OWNER_SHIFT = 5 - Log2<V>::value;
-  const int64_t stride = (int64_t)gridDim.x * ka.round;
+  int round = ka.round;
+  if (SEG) {   // the lists' true length: as few rounds as their size allows, the rows spread evenly over them
+    const int64_t share = (n + gridDim.x - 1) / gridDim.x, rounds = (share + FEW_ROUND - 1) / FEW_ROUND;
+    constexpr int kStep = FEW_WARPS * FEW_ROWS;
+    round = n > 0 ? (int)min((int64_t)FEW_ROUND, ((share + rounds - 1) / rounds + kStep - 1) / kStep * kStep) : kStep;
+  }
+  const int64_t stride = (int64_t)gridDim.x * round;
   int cur = 0;   // SEG: the list of the current position
-  for (int64_t r0 = (int64_t)blockIdx.x * ka.round; r0 < n; r0 += stride) {
-    const int64_t r1 = min(n, r0 + ka.round);
-    for (int64_t n0 = r0 + warp * FEW_ROWS; n0 < r1; n0 += FEW_WARPS * FEW_ROWS) {
-      bool live[FEW_ROWS];
-      uint32_t rid[FEW_ROWS];
-      uint64_t rmask[FEW_ROWS];
+  // rows n0 .. of the warp's step; a row that no query of the batch may see is not live, and not read
+  auto locate = [&](int64_t n0, int64_t r1, uint32_t (&rid)[FEW_ROWS], uint64_t (&rmask)[FEW_ROWS], bool (&live)[FEW_ROWS]) {
 #pragma unroll
-      for (int r = 0; r < FEW_ROWS; ++r) {
-        const int64_t at = n0 + r;
-        const bool has = at < r1;
-        rid[r] = has ? (uint32_t)at : 0u;
-        if (SEG && has) {   // positions only grow: the warp's current list serves until the next one starts
-          while (cur + 1 < a.nprobe && seg_pos[cur + 1] <= at) ++cur;
-          rid[r] = (uint32_t)(seg_row[cur] + (at - seg_pos[cur]));
-        }
-        rmask[r] = (a.row_masks && has) ? __ldg(a.row_masks + rid[r]) : ~0ull;
-        live[r] = has && (rmask[r] & any_mask) != 0;   // a row no query may see is not read
+    for (int r = 0; r < FEW_ROWS; ++r) {
+      const int64_t at = n0 + r;
+      const bool has = at < r1;
+      rid[r] = has ? (uint32_t)at : 0u;
+      if (SEG && has) {   // positions only grow: the warp's current list serves until the next one starts
+        while (cur + 1 < a.nprobe && seg_pos[cur + 1] <= at) ++cur;
+        rid[r] = (uint32_t)(seg_row[cur] + (at - seg_pos[cur]));
       }
-      float acc[V];
+      rmask[r] = (a.row_masks && has) ? __ldg(a.row_masks + rid[r]) : ~0ull;
+      live[r] = has && (rmask[r] & any_mask) != 0;
+    }
+  };
+  // the step's partial sums to values, and those at or below the threshold to the lists
+  auto list_step = [&](float (&acc)[V], int64_t n0, const uint32_t (&rid)[FEW_ROWS], const uint64_t (&rmask)[FEW_ROWS], const bool (&live)[FEW_ROWS]) {
+    warp_reduce_scatter<V>(acc, lane);
+    if ((lane & ((1 << OWNER_SHIFT) - 1)) == 0) {
+      const int j = lane >> OWNER_SHIFT;
+      const int r = j / NQ, i = j - r * NQ;
+      bool liver = live[0];
+      uint32_t ridr = rid[0];
+      uint64_t rmaskr = rmask[0];
 #pragma unroll
-      for (int j = 0; j < V; ++j) acc[j] = 0.f;
-      stream_accumulate<METRIC, NQ, VEC, FEW_ROWS>(acc, a.x, dim, sq, rid, live, lane);
-      warp_reduce_scatter<V>(acc, lane);
-      if ((lane & ((1 << OWNER_SHIFT) - 1)) == 0) {
-        const int j = lane >> OWNER_SHIFT;
-        const int r = j / NQ, i = j - r * NQ;
-        bool liver = live[0];
-        uint32_t ridr = rid[0];
-        uint64_t rmaskr = rmask[0];
-#pragma unroll
-        for (int t = 1; t < FEW_ROWS; ++t)
-          if (r == t) { liver = live[t]; ridr = rid[t]; rmaskr = rmask[t]; }
-        if (liver && i < nq_here && (rmaskr & s_qm[i]) != 0) {
-          float v = acc[0];
-          if (METRIC == VSK_METRIC_COSINE) v = 1.0f - v / (s_qn[i] * __ldg(a.xnorm + ridr) + 1e-8f);
-          else if (METRIC == VSK_METRIC_DOT_PRODUCT) v = -v;
-          // (the id is looked up only for a value that can be listed: the load would be on every step's path)
-          if (float_to_ordered(v) <= (uint32_t)(s_thr[i] >> 32)) {
-            const uint32_t id = a.id_remap ? (uint32_t)__ldg(a.id_remap + ridr) : ridr;
-            const uint64_t key = make_key(v, id);
-            // a value that is not a number is listed among the first rows only, as the chunked schedule does
-            if (key <= s_thr[i] && (!isnan(v) || n0 + r < a.nan_rows)) lists[i * FEW_LIST + atomicAdd(&s_cnt[i], 1)] = key;
-          }
-        }
+      for (int t = 1; t < FEW_ROWS; ++t)
+        if (r == t) { liver = live[t]; ridr = rid[t]; rmaskr = rmask[t]; }
+      if (liver && i < nq_here && (rmaskr & s_qm[i]) != 0) {
+        float v = acc[0];
+        if (METRIC == VSK_METRIC_COSINE) v = 1.0f - v / (s_qn[i] * __ldg(a.xnorm + ridr) + 1e-8f);
+        else if (METRIC == VSK_METRIC_DOT_PRODUCT) v = -v;
+        // With ids of their own (id_remap) rows are listed by number and get their ids at the round's end, all at once: by
+        // value, that is, and one that only ties the threshold is listed whatever its id.
+        const uint64_t key = make_key(v, a.id_remap ? 0u : ridr);
+        // a value that is not a number is listed among the first rows only, as the chunked schedule does
+        if (key <= s_thr[i] && (!isnan(v) || n0 + r < a.nan_rows))
+          lists[i * FEW_LIST + atomicAdd(&s_cnt[i], 1)] = make_key(v, ridr);
       }
     }
-    few_end_round(lists, nq_here, k, r0 + stride >= n, s_cnt, s_thr, fs);
+  };
+  int done = 0;   // keys of the list that carry their ids already (id_remap comes with one query per CTA)
+  for (int64_t r0 = (int64_t)blockIdx.x * round; r0 < n; r0 += stride) {
+    const int64_t r1 = min(n, r0 + round);
+    int64_t n0 = r0 + warp * FEW_ROWS;
+    if constexpr (CH > 0) {
+      const int nv = dim >> 2;
+      const float4* sq4 = reinterpret_cast<const float4*>(sq);
+      float4 qv[CH];
+#pragma unroll
+      for (int c = 0; c < CH; ++c) qv[c] = lane + 32 * c < nv ? sq4[lane + 32 * c] : make_float4(0.f, 0.f, 0.f, 0.f);
+      // (one query: a live row is one the query may see, its mask is not needed again)
+      uint64_t rmask[FEW_ROWS];
+      uint32_t rid[FEW_ROWS];
+      float4 x[FEW_ROWS][CH];
+      auto fetch = [&](const bool (&live)[FEW_ROWS]) {
+#pragma unroll
+        for (int r = 0; r < FEW_ROWS; ++r)
+#pragma unroll
+          for (int c = 0; c < CH; ++c)
+            x[r][c] = (live[r] && lane + 32 * c < nv) ? __ldg(reinterpret_cast<const float4*>(a.x + (int64_t)rid[r] * dim) + lane + 32 * c)
+                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+      };
+      bool live[FEW_ROWS];
+      if (n0 < r1) {
+        locate(n0, r1, rid, rmask, live);
+        fetch(live);
+      }
+      for (; n0 < r1; n0 += FEW_WARPS * FEW_ROWS) {
+        float acc[V];
+#pragma unroll
+        for (int r = 0; r < FEW_ROWS; ++r) {
+          acc[r] = 0.f;
+#pragma unroll
+          for (int c = 0; c < CH; ++c) {
+            if (lane + 32 * c >= nv) continue;
+            tile::accum<METRIC>(acc[r], qv[c].x, x[r][c].x);
+            tile::accum<METRIC>(acc[r], qv[c].y, x[r][c].y);
+            tile::accum<METRIC>(acc[r], qv[c].z, x[r][c].z);
+            tile::accum<METRIC>(acc[r], qv[c].w, x[r][c].w);
+          }
+        }
+        // the next step's rows are on their way while this one's sums are exchanged and listed
+        uint32_t was[FEW_ROWS];
+        bool had[FEW_ROWS];
+#pragma unroll
+        for (int r = 0; r < FEW_ROWS; ++r) {
+          was[r] = rid[r];
+          had[r] = live[r];
+          rmask[r] = ~0ull;
+        }
+        const int64_t n1 = n0 + FEW_WARPS * FEW_ROWS;
+        if (n1 < r1) {
+          locate(n1, r1, rid, rmask, live);
+          fetch(live);
+#pragma unroll
+          for (int r = 0; r < FEW_ROWS; ++r) rmask[r] = ~0ull;
+        }
+        list_step(acc, n0, was, rmask, had);
+      }
+    } else {
+      for (; n0 < r1; n0 += FEW_WARPS * FEW_ROWS) {
+        bool live[FEW_ROWS];
+        uint32_t rid[FEW_ROWS];
+        uint64_t rmask[FEW_ROWS];
+        locate(n0, r1, rid, rmask, live);
+        float acc[V];
+#pragma unroll
+        for (int j = 0; j < V; ++j) acc[j] = 0.f;
+        stream_accumulate<METRIC, NQ, VEC, FEW_ROWS>(acc, a.x, dim, sq, rid, live, lane);
+        list_step(acc, n0, rid, rmask, live);
+      }
+    }
+    if (NQ == 1 && a.id_remap) {
+      __syncthreads();
+      const int cnt = s_cnt[0];
+      for (int j = done + threadIdx.x; j < cnt; j += FEW_THREADS)
+        lists[j] = (lists[j] & 0xffffffff00000000ull) | (uint32_t)*VSK_CHK(a.id_remap + (uint32_t)lists[j]);
+    }
+    few_end_round(lists, nq_here, k, ka.stride, r0 + stride >= n, s_cnt, s_thr, fs);
+    done = s_cnt[0];
   }
   // ---- this CTA's lists, and the merge by the last one to arrive ----
-  few_write_lists(ka, lists, qp, nq_here, k, s_cnt);
+  few_write_lists(ka, lists, qp, nq_here, s_cnt);
   if (NQ > 1) return;   // several queries: few_merge_kernel merges them side by side
   __threadfence();
   __syncthreads();
@@ -323,7 +441,7 @@ struct FewHalf {
   float inv_scale;        // 1 / s
   float err, norm;        // largest |s x - x16| / s and |x16| / s of a row
   float max_norm, min_norm_nz;
-  int32_t* flags;         // [nq], set to 0 or 1
+  int32_t* flags;         // [nq] (pinned host memory), set to 0 or 1
 };
 
 // |coarse - exact| for every row, in coarse units (bound_kernel's terms with an unrounded query)
@@ -341,8 +459,13 @@ __device__ __forceinline__ float few_eps(const FewHalf& h, int dim, float qn) {
   return e * 1.0001f + 1e-30f;
 }
 
-template <int METRIC, int NQ>
-__global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_coarse_kernel(FewKernelArgs ka, FewHalf h) {
+template <int METRIC>
+__device__ __forceinline__ void few_refine(const FewKernelArgs& ka, const FewHalf& h, int lists, int64_t pos, const float* q, uint64_t* list,
+                                           unsigned short* cand, FewScratch& fs);
+
+template <int METRIC, int NQ, bool INL>
+__global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_coarse_kernel(const __grid_constant__ FewKernelArgs ka, FewHalf h,
+                                                                                const __grid_constant__ FewInline<INL> iq) {
   const FewArgs& a = ka.a;
   extern __shared__ __align__(16) uint8_t smem[];
   uint64_t* lists = reinterpret_cast<uint64_t*>(smem);                       // [NQ][FEW_LIST]
@@ -361,7 +484,7 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_coarse_kernel
   for (int i = warp; i < NQ; i += FEW_WARPS) {
     float ss = 0.f;
     for (int c = lane; c < dim; c += 32) {
-      const float v = i < nq ? __ldg(a.q + (int64_t)i * dim + c) : 0.f;
+      const float v = i < nq ? few_query<INL>(iq, a.q, (int64_t)i * dim + c) : 0.f;
       ss = fmaf(v, v, ss);
     }
 #pragma unroll
@@ -369,7 +492,7 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_coarse_kernel
     const float qn = sqrtf(ss), f = METRIC == VSK_METRIC_COSINE ? (qn > 0.f ? 1.0f / qn : 0.f) : 1.0f;
     if (lane == 0) s_qn[i] = qn;
     for (int c = lane; c < h.dim16; c += 32) {
-      const float v = (i < nq && c < dim) ? __ldg(a.q + (int64_t)i * dim + c) * f : 0.f;
+      const float v = (i < nq && c < dim) ? few_query<INL>(iq, a.q, (int64_t)i * dim + c) * f : 0.f;
       reinterpret_cast<float*>(sq)[((i * 2 + ((c >> 2) & 1)) * nv + (c >> 3)) * 4 + (c & 3)] = v;
     }
   }
@@ -422,28 +545,38 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_coarse_kernel
         }
       }
     }
-    few_end_round(lists, nq, keep, r0 + stride >= n, s_cnt, s_thr, fs);
+    few_end_round(lists, nq, keep, ka.stride, r0 + stride >= n, s_cnt, s_thr, fs);
   }
-  few_write_lists(ka, lists, 0, nq, keep, s_cnt);
+  few_write_lists(ka, lists, 0, nq, s_cnt);
+  if (NQ > 1) return;   // several queries: few_refine_kernel takes them side by side
+  __shared__ unsigned s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(ka.ticket, 1u);
+  __syncthreads();
+  if (s_last != gridDim.x - 1) return;
+  __threadfence();
+  if (threadIdx.x == 0) *VSK_CHK_W(ka.ticket) = 0u;
+  // the query as it is, where its halves were; behind it the list numbers
+  float* qs = reinterpret_cast<float*>(sq);
+  for (int c = threadIdx.x; c < dim; c += FEW_THREADS) qs[c] = few_query<INL>(iq, a.q, c);
+  __syncthreads();
+  few_refine<METRIC>(ka, h, (int)gridDim.x, 0, qs, lists, reinterpret_cast<unsigned short*>(qs + h.dim16), fs);
 }
 
-// One CTA per query: the rows within 2 eps of the k-th best coarse value, re-scored with the direct formulas and ordered.
+// The rows within 2 eps of the k-th best coarse value, re-scored with the direct formulas and ordered.
 template <int METRIC>
-__global__ void __launch_bounds__(FEW_THREADS) few_refine_kernel(FewKernelArgs ka, FewHalf h, int lists) {
-  __shared__ uint64_t list[FEW_LIST];
-  __shared__ unsigned short cand[FEW_MAX_CTAS];
-  __shared__ FewScratch fs;
+__device__ __forceinline__ void few_refine(const FewKernelArgs& ka, const FewHalf& h, int lists, int64_t pos, const float* q, uint64_t* list,
+                                           unsigned short* cand, FewScratch& fs) {
   __shared__ int n_cand, n_list, n_have, s_bad;
   __shared__ float s_qn;
   const FewArgs& a = ka.a;
   const int k = a.k, keep = k + kFewMargin, dim = a.dim;
-  const int64_t pos = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const float* q = a.q + pos * dim;
   if (threadIdx.x == 0) { n_cand = 0; n_list = 0; n_have = 0; s_bad = 0; }
   if (warp == 0) {
     float ss = 0.f;
-    for (int c = lane; c < dim; c += 32) ss = fmaf(__ldg(q + c), __ldg(q + c), ss);
+    for (int c = lane; c < dim; c += 32) ss = fmaf(*VSK_CHK(q + c), *VSK_CHK(q + c), ss);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if (lane == 0) s_qn = sqrtf(ss);
@@ -477,7 +610,7 @@ __global__ void __launch_bounds__(FEW_THREADS) few_refine_kernel(FewKernelArgs k
     const int m = __ldcg(VSK_CHK(ka.part_n + l));
     bool all = m >= keep;   // a shortened list whose every key is within the bound may have dropped such a row
     for (int i = lane; i < m; i += 32) {
-      const uint64_t v = __ldcg(VSK_CHK(ka.part + l * keep + i));
+      const uint64_t v = __ldcg(VSK_CHK(ka.part + l * ka.stride + i));
       if (v <= bound) {
         const int at = atomicAdd(&n_list, 1);
         if (at < FEW_LIST) list[at] = v;
@@ -519,7 +652,7 @@ __global__ void __launch_bounds__(FEW_THREADS) few_refine_kernel(FewKernelArgs k
       s[r] = 0.f;
     }
     for (int i = lane; i < dim; i += 32) {
-      const float qv = __ldg(q + i);
+      const float qv = *VSK_CHK(q + i);
 #pragma unroll
       for (int r = 0; r < RR; ++r) {
         const float xv = __ldg(a.x + (int64_t)id[r] * dim + i);
@@ -540,22 +673,16 @@ __global__ void __launch_bounds__(FEW_THREADS) few_refine_kernel(FewKernelArgs k
     }
   }
   __syncthreads();
-  const int P = next_pow2(cnt);
-  for (int i = cnt + threadIdx.x; i < P; i += FEW_THREADS) list[i] = kEmptyKey;
-  __syncthreads();
-  bitonic_sort(list, P);
-  for (int j = threadIdx.x; j < k; j += FEW_THREADS) {
-    float d = CUDART_INF_F;
-    int64_t id = -1;
-    if (j < cnt) {
-      d = ordered_to_float((uint32_t)(list[j] >> 32));
-      if (METRIC == VSK_METRIC_EUCLIDEAN) d = sqrtf(d);
-      id = (int64_t)(uint32_t)list[j] + a.id_base;
-    }
-    *VSK_CHK_W(a.out_dist + pos * k + j) = d;
-    *VSK_CHK_W(a.out_ids + pos * k + j) = id;
-  }
+  few_order(list, cnt, k, METRIC == VSK_METRIC_EUCLIDEAN, a.id_base, a.out_dist + pos * k, a.out_ids + pos * k);
   if (threadIdx.x == 0) *VSK_CHK_W(h.flags + pos) = 0;
+}
+
+template <int METRIC>
+__global__ void __launch_bounds__(FEW_THREADS) few_refine_kernel(FewKernelArgs ka, FewHalf h, int lists) {
+  __shared__ uint64_t list[FEW_LIST];
+  __shared__ unsigned short cand[FEW_MAX_CTAS];
+  __shared__ FewScratch fs;
+  few_refine<METRIC>(ka, h, lists, blockIdx.x, ka.a.q + (int64_t)blockIdx.x * ka.a.dim, list, cand, fs);
 }
 
 __global__ void __launch_bounds__(FEW_THREADS) few_merge_kernel(FewKernelArgs ka, int lists) {
@@ -574,30 +701,39 @@ size_t few_smem(const FewArgs& a) {
 }
 constexpr size_t kFewMaxSmem = 110 * 1024;   // two CTAs per SM
 
-template <int METRIC, int NQ, bool VEC, bool SEG>
-int32_t few_launch(Ctx* ctx, FewKernelArgs ka) {
+// The query of a host call that has not been copied to the device yet (HostQuery), when it fits the arguments.
+const float* few_inline_query(const Ctx* ctx, const FewArgs& a) {
+  return a.nq == 1 && a.dim <= kFewInline && ctx->host_query.pending && ctx->host_query.dev == a.q ? ctx->host_query.host : nullptr;
+}
+
+template <int METRIC, int NQ, bool VEC, bool SEG, int ROWS, int CH, bool INL>
+int32_t few_launch_as(Ctx* ctx, FewKernelArgs ka, const float* host_q) {
   const FewArgs& a = ka.a;
-  auto kern = few_topk_kernel<METRIC, NQ, VEC, SEG>;
+  auto kern = few_topk_kernel<METRIC, NQ, VEC, SEG, ROWS, CH, INL>;
   const size_t smem = few_smem<NQ>(a);
   if (smem > 48 * 1024) VSK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int sms = ctx->prop.multiProcessorCount;
   const int per_sm = std::max(1, std::min(NQ > 4 ? 2 : 3, (int)(220 * 1024 / (smem + 3072))));
-  // at least two warp steps of rows per CTA; per-query lists share the machine
-  const int64_t rows = std::max<int64_t>(a.n, 1);   // SEG: an estimate, the kernel takes the lists' true lengths
+  // 32 rows per CTA at least; per-query lists share the machine.  SEG: the mean list's length is known, but probed lists are the
+  // longer ones, and the kernel takes their true lengths
+  const int64_t rows = std::max<int64_t>(SEG ? 2 * a.n : a.n, 1);
   const int64_t nseg = SEG ? a.nq : 1;
-  constexpr int kStep = FEW_WARPS * FEW_ROWS;
-  const int64_t grid = std::min({ceil_div(rows, 2 * kStep), std::max<int64_t>(1, (int64_t)sms * per_sm / nseg), (int64_t)FEW_MAX_CTAS});
+  constexpr int kStep = FEW_WARPS * ROWS;
+  const int64_t grid = std::min({ceil_div(rows, 32), std::max<int64_t>(1, (int64_t)sms * per_sm / nseg), (int64_t)FEW_MAX_CTAS});
   // rounds of whole warp steps, such that the last one is spread evenly
   const int64_t share = ceil_div(rows, grid);
   ka.round = (int32_t)std::min<int64_t>(FEW_ROUND, ceil_div(ceil_div(share, ceil_div(share, (int64_t)FEW_ROUND)), kStep) * kStep);
+  ka.stride = std::max(a.k, kFewShort);
   void* p;
   const size_t lists = (size_t)a.nq * grid;
-  VSK_TRY(scratch(ctx, SLOT_FEW, lists * ((size_t)a.k * 8 + 8 + 4), &p));
+  VSK_TRY(scratch(ctx, SLOT_FEW, lists * ((size_t)ka.stride * 8 + 8 + 4), &p));
   ka.part = (uint64_t*)p;
-  ka.part_min = ka.part + lists * a.k;
+  ka.part_min = ka.part + lists * ka.stride;
   ka.part_n = (int32_t*)(ka.part_min + lists);
+  FewInline<INL> iq;
+  if constexpr (INL) memcpy(iq.q, host_q, (size_t)a.dim * sizeof(float));
   prof_begin(ctx);
-  kern<<<dim3((unsigned)grid, (unsigned)nseg), FEW_THREADS, smem, ctx->stream>>>(ka);
+  kern<<<dim3((unsigned)grid, (unsigned)nseg), FEW_THREADS, smem, ctx->stream>>>(ka, iq);
   prof_end(ctx);
   ctx->stats.kernel_launches++;
   if (NQ > 1) {
@@ -606,6 +742,26 @@ int32_t few_launch(Ctx* ctx, FewKernelArgs ka) {
   }
   VSK_CUDA(ctx, cudaGetLastError());
   return VSK_OK;
+}
+
+// One query over rows of at most 256 dimensions: four 16-byte loads per lane and step, the next step's already on their way
+// (the general form takes two rows per step and waits for them).
+template <int METRIC, int NQ, bool VEC, bool SEG, bool INL>
+int32_t few_launch_one(Ctx* ctx, const FewKernelArgs& ka, const float* host_q) {
+  if constexpr (VEC) {
+    if (ka.a.dim <= 128) return few_launch_as<METRIC, NQ, VEC, SEG, 4, 1, INL>(ctx, ka, host_q);
+    if (ka.a.dim <= 256) return few_launch_as<METRIC, NQ, VEC, SEG, 2, 2, INL>(ctx, ka, host_q);
+  }
+  return few_launch_as<METRIC, NQ, VEC, SEG, 2, 0, INL>(ctx, ka, host_q);
+}
+
+template <int METRIC, int NQ, bool VEC, bool SEG>
+int32_t few_launch(Ctx* ctx, const FewKernelArgs& ka) {
+  if constexpr (NQ == 1)
+    if (const float* host_q = few_inline_query(ctx, ka.a)) return few_launch_one<METRIC, NQ, VEC, SEG, true>(ctx, ka, host_q);
+  VSK_TRY(host_query_upload(ctx));
+  if constexpr (NQ == 1) return few_launch_one<METRIC, NQ, VEC, SEG, false>(ctx, ka, nullptr);
+  else return few_launch_as<METRIC, NQ, VEC, SEG, 2, 0, false>(ctx, ka, nullptr);
 }
 
 template <int METRIC>
@@ -621,41 +777,60 @@ int32_t few_metric(Ctx* ctx, const FewKernelArgs& ka, bool vec) {
 
 namespace {
 
-template <int METRIC, int NQ>
-int32_t few_half_launch(Ctx* ctx, FewKernelArgs ka, const FewHalf& h) {
+template <int METRIC, int NQ, bool INL>
+int32_t few_half_launch(Ctx* ctx, FewKernelArgs ka, const FewHalf& h, const float* host_q) {
   const FewArgs& a = ka.a;
-  auto kern = few_coarse_kernel<METRIC, NQ>;
-  const size_t smem = (size_t)NQ * (FEW_LIST * 8 + (size_t)h.dim16 * 4);
+  auto kern = few_coarse_kernel<METRIC, NQ, INL>;
+  const size_t smem = (size_t)NQ * (FEW_LIST * 8 + (size_t)h.dim16 * 4) + (NQ == 1 ? FEW_MAX_CTAS * sizeof(unsigned short) : 0);
   if (smem > 48 * 1024) VSK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int per_sm = std::max(1, std::min(NQ > 4 ? 2 : 3, (int)(220 * 1024 / (smem + 3072))));
   constexpr int kStep = FEW_WARPS * FEWH_ROWS;
   const int64_t grid = std::min<int64_t>(ceil_div(a.n, kStep), (int64_t)ctx->prop.multiProcessorCount * per_sm);
   const int64_t share = ceil_div(a.n, grid);
   ka.round = (int32_t)std::min<int64_t>(FEW_ROUND, ceil_div(ceil_div(share, ceil_div(share, (int64_t)FEW_ROUND)), kStep) * kStep);
+  ka.stride = a.k + kFewMargin;
   void* p;
-  const size_t lists = (size_t)a.nq * grid, keep = (size_t)a.k + kFewMargin;
-  VSK_TRY(scratch(ctx, SLOT_FEW, lists * (keep * 8 + 8 + 4), &p));
+  const size_t lists = (size_t)a.nq * grid;
+  VSK_TRY(scratch(ctx, SLOT_FEW, lists * ((size_t)ka.stride * 8 + 8 + 4), &p));
   ka.part = (uint64_t*)p;
-  ka.part_min = ka.part + lists * keep;
+  ka.part_min = ka.part + lists * ka.stride;
   ka.part_n = (int32_t*)(ka.part_min + lists);
+  FewInline<INL> iq;
+  if constexpr (INL) memcpy(iq.q, host_q, (size_t)a.dim * sizeof(float));
   prof_begin(ctx);
-  kern<<<(unsigned)grid, FEW_THREADS, smem, ctx->stream>>>(ka, h);
+  kern<<<(unsigned)grid, FEW_THREADS, smem, ctx->stream>>>(ka, h, iq);
   prof_end(ctx);
-  few_refine_kernel<METRIC><<<(unsigned)a.nq, FEW_THREADS, 0, ctx->stream>>>(ka, h, (int)grid);
-  ctx->stats.kernel_launches += 2;
+  ctx->stats.kernel_launches++;
+  if (NQ > 1) {
+    few_refine_kernel<METRIC><<<(unsigned)a.nq, FEW_THREADS, 0, ctx->stream>>>(ka, h, (int)grid);
+    ctx->stats.kernel_launches++;
+  }
   VSK_CUDA(ctx, cudaGetLastError());
   return VSK_OK;
 }
 
 template <int METRIC>
 int32_t few_half_metric(Ctx* ctx, const FewKernelArgs& ka, const FewHalf& h) {
-  if (ka.a.nq <= 1) return few_half_launch<METRIC, 1>(ctx, ka, h);
-  if (ka.a.nq <= 2) return few_half_launch<METRIC, 2>(ctx, ka, h);
-  if (ka.a.nq <= 4) return few_half_launch<METRIC, 4>(ctx, ka, h);
-  return few_half_launch<METRIC, 8>(ctx, ka, h);
+  if (const float* host_q = few_inline_query(ctx, ka.a)) return few_half_launch<METRIC, 1, true>(ctx, ka, h, host_q);
+  VSK_TRY(host_query_upload(ctx));
+  if (ka.a.nq <= 1) return few_half_launch<METRIC, 1, false>(ctx, ka, h, nullptr);
+  if (ka.a.nq <= 2) return few_half_launch<METRIC, 2, false>(ctx, ka, h, nullptr);
+  if (ka.a.nq <= 4) return few_half_launch<METRIC, 4, false>(ctx, ka, h, nullptr);
+  return few_half_launch<METRIC, 8, false>(ctx, ka, h, nullptr);
 }
 
 }  // namespace
+
+// zeroed once: the last CTA of a query leaves its ticket at zero
+static int32_t few_tickets(Ctx* ctx, unsigned** out) {
+  unsigned*& tickets = ctx->few_tickets[ctx->lane];
+  if (!tickets) {
+    VSK_TRY(dev_alloc(ctx, (void**)&tickets, kStreamScanMaxSegQueries * sizeof(unsigned)));
+    VSK_CUDA(ctx, cudaMemsetAsync(tickets, 0, kStreamScanMaxSegQueries * sizeof(unsigned), ctx->stream));
+  }
+  *out = tickets;
+  return VSK_OK;
+}
 
 int32_t few_search_half(Index* ix, const FewArgs& a, bool* handled) {
   VSK_TRACE("vsk:few_search_half");
@@ -675,19 +850,17 @@ int32_t few_search_half(Index* ix, const FewArgs& a, bool* handled) {
   h.norm = ix->max_xnorm16 * h.inv_scale;
   h.max_norm = ix->max_xnorm;
   h.min_norm_nz = ix->min_xnorm_nz;
-  void* p;
-  VSK_TRY(scratch(ctx, SLOT_CAND_FLAGS, (size_t)a.nq * sizeof(int32_t), &p));
-  h.flags = (int32_t*)p;
-  PinnedBuf& hb = ctx->host_flags[ctx->lane];
+  PinnedBuf& hb = ctx->host_flags[ctx->lane];   // the kernel's flags go straight to the host
   VSK_TRY(pinned_reserve(ctx, &hb, (size_t)a.nq * 4));
+  h.flags = (int32_t*)hb.p;
   FewKernelArgs ka{};
   ka.a = a;
+  VSK_TRY(few_tickets(ctx, &ka.ticket));
   switch (a.metric) {
     case VSK_METRIC_EUCLIDEAN: VSK_TRY(few_half_metric<VSK_METRIC_EUCLIDEAN>(ctx, ka, h)); break;
     case VSK_METRIC_COSINE: VSK_TRY(few_half_metric<VSK_METRIC_COSINE>(ctx, ka, h)); break;
     default: VSK_TRY(few_half_metric<VSK_METRIC_DOT_PRODUCT>(ctx, ka, h)); break;
   }
-  VSK_CUDA(ctx, cudaMemcpyAsync(hb.p, h.flags, (size_t)a.nq * 4, cudaMemcpyDeviceToHost, ctx->stream));
   VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   int64_t bad = 0;
   for (int64_t i = 0; i < a.nq; ++i) bad += ((const int32_t*)hb.p)[i] != 0;
@@ -710,12 +883,7 @@ int32_t few_search(Ctx* ctx, const FewArgs& a) {
   FewKernelArgs ka{};
   ka.a = a;
   ka.a.nan_rows = schedule_dense_rows(ctx, a.k);
-  unsigned*& tickets = ctx->few_tickets[ctx->lane];
-  if (!tickets) {   // zeroed once: the last CTA of a query leaves its ticket at zero
-    VSK_TRY(dev_alloc(ctx, (void**)&tickets, kStreamScanMaxSegQueries * sizeof(unsigned)));
-    VSK_CUDA(ctx, cudaMemsetAsync(tickets, 0, kStreamScanMaxSegQueries * sizeof(unsigned), ctx->stream));
-  }
-  ka.ticket = tickets;
+  VSK_TRY(few_tickets(ctx, &ka.ticket));
   const bool vec = a.dim % 4 == 0 && (reinterpret_cast<uintptr_t>(a.x) & 15) == 0;
   if (a.probes)
     return vec ? few_launch<VSK_METRIC_EUCLIDEAN, 1, true, true>(ctx, ka) : few_launch<VSK_METRIC_EUCLIDEAN, 1, false, true>(ctx, ka);

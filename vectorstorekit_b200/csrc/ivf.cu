@@ -708,6 +708,7 @@ int32_t ivf_search_dev(Index* ix, const float* q, int64_t nq, int32_t k, int32_t
         VSK_TRY(few_search(ctx, g));
       }
     } else {
+      VSK_TRY(host_query_upload(ctx));
       ExactScanArgs c{};
       c.metric = VSK_METRIC_EUCLIDEAN;
       c.q = qb;
@@ -772,6 +773,7 @@ int32_t ivf_search_dev(Index* ix, const float* q, int64_t nq, int32_t k, int32_t
         VSK_TRY(few_search(ctx, f));
         continue;
       }
+      VSK_TRY(host_query_upload(ctx));
       bool few = false;
       VSK_TRY(ivf_search_few(ctx, ix, qb, bn, (const int64_t*)pi, nprobe, k, mb, out_dist + b * k, out_ids + b * k, &few));
       if (few) continue;
@@ -933,8 +935,10 @@ int32_t vsk_ivf_search_filtered(vsk_index* i, const float* q, int64_t nq, int32_
   if (k <= 0) return fail(ctx, VSK_ERR_INVALID_INPUT, "k must be positive");
   if (!q || !out_dist || !out_ids) return fail(ctx, VSK_ERR_INVALID_INPUT, "null pointer");
   HostCall c;
-  VSK_TRY(host_call_begin(ctx, q, nq, ix->dim, qmasks, k, &c));
-  VSK_TRY(ivf_search_dev(ix, c.q, nq, k, nprobe, c.masks, c.dist, c.ids));
+  VSK_TRY(host_call_begin(ctx, q, nq, ix->dim, qmasks, k, &c, true));
+  const int32_t st = ivf_search_dev(ix, c.q, nq, k, nprobe, c.masks, c.dist, c.ids);
+  ctx->host_query.pending = false;
+  VSK_TRY(st);
   VSK_TRY(host_call_end(ctx, c, nq, ix->dim, k, out_dist, out_ids));
   return VSK_OK;
 }
