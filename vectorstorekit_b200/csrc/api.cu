@@ -593,17 +593,17 @@ static int32_t flat_search_dev(Index* ix, const float* q, int64_t nq, int32_t k,
       }
     }
     VSK_TRY(host_query_upload(ctx));
+    // Euclidean, cosine and dot-product batches take the tensor path, filtered or not (the filter is applied to the
+    // hits in the contraction's epilogue).  A batch of a few queries is bound by the bytes it reads, not by the
+    // contraction: the fp32 streaming scan reads each eligible fp32 row once.
+    const bool tensor = tensor_metric && !(mb && bn <= kStreamScanMaxQueries);
     float* qnorm = nullptr;
-    if (ix->metric == VSK_METRIC_COSINE) {
+    if (ix->metric == VSK_METRIC_COSINE && (mb || !tensor)) {   // (the tensor path measures its queries itself)
       void* p;
       VSK_TRY(scratch(ctx, SLOT_QNORM, bn * sizeof(float), &p));
       qnorm = (float*)p;
       VSK_TRY(launch_row_norms(ctx, qb, bn, ix->dim, 0, qnorm));
     }
-    // Euclidean, cosine and dot-product batches take the tensor path, filtered or not (the filter is applied to the
-    // hits in the contraction's epilogue).  A batch of a few queries is bound by the bytes it reads, not by the
-    // contraction: the fp32 streaming scan reads each eligible fp32 row once.
-    const bool tensor = tensor_metric && !(mb && bn <= kStreamScanMaxQueries);
     bool grouped = false;
     L1Call l1;
     l1.queries = bn;

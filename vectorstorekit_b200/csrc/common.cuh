@@ -140,6 +140,8 @@ struct ShardPending {
   const float* eps = nullptr;
   int32_t* err = nullptr;
   unsigned long long* rr_total = nullptr;
+  bool fused = false;         // the second half is one launch (finish_kernel), with ...
+  int32_t dense_count = -1;   // ... the length of a list that only the dense first chunk has written
   // second half issued, results not yet looked at by the host
   bool issued = false;
   float* out_dist = nullptr;

@@ -33,6 +33,7 @@
 #include <climits>
 #include <cmath>
 
+#include "block_select.cuh"
 #include "common.cuh"
 #include "tensor_scan.cuh"
 #include "tc_ptx.cuh"
@@ -84,7 +85,8 @@ struct TcArgs {
   int32_t stage_kblocks;      // K blocks per ring stage: 1 (four stages of 48 KB) or 2 (two stages of 96 KB: half the
                               // hand-overs between producer, MMA issuer and ring)
   int mode;                   // SCAN_DENSE or SCAN_THRESHOLD
-  const float* alpha;         // device scalar: value = alpha * acc + beta[row]
+  const float* alpha;         // value = alpha * acc + beta[row]: device scalar ...
+  int32_t alpha_per_query;    // ... or [nq] by list position
   const float* beta;          // [n] or null (treated as 0)
   CandLists cand;
   int32_t cap;                // keys per candidate list (SCAN_THRESHOLD)
@@ -289,7 +291,7 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     const int ew = warp - 2;                      // epilogue warp 0..7
     const int part = ew >> 2;                     // which part of the tile's columns this warp takes
     const int c0 = part * EPI_GROUPS;             // first 32-column group of that part
-    const float alpha = __ldg(a.alpha);
+    float alpha = a.alpha_per_query ? -1.0f : __ldg(a.alpha);
     int64_t local = 0;
     bool ok = true;
     int run_cnt = 0;                 // row-tile-fastest order: keys this thread has stored for its query so far
@@ -363,6 +365,7 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       }
       float thr = CUDART_INF_F;
       if (MODE == SCAN_THRESHOLD && qok) thr = a.tiles ? thr_tile : a.cand.thr[q];
+      if (a.alpha_per_query && qok) alpha = __ldg(a.alpha + q);
       uint64_t qm = 0ull;   // this query's filter mask: a row is eligible iff (row mask & qm) != 0
       if (HAS_MASK && qok) qm = __ldg(a.q_masks + q);
       // every lane of the warp must take part in the wait result
@@ -1499,19 +1502,21 @@ __global__ void absmax_kernel(const float* __restrict__ x, int64_t total, unsign
 // scale = 2^e with 2^13 < absmax * scale <= 2^14 (1 when absmax is 0 or not finite); cosine: 2^14
 // fold != 0 (queries against folded rows, see FoldArgs): the scale is also kept where the folded constant
 // s 2^-exp is a normal fp16 number.
-__global__ void choose_scale_kernel(const unsigned* absmax, int cosine, float* scale, int fold = 0, int fold_exp = 0) {
+__device__ __forceinline__ float operand_scale(bool cosine, float absmax, bool fold, int fold_exp) {
   float s = 16384.f;
   if (!cosine) {
-    const float m = __uint_as_float(*absmax);
     s = 1.f;
-    if (m > 0.f && m < CUDART_INF_F) {
+    if (absmax > 0.f && absmax < CUDART_INF_F) {
       int e;
-      frexpf(m, &e);               // m = f * 2^e, f in [0.5, 1)
+      frexpf(absmax, &e);          // absmax = f * 2^e, f in [0.5, 1)
       s = ldexpf(1.f, 14 - e);
     }
   }
   if (fold) s = fmaxf(fminf(s, ldexpf(1.f, fold_exp + 13)), ldexpf(1.f, fold_exp - 14));   // 4u <= 2^15, 2u normal
-  *scale = s;
+  return s;
+}
+__global__ void choose_scale_kernel(const unsigned* absmax, int cosine, float* scale, int fold = 0, int fold_exp = 0) {
+  *scale = operand_scale(cosine != 0, __uint_as_float(*absmax), fold != 0, fold_exp);
 }
 
 // One warp per row: fp32 row -> fp16 operand row x' = fp16(s * x) (cosine: s * x/|x|), padded with
@@ -1625,14 +1630,7 @@ struct BoundConsts {
 //   cosine adds the effect of the reference's +1e-8 in the denominator and of normalising in fp32.
 // Also writes alpha = coefficient / (s_q s_x).
 template <int METRIC>
-__global__ void bound_kernel(const float* __restrict__ qn16, const float* __restrict__ qe16,
-                             const float* __restrict__ qnorm, int64_t nq, const float* scale_q, BoundConsts c,
-                             float* __restrict__ eps, float* alpha) {
-  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const float inv = 1.0f / ((*scale_q) * c.scale_x);
-  if (q == 0) *alpha = (METRIC == VSK_METRIC_EUCLIDEAN ? -2.0f : -1.0f) * inv;
-  if (q >= nq) return;
-  const float a = qn16[q], e = qe16[q];
+__device__ __forceinline__ float query_eps(float a, float e, float qn, float inv, const BoundConsts& c) {
   float dot_err = (a * c.max_err16 + e * c.max_norm16 + e * c.max_err16) + (float)c.dim16 * 2.3841858e-7f * a * c.max_norm16;
   dot_err *= inv;
   // folded per-row term (true units): its products pass through the same fp32 accumulation, and three fp16 pieces
@@ -1641,18 +1639,94 @@ __global__ void bound_kernel(const float* __restrict__ qn16, const float* __rest
   float r;
   if (METRIC == VSK_METRIC_EUCLIDEAN) {
     // + fp32 rounding of the stored |x|^2 (a sum of dim squares) and of the final multiply-add
-    const float qn = qnorm[q];
     r = 2.0f * dot_err + 4.0f * 5.9604645e-8f * (float)c.dim16 * c.max_norm * c.max_norm +
         2.0f * 5.9604645e-8f * (c.max_norm * c.max_norm + 2.0f * qn * c.max_norm);
   } else if (METRIC == VSK_METRIC_COSINE) {
-    const float qn = qnorm[q];
     const float den = qn * c.min_norm_nz;
     r = dot_err + 1e-8f / (den + 1e-8f) + 4.0f * 5.9604645e-8f;
     if (!(den > 0.f)) r = dot_err + 4.0f * 5.9604645e-8f;  // zero query (or no nonzero row): every value is exactly 0
   } else {
     r = dot_err;
   }
-  eps[q] = r * 1.0001f + 1e-30f;
+  return r * 1.0001f + 1e-30f;
+}
+
+template <int METRIC>
+__global__ void bound_kernel(const float* __restrict__ qn16, const float* __restrict__ qe16,
+                             const float* __restrict__ qnorm, int64_t nq, const float* scale_q, BoundConsts c,
+                             float* __restrict__ eps, float* alpha) {
+  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const float inv = 1.0f / ((*scale_q) * c.scale_x);
+  if (q == 0) *alpha = (METRIC == VSK_METRIC_EUCLIDEAN ? -2.0f : -1.0f) * inv;
+  if (q >= nq) return;
+  eps[q] = query_eps<METRIC>(qn16[q], qe16[q], qnorm[q], inv, c);
+}
+
+// All a flat search needs of its queries in one launch, a warp per query: a power-of-two scale of the query's own (as
+// choose_scale_kernel picks the batch's), the fp16 operand row with its fold constants, |q|, the error bound, the coefficient of
+// the values, and empty candidate lists.  With a scale for the whole batch this took a pass over the queries for it and five
+// launches more, 30 of the 207 us of 1 000 queries over 100 000 x 128.
+struct QueryPrep {
+  const float* q;
+  int64_t nq;
+  int32_t dim, dim16;
+  BoundConsts c;
+  FoldArgs fold;            // side 2 or 0
+  __half* out;
+  float *alpha, *eps, *norm;
+  CandLists cand;
+  uint64_t* words;          // eight words to be zeroed (error word, counters)
+};
+
+template <int METRIC>
+__global__ void __launch_bounds__(256) query_prep_kernel(QueryPrep a) {
+  if (blockIdx.x == 0 && threadIdx.x < 8) *VSK_CHK_W(a.words + threadIdx.x) = 0ull;
+  const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= a.nq) return;
+  const int lane = threadIdx.x & 31;
+  const float* p = a.q + row * a.dim;
+  float ss = 0.f, top = 0.f;
+  for (int i = lane; i < a.dim; i += 32) {
+    const float v = __ldg(p + i);
+    ss = fmaf(v, v, ss);
+    top = fmaxf(top, fabsf(v));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+  }
+  const float norm = sqrtf(ss);
+  const float unit = (METRIC == VSK_METRIC_COSINE) ? (norm > 0.f ? 1.0f / norm : 0.f) : 1.0f;
+  const float s = operand_scale(METRIC == VSK_METRIC_COSINE, top, a.fold.side != 0, a.fold.exp);
+  float n2 = 0.f, e2 = 0.f;
+  __half* out = a.out + row * a.dim16;
+  for (int i = lane; i < a.dim16; i += 32) {
+    float t = 0.f;
+    if (i < a.dim) t = (METRIC == VSK_METRIC_COSINE) ? (__ldg(p + i) * unit) * s : __ldg(p + i) * s;
+    __half h = __float2half_rn(t);
+    const float back = __half2float(h);
+    n2 = fmaf(back, back, n2);
+    const float e = t - back;
+    e2 = fmaf(e, e, e2);
+    const int f = i - a.fold.col0;   // 4u against the four copies of p0 and of p1, 2u against the eight copies of p2
+    if (a.fold.side != 0 && f >= 0 && f < kFoldCols) h = __float2half_rn(ldexpf(s, (f < 8 ? 2 : 1) - a.fold.exp));
+    *VSK_CHK_W(out + i) = h;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+    e2 += __shfl_xor_sync(0xffffffffu, e2, o);
+  }
+  if (lane == 0) {
+    const float up = 1.0f + 1e-5f, inv = 1.0f / (s * a.c.scale_x);
+    *VSK_CHK_W(a.alpha + row) = (METRIC == VSK_METRIC_EUCLIDEAN ? -2.0f : -1.0f) * inv;
+    *VSK_CHK_W(a.eps + row) = query_eps<METRIC>(sqrtf(n2) * up, sqrtf(e2) * up, norm, inv, a.c);
+    *VSK_CHK_W(a.norm + row) = norm;
+    *VSK_CHK_W(a.cand.count + row) = 0;
+    *VSK_CHK_W(a.cand.thr + row) = CUDART_INF_F;
+    *VSK_CHK_W(a.cand.flags + row) = 0;
+  }
 }
 
 // ---- int8-coded rows -----------------------------------------------------------------------
@@ -1810,6 +1884,156 @@ __global__ void __launch_bounds__(256) rerank_kernel(const float* __restrict__ q
       }
     }
   }
+}
+
+// ---- the second half of a flat search in one launch -------------------------------------------
+// One CTA per query: the last compaction with its certificate (select_kernel's, see there), the exact values of the rows it
+// keeps (rerank_kernel's formulas, summed in its order), the final order, and the query's flags (low byte) with the number of
+// re-scored rows to the host.  The kept keys never leave shared memory, the rows of one query are fetched while another one's
+// list is ordered, and two launches, the copies of the flags and the gaps between them are gone.
+struct FinishArgs {
+  CandLists cand;
+  int32_t dense_count;        // >= 0: the list holds exactly this many slots
+  const float *q, *x, *qnorm, *xnorm;
+  int32_t dim, k;
+  const float* eps;
+  const float* ext_bound;     // or null (SelectArgs::ext_bound)
+  float* out_dist;
+  int64_t* out_ids;
+  int64_t id_base;
+  const int32_t* err;         // device error word of the scans
+  int32_t* host_err;          // pinned host memory ...
+  int32_t* host_flags;        // [nq]
+};
+template <int NT> constexpr int kFinishMinBlocks = NT == 128 ? 8 : 2;
+
+template <int METRIC, int NT>
+__global__ void __launch_bounds__(NT, kFinishMinBlocks<NT>) finish_kernel(FinishArgs a) {
+  extern __shared__ __align__(16) uint64_t s_keys[];
+  constexpr int CAPACITY = NT * SEL_ITEMS;
+  float* qs = reinterpret_cast<float*>(s_keys + CAPACITY);
+  __shared__ int hist[256];
+  __shared__ int s_valid, s_bin, s_less, s_in_bin, s_out;
+  const int64_t qi = blockIdx.x;
+  const uint64_t* keys = a.cand.keys + qi * kCandCap;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int raw = a.dense_count >= 0 ? a.dense_count : *VSK_CHK(a.cand.count + qi);
+  const int c = min(raw, CAPACITY);
+  uint64_t key[SEL_ITEMS];
+  int nvalid = 0;
+#pragma unroll
+  for (int i = 0; i < SEL_ITEMS; ++i) {
+    const int idx = threadIdx.x + i * NT;
+    key[i] = idx < c ? *VSK_CHK(keys + idx) : kEmptyKey;
+    nvalid += key[i] != kEmptyKey;
+  }
+  for (int i = threadIdx.x; i < a.dim; i += NT) qs[i] = *VSK_CHK(a.q + qi * a.dim + i);
+  if (threadIdx.x == 0) { s_valid = 0; s_out = 0; }
+  __syncthreads();
+  nvalid = __reduce_add_sync(0xffffffffu, nvalid);
+  if (lane == 0) atomicAdd(&s_valid, nvalid);
+  __syncthreads();
+  // a row of the true top-k has coarse value <= c_k + 2 eps; the list is complete only below the threshold that filtered the scan
+  float bound = CUDART_INF_F;
+  bool have = false;
+  if (s_valid >= a.k) {
+    const uint64_t kth = block_radix_select(key, a.k, hist, &s_bin, &s_less, &s_in_bin);
+    bound = ordered_to_float((uint32_t)(kth >> 32)) + 2.0f * *VSK_CHK(a.eps + qi);
+    have = true;
+  }
+  if (a.ext_bound != nullptr && *VSK_CHK(a.ext_bound + qi) < CUDART_INF_F) {
+    bound = fminf(bound, *VSK_CHK(a.ext_bound + qi) + *VSK_CHK(a.eps + qi));
+    have = true;
+  }
+  uint64_t pivot = kEmptyKey - 1;
+  if (have) {
+    pivot = ((uint64_t)float_to_ordered(bound) << 32) | 0xffffffffull;
+    if (pivot == kEmptyKey) pivot = kEmptyKey - 1;
+  }
+#pragma unroll
+  for (int i = 0; i < SEL_ITEMS; ++i)
+    if (key[i] <= pivot && key[i] != kEmptyKey) s_keys[atomicAdd(&s_out, 1)] = key[i];
+  __syncthreads();
+  const int cnt = s_out;
+  if (threadIdx.x == 0) {
+    int flags = *VSK_CHK(a.cand.flags + qi);
+    if (raw > CAPACITY) flags |= 1;
+    if (have && !(bound < *VSK_CHK(a.cand.thr + qi))) flags |= 2;
+    *VSK_CHK_W(a.host_flags + qi) = flags | (cnt << 8);
+    if (qi == 0) *VSK_CHK_W(a.host_err) = *VSK_CHK(a.err);
+  }
+  // exact values: four rows per warp step, four loads of each in flight
+  const float qn = (METRIC == VSK_METRIC_COSINE) ? *VSK_CHK(a.qnorm + qi) : 0.f;
+  constexpr int RR = 4, U = 4;
+  for (int c0 = warp * RR; c0 < cnt; c0 += (NT / 32) * RR) {
+    uint32_t id[RR];
+    const float* xr[RR];
+    float sum[RR];
+#pragma unroll
+    for (int r = 0; r < RR; ++r) {
+      id[r] = (uint32_t)s_keys[min(c0 + r, cnt - 1)];
+      xr[r] = a.x + (int64_t)id[r] * a.dim;
+      sum[r] = 0.f;
+    }
+    for (int i0 = lane; i0 < a.dim; i0 += 32 * U) {
+      float xv[RR][U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int r = 0; r < RR; ++r) xv[r][u] = i0 + 32 * u < a.dim ? __ldg(xr[r] + i0 + 32 * u) : 0.f;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const float qv = i0 + 32 * u < a.dim ? qs[i0 + 32 * u] : 0.f;
+#pragma unroll
+        for (int r = 0; r < RR; ++r) {
+          if (METRIC == VSK_METRIC_EUCLIDEAN) {
+            const float d = qv - xv[r][u];
+            sum[r] = fmaf(d, d, sum[r]);
+          } else {
+            sum[r] = fmaf(qv, xv[r][u], sum[r]);
+          }
+        }
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < RR; ++r) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o);
+      if (lane == 0 && c0 + r < cnt) {
+        float v;
+        if (METRIC == VSK_METRIC_COSINE) v = 1.0f - sum[r] / (qn * __ldg(a.xnorm + id[r]) + 1e-8f);
+        else if (METRIC == VSK_METRIC_DOT_PRODUCT) v = -sum[r];
+        else v = sum[r];
+        s_keys[c0 + r] = make_key(v, id[r]);
+      }
+    }
+  }
+  __syncthreads();
+  auto put = [&](int j, uint64_t key1, bool has) {
+    float d = has ? ordered_to_float((uint32_t)(key1 >> 32)) : CUDART_INF_F;
+    if (has && METRIC == VSK_METRIC_EUCLIDEAN) d = sqrtf(d);
+    *VSK_CHK_W(a.out_dist + qi * a.k + j) = d;
+    *VSK_CHK_W(a.out_ids + qi * a.k + j) = has ? (int64_t)(uint32_t)key1 + a.id_base : -1;
+  };
+  if (cnt <= 2 * NT) {   // keys are distinct: a key's place is the number of smaller ones
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int at = threadIdx.x + h * NT;
+      if (at >= cnt) continue;
+      const uint64_t mine = s_keys[at];
+      int below = 0;
+      for (int j = 0; j < cnt; ++j) below += s_keys[j] < mine;
+      if (below < a.k) put(below, mine, true);
+    }
+    for (int j = cnt + threadIdx.x; j < a.k; j += NT) put(j, 0ull, false);
+    return;
+  }
+  const int P = next_pow2(cnt);
+  for (int i = cnt + threadIdx.x; i < P; i += NT) s_keys[i] = kEmptyKey;
+  __syncthreads();
+  bitonic_sort(s_keys, P);
+  for (int j = threadIdx.x; j < a.k; j += NT) put(j, j < cnt ? s_keys[j] : 0ull, j < cnt);
 }
 
 // ---- host side ------------------------------------------------------------------------------
@@ -2383,10 +2607,11 @@ int32_t make_map_rows_f32(Ctx* ctx, const float* base, int64_t rows, int32_t dim
   return VSK_OK;
 }
 
-// ---- query operands of a flat search ------------------------------------------------------------------
-// fp16 operand rows of the queries, their error bound eps[q], the output coefficient alpha, and the small words a
+// ---- query operands of a search -----------------------------------------------------------------------
+// Over int8 codes or product-quantised rows: fp16 operand rows of the queries, their error bound eps[q], the output coefficient alpha, and the small words a
 // search needs (device error word, re-scored row counter), all in the current lane's scratch.
 struct QueryOperands {
+  float* norm = nullptr;    // [nq] |q| (flat_query_operands)
   __half* q16 = nullptr;
   float* eps = nullptr;
   float* alpha = nullptr;
@@ -2399,8 +2624,7 @@ int32_t prepare_query_operands(Index* ix, const float* q, int64_t nq, QueryOpera
   VSK_TRACE("vsk:query_operands");
   Ctx* ctx = ix->ctx;
   prefer_shared_carveout(ctx, absmax_kernel, choose_scale_kernel, scale_queries_kernel, prep_rows_kernel<VSK_METRIC_EUCLIDEAN>,
-                         prep_rows_kernel<VSK_METRIC_COSINE>, prep_rows_kernel<VSK_METRIC_DOT_PRODUCT>, bound_kernel<VSK_METRIC_EUCLIDEAN>,
-                         bound_kernel<VSK_METRIC_COSINE>, bound_kernel<VSK_METRIC_DOT_PRODUCT>, bound_i8_kernel<VSK_METRIC_EUCLIDEAN>,
+                         prep_rows_kernel<VSK_METRIC_COSINE>, prep_rows_kernel<VSK_METRIC_DOT_PRODUCT>, bound_kernel<VSK_METRIC_EUCLIDEAN>, bound_i8_kernel<VSK_METRIC_EUCLIDEAN>,
                          bound_i8_kernel<VSK_METRIC_DOT_PRODUCT>, rerank_kernel<VSK_METRIC_EUCLIDEAN>, rerank_kernel<VSK_METRIC_COSINE>,
                          rerank_kernel<VSK_METRIC_DOT_PRODUCT>, rerank_i8_kernel<VSK_METRIC_EUCLIDEAN>, rerank_i8_kernel<VSK_METRIC_DOT_PRODUCT>);
   const int metric = ix->metric;
@@ -2422,7 +2646,6 @@ int32_t prepare_query_operands(Index* ix, const float* q, int64_t nq, QueryOpera
   int32_t* err = (int32_t*)p + 3;
   unsigned long long* rr_total = (unsigned long long*)((char*)p + 16);
   VSK_CUDA(ctx, cudaMemsetAsync(p, 0, 64, ctx->stream));
-  const bool cosine = metric == VSK_METRIC_COSINE;
   const bool i8 = ix->kind == INDEX_FLAT_I8;
   if (i8 && metric != VSK_METRIC_EUCLIDEAN && metric != VSK_METRIC_DOT_PRODUCT)
     return fail(ctx, VSK_ERR_UNSUPPORTED_OPERATION, "the tensor path over int8 codes covers euclidean and dotProduct");
@@ -2438,14 +2661,12 @@ int32_t prepare_query_operands(Index* ix, const float* q, int64_t nq, QueryOpera
     q_true_norm = (float*)p;
     VSK_TRY(launch_row_norms(ctx, q, nq, dim, 0, q_true_norm));
   }
-  if (!cosine) {
-    absmax_kernel<<<296, 256, 0, ctx->stream>>>(qsrc, nq * (int64_t)dim, q_absmax);
-    ctx->stats.kernel_launches++;
-  }
+  absmax_kernel<<<296, 256, 0, ctx->stream>>>(qsrc, nq * (int64_t)dim, q_absmax);
+  ctx->stats.kernel_launches++;
   const bool fold = ix->fold16;
   const FoldArgs qfold{fold ? 2 : 0, fold_col0(ix->dim), ix->fold_exp};
   // (a product-quantised index may put twice the constants into the fold columns, list_scan_kernel)
-  choose_scale_kernel<<<1, 1, 0, ctx->stream>>>(q_absmax, cosine ? 1 : 0, q_scale, fold ? 1 : 0,
+  choose_scale_kernel<<<1, 1, 0, ctx->stream>>>(q_absmax, 0, q_scale, fold ? 1 : 0,
                                                 ix->fold_exp - (ix->kind == INDEX_PQ ? 1 : 0));
   ctx->stats.kernel_launches++;
   BoundConsts bc{ix->scale16, ix->max_xnorm16, ix->max_xerr16, ix->max_xnorm, ix->min_xnorm_nz, dim16, fold ? ix->fold_bmax : 0.f};
@@ -2456,20 +2677,9 @@ int32_t prepare_query_operands(Index* ix, const float* q, int64_t nq, QueryOpera
       bound_i8_kernel<VSK_METRIC_EUCLIDEAN><<<bgrid, 256, 0, ctx->stream>>>(qn16, qe16, qn_tmp, q_true_norm, nq, q_scale, bc, eps, alpha);
     else
       bound_i8_kernel<VSK_METRIC_DOT_PRODUCT><<<bgrid, 256, 0, ctx->stream>>>(qn16, qe16, qn_tmp, q_true_norm, nq, q_scale, bc, eps, alpha);
-  } else
-  switch (metric) {
-    case VSK_METRIC_EUCLIDEAN:
-      launch_prep<VSK_METRIC_EUCLIDEAN>(ctx, q, nq, dim, dim16, q_scale, q16, nullptr, qn16, qe16, qn_tmp, nullptr, qfold);
-      bound_kernel<VSK_METRIC_EUCLIDEAN><<<bgrid, 256, 0, ctx->stream>>>(qn16, qe16, qn_tmp, nq, q_scale, bc, eps, alpha);
-      break;
-    case VSK_METRIC_COSINE:
-      launch_prep<VSK_METRIC_COSINE>(ctx, q, nq, dim, dim16, q_scale, q16, nullptr, qn16, qe16, qn_tmp, nullptr);
-      bound_kernel<VSK_METRIC_COSINE><<<bgrid, 256, 0, ctx->stream>>>(qn16, qe16, qn_tmp, nq, q_scale, bc, eps, alpha);
-      break;
-    default:
-      launch_prep<VSK_METRIC_DOT_PRODUCT>(ctx, q, nq, dim, dim16, q_scale, q16, nullptr, qn16, qe16, qn_tmp, nullptr);
-      bound_kernel<VSK_METRIC_DOT_PRODUCT><<<bgrid, 256, 0, ctx->stream>>>(qn16, qe16, qn_tmp, nq, q_scale, bc, eps, alpha);
-      break;
+  } else {
+    launch_prep<VSK_METRIC_EUCLIDEAN>(ctx, q, nq, dim, dim16, q_scale, q16, nullptr, qn16, qe16, qn_tmp, nullptr, qfold);
+    bound_kernel<VSK_METRIC_EUCLIDEAN><<<bgrid, 256, 0, ctx->stream>>>(qn16, qe16, qn_tmp, nq, q_scale, bc, eps, alpha);
   }
   ctx->stats.kernel_launches++;
   VSK_CUDA(ctx, cudaGetLastError());
@@ -2480,6 +2690,48 @@ int32_t prepare_query_operands(Index* ix, const float* q, int64_t nq, QueryOpera
   out->scale = q_scale;
   out->err = err;
   out->rr_total = rr_total;
+  return VSK_OK;
+}
+
+// The same for a flat fp32 index, with a scale and a coefficient per query (alpha is an array), and the lists emptied.
+int32_t flat_query_operands(Index* ix, const float* q, int64_t nq, const CandLists& cand, QueryOperands* out) {
+  VSK_TRACE("vsk:query_operands");
+  Ctx* ctx = ix->ctx;
+  prefer_shared_carveout(ctx, query_prep_kernel<VSK_METRIC_EUCLIDEAN>, query_prep_kernel<VSK_METRIC_COSINE>, query_prep_kernel<VSK_METRIC_DOT_PRODUCT>,
+                         finish_kernel<VSK_METRIC_EUCLIDEAN, 128>, finish_kernel<VSK_METRIC_COSINE, 128>, finish_kernel<VSK_METRIC_DOT_PRODUCT, 128>,
+                         finish_kernel<VSK_METRIC_EUCLIDEAN, 512>, finish_kernel<VSK_METRIC_COSINE, 512>, finish_kernel<VSK_METRIC_DOT_PRODUCT, 512>);
+  QueryPrep a{};
+  void* p;
+  VSK_TRY(scratch(ctx, SLOT_Q16, (size_t)nq * ix->dim16 * sizeof(__half), &p));
+  a.out = (__half*)p;
+  VSK_TRY(scratch(ctx, SLOT_QAUX, (size_t)nq * 4 * sizeof(float) + 64, &p));
+  a.alpha = (float*)p;
+  a.eps = a.alpha + nq;
+  a.norm = a.eps + nq;
+  VSK_TRY(scratch(ctx, SLOT_TC_B, 64, &p));
+  a.words = (uint64_t*)p;
+  a.q = q;
+  a.nq = nq;
+  a.dim = ix->dim;
+  a.dim16 = ix->dim16;
+  a.c = BoundConsts{ix->scale16, ix->max_xnorm16, ix->max_xerr16, ix->max_xnorm, ix->min_xnorm_nz, ix->dim16, ix->fold16 ? ix->fold_bmax : 0.f};
+  a.fold = FoldArgs{ix->fold16 ? 2 : 0, fold_col0(ix->dim), ix->fold_exp};
+  a.cand = cand;
+  const unsigned grid = (unsigned)ceil_div(nq, 8);
+  switch (ix->metric) {
+    case VSK_METRIC_EUCLIDEAN: query_prep_kernel<VSK_METRIC_EUCLIDEAN><<<grid, 256, 0, ctx->stream>>>(a); break;
+    case VSK_METRIC_COSINE: query_prep_kernel<VSK_METRIC_COSINE><<<grid, 256, 0, ctx->stream>>>(a); break;
+    default: query_prep_kernel<VSK_METRIC_DOT_PRODUCT><<<grid, 256, 0, ctx->stream>>>(a); break;
+  }
+  ctx->stats.kernel_launches++;
+  VSK_CUDA(ctx, cudaGetLastError());
+  tl_mark(ctx, "query_operands");
+  out->q16 = a.out;
+  out->eps = a.eps;
+  out->alpha = a.alpha;
+  out->norm = a.norm;
+  out->err = (int32_t*)p;
+  out->rr_total = (unsigned long long*)((char*)p + 16);
   return VSK_OK;
 }
 
@@ -2497,6 +2749,25 @@ int32_t cand_lists(Ctx* ctx, int64_t nq, CandLists* cand) {
   return VSK_OK;
 }
 
+// Whether a query row fits beside the largest list in finish_kernel's shared memory.
+bool finish_applies(int dim) { return (size_t)dim * sizeof(float) <= 160 * 1024; }
+
+template <int METRIC, int NT>
+int32_t launch_finish_as(Ctx* ctx, const FinishArgs& f, int64_t nq) {
+  const size_t smem = (size_t)NT * SEL_ITEMS * sizeof(uint64_t) + (size_t)f.dim * sizeof(float);
+  if (smem > 48 * 1024) VSK_CUDA(ctx, cudaFuncSetAttribute(finish_kernel<METRIC, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  finish_kernel<METRIC, NT><<<(unsigned)nq, NT, smem, ctx->stream>>>(f);
+  tl_mark(ctx, "finish");
+  ctx->stats.kernel_launches++;
+  VSK_CUDA(ctx, cudaGetLastError());
+  return VSK_OK;
+}
+// small: no list holds more than 1 024 keys
+template <int METRIC>
+int32_t launch_finish(Ctx* ctx, const FinishArgs& f, int64_t nq, bool small) {
+  return small ? launch_finish_as<METRIC, 128>(ctx, f, nq) : launch_finish_as<METRIC, 512>(ctx, f, nq);
+}
+
 // The search in two halves.  `begin` runs the scan and its compactions; `finish` certifies, re-scores and orders.
 // A plain search calls them back to back.  A shard of a row-sharded search passes `bound_out` (and the number of
 // shards): the last compaction is then left to `finish`, and bound_out[q] gets a value that this shard's
@@ -2512,20 +2783,28 @@ int32_t tensor_search_begin(Index* ix, const float* q, int64_t nq, int32_t k, co
   const int metric = ix->metric;
   const int dim16 = ix->dim16;
   const int32_t keep = std::min<int32_t>(kCandCap / 2, k + std::max(8, k / 8));
+  // An fp32 index's second half is one launch, the last compaction in it (finish_kernel); rows too wide for its shared memory,
+  // and codes, keep the separate ones.
+  const bool fused = ix->kind == INDEX_FLAT_F32 && finish_applies(ix->dim);
+  CandLists cand;
+  VSK_TRY(cand_lists(ctx, nq, &cand));
   QueryOperands qo;
-  VSK_TRY(prepare_query_operands(ix, q, nq, &qo));
+  if (ix->kind == INDEX_FLAT_F32) {
+    VSK_TRY(flat_query_operands(ix, q, nq, cand, &qo));
+    if (!qnorm) qnorm = qo.norm;
+  } else {
+    VSK_TRY(prepare_query_operands(ix, q, nq, &qo));
+    VSK_TRY(launch_init_cand(ctx, cand, nq));
+  }
   const bool fold = ix->fold16;
 
   CUtensorMap mq, mx;
   VSK_TRY(make_map(ctx, qo.q16, nq, dim16, TM, &mq));
   VSK_TRY(make_map(ctx, ix->rows16, ix->n, dim16, TN, &mx));
 
-  // ---- candidate lists and the chunk schedule ----
-  CandLists cand;
-  VSK_TRY(cand_lists(ctx, nq, &cand));
-  VSK_TRY(launch_init_cand(ctx, cand, nq));
-
+  // ---- the chunk schedule ----
   TcArgs a{};
+  a.alpha_per_query = ix->kind == INDEX_FLAT_F32 ? 1 : 0;
   a.nq = nq;
   a.kblocks = dim16 / TK;
   a.k16_last = k16_last_of(fold ? fold_col0(ix->dim) + kFoldCols : ix->dim, dim16);
@@ -2555,8 +2834,11 @@ int32_t tensor_search_begin(Index* ix, const float* q, int64_t nq, int32_t k, co
   sel.k = k;
   // the compaction after the last chunk keeps what the exact re-scoring needs and certifies the query; a shard
   // only measures its bound there and leaves that compaction to the second half
+  bool skip_last = false;
   auto last_select = [&]() {
-    if (bound_out == nullptr) {
+    if (bound_out == nullptr && fused) {
+      skip_last = true;
+    } else if (bound_out == nullptr) {
       sel.cert_eps = qo.eps;
     } else {
       sel.bound_out = bound_out;
@@ -2565,7 +2847,9 @@ int32_t tensor_search_begin(Index* ix, const float* q, int64_t nq, int32_t k, co
     }
   };
   if (seen == n) last_select();
-  VSK_TRY(launch_select(ctx, sel));
+  if (!skip_last) VSK_TRY(launch_select(ctx, sel));
+  // (a dense list that was only measured has had its count written)
+  const int32_t dense_left = skip_last ? sel.dense_count : -1;
   sel.dense_count = -1;
   a.mode = SCAN_THRESHOLD;
   // A small batch is bound by its launches, not by its hits: fewer, faster-growing chunks (each still within what a
@@ -2591,7 +2875,7 @@ int32_t tensor_search_begin(Index* ix, const float* q, int64_t nq, int32_t k, co
     sel.max_count = schedule_max_count(seen, chunk, keep);
     seen += chunk;
     if (seen == n) last_select();
-    VSK_TRY(launch_select(ctx, sel));
+    if (!skip_last) VSK_TRY(launch_select(ctx, sel));
   }
   ShardPending& pd = ctx->pending[ctx->lane];
   pd.active = true;
@@ -2609,6 +2893,8 @@ int32_t tensor_search_begin(Index* ix, const float* q, int64_t nq, int32_t k, co
   pd.keep = keep;
   pd.max_count = sel.max_count;
   pd.need_cert = bound_out != nullptr;
+  pd.fused = fused;
+  pd.dense_count = dense_left;
   return VSK_OK;
 }
 
@@ -2628,6 +2914,37 @@ int32_t tensor_search_finish_issue(Index* ix, const float* ext_bound, float* out
   const int metric = ix->metric;
   const int dim = ix->dim;
   const bool i8 = ix->kind == INDEX_FLAT_I8;
+  PinnedBuf& hb = ctx->host_flags[ctx->lane];
+  VSK_TRY(pinned_reserve(ctx, &hb, (size_t)nq * 4 + 16));
+  if (pd.fused) {
+    FinishArgs f{};
+    f.cand = cand;
+    f.dense_count = pd.dense_count;
+    f.q = q;
+    f.x = ix->rows;
+    f.qnorm = qnorm;
+    f.xnorm = ix->row_norm;
+    f.dim = dim;
+    f.k = k;
+    f.eps = pd.eps;
+    f.ext_bound = ext_bound;
+    f.out_dist = out_dist;
+    f.out_ids = out_ids;
+    f.id_base = ix->id_base;
+    f.err = pd.err;
+    f.host_err = (int32_t*)hb.p;
+    f.host_flags = (int32_t*)hb.p + 4;
+    const bool small = pd.max_count <= 128 * SEL_ITEMS && pd.dense_count <= 128 * SEL_ITEMS;
+    switch (metric) {
+      case VSK_METRIC_EUCLIDEAN: VSK_TRY(launch_finish<VSK_METRIC_EUCLIDEAN>(ctx, f, nq, small)); break;
+      case VSK_METRIC_COSINE: VSK_TRY(launch_finish<VSK_METRIC_COSINE>(ctx, f, nq, small)); break;
+      default: VSK_TRY(launch_finish<VSK_METRIC_DOT_PRODUCT>(ctx, f, nq, small)); break;
+    }
+    pd.issued = true;
+    pd.out_dist = out_dist;
+    pd.out_ids = out_ids;
+    return VSK_OK;
+  }
   if (pd.need_cert) {
     SelectArgs sel{};
     sel.cand = cand;
@@ -2681,8 +2998,6 @@ int32_t tensor_search_finish_issue(Index* ix, const float* ext_bound, float* out
   VSK_TRY(launch_select(ctx, fin));
 
   // ---- flag words to the host: bounded-wait expiry, overflowed lists, failed certificates ----
-  PinnedBuf& hb = ctx->host_flags[ctx->lane];
-  VSK_TRY(pinned_reserve(ctx, &hb, (size_t)nq * 4 + 16));
   char* h = (char*)hb.p;
   VSK_CUDA(ctx, cudaMemcpyAsync(h, pd.err, 4, cudaMemcpyDeviceToHost, ctx->stream));
   VSK_CUDA(ctx, cudaMemcpyAsync(h + 8, pd.rr_total, 8, cudaMemcpyDeviceToHost, ctx->stream));
@@ -2709,12 +3024,16 @@ int32_t tensor_search_finish_collect(Index* ix, int from_lane) {
   memcpy(&herr, h, 4);
   memcpy(&hrr, h + 8, 8);
   const int32_t* flags = (const int32_t*)(h + 16);
+  if (pd.fused) {   // the words of finish_kernel: flags in the low byte, re-scored rows above
+    hrr = 0;
+    for (int64_t i = 0; i < pd.nq; ++i) hrr += (unsigned)flags[i] >> 8;
+  }
   ctx->stats.reranked_rows += (int64_t)hrr;
   if (herr != 0)
     return fail(ctx, VSK_ERR_TIMEOUT, "tensor-core scan: a bounded pipeline wait ran out (role %d)", herr);
   std::vector<int32_t> bad;
   for (int64_t i = 0; i < pd.nq; ++i)
-    if (flags[i]) bad.push_back((int32_t)i);
+    if (flags[i] & 0xff) bad.push_back((int32_t)i);
   if (!bad.empty()) VSK_TRY(fp32_search_subset(ix, pd.q, bad, pd.k, pd.qnorm, pd.qmasks, pd.out_dist, pd.out_ids));
   return VSK_OK;
 }
@@ -2790,15 +3109,15 @@ int32_t tensor_coarse_values(Index* ix, const float* q, int64_t nq, int64_t rows
   if (rows <= 0 || rows > kCandCap || rows > ix->n)
     return fail(ctx, VSK_ERR_INVALID_BUFFER_SIZE, "rows must be in [1, min(%d, index size)]", kCandCap);
   VSK_TRY(tensor_prepare(ix));
+  CandLists cand;
+  VSK_TRY(cand_lists(ctx, nq, &cand));
   QueryOperands qo;
-  VSK_TRY(prepare_query_operands(ix, q, nq, &qo));
+  VSK_TRY(flat_query_operands(ix, q, nq, cand, &qo));
   CUtensorMap mq, mx;
   VSK_TRY(make_map(ctx, qo.q16, nq, ix->dim16, TM, &mq));
   VSK_TRY(make_map(ctx, ix->rows16, ix->n, ix->dim16, TN, &mx));
-  CandLists cand;
-  VSK_TRY(cand_lists(ctx, nq, &cand));
-  VSK_TRY(launch_init_cand(ctx, cand, nq));
   TcArgs a{};
+  a.alpha_per_query = 1;
   a.nq = nq;
   a.kblocks = ix->dim16 / TK;
   a.k16_last = k16_last_of(ix->fold16 ? fold_col0(ix->dim) + kFoldCols : ix->dim, ix->dim16);
