@@ -143,3 +143,39 @@ def test_a_bounded_wait_of_the_row_lists_runs_out(vsk, cpu_oracle):
         ix.close()
     finally:
         dev.close()
+
+
+def test_decoded_values_are_divided_as_the_decoder_divides(vsk, dev):
+    """Queries along one axis: a distance is minus one decoded value, which has to carry the bits of
+    (code - offset) / scale, each operation rounded by itself - ordinary scales, powers of two, and scales and offsets beyond
+    the range in which the division is done by a reciprocal."""
+    rng = np.random.default_rng(77)
+    n, d, k = 20_000, 48, 200
+    codes = rng.integers(-128, 128, (n, d)).astype(np.int8)
+    scale = np.exp(rng.uniform(-8, 8, d)).astype(np.float32)
+    offset = (100 * rng.standard_normal(d)).astype(np.float32)
+    scale[:6] = [1.0, 0.25, 3.0, 1.0 / 3.0, 2.0, 7.0]
+    offset[:6] = [0.0, 5.0, -17.0, 0.5, 1e-18, 128.0]
+    ix = vsk.QuantizedFlatIndex(dev, d, vsk.DistanceMetric.dotProduct, scale, offset)
+    ix.add(codes)
+    q = np.eye(d, dtype=np.float32)
+    dist, ids = ix.batchSearch(q, k)
+    x = ((codes.astype(np.float32) - offset) / scale).astype(np.float32)
+    for j in range(d):
+        assert np.array_equal(dist[j], -x[ids[j], j])
+        assert np.array_equal(dist[j], np.sort(-x[:, j])[:k])
+
+
+def test_decoded_values_with_extreme_parameters(vsk, dev):
+    rng = np.random.default_rng(78)
+    n, d, k = 20_000, 32, 100
+    codes = rng.integers(-128, 128, (n, d)).astype(np.int8)
+    for s, o in ((1e-13, 3.0), (1e13, 3.0), (0.7, 1e16), (0.7, 1e-16)):
+        scale, offset = np.full(d, s, np.float32), np.full(d, o, np.float32)
+        ix = vsk.QuantizedFlatIndex(dev, d, vsk.DistanceMetric.dotProduct, scale, offset)
+        ix.add(codes)
+        dist, ids = ix.batchSearch(np.eye(d, dtype=np.float32), k)
+        x = ((codes.astype(np.float32) - offset) / scale).astype(np.float32)
+        for j in range(d):
+            assert np.array_equal(dist[j], -x[ids[j], j])
+        ix.close()

@@ -60,13 +60,17 @@ template <int EW> struct Epi {
   static constexpr int THREADS = 64 + 32 * EW;
 };
 
-template <int EW>
+// A launch that lists every row (tile-table mode, no thresholds yet); beside the modes of ScanMode.
+constexpr int SCAN_ALL = 4;
+
+constexpr int kTcQueue = 8;   // hits a lane can hold before they go to its query's list
+
+template <int EW, bool HAS_BETA>
 struct TcSmemT {
   // stage buffers first: each must start on a 1024-byte boundary for the 128B swizzle
   uint8_t ring[RING_BYTES];
-  float beta[2][EW][Epi<EW>::COLS];   // per accumulator buffer and epilogue warp: its columns' per-row terms
-  uint32_t masks[EW * 32][Epi<EW>::GROUPS + 1];  // per epilogue thread: pass bits of its values (padded row)
-  float hitval[EW * 32][Epi<EW>::GROUPS + 1];    // ... and per group the value of its last hit
+  float beta[HAS_BETA ? 2 : 1][HAS_BETA ? EW : 1][Epi<EW>::COLS];   // per accumulator buffer and epilogue warp: its columns' per-row terms
+  uint2 queue[EW][kTcQueue][32];   // per epilogue lane: its hits {value, column}; the dense mode's keys on their way out
   uint64_t full[STAGES];
   uint64_t empty[STAGES];
   uint64_t tmem_full[2];
@@ -75,7 +79,32 @@ struct TcSmemT {
   uint32_t tmem_base;
   volatile int abort_flag;
 };
-template <int EW> constexpr size_t tc_smem_bytes() { return sizeof(TcSmemT<EW>) + 1024; }   // + alignment slack
+template <int EW, bool HAS_BETA> constexpr size_t tc_smem_bytes() { return sizeof(TcSmemT<EW, HAS_BETA>) + 1024; }   // + alignment slack
+
+// The tiles of a unit, one after the other, without a division per tile.  (All counts of tiles are below 2^31.)
+struct TcTiles {
+  int mode;                           // 0: query tile fastest, 1: row tile fastest (a unit owns whole query tiles), 2: tile table
+  uint32_t qtiles, ntiles, units, dq, dn;   // (tile table: ntiles is the table's length)
+};
+struct TcWalk {
+  uint32_t qt, nt;   // query tile and row tile (tile table: nt is the tile's index in it)
+  __device__ __forceinline__ void start(const TcTiles& t, uint32_t unit) {
+    nt = t.mode == 2 ? unit : t.mode == 1 ? 0u : unit / t.qtiles;
+    qt = t.mode == 2 ? 0u : t.mode == 1 ? unit : unit - nt * t.qtiles;
+  }
+  __device__ __forceinline__ bool valid(const TcTiles& t) const { return nt < t.ntiles && qt < t.qtiles; }
+  __device__ __forceinline__ void advance(const TcTiles& t) {
+    if (t.mode == 2) {
+      nt += t.units;
+    } else if (t.mode == 1) {
+      if (++nt == t.ntiles) { nt = 0u; qt += t.units; }
+    } else {
+      nt += t.dn;
+      qt += t.dq;
+      if (qt >= t.qtiles) { qt -= t.qtiles; ++nt; }
+    }
+  }
+};
 
 struct TcArgs {
   int64_t nq;                 // queries (list positions)
@@ -114,6 +143,14 @@ struct TcArgs {
 };
 
 
+// The accumulator a value must reach to be a hit: alpha * acc <= thr with alpha < 0 holds for every acc >= thr / alpha;
+// thr * (1 / alpha) and the product alpha * acc each differ from the exact quotient by a few units in the last place,
+// so the bar is lowered by 2^-20 of its size (and a denormal's worth): no hit of the product form is lost.
+__device__ __forceinline__ float as_bar(float thr, float inv_alpha) {
+  const float b = thr * inv_alpha;
+  return b - fabsf(b) * 9.5367431640625e-7f - 1e-37f;
+}
+
 // I8 (threshold mode, plain grid): both operands are 8-bit integers, 128 to a K block, and the accumulators exact 32-bit
 // integers.  cand.thr then holds, as integer bits, the accumulator a row must reach; a listed key carries the row only
 // (its value is formed by the re-scoring).
@@ -121,7 +158,7 @@ template <int MODE, bool HAS_BETA, bool HAS_MASK, int EW, bool I8 = false>
 __global__ void __launch_bounds__(Epi<EW>::THREADS, 1)
 tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_x, TcArgs a) {
   extern __shared__ uint8_t smem_raw[];
-  using TcSmem = TcSmemT<EW>;
+  using TcSmem = TcSmemT<EW, HAS_BETA>;
   constexpr int EPI_WARPS = EW, EPI_COLS = Epi<EW>::COLS, EPI_GROUPS = Epi<EW>::GROUPS, EPI_PARTS = Epi<EW>::PARTS;
   TcSmem* sm = reinterpret_cast<TcSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -137,29 +174,16 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   const int64_t qtiles = (a.nq + QT - 1) / QT;
   const int64_t ntiles = (a.row_end - a.row_begin + TN - 1) / TN;
   const int64_t tiles = qtiles * ntiles;
-  // i-th tile of this unit.  Query-tile-fastest order interleaves units over the tile list (units that run
+  // The tiles of this unit.  Query-tile-fastest order interleaves units over the tile list (units that run
   // together read the same rows).  In row-tile-fastest order a unit OWNS whole query tiles and walks all their
   // row tiles in turn, so a query's running state (slot count, best key) stays in its thread's registers.
-  auto tile_at = [&](int64_t i, int64_t& qt, int64_t& nt) -> bool {
-    if (a.tiles) {   // explicit tile list: nt is the tile's index in the table
-      const int64_t t = unit + i * units;
-      if (t >= a.num_tiles) return false;
-      nt = t;
-      qt = 0;
-      return true;
-    }
-    if (a.row_tile_fastest) {
-      const int64_t qi = i / ntiles;
-      nt = i - qi * ntiles;
-      qt = unit + qi * units;
-      return qt < qtiles;
-    }
-    const int64_t t = unit + i * units;
-    if (t >= tiles) return false;
-    nt = t / qtiles;
-    qt = t - nt * qtiles;
-    return true;
-  };
+  TcTiles walk;
+  walk.mode = a.tiles ? 2 : (a.row_tile_fastest ? 1 : 0);
+  walk.units = (uint32_t)units;
+  walk.qtiles = a.tiles ? 1u : (uint32_t)qtiles;
+  walk.ntiles = a.tiles ? (uint32_t)a.num_tiles : (uint32_t)ntiles;
+  walk.dn = walk.units / walk.qtiles;
+  walk.dq = walk.units - walk.dn * walk.qtiles;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -197,9 +221,10 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       // table look-up (a global load) is not on the producer's critical path
       int4 entry_next = make_int4(0, 0, 0, 0);
       if (a.tiles && unit < a.num_tiles) entry_next = __ldg(&a.tiles[unit]);
-      for (int64_t i = 0; ok; ++i) {
-        int64_t qt, nt;
-        if (!tile_at(i, qt, nt)) break;
+      TcWalk w;
+      w.start(walk, blockIdx.x);
+      for (bool first = true; ok && w.valid(walk); w.advance(walk), first = false) {
+        const int64_t qt = w.qt, nt = w.nt;
         const int4 entry = entry_next;
         if (a.tiles && nt + units < a.num_tiles) entry_next = __ldg(&a.tiles[nt + units]);
         const int32_t qrow = a.tiles ? entry.x : (int32_t)(qt * QT);
@@ -208,7 +233,7 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           if (!mbar_wait(&sm->empty[s], ph ^ 1, &sm->abort_flag, a.err, 1, wait_limit)) { ok = false; break; }
           uint8_t* st = sm->ring + s * kps * STAGE_BYTES;
           const int nkb = min(kps, a.kblocks - kb);
-          if (a.stall_kblock >= 0 && unit == 0 && i == 0 && kb == a.stall_kblock) {
+          if (a.stall_kblock >= 0 && unit == 0 && first && kb == a.stall_kblock) {
             // testing only: this stage is never filled, the consumer's bounded wait for it runs out
           } else {
             mbar_expect_tx(&sm->full[s], (uint32_t)(nkb * STAGE_BYTES));
@@ -285,62 +310,96 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       }
     }
   } else {
-    // ---------------- epilogue: one query per thread, half of the tile's columns per warp ----------------
+    // ---------------- epilogue: one query per thread, a part of the tile's columns per warp ----------------
     const int quarter = warp & 3;                 // tensor-memory lanes this warp may read
     const int et = quarter * 32 + lane;           // row of the tile owned by this thread
-    const int ew = warp - 2;                      // epilogue warp 0..7
+    const int ew = warp - 2;                      // epilogue warp 0..
     const int part = ew >> 2;                     // which part of the tile's columns this warp takes
     const int c0 = part * EPI_GROUPS;             // first 32-column group of that part
-    float alpha = a.alpha_per_query ? -1.0f : __ldg(a.alpha);
-    int64_t local = 0;
+    const float alpha0 = a.alpha_per_query ? -1.0f : __ldg(a.alpha);
+    const bool owned = a.row_tile_fastest != 0;
+    const int32_t row_begin = (int32_t)a.row_begin, row_end_all = (int32_t)a.row_end;   // (an index holds fewer than 2^31 rows)
     bool ok = true;
     int run_cnt = 0;                 // row-tile-fastest order: keys this thread has stored for its query so far
     float run_bv = CUDART_INF_F;     // ... and its best value / row so far (SCAN_ARGMIN)
     int64_t run_bn = 0;
-    // Tile-table mode: the tile's entry, then this lane's pair and threshold (both indexed by the entry), are a
-    // chain of dependent global loads.  The chain is pipelined over the tiles: the entry is loaded two tiles ahead,
-    // the pair and threshold one tile ahead, so neither load is waited for (with short contractions the epilogue,
-    // not the MMA, sets the pace).  pair_info / pair_thr are padded by one tile, so the loads need no bounds test.
-    struct Ahead { int4 e; uint32_t info; float thr; };
-    auto entry_at = [&](int64_t i) {
-      const int64_t t = unit + i * units;
-      return (a.tiles && t < a.num_tiles) ? __ldg(&a.tiles[t]) : make_int4(0, 0, 0, 0);
+    // What a lane needs to know of a tile before it can look at its values - the tile's entry and the pair behind it in
+    // tile-table mode, the query's threshold and coefficient - are dependent global loads.  They are pipelined over the
+    // tiles: the entry is loaded two tiles ahead, the rest one tile ahead, so that none is waited for (with short
+    // contractions the epilogue, not the MMA, sets the pace).  pair_info / pair_thr are padded by one tile, so the loads
+    // need no bounds test.
+    struct Ahead {
+      int4 e;
+      uint32_t info;
+      float thr, alpha;
+      bool qok;
     };
-    auto pair_at = [&](const int4& e) {
-      Ahead h{e, 0u, -CUDART_INF_F};
+    TcWalk w, wn;   // this tile and the next
+    w.start(walk, blockIdx.x);
+    wn = w;
+    auto entry_of = [&](const TcWalk& t) { return (a.tiles && t.valid(walk)) ? __ldg(&a.tiles[t.nt]) : make_int4(0, 0, 0, 0); };
+    auto look_ahead = [&](const TcWalk& t, const int4& e) {
+      Ahead h{e, 0u, -CUDART_INF_F, alpha0, false};
       if (a.tiles) {
         h.info = __ldg(a.pair_info + e.x + et);
-        if (MODE == SCAN_THRESHOLD) h.thr = __ldg(a.pair_thr + e.x + et);
+        if (MODE == SCAN_THRESHOLD || MODE == SCAN_ALL) h.thr = __ldg(a.pair_thr + e.x + et);
+        h.qok = et < e.w;
+      } else if (t.valid(walk)) {
+        const int64_t q = (int64_t)t.qt * QT + et;
+        h.qok = q < a.nq;
+        if (MODE == SCAN_THRESHOLD && h.qok) h.thr = __ldg(a.cand.thr + q);
+        if (a.alpha_per_query && h.qok) h.alpha = __ldg(a.alpha + q);
       }
       return h;
     };
-    Ahead ahead = pair_at(entry_at(0));
-    int4 entry_next = entry_at(1);
-    for (;; ++local) {
-      int64_t qt, nt;
-      if (!ok || !tile_at(local, qt, nt)) break;
-      const int acc = (int)(local & 1);
-      const uint32_t aph = (uint32_t)((local >> 1) & 1);
-      const Ahead cur = ahead;
-      if (a.tiles) {
-        ahead = pair_at(entry_next);
-        entry_next = entry_at(local + 2);
+    Ahead ahead = look_ahead(w, entry_of(w));
+    wn.advance(walk);
+    int4 entry_next = entry_of(wn);
+    // Hits wait in the lane's queue while their slots are reserved (the atomic's round trip is not waited for): they go to
+    // the lists when the next tile's values are on their way from tensor memory, or when a queue is full.
+    constexpr int QCAP = kTcQueue;
+    uint2(*queue)[32] = sm->queue[ew];
+    int pend_cnt = 0, pend_base = 0;
+    int32_t pend_q = 0;
+    uint32_t pend_row = 0u;
+    float pend_alpha = alpha0;
+    const int cap_here = owned ? a.cap / EPI_PARTS : a.cap;
+    auto flush = [&]() {
+      if (MODE != SCAN_THRESHOLD || !__any_sync(0xffffffffu, pend_cnt != 0)) return;
+      uint64_t* dst = a.cand.keys + (int64_t)pend_q * a.cap + (owned ? part * cap_here : 0) + pend_base;
+      const int n = min(pend_cnt, cap_here - pend_base);
+      for (int e = 0; __any_sync(0xffffffffu, e < pend_cnt); ++e) {
+        const uint2 h = queue[e][lane];
+        const float x = __uint_as_float(h.x);
+        if (e < n) *VSK_CHK_W(dst + e) = make_key(I8 ? 0.f : HAS_BETA ? -x : x * pend_alpha, pend_row + h.y);
       }
-      int64_t q = qt * QT + et;
-      const bool owned = a.row_tile_fastest != 0;
-      if (owned && nt == 0) { run_cnt = 0; run_bv = CUDART_INF_F; run_bn = 0; }
-      int64_t n0 = a.row_begin + nt * TN;
-      int64_t row_end = a.row_end;
-      bool qok = q < a.nq;
-      float thr_tile = -CUDART_INF_F;
+      __syncwarp();
+      pend_cnt = 0;
+    };
+    uint32_t local = 0;
+    for (; ok && w.valid(walk); w = wn, wn.advance(walk), ++local) {
+      const int acc = (int)(local & 1);
+      const uint32_t aph = (local >> 1) & 1u;
+      const Ahead cur = ahead;
+      ahead = look_ahead(wn, entry_next);
+      if (a.tiles) {
+        TcWalk w2 = wn;
+        w2.advance(walk);
+        entry_next = entry_of(w2);
+      }
+      int32_t q = (int32_t)(w.qt * (uint32_t)QT) + et;
+      if (owned && w.nt == 0u) { run_cnt = 0; run_bv = CUDART_INF_F; run_bn = 0; }
+      int32_t n0 = row_begin + (int32_t)(w.nt * (uint32_t)TN);
+      int32_t row_end = row_end_all;
+      const bool qok = cur.qok;
+      const float alpha = cur.alpha;
+      float thr = cur.thr;
       if (a.tiles) {
         n0 = cur.e.y;
-        row_end = (int64_t)cur.e.y + (cur.e.z & 0x3fffffff);
-        qok = et < cur.e.w;
-        q = cur.info & 0x7fffffffu;
+        row_end = cur.e.y + (cur.e.z & 0x3fffffff);
+        q = (int32_t)(cur.info & 0x7fffffffu);
         // a remainder item (the rest of a query's nearest list) skips the tiles inside the pilot window
-        const bool skip = (cur.info >> 31) != 0u && ((cur.e.z >> 30) & 1) != 0;
-        if (qok && !skip) thr_tile = cur.thr;
+        if ((cur.info >> 31) != 0u && ((cur.e.z >> 30) & 1) != 0) thr = -CUDART_INF_F;
       }
       // The tile's per-row terms; each warp stages its own copy, so no CTA-wide barrier is needed.  The first tile
       // loads them directly; after that they are fetched one tile ahead into registers (the loads fly while this
@@ -349,25 +408,53 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       if (HAS_BETA) {
         if (local == 0) {
           for (int i = lane; i < EPI_COLS; i += 32)
-            sm->beta[acc][ew][i] = (n0 + c0 * 32 + i < row_end) ? __ldg(a.beta + n0 + c0 * 32 + i) : 0.f;
+            sm->beta[HAS_BETA ? acc : 0][HAS_BETA ? ew : 0][i] = (n0 + c0 * 32 + i < row_end) ? __ldg(a.beta + n0 + c0 * 32 + i) : 0.f;
           __syncwarp();
         }
-        int64_t nqt, nnt, nn0 = 0, nrow_end = 0;
-        if (tile_at(local + 1, nqt, nnt)) {
-          if (a.tiles) { nn0 = ahead.e.y; nrow_end = (int64_t)ahead.e.y + (ahead.e.z & 0x3fffffff); }
-          else { nn0 = a.row_begin + nnt * TN; nrow_end = a.row_end; }
+        int32_t nn0 = 0, nrow_end = 0;
+        if (wn.valid(walk)) {
+          if (a.tiles) { nn0 = ahead.e.y; nrow_end = ahead.e.y + (ahead.e.z & 0x3fffffff); }
+          else { nn0 = row_begin + (int32_t)(wn.nt * (uint32_t)TN); nrow_end = row_end_all; }
         }
 #pragma unroll
         for (int i = 0; i < EPI_COLS / 32; ++i) {
-          const int64_t r = nn0 + c0 * 32 + lane + 32 * i;
+          const int32_t r = nn0 + c0 * 32 + lane + 32 * i;
           beta_next[i] = r < nrow_end ? __ldg(a.beta + r) : 0.f;
         }
       }
-      float thr = CUDART_INF_F;
-      if (MODE == SCAN_THRESHOLD && qok) thr = a.tiles ? thr_tile : a.cand.thr[q];
-      if (a.alpha_per_query && qok) alpha = __ldg(a.alpha + q);
       uint64_t qm = 0ull;   // this query's filter mask: a row is eligible iff (row mask & qm) != 0
-      if (HAS_MASK && qok) qm = __ldg(a.q_masks + q);
+      uint64_t rmask[EPI_GROUPS];   // the masks of the warp's columns lane, lane + 32, ..
+      if (HAS_MASK) {
+        if (qok) qm = __ldg(a.q_masks + q);
+        if (MODE == SCAN_THRESHOLD || MODE == SCAN_ALL) {
+#pragma unroll
+          for (int g = 0; g < EPI_GROUPS; ++g) {
+            const int32_t r = n0 + (c0 + g) * 32 + lane;
+            rmask[g] = r < row_end ? __ldg(a.row_masks + r) : 0ull;
+          }
+        }
+      }
+      // SCAN_ALL: which columns are listed does not depend on their values, so their slots are asked for before the wait
+      uint32_t all_bits[EPI_GROUPS];
+      int all_base = 0;
+      if constexpr (MODE == SCAN_ALL) {
+        int n = 0;
+#pragma unroll
+        for (int g = 0; g < EPI_GROUPS; ++g) {
+          const int left = row_end - (n0 + (c0 + g) * 32);
+          uint32_t bits = left >= 32 ? 0xffffffffu : (left > 0 ? (1u << left) - 1u : 0u);
+          if (!qok || !(thr > -CUDART_INF_F)) bits = 0u;
+          if (HAS_MASK) {
+            for (int j = 0; j < 32; ++j) {
+              const uint64_t m = __shfl_sync(0xffffffffu, rmask[g], j);
+              if ((m & qm) == 0ull) bits &= ~(1u << j);
+            }
+          }
+          all_bits[g] = bits;
+          n += __popc(bits);
+        }
+        if (n) all_base = atomicAdd(&a.cand.count[q], n);
+      }
       // every lane of the warp must take part in the wait result
       bool got = mbar_wait(&sm->tmem_full[acc], aph, &sm->abort_flag, a.err, 4, wait_limit);
       got = __all_sync(0xffffffffu, got);
@@ -375,29 +462,36 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       tc_fence_after();
       const uint32_t trow = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * TN);
       if (MODE == SCAN_DENSE) {
+        // Eight columns at a time through shared memory: stored by their own lanes, the keys of 32 queries would go to 32
+        // different lines per instruction, which bound this epilogue; turned around, eight lanes store 64 bytes of one query.
+        uint64_t* buf = reinterpret_cast<uint64_t*>(&queue[0][0]);
+        constexpr int W = 8;   // columns per turn
+        static_assert(QCAP * sizeof(uint2) >= W * sizeof(uint64_t), "room for the turned keys");
 #pragma unroll 1
         for (int c = c0; c < c0 + EPI_GROUPS; ++c) {
           float v[32];
           tc_ld32(trow + (uint32_t)(c * 32), v);
-          const int64_t nc = n0 + c * 32;
-          if (!qok) continue;
-          uint64_t* dst = a.cand.keys + q * kCandCap + (nc - a.row_begin);
-          // a query's keys are contiguous (16-byte aligned at every even column): two keys per store halve the
-          // number of scattered store transactions, which is what bounds this epilogue
+          const int32_t nc = n0 + c * 32;
 #pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const float v0 = HAS_BETA ? fmaf(v[j], alpha, sm->beta[acc][ew][(c - c0) * 32 + j]) : v[j] * alpha;
-            const float v1 = HAS_BETA ? fmaf(v[j + 1], alpha, sm->beta[acc][ew][(c - c0) * 32 + j + 1]) : v[j + 1] * alpha;
-            uint64_t k0 = make_key(v0, (uint32_t)(nc + j)), k1 = make_key(v1, (uint32_t)(nc + j + 1));
-            if (HAS_MASK) {
+          for (int t = 0; t < 32 / W; ++t) {
+#pragma unroll
+            for (int j = 0; j < W; ++j) {
+              const int col = t * W + j;
+              const float val = HAS_BETA ? fmaf(v[col], alpha, sm->beta[HAS_BETA ? acc : 0][HAS_BETA ? ew : 0][(c - c0) * 32 + col]) : v[col] * alpha;
+              uint64_t key = make_key(val, (uint32_t)(nc + col));
               // the same row mask for every lane (a broadcast load); an ineligible row leaves an empty slot
-              if (nc + j < a.row_end && (__ldg(a.row_masks + nc + j) & qm) == 0ull) k0 = kEmptyKey;
-              if (nc + j + 1 < a.row_end && (__ldg(a.row_masks + nc + j + 1) & qm) == 0ull) k1 = kEmptyKey;
+              if (HAS_MASK && nc + col < row_end && (__ldg(a.row_masks + nc + col) & qm) == 0ull) key = kEmptyKey;
+              buf[lane * W + (j ^ (lane & (W - 1)))] = key;
             }
-            if (nc + j + 1 < a.row_end)
-              *reinterpret_cast<ulonglong2*>(dst + j) = make_ulonglong2(k0, k1);
-            else if (nc + j < a.row_end)
-              dst[j] = k0;
+            __syncwarp();
+#pragma unroll
+            for (int r0 = 0; r0 < 32; r0 += 32 / W) {
+              const int r = r0 + lane / W, j = lane & (W - 1);
+              const int32_t qr = q - lane + r, row = nc + t * W + j;
+              if (qr < a.nq && row < row_end)
+                *VSK_CHK_W(a.cand.keys + (int64_t)qr * kCandCap + (row - row_begin)) = buf[r * W + (j ^ (r & (W - 1)))];
+            }
+            __syncwarp();
           }
         }
       } else if (MODE == SCAN_ARGMIN) {
@@ -408,163 +502,171 @@ tc_scan_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         for (int c = c0; c < c0 + EPI_GROUPS; ++c) {
           float v[32];
           tc_ld32(trow + (uint32_t)(c * 32), v);
-          const int64_t left = a.row_end - (n0 + c * 32);
+          const int left = row_end - (n0 + c * 32);
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            const float val = HAS_BETA ? fmaf(v[j], alpha, sm->beta[acc][ew][(c - c0) * 32 + j]) : v[j] * alpha;
+            const float val = HAS_BETA ? fmaf(v[j], alpha, sm->beta[HAS_BETA ? acc : 0][HAS_BETA ? ew : 0][(c - c0) * 32 + j]) : v[j] * alpha;
             if (j < left && val < bv) { bv = val; bj = c * 32 + j; }   // strict '<': the lowest row wins ties
           }
         }
         if (owned) {
           if (bv < run_bv) { run_bv = bv; run_bn = n0 + bj; }   // row tiles come in ascending order: '<' keeps the lowest row
-          if (nt == ntiles - 1 && qok && run_bv < CUDART_INF_F)
+          if (w.nt == walk.ntiles - 1u && qok && run_bv < CUDART_INF_F)
             atomicMin(a.best + q, (unsigned long long)make_key(run_bv, (uint32_t)run_bn));
         } else if (qok && bv < CUDART_INF_F) {
           atomicMin(a.best + q, (unsigned long long)make_key(bv, (uint32_t)(n0 + bj)));
         }
       } else {
-        // Pass 1: which of this query's 256 values pass the threshold (one bit each).  A thread then
-        // reserves all its slots with ONE atomic per tile; pass 2 re-reads the accumulator groups that
-        // have a passing value and stores the keys.  A per-value atomic would serialise the warp on an
-        // L2 round trip for every column in which any of its 32 queries has a hit.
-        // The masks live in shared memory so that both loops stay rolled (small code, no dynamic
-        // register indexing).
-        uint32_t* m = sm->masks[ew * 32 + lane];
-        float* mv = sm->hitval[ew * 32 + lane];
-        int cnt = 0;
-#pragma unroll 1
-        for (int c = c0; c < c0 + EPI_GROUPS; ++c) {
-          float v[32];
-          tc_ld32(trow + (uint32_t)(c * 32), v);
-          const int64_t left = row_end - (n0 + c * 32);   // columns of this group inside the launch (tile)
-          // Cheap test first: the smallest of the group's 32 values against the threshold.  Most groups of a late
-          // chunk hold no hit for any of the warp's queries and then cost two instructions per value, not five.
-          float vmin = CUDART_INF_F;
-          if constexpr (I8) {
-            int top = __float_as_int(v[0]);
-#pragma unroll
-            for (int j = 1; j < 32; ++j) top = max(top, __float_as_int(v[j]));
-            if (left >= 32 && !__any_sync(0xffffffffu, qok && top >= __float_as_int(thr))) {
-              m[c - c0] = 0u;
-              continue;
-            }
-          } else if (!HAS_BETA && alpha < 0.f) {
-            // value = alpha * accumulator with alpha < 0: the smallest value is alpha times the largest accumulator
-            // (the multiplication is monotone, so this is the same number), one instruction per value; the values
-            // themselves are only formed for a group that has a hit
-            float amax = v[0];
-#pragma unroll
-            for (int j = 1; j < 32; ++j) amax = fmaxf(amax, v[j]);
-            vmin = amax * alpha;
-            if (left >= 32 && !__any_sync(0xffffffffu, qok && vmin <= thr)) {
-              m[c - c0] = 0u;
-              continue;
-            }
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] *= alpha;
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              v[j] = HAS_BETA ? fmaf(v[j], alpha, sm->beta[acc][ew][(c - c0) * 32 + j]) : v[j] * alpha;
-              vmin = fminf(vmin, v[j]);
-            }
-            if (left >= 32 && !__any_sync(0xffffffffu, qok && vmin <= thr)) {
-              m[c - c0] = 0u;
-              continue;
-            }
-          }
-          const uint32_t colmask = left >= 32 ? 0xffffffffu : (left > 0 ? ((1u << (int)left) - 1u) : 0u);
-          uint32_t bits = 0;
-          float hv = 0.f;   // the value of the (last) hit: all that pass 2 needs when a query has one hit in the group
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float val = v[j];
-            const bool hit = I8 ? __float_as_int(val) >= __float_as_int(thr) : val <= thr;
-            bits |= hit ? (1u << j) : 0u;
-            hv = hit ? val : hv;
-          }
-          bits = qok ? (bits & colmask) : 0u;
+        // alpha < 0 and a power of two (but for the per-row term): value <= threshold is accumulator >= threshold / alpha, so a
+        // value that is not listed costs one instruction, the running maximum of its eight columns.  The accumulator goes back
+        // as soon as its last columns are in registers.  Only eights in which some lane has a hit are looked at one by one.
+        const float bar = I8 ? (qok ? thr : __int_as_float(0x7fffffff)) : !qok ? CUDART_INF_F : HAS_BETA ? -thr : as_bar(thr, 1.0f / alpha);
+        auto reaches = [&](float v, float b) { return I8 ? __float_as_int(v) >= __float_as_int(b) : v >= b; };
+        int cnt = 0;          // hits in the queue
+        int tile_cnt = 0;     // ... and of the tile in all (owned order)
+        const uint32_t row0 = (uint32_t)(n0 + c0 * 32);
+        // the queue's hits: those the filter lets through stay, and their slots are asked for
+        auto reserve = [&]() {
           if (HAS_MASK) {
-            // Only hits are tested against the filter (a few per query and tile once the threshold is tight): the
-            // row masks of a tile are 2 KB and stay in L1 for the CTA's 128 queries.
-            uint32_t b = bits;
-            while (b) {
-              const int j = __ffs((int)b) - 1;
-              b &= b - 1u;
-              if ((__ldg(a.row_masks + n0 + c * 32 + j) & qm) == 0ull) bits &= ~(1u << j);
+            int kept = 0;
+            for (int e = 0; __any_sync(0xffffffffu, e < cnt); ++e) {
+              const uint2 h = queue[e][lane];
+              uint64_t m = 0ull;
+#pragma unroll
+              for (int g = 0; g < EPI_GROUPS; ++g) {
+                const uint64_t x = __shfl_sync(0xffffffffu, rmask[g], h.y & 31u);
+                if ((h.y >> 5) == (uint32_t)g) m = x;
+              }
+              if (e < cnt && (m & qm) != 0ull) queue[kept++][lane] = h;
             }
+            cnt = kept;
           }
-          m[c - c0] = bits;
-          mv[c - c0] = hv;
-          cnt += __popc(bits);
-        }
-        // Slot reservation.  Interleaved order: one atomic per tile.  Owned order: this warp's half of the
-        // columns appends to its own half of the query's list, counted in a register; the two 16-bit counts are
-        // stored after the last row tile.
-        int base = 0;
-        const int cap_here = owned ? a.cap / EPI_PARTS : a.cap;
-        if (owned) base = run_cnt;
-        else if (cnt) base = atomicAdd(&a.cand.count[q], cnt);
+          pend_cnt = cnt;
+          pend_q = q;
+          pend_row = row0;
+          pend_alpha = alpha;
+          pend_base = owned ? run_cnt + tile_cnt : (cnt ? atomicAdd(&a.cand.count[q], cnt) : 0);
+          tile_cnt += cnt;
+          cnt = 0;
+        };
+        if constexpr (MODE == SCAN_ALL) {
+          // the keys turned around as in the dense mode
+          constexpr int W = 8;
+          uint64_t* buf = reinterpret_cast<uint64_t*>(&queue[0][0]);
+          int base = all_base;
+#pragma unroll
+          for (int h = 0; h < EPI_GROUPS; ++h) {
+            const uint32_t bits = all_bits[h];
+            const uint32_t who = __ballot_sync(0xffffffffu, bits != 0u);   // (lists are short of a tile's 128 pairs as a rule)
+            if (who == 0u) continue;
+            float v[32];
+            tc_ld32(trow + (uint32_t)((c0 + h) * 32), v);
+#pragma unroll
+            for (int t = 0; t < 32 / W; ++t) {
+#pragma unroll
+              for (int j = 0; j < W; ++j) {
+                const int col = t * W + j;
+                const float val = HAS_BETA ? fmaf(v[col], alpha, sm->beta[HAS_BETA ? acc : 0][HAS_BETA ? ew : 0][h * 32 + col]) : v[col] * alpha;
+                buf[lane * W + (j ^ (lane & (W - 1)))] = make_key(I8 ? 0.f : val, row0 + (uint32_t)(h * 32 + col));
+              }
+              __syncwarp();
+#pragma unroll
+              for (int r0 = 0; r0 < 32; r0 += 32 / W) {
+                if (((who >> r0) & ((1u << (32 / W)) - 1u)) == 0u) continue;
+                const int r = r0 + lane / W, j = lane & (W - 1), col = t * W + j;
+                const uint32_t rb = __shfl_sync(0xffffffffu, bits, r);
+                const int at = __shfl_sync(0xffffffffu, base, r) + __popc(rb & ((1u << col) - 1u));
+                const int32_t qr = __shfl_sync(0xffffffffu, q, r);
+                if (((rb >> col) & 1u) != 0u && at < a.cap) *VSK_CHK_W(a.cand.keys + (int64_t)qr * a.cap + at) = buf[r * W + (j ^ (r & (W - 1)))];
+              }
+              __syncwarp();
+            }
+            base += __popc(bits);
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sm->tmem_empty[acc]);
+        } else {
 #pragma unroll 1
-        for (int c = c0; c < c0 + EPI_GROUPS; ++c) {
-          const uint32_t bits = m[c - c0];
-          const uint32_t colbits = __reduce_or_sync(0xffffffffu, bits);   // columns in which any query has a hit
-          if (colbits == 0u) continue;
-          if (!HAS_MASK && !__any_sync(0xffffffffu, (bits & (bits - 1u)) != 0u) && n0 + c * 32 + 32 <= row_end) {
-            // no query has more than one hit in this (whole) group: its value was kept by pass 1
-            const uint32_t ok1 = (bits != 0u && base < cap_here) ? 1u : 0u;
-            const uint64_t key1 = make_key(I8 ? 0.f : mv[c - c0], (uint32_t)(n0 + c * 32 + (__ffs((int)bits) - 1)));
-            uint64_t* d1 = a.cand.keys + q * a.cap + (owned ? part * cap_here : 0) + base;
-            asm volatile(
-                "{\n\t.reg .pred p;\n\t"
-                "setp.ne.u32 p, %2, 0;\n\t"
-                "@p st.global.u64 [%0], %1;\n\t}" ::"l"(d1),
-                "l"(key1), "r"(ok1)
-                : "memory");
-            base += bits != 0u ? 1 : 0;
-            continue;
-          }
+        for (int h = 0; h < EPI_GROUPS; ++h) {   // 32 columns at a time
           float v[32];
-          if constexpr (!I8) tc_ld32(trow + (uint32_t)(c * 32), v);
-          const int64_t nc = n0 + c * 32;
-          uint64_t* dst = a.cand.keys + q * a.cap + (owned ? part * cap_here : 0) + base;
-          // Straight-line code with predicated stores: a branch around every store makes the warp wait out each
-          // store's address chain in turn (measured: four times the cost of this form at 1 hit in 150 values).
-          // Only whole octets of columns without any hit are skipped, on a warp-uniform test.
+          tc_ld32_issue(trow + (uint32_t)((c0 + h) * 32), v);
+          if (h == 0) flush();   // the last tile's hits
+          tc_ld_wait();
+          if (h + 1 == EPI_GROUPS) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm->tmem_empty[acc]);
+          }
+          if (HAS_BETA) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = -fmaf(v[j], alpha, sm->beta[HAS_BETA ? acc : 0][HAS_BETA ? ew : 0][h * 32 + j]);
+          }
+          const int left = row_end - (n0 + (c0 + h) * 32);   // columns inside the launch (tile)
+          float top[4];
 #pragma unroll
           for (int o = 0; o < 4; ++o) {
-            if (((colbits >> (8 * o)) & 0xffu) == 0u) continue;
+            const float* x = &v[o * 8];
+            if constexpr (I8) {
+              int t = __float_as_int(x[0]);
 #pragma unroll
-            for (int jj = 0; jj < 8; ++jj) {
-              const int j = o * 8 + jj;
-              const float val = I8 ? 0.f : HAS_BETA ? fmaf(v[j], alpha, sm->beta[acc][ew][(c - c0) * 32 + j]) : v[j] * alpha;
-              const int rank = __popc(bits & ((1u << j) - 1u));
-              const uint32_t ok = (((bits >> j) & 1u) != 0u && base + rank < cap_here) ? 1u : 0u;
-              const uint64_t key = make_key(val, (uint32_t)(nc + j));
-              asm volatile(
-                  "{\n\t.reg .pred p;\n\t"
-                  "setp.ne.u32 p, %2, 0;\n\t"
-                  "@p st.global.u64 [%0], %1;\n\t}" ::"l"(dst + rank),
-                  "l"(key), "r"(ok)
-                  : "memory");
+              for (int j = 1; j < 8; ++j) t = max(t, __float_as_int(x[j]));
+              top[o] = __int_as_float(t);
+            } else {
+              top[o] = max3(x[6], x[7], fmaxf(max3(x[0], x[1], x[2]), max3(x[3], x[4], x[5])));
             }
           }
-          base += __popc(bits);
+          if (!__any_sync(0xffffffffu, reaches(top[0], bar) || reaches(top[1], bar) || reaches(top[2], bar) || reaches(top[3], bar))) continue;
+          uint32_t todo = 0u;   // fours of columns to be looked at, the same in every lane
+#pragma unroll
+          for (int o = 0; o < 4; ++o) todo |= __any_sync(0xffffffffu, reaches(top[o], bar)) ? 3u << (2 * o) : 0u;
+          const uint32_t col0 = (uint32_t)(h * 32);
+          while (todo != 0u) {
+            bool full = false;
+#pragma unroll
+            for (int f = 0; f < 8; ++f) {
+              if (((todo >> f) & 1u) == 0u || full) continue;
+              full = __any_sync(0xffffffffu, cnt > QCAP - 4);
+              if (full) continue;
+              todo &= ~(1u << f);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float x = v[f * 4 + j];
+                if (reaches(x, bar) && f * 4 + j < left) {
+                  queue[cnt][lane] = make_uint2(__float_as_uint(x), col0 + (uint32_t)(f * 4 + j));
+                  ++cnt;
+                }
+              }
+            }
+            if (full) {   // a queue without room: the hits so far go to their lists first
+              __syncwarp();
+              reserve();
+              flush();
+            }
+          }
         }
-        if (owned) {
-          run_cnt += cnt;
-          if (nt == ntiles - 1 && qok)
-            reinterpret_cast<unsigned char*>(a.cand.count)[q * 4 + part] = (unsigned char)min(run_cnt, 255);
+        __syncwarp();
+        reserve();
+        }
+        if (MODE == SCAN_THRESHOLD && owned) {
+          run_cnt += tile_cnt;
+          if (w.nt == walk.ntiles - 1u && qok)
+            reinterpret_cast<unsigned char*>(a.cand.count)[(int64_t)q * 4 + part] = (unsigned char)min(run_cnt, 255);
         }
       }
       if (HAS_BETA) {
 #pragma unroll
-        for (int i = 0; i < EPI_COLS / 32; ++i) sm->beta[acc ^ 1][ew][lane + 32 * i] = beta_next[i];
+        for (int i = 0; i < EPI_COLS / 32; ++i) sm->beta[HAS_BETA ? acc ^ 1 : 0][HAS_BETA ? ew : 0][lane + 32 * i] = beta_next[i];
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm->tmem_empty[acc]);
+      if (MODE == SCAN_DENSE || MODE == SCAN_ARGMIN) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm->tmem_empty[acc]);
+      } else if (HAS_BETA) {
+        __syncwarp();
+      }
     }
+    flush();
   }
 
   // ---------------- teardown ----------------
@@ -641,14 +743,6 @@ struct AsArgs {
   int32_t* err;
   uint32_t wait_limit;
 };
-
-// The accumulator a value must reach to be a hit: alpha * acc <= thr with alpha < 0 holds for every acc >= thr / alpha;
-// thr * (1 / alpha) and the product alpha * acc each differ from the exact quotient by a few units in the last place,
-// so the bar is lowered by 2^-20 of its size (and a denormal's worth): no hit of the product form is lost.
-__device__ __forceinline__ float as_bar(float thr, float inv_alpha) {
-  const float b = thr * inv_alpha;
-  return b - fabsf(b) * 9.5367431640625e-7f - 1e-37f;
-}
 
 template <int MODE>
 __global__ void __launch_bounds__(AS_THREADS, 1)
@@ -1662,6 +1756,21 @@ __global__ void bound_kernel(const float* __restrict__ qn16, const float* __rest
   eps[q] = query_eps<METRIC>(qn16[q], qe16[q], qnorm[q], inv, c);
 }
 
+// eps for int8-coded rows (operand residual of the rows is zero; the query operand is fp16(s_q q~), q~ = q / scale):
+//   contraction   |e_q| C + dim16 2^-22 |q'| C, divided by s_q          (C = max |code row|)
+//   formula       2^-22 (|q| max|x^| + |q~| C): fp32 rounding of x^ = (code - offset)/scale and of q~
+// doubled for euclidean (value = |x^|^2 - 2 q.x^) plus the rounding of |x^|^2 and of the final multiply-add.
+template <int METRIC>
+__device__ __forceinline__ float query_eps_i8(float a, float e, float qt_norm, float q_norm, float inv, const BoundConsts& c) {
+  float dot_err = (e * c.max_norm16 + (float)c.dim16 * 2.3841858e-7f * a * c.max_norm16) * inv;
+  dot_err += 2.3841858e-7f * (q_norm * c.max_norm + qt_norm * c.max_norm16);
+  float r = dot_err;
+  if (METRIC == VSK_METRIC_EUCLIDEAN)
+    r = 2.0f * dot_err + 4.0f * 5.9604645e-8f * (float)c.dim16 * c.max_norm * c.max_norm +
+        2.0f * 5.9604645e-8f * (c.max_norm * c.max_norm + 2.0f * q_norm * c.max_norm);
+  return r * 1.0001f + 1e-30f;
+}
+
 // All a flat search needs of its queries in one launch, a warp per query: a power-of-two scale of the query's own (as
 // choose_scale_kernel picks the batch's), the fp16 operand row with its fold constants, |q|, the error bound, the coefficient of
 // the values, and empty candidate lists.  With a scale for the whole batch this took a pass over the queries for it and five
@@ -1676,24 +1785,29 @@ struct QueryPrep {
   float *alpha, *eps, *norm;
   CandLists cand;
   uint64_t* words;          // eight words to be zeroed (error word, counters)
+  const float* sq_scale;    // I8: the operand is made from q / scale (the codes are the row operand)
 };
 
-template <int METRIC>
+template <int METRIC, bool I8 = false>
 __global__ void __launch_bounds__(256) query_prep_kernel(QueryPrep a) {
+  static_assert(!I8 || METRIC != VSK_METRIC_COSINE, "no cosine over codes");
   if (blockIdx.x == 0 && threadIdx.x < 8) *VSK_CHK_W(a.words + threadIdx.x) = 0ull;
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= a.nq) return;
   const int lane = threadIdx.x & 31;
   const float* p = a.q + row * a.dim;
-  float ss = 0.f, top = 0.f;
+  auto value = [&](int i) { return I8 ? __fdiv_rn(__ldg(p + i), __ldg(a.sq_scale + i)) : __ldg(p + i); };
+  float ss = 0.f, st = 0.f, top = 0.f;
   for (int i = lane; i < a.dim; i += 32) {
-    const float v = __ldg(p + i);
+    const float v = __ldg(p + i), t = value(i);
     ss = fmaf(v, v, ss);
-    top = fmaxf(top, fabsf(v));
+    if (I8) st = fmaf(t, t, st);
+    top = fmaxf(top, fabsf(t));
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (I8) st += __shfl_xor_sync(0xffffffffu, st, o);
     top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
   }
   const float norm = sqrtf(ss);
@@ -1703,7 +1817,7 @@ __global__ void __launch_bounds__(256) query_prep_kernel(QueryPrep a) {
   __half* out = a.out + row * a.dim16;
   for (int i = lane; i < a.dim16; i += 32) {
     float t = 0.f;
-    if (i < a.dim) t = (METRIC == VSK_METRIC_COSINE) ? (__ldg(p + i) * unit) * s : __ldg(p + i) * s;
+    if (i < a.dim) t = (METRIC == VSK_METRIC_COSINE) ? (__ldg(p + i) * unit) * s : value(i) * s;
     __half h = __float2half_rn(t);
     const float back = __half2float(h);
     n2 = fmaf(back, back, n2);
@@ -1719,9 +1833,10 @@ __global__ void __launch_bounds__(256) query_prep_kernel(QueryPrep a) {
     e2 += __shfl_xor_sync(0xffffffffu, e2, o);
   }
   if (lane == 0) {
-    const float up = 1.0f + 1e-5f, inv = 1.0f / (s * a.c.scale_x);
+    const float up = 1.0f + 1e-5f, inv = 1.0f / (I8 ? s : s * a.c.scale_x);
     *VSK_CHK_W(a.alpha + row) = (METRIC == VSK_METRIC_EUCLIDEAN ? -2.0f : -1.0f) * inv;
-    *VSK_CHK_W(a.eps + row) = query_eps<METRIC>(sqrtf(n2) * up, sqrtf(e2) * up, norm, inv, a.c);
+    *VSK_CHK_W(a.eps + row) = I8 ? query_eps_i8<METRIC>(sqrtf(n2) * up, sqrtf(e2) * up, sqrtf(st), norm, inv, a.c)
+                                 : query_eps<METRIC>(sqrtf(n2) * up, sqrtf(e2) * up, norm, inv, a.c);
     *VSK_CHK_W(a.norm + row) = norm;
     *VSK_CHK_W(a.cand.count + row) = 0;
     *VSK_CHK_W(a.cand.thr + row) = CUDART_INF_F;
@@ -1766,36 +1881,55 @@ __global__ void prep_codes_kernel(const int8_t* __restrict__ codes, int64_t n, i
 
 // q~ = q / scale per dimension: sum_i q_i x^_i = sum_i q~_i code_i - sum_i q_i offset_i / scale_i, and the
 // second term does not depend on the row.
-__global__ void scale_queries_kernel(const float* __restrict__ q, int64_t total, int dim,
-                                     const float* __restrict__ scale, float* __restrict__ out) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < total) out[i] = __fdiv_rn(q[i], __ldg(scale + (int)(i % dim)));
+// a / b rounded once, with y = 1 / b rounded once: Markstein's correction (IBM J. Res. Dev. 34, 1990) - the remainder of the
+// product a y is exact in a fused operation, and adding its share rounds correctly while nothing over- or underflows.
+// `plain`: b is where that holds (div_plain); a value too small or too large for it is divided.
+__device__ __forceinline__ bool div_plain(float b) { return fabsf(b) >= 1e-12f && fabsf(b) <= 1e12f; }
+__device__ __forceinline__ float div_rn_by(float a, float b, float y, bool plain) {
+  const float q = a * y, size = fabsf(a);
+  float r = fmaf(fmaf(-q, b, a), y, q);
+  if (!plain || !(size <= 1e15f) || (size < 1e-15f && a != 0.f)) r = __fdiv_rn(a, b);
+  return r;
 }
 
-// eps for int8-coded rows (operand residual of the rows is zero; the query operand is fp16(s_q q~)):
-//   contraction   |e_q| C + dim16 2^-22 |q'| C, divided by s_q          (C = max |code row|)
-//   formula       2^-22 (|q| max|x^| + |q~| C): fp32 rounding of x^ = (code - offset)/scale and of q~
-// doubled for euclidean (value = |x^|^2 - 2 q.x^) plus the rounding of |x^|^2 and of the final multiply-add.
-template <int METRIC>
-__global__ void bound_i8_kernel(const float* __restrict__ qn16, const float* __restrict__ qe16,
-                                const float* __restrict__ qt_norm, const float* __restrict__ q_norm, int64_t nq,
-                                const float* scale_q, BoundConsts c, float* __restrict__ eps, float* alpha) {
-  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const float inv = 1.0f / (*scale_q);
-  if (q == 0) *alpha = (METRIC == VSK_METRIC_EUCLIDEAN ? -2.0f : -1.0f) * inv;
-  if (q >= nq) return;
-  const float a = qn16[q], e = qe16[q];
-  float dot_err = (e * c.max_norm16 + (float)c.dim16 * 2.3841858e-7f * a * c.max_norm16) * inv;
-  dot_err += 2.3841858e-7f * (q_norm[q] * c.max_norm + qt_norm[q] * c.max_norm16);
-  float r = dot_err;
-  if (METRIC == VSK_METRIC_EUCLIDEAN)
-    r = 2.0f * dot_err + 4.0f * 5.9604645e-8f * (float)c.dim16 * c.max_norm * c.max_norm +
-        2.0f * 5.9604645e-8f * (c.max_norm * c.max_norm + 2.0f * q_norm[q] * c.max_norm);
-  eps[q] = r * 1.0001f + 1e-30f;
+// Sums of RR rows of codes against the query in shared memory: the metric between the fp32 query and x^ = (code - offset)/scale,
+// every operation of x^ rounded by itself (ScalarQuantizer.swift:576-578).  A lane's dimensions are lane, lane + 32, ..; the
+// parameters of a dimension serve all rows, and their reciprocal replaces the rows' divisions.
+template <int METRIC, int RR>
+__device__ __forceinline__ void i8_row_sums(const float* qs, const int8_t* __restrict__ codes, int dim, const float* __restrict__ scale,
+                                            const float* __restrict__ offset, const uint32_t (&id)[RR], int lane, float (&sum)[RR]) {
+  const int8_t* xr[RR];
+#pragma unroll
+  for (int r = 0; r < RR; ++r) {
+    xr[r] = codes + (int64_t)id[r] * dim;
+    sum[r] = 0.f;
+  }
+#pragma unroll 2
+  for (int i = lane; i < dim; i += 32) {
+    int8_t code[RR];
+#pragma unroll
+    for (int r = 0; r < RR; ++r) code[r] = __ldg(xr[r] + i);
+    const float sc = __ldg(scale + i), of = __ldg(offset + i), qv = qs[i], y = __frcp_rn(sc);
+    const bool plain = div_plain(sc);
+#pragma unroll
+    for (int r = 0; r < RR; ++r) {
+      const float xv = div_rn_by(__fsub_rn((float)code[r], of), sc, y, plain);
+      if (METRIC == VSK_METRIC_EUCLIDEAN) {
+        const float d = qv - xv;
+        sum[r] = fmaf(d, d, sum[r]);
+      } else {
+        sum[r] = fmaf(qv, xv, sum[r]);
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < RR; ++r)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o);
 }
 
-// Exact re-scoring against dequantised rows (the int8 scan's definition: the metric between the fp32 query
-// and x^ = (code - offset)/scale, ScalarQuantizer.swift:576-578).
+// Exact re-scoring against dequantised rows.  Four rows per warp step share a dimension's parameters and reciprocal: a row at a
+// time, each code divided by its scale, the seven launches of 10 000 queries over 6.25 million x 384 took 2.84 ms.
 template <int METRIC>
 __global__ void __launch_bounds__(256) rerank_i8_kernel(const float* __restrict__ q, const int8_t* __restrict__ codes,
                                                         int dim, const float* __restrict__ scale,
@@ -1809,23 +1943,16 @@ __global__ void __launch_bounds__(256) rerank_i8_kernel(const float* __restrict_
   if (threadIdx.x == 0) atomicAdd(total, (unsigned long long)cnt);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  for (int c = warp; c < cnt; c += nwarps) {
-    const uint32_t id = (uint32_t)keys[c];
-    const int8_t* xr = codes + (int64_t)id * dim;
-    float s = 0.f;
-    for (int i = lane; i < dim; i += 32) {
-      const float xv = __fdiv_rn(__fsub_rn((float)xr[i], __ldg(offset + i)), __ldg(scale + i));
-      const float qv = qs[i];
-      if (METRIC == VSK_METRIC_EUCLIDEAN) {
-        const float d = qv - xv;
-        s = fmaf(d, d, s);
-      } else {
-        s = fmaf(qv, xv, s);
-      }
-    }
+  constexpr int RR = 4;
+  for (int c0 = warp * RR; c0 < cnt; c0 += nwarps * RR) {
+    uint32_t id[RR];
+    float sum[RR];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) keys[c] = make_key(METRIC == VSK_METRIC_EUCLIDEAN ? s : -s, id);
+    for (int r = 0; r < RR; ++r) id[r] = (uint32_t)keys[min(c0 + r, cnt - 1)];
+    i8_row_sums<METRIC, RR>(qs, codes, dim, scale, offset, id, lane, sum);
+#pragma unroll
+    for (int r = 0; r < RR; ++r)
+      if (lane == r && c0 + r < cnt) *VSK_CHK_W(keys + c0 + r) = make_key(METRIC == VSK_METRIC_EUCLIDEAN ? sum[r] : -sum[r], id[r]);
   }
 }
 
@@ -1895,6 +2022,8 @@ struct FinishArgs {
   CandLists cand;
   int32_t dense_count;        // >= 0: the list holds exactly this many slots
   const float *q, *x, *qnorm, *xnorm;
+  const int8_t* codes;        // I8: the rows, with ...
+  const float *sq_scale, *sq_offset;
   int32_t dim, k;
   const float* eps;
   const float* ext_bound;     // or null (SelectArgs::ext_bound)
@@ -1907,7 +2036,7 @@ struct FinishArgs {
 };
 template <int NT> constexpr int kFinishMinBlocks = NT == 128 ? 8 : 2;
 
-template <int METRIC, int NT>
+template <int METRIC, int NT, bool I8 = false>
 __global__ void __launch_bounds__(NT, kFinishMinBlocks<NT>) finish_kernel(FinishArgs a) {
   extern __shared__ __align__(16) uint64_t s_keys[];
   constexpr int CAPACITY = NT * SEL_ITEMS;
@@ -1966,6 +2095,18 @@ __global__ void __launch_bounds__(NT, kFinishMinBlocks<NT>) finish_kernel(Finish
   const float qn = (METRIC == VSK_METRIC_COSINE) ? *VSK_CHK(a.qnorm + qi) : 0.f;
   constexpr int RR = 4, U = 4;
   for (int c0 = warp * RR; c0 < cnt; c0 += (NT / 32) * RR) {
+    if constexpr (I8) {
+      uint32_t id[RR];
+      float sum[RR];
+#pragma unroll
+      for (int r = 0; r < RR; ++r) id[r] = (uint32_t)s_keys[min(c0 + r, cnt - 1)];
+      i8_row_sums<METRIC, RR>(qs, a.codes, a.dim, a.sq_scale, a.sq_offset, id, lane, sum);
+      __syncwarp();
+#pragma unroll
+      for (int r = 0; r < RR; ++r)
+        if (lane == r && c0 + r < cnt) s_keys[c0 + r] = make_key(METRIC == VSK_METRIC_EUCLIDEAN ? sum[r] : -sum[r], id[r]);
+      continue;
+    }
     uint32_t id[RR];
     const float* xr[RR];
     float sum[RR];
@@ -2228,15 +2369,16 @@ template <int MODE, int EW, bool I8 = false>
 int32_t launch_tc_ew(Ctx* ctx, const CUtensorMap& mq, const CUtensorMap& mx, const TcArgs& a, bool has_beta) {
   const bool has_mask = MODE != SCAN_ARGMIN && a.row_masks != nullptr && a.q_masks != nullptr;
   void (*kern)(CUtensorMap, CUtensorMap, TcArgs);
+  constexpr bool BETA = EW == 8 && !I8;   // (tc_epilogue_warps: a per-row term comes with eight warps)
   if constexpr (I8) {
     kern = tc_scan_kernel<MODE, false, false, EW, true>;
   } else if constexpr (MODE == SCAN_ARGMIN) {
-    kern = has_beta ? tc_scan_kernel<MODE, true, false, EW> : tc_scan_kernel<MODE, false, false, EW>;
+    kern = has_beta ? tc_scan_kernel<MODE, BETA, false, EW> : tc_scan_kernel<MODE, false, false, EW>;
   } else {
-    kern = has_mask ? (has_beta ? tc_scan_kernel<MODE, true, true, EW> : tc_scan_kernel<MODE, false, true, EW>)
-                    : (has_beta ? tc_scan_kernel<MODE, true, false, EW> : tc_scan_kernel<MODE, false, false, EW>);
+    kern = has_mask ? (has_beta ? tc_scan_kernel<MODE, BETA, true, EW> : tc_scan_kernel<MODE, false, true, EW>)
+                    : (has_beta ? tc_scan_kernel<MODE, BETA, false, EW> : tc_scan_kernel<MODE, false, false, EW>);
   }
-  constexpr size_t smem = tc_smem_bytes<EW>();
+  const size_t smem = has_beta ? tc_smem_bytes<EW, BETA>() : tc_smem_bytes<EW, false>();
   VSK_CUDA(ctx, opt_in_shared(ctx, kern, smem));
   const int64_t tiles = a.tiles ? a.num_tiles : ceil_div(a.nq, TM) * ceil_div(a.row_end - a.row_begin, TN);
   if (tiles <= 0) return VSK_OK;
@@ -2260,12 +2402,13 @@ int32_t launch_tc_ew(Ctx* ctx, const CUtensorMap& mq, const CUtensorMap& mx, con
   return VSK_OK;
 }
 
-// Epilogue warps by contraction length (see Epi): 16 up to four K blocks (d <= 256), 8 beyond.
-inline int tc_epilogue_warps(int kblocks) { return kblocks <= 4 ? 16 : 8; }
+// Epilogue warps by contraction length (see Epi): 16 up to four K blocks (d <= 256), 8 beyond and with a per-row term, which needs more
+// registers than sixteen warps have (2 000 queries over 500 000 x 200 int8 rows, euclidean: 0.76 ms with eight, 1.24 with sixteen).
+inline int tc_epilogue_warps(int kblocks, bool has_beta) { return kblocks <= 4 && !has_beta ? 16 : 8; }
 
 template <int MODE>
 int32_t launch_tc(Ctx* ctx, const CUtensorMap& mq, const CUtensorMap& mx, const TcArgs& a, bool has_beta) {
-  if (tc_epilogue_warps(a.kblocks) == 16) return launch_tc_ew<MODE, 16>(ctx, mq, mx, a, has_beta);
+  if (tc_epilogue_warps(a.kblocks, has_beta) == 16) return launch_tc_ew<MODE, 16>(ctx, mq, mx, a, false);
   return launch_tc_ew<MODE, 8>(ctx, mq, mx, a, has_beta);
 }
 
@@ -2608,7 +2751,7 @@ int32_t make_map_rows_f32(Ctx* ctx, const float* base, int64_t rows, int32_t dim
 }
 
 // ---- query operands of a search -----------------------------------------------------------------------
-// Over int8 codes or product-quantised rows: fp16 operand rows of the queries, their error bound eps[q], the output coefficient alpha, and the small words a
+// fp16 operand rows of the queries, their error bound eps[q], the output coefficient alpha, and the small words a
 // search needs (device error word, re-scored row counter), all in the current lane's scratch.
 struct QueryOperands {
   float* norm = nullptr;    // [nq] |q| (flat_query_operands)
@@ -2620,17 +2763,14 @@ struct QueryOperands {
   unsigned long long* rr_total = nullptr;
 };
 
+// Over product-quantised rows: one scale and coefficient for the batch, operand rows up to list_scan_kernel's whole blocks.
 int32_t prepare_query_operands(Index* ix, const float* q, int64_t nq, QueryOperands* out) {
   VSK_TRACE("vsk:query_operands");
   Ctx* ctx = ix->ctx;
-  prefer_shared_carveout(ctx, absmax_kernel, choose_scale_kernel, scale_queries_kernel, prep_rows_kernel<VSK_METRIC_EUCLIDEAN>,
-                         prep_rows_kernel<VSK_METRIC_COSINE>, prep_rows_kernel<VSK_METRIC_DOT_PRODUCT>, bound_kernel<VSK_METRIC_EUCLIDEAN>, bound_i8_kernel<VSK_METRIC_EUCLIDEAN>,
-                         bound_i8_kernel<VSK_METRIC_DOT_PRODUCT>, rerank_kernel<VSK_METRIC_EUCLIDEAN>, rerank_kernel<VSK_METRIC_COSINE>,
-                         rerank_kernel<VSK_METRIC_DOT_PRODUCT>, rerank_i8_kernel<VSK_METRIC_EUCLIDEAN>, rerank_i8_kernel<VSK_METRIC_DOT_PRODUCT>);
-  const int metric = ix->metric;
+  prefer_shared_carveout(ctx, absmax_kernel, choose_scale_kernel, prep_rows_kernel<VSK_METRIC_EUCLIDEAN>, bound_kernel<VSK_METRIC_EUCLIDEAN>);
   const int dim = ix->dim, dim16 = ix->dim16;
   void* p;
-  const int64_t nq_pad = ix->kind == INDEX_PQ ? ceil_div(nq, TN) * TN : nq;   // (list_scan_kernel's whole blocks)
+  const int64_t nq_pad = ceil_div(nq, TN) * TN;
   VSK_TRY(scratch(ctx, SLOT_Q16, (size_t)nq_pad * dim16 * sizeof(__half), &p));
   __half* q16 = (__half*)p;
   if (nq_pad > nq) VSK_CUDA(ctx, cudaMemsetAsync(q16 + nq * dim16, 0, (size_t)(nq_pad - nq) * dim16 * sizeof(__half), ctx->stream));
@@ -2646,42 +2786,15 @@ int32_t prepare_query_operands(Index* ix, const float* q, int64_t nq, QueryOpera
   int32_t* err = (int32_t*)p + 3;
   unsigned long long* rr_total = (unsigned long long*)((char*)p + 16);
   VSK_CUDA(ctx, cudaMemsetAsync(p, 0, 64, ctx->stream));
-  const bool i8 = ix->kind == INDEX_FLAT_I8;
-  if (i8 && metric != VSK_METRIC_EUCLIDEAN && metric != VSK_METRIC_DOT_PRODUCT)
-    return fail(ctx, VSK_ERR_UNSUPPORTED_OPERATION, "the tensor path over int8 codes covers euclidean and dotProduct");
-  const float* qsrc = q;   // what the query operand is made from
-  float* q_true_norm = nullptr;
-  if (i8) {
-    VSK_TRY(scratch(ctx, SLOT_TC_C, (size_t)nq * dim * sizeof(float), &p));
-    float* qt = (float*)p;
-    scale_queries_kernel<<<(unsigned)ceil_div(nq * (int64_t)dim, 256), 256, 0, ctx->stream>>>(q, nq * (int64_t)dim, dim, ix->sq_scale, qt);
-    ctx->stats.kernel_launches++;
-    qsrc = qt;
-    VSK_TRY(scratch(ctx, SLOT_TC_D, (size_t)nq * sizeof(float), &p));
-    q_true_norm = (float*)p;
-    VSK_TRY(launch_row_norms(ctx, q, nq, dim, 0, q_true_norm));
-  }
-  absmax_kernel<<<296, 256, 0, ctx->stream>>>(qsrc, nq * (int64_t)dim, q_absmax);
-  ctx->stats.kernel_launches++;
+  absmax_kernel<<<296, 256, 0, ctx->stream>>>(q, nq * (int64_t)dim, q_absmax);
   const bool fold = ix->fold16;
   const FoldArgs qfold{fold ? 2 : 0, fold_col0(ix->dim), ix->fold_exp};
-  // (a product-quantised index may put twice the constants into the fold columns, list_scan_kernel)
-  choose_scale_kernel<<<1, 1, 0, ctx->stream>>>(q_absmax, 0, q_scale, fold ? 1 : 0,
-                                                ix->fold_exp - (ix->kind == INDEX_PQ ? 1 : 0));
-  ctx->stats.kernel_launches++;
+  // (list_scan_kernel may put twice the constants into the fold columns)
+  choose_scale_kernel<<<1, 1, 0, ctx->stream>>>(q_absmax, 0, q_scale, fold ? 1 : 0, ix->fold_exp - 1);
   BoundConsts bc{ix->scale16, ix->max_xnorm16, ix->max_xerr16, ix->max_xnorm, ix->min_xnorm_nz, dim16, fold ? ix->fold_bmax : 0.f};
-  const unsigned bgrid = (unsigned)ceil_div(nq, 256);
-  if (i8) {
-    launch_prep<VSK_METRIC_DOT_PRODUCT>(ctx, qsrc, nq, dim, dim16, q_scale, q16, nullptr, qn16, qe16, qn_tmp, nullptr);
-    if (metric == VSK_METRIC_EUCLIDEAN)
-      bound_i8_kernel<VSK_METRIC_EUCLIDEAN><<<bgrid, 256, 0, ctx->stream>>>(qn16, qe16, qn_tmp, q_true_norm, nq, q_scale, bc, eps, alpha);
-    else
-      bound_i8_kernel<VSK_METRIC_DOT_PRODUCT><<<bgrid, 256, 0, ctx->stream>>>(qn16, qe16, qn_tmp, q_true_norm, nq, q_scale, bc, eps, alpha);
-  } else {
-    launch_prep<VSK_METRIC_EUCLIDEAN>(ctx, q, nq, dim, dim16, q_scale, q16, nullptr, qn16, qe16, qn_tmp, nullptr, qfold);
-    bound_kernel<VSK_METRIC_EUCLIDEAN><<<bgrid, 256, 0, ctx->stream>>>(qn16, qe16, qn_tmp, nq, q_scale, bc, eps, alpha);
-  }
-  ctx->stats.kernel_launches++;
+  launch_prep<VSK_METRIC_EUCLIDEAN>(ctx, q, nq, dim, dim16, q_scale, q16, nullptr, qn16, qe16, qn_tmp, nullptr, qfold);
+  bound_kernel<VSK_METRIC_EUCLIDEAN><<<(unsigned)ceil_div(nq, 256), 256, 0, ctx->stream>>>(qn16, qe16, qn_tmp, nq, q_scale, bc, eps, alpha);
+  ctx->stats.kernel_launches += 3;
   VSK_CUDA(ctx, cudaGetLastError());
   tl_mark(ctx, "query_operands");
   out->q16 = q16;
@@ -2693,14 +2806,21 @@ int32_t prepare_query_operands(Index* ix, const float* q, int64_t nq, QueryOpera
   return VSK_OK;
 }
 
-// The same for a flat fp32 index, with a scale and a coefficient per query (alpha is an array), and the lists emptied.
+// Over a flat index, fp32 rows or int8 codes: a scale and a coefficient per query (alpha is an array), and the lists emptied.
 int32_t flat_query_operands(Index* ix, const float* q, int64_t nq, const CandLists& cand, QueryOperands* out) {
   VSK_TRACE("vsk:query_operands");
   Ctx* ctx = ix->ctx;
   prefer_shared_carveout(ctx, query_prep_kernel<VSK_METRIC_EUCLIDEAN>, query_prep_kernel<VSK_METRIC_COSINE>, query_prep_kernel<VSK_METRIC_DOT_PRODUCT>,
                          finish_kernel<VSK_METRIC_EUCLIDEAN, 128>, finish_kernel<VSK_METRIC_COSINE, 128>, finish_kernel<VSK_METRIC_DOT_PRODUCT, 128>,
-                         finish_kernel<VSK_METRIC_EUCLIDEAN, 512>, finish_kernel<VSK_METRIC_COSINE, 512>, finish_kernel<VSK_METRIC_DOT_PRODUCT, 512>);
+                         finish_kernel<VSK_METRIC_EUCLIDEAN, 512>, finish_kernel<VSK_METRIC_COSINE, 512>, finish_kernel<VSK_METRIC_DOT_PRODUCT, 512>,
+                         query_prep_kernel<VSK_METRIC_EUCLIDEAN, true>, query_prep_kernel<VSK_METRIC_DOT_PRODUCT, true>,
+                         finish_kernel<VSK_METRIC_EUCLIDEAN, 128, true>, finish_kernel<VSK_METRIC_DOT_PRODUCT, 128, true>,
+                         finish_kernel<VSK_METRIC_EUCLIDEAN, 512, true>, finish_kernel<VSK_METRIC_DOT_PRODUCT, 512, true>);
+  const bool i8 = ix->kind == INDEX_FLAT_I8;
+  if (i8 && ix->metric != VSK_METRIC_EUCLIDEAN && ix->metric != VSK_METRIC_DOT_PRODUCT)
+    return fail(ctx, VSK_ERR_UNSUPPORTED_OPERATION, "the tensor path over int8 codes covers euclidean and dotProduct");
   QueryPrep a{};
+  a.sq_scale = ix->sq_scale;
   void* p;
   VSK_TRY(scratch(ctx, SLOT_Q16, (size_t)nq * ix->dim16 * sizeof(__half), &p));
   a.out = (__half*)p;
@@ -2718,6 +2838,10 @@ int32_t flat_query_operands(Index* ix, const float* q, int64_t nq, const CandLis
   a.fold = FoldArgs{ix->fold16 ? 2 : 0, fold_col0(ix->dim), ix->fold_exp};
   a.cand = cand;
   const unsigned grid = (unsigned)ceil_div(nq, 8);
+  if (i8) {
+    if (ix->metric == VSK_METRIC_EUCLIDEAN) query_prep_kernel<VSK_METRIC_EUCLIDEAN, true><<<grid, 256, 0, ctx->stream>>>(a);
+    else query_prep_kernel<VSK_METRIC_DOT_PRODUCT, true><<<grid, 256, 0, ctx->stream>>>(a);
+  } else
   switch (ix->metric) {
     case VSK_METRIC_EUCLIDEAN: query_prep_kernel<VSK_METRIC_EUCLIDEAN><<<grid, 256, 0, ctx->stream>>>(a); break;
     case VSK_METRIC_COSINE: query_prep_kernel<VSK_METRIC_COSINE><<<grid, 256, 0, ctx->stream>>>(a); break;
@@ -2752,20 +2876,20 @@ int32_t cand_lists(Ctx* ctx, int64_t nq, CandLists* cand) {
 // Whether a query row fits beside the largest list in finish_kernel's shared memory.
 bool finish_applies(int dim) { return (size_t)dim * sizeof(float) <= 160 * 1024; }
 
-template <int METRIC, int NT>
+template <int METRIC, int NT, bool I8>
 int32_t launch_finish_as(Ctx* ctx, const FinishArgs& f, int64_t nq) {
   const size_t smem = (size_t)NT * SEL_ITEMS * sizeof(uint64_t) + (size_t)f.dim * sizeof(float);
-  if (smem > 48 * 1024) VSK_CUDA(ctx, cudaFuncSetAttribute(finish_kernel<METRIC, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  finish_kernel<METRIC, NT><<<(unsigned)nq, NT, smem, ctx->stream>>>(f);
+  if (smem > 48 * 1024) VSK_CUDA(ctx, cudaFuncSetAttribute(finish_kernel<METRIC, NT, I8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  finish_kernel<METRIC, NT, I8><<<(unsigned)nq, NT, smem, ctx->stream>>>(f);
   tl_mark(ctx, "finish");
   ctx->stats.kernel_launches++;
   VSK_CUDA(ctx, cudaGetLastError());
   return VSK_OK;
 }
 // small: no list holds more than 1 024 keys
-template <int METRIC>
+template <int METRIC, bool I8 = false>
 int32_t launch_finish(Ctx* ctx, const FinishArgs& f, int64_t nq, bool small) {
-  return small ? launch_finish_as<METRIC, 128>(ctx, f, nq) : launch_finish_as<METRIC, 512>(ctx, f, nq);
+  return small ? launch_finish_as<METRIC, 128, I8>(ctx, f, nq) : launch_finish_as<METRIC, 512, I8>(ctx, f, nq);
 }
 
 // The search in two halves.  `begin` runs the scan and its compactions; `finish` certifies, re-scores and orders.
@@ -2783,19 +2907,14 @@ int32_t tensor_search_begin(Index* ix, const float* q, int64_t nq, int32_t k, co
   const int metric = ix->metric;
   const int dim16 = ix->dim16;
   const int32_t keep = std::min<int32_t>(kCandCap / 2, k + std::max(8, k / 8));
-  // An fp32 index's second half is one launch, the last compaction in it (finish_kernel); rows too wide for its shared memory,
-  // and codes, keep the separate ones.
-  const bool fused = ix->kind == INDEX_FLAT_F32 && finish_applies(ix->dim);
+  // The second half is one launch, the last compaction in it (finish_kernel); rows too wide for its shared memory keep the
+  // separate ones.
+  const bool fused = finish_applies(ix->dim);
   CandLists cand;
   VSK_TRY(cand_lists(ctx, nq, &cand));
   QueryOperands qo;
-  if (ix->kind == INDEX_FLAT_F32) {
-    VSK_TRY(flat_query_operands(ix, q, nq, cand, &qo));
-    if (!qnorm) qnorm = qo.norm;
-  } else {
-    VSK_TRY(prepare_query_operands(ix, q, nq, &qo));
-    VSK_TRY(launch_init_cand(ctx, cand, nq));
-  }
+  VSK_TRY(flat_query_operands(ix, q, nq, cand, &qo));
+  if (!qnorm) qnorm = qo.norm;
   const bool fold = ix->fold16;
 
   CUtensorMap mq, mx;
@@ -2804,7 +2923,7 @@ int32_t tensor_search_begin(Index* ix, const float* q, int64_t nq, int32_t k, co
 
   // ---- the chunk schedule ----
   TcArgs a{};
-  a.alpha_per_query = ix->kind == INDEX_FLAT_F32 ? 1 : 0;
+  a.alpha_per_query = 1;
   a.nq = nq;
   a.kblocks = dim16 / TK;
   a.k16_last = k16_last_of(fold ? fold_col0(ix->dim) + kFoldCols : ix->dim, dim16);
@@ -2914,6 +3033,7 @@ int32_t tensor_search_finish_issue(Index* ix, const float* ext_bound, float* out
   const int metric = ix->metric;
   const int dim = ix->dim;
   const bool i8 = ix->kind == INDEX_FLAT_I8;
+  if (i8 && dim > 12 * 1024) return fail(ctx, VSK_ERR_INVALID_BUFFER_SIZE, "dimension %d is too large for the int8 rerank kernel", dim);
   PinnedBuf& hb = ctx->host_flags[ctx->lane];
   VSK_TRY(pinned_reserve(ctx, &hb, (size_t)nq * 4 + 16));
   if (pd.fused) {
@@ -2924,6 +3044,9 @@ int32_t tensor_search_finish_issue(Index* ix, const float* ext_bound, float* out
     f.x = ix->rows;
     f.qnorm = qnorm;
     f.xnorm = ix->row_norm;
+    f.codes = ix->codes;
+    f.sq_scale = ix->sq_scale;
+    f.sq_offset = ix->sq_offset;
     f.dim = dim;
     f.k = k;
     f.eps = pd.eps;
@@ -2935,6 +3058,10 @@ int32_t tensor_search_finish_issue(Index* ix, const float* ext_bound, float* out
     f.host_err = (int32_t*)hb.p;
     f.host_flags = (int32_t*)hb.p + 4;
     const bool small = pd.max_count <= 128 * SEL_ITEMS && pd.dense_count <= 128 * SEL_ITEMS;
+    if (i8) {
+      if (metric == VSK_METRIC_EUCLIDEAN) VSK_TRY((launch_finish<VSK_METRIC_EUCLIDEAN, true>(ctx, f, nq, small)));
+      else VSK_TRY((launch_finish<VSK_METRIC_DOT_PRODUCT, true>(ctx, f, nq, small)));
+    } else
     switch (metric) {
       case VSK_METRIC_EUCLIDEAN: VSK_TRY(launch_finish<VSK_METRIC_EUCLIDEAN>(ctx, f, nq, small)); break;
       case VSK_METRIC_COSINE: VSK_TRY(launch_finish<VSK_METRIC_COSINE>(ctx, f, nq, small)); break;
@@ -2967,13 +3094,6 @@ int32_t tensor_search_finish_issue(Index* ix, const float* ext_bound, float* out
       VSK_CUDA(ctx, cudaFuncSetAttribute(rerank_kernel<M_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qsm)); \
     rerank_kernel<M_><<<(unsigned)nq, 256, qsm, ctx->stream>>>(q, ix->rows, dim, qnorm, ix->row_norm, cand, pd.rr_total); \
   } while (0)
-  if (i8) {
-    if (qsm > 48 * 1024) return fail(ctx, VSK_ERR_INVALID_BUFFER_SIZE, "dimension %d is too large for the int8 rerank kernel", dim);
-    if (metric == VSK_METRIC_EUCLIDEAN)
-      rerank_i8_kernel<VSK_METRIC_EUCLIDEAN><<<(unsigned)nq, 256, qsm, ctx->stream>>>(q, ix->codes, dim, ix->sq_scale, ix->sq_offset, cand, pd.rr_total);
-    else
-      rerank_i8_kernel<VSK_METRIC_DOT_PRODUCT><<<(unsigned)nq, 256, qsm, ctx->stream>>>(q, ix->codes, dim, ix->sq_scale, ix->sq_offset, cand, pd.rr_total);
-  } else
   switch (metric) {
     case VSK_METRIC_EUCLIDEAN: VSK_RERANK(VSK_METRIC_EUCLIDEAN); break;
     case VSK_METRIC_COSINE: VSK_RERANK(VSK_METRIC_COSINE); break;
@@ -3417,7 +3537,8 @@ int32_t ivf_tensor_search(Index* ix, const float* q, int64_t nq, const int64_t* 
     a.tiles = (const int4*)p;
     a.num_tiles = total;
     a.pair_thr = pair_thr;
-    VSK_TRY(launch_tc<SCAN_THRESHOLD>(ctx, mq, mx, a, !fold));
+    if (stage == 0) VSK_TRY(launch_tc<SCAN_ALL>(ctx, mq, mx, a, !fold));
+    else VSK_TRY(launch_tc<SCAN_THRESHOLD>(ctx, mq, mx, a, !fold));
     if (stage == 0) {
       // the pilot appended up to 1 024 rows per query: keep the best few by coarse value and re-score only those
       SelectArgs pre = sel;
@@ -4207,7 +4328,7 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
       la.cand = cand;
       la.err = err;
       VSK_TRY(launch_list_scan<true>(ctx, mx, mq, mx, mb, la, stride));
-    } else if (tc_epilogue_warps(a.kblocks) == 16) VSK_TRY((launch_tc_ew<SCAN_THRESHOLD, 16, true>(ctx, mq, mx, a, false)));
+    } else if (tc_epilogue_warps(a.kblocks, false) == 16) VSK_TRY((launch_tc_ew<SCAN_THRESHOLD, 16, true>(ctx, mq, mx, a, false)));
     else VSK_TRY((launch_tc_ew<SCAN_THRESHOLD, 8, true>(ctx, mq, mx, a, false)));
     rerank_i8_kernel<VSK_METRIC_DOT_PRODUCT><<<(unsigned)nq, 256, qsm, ctx->stream>>>(q, ix->codes, dim, ix->sq_scale, ix->sq_offset, cand, rr_total);
     ctx->stats.kernel_launches++;
@@ -4441,7 +4562,7 @@ int32_t tensor_assign(Ctx* ctx, TensorAssign* ta, const float* rows, const float
   a.mode = SCAN_THRESHOLD;
   VSK_TRY(launch_tc<SCAN_THRESHOLD>(ctx, mr, mc, a, true));
   assign_exact_kernel<<<(unsigned)ceil_div(n, 8), 256, 0, ctx->stream>>>(rows, n, dim, centroids, ta->keys, ta->count, assign, dist,
-                                                                         ta->bad_rows, (int32_t*)(sm + 6), tc_epilogue_warps(a.kblocks) / 4);
+                                                                         ta->bad_rows, (int32_t*)(sm + 6), tc_epilogue_warps(a.kblocks, true) / 4);
   ctx->stats.kernel_launches += 2;
   VSK_CUDA(ctx, cudaGetLastError());
   }
