@@ -1883,42 +1883,54 @@ __global__ void prep_codes_kernel(const int8_t* __restrict__ codes, int64_t n, i
 // second term does not depend on the row.
 // a / b rounded once, with y = 1 / b rounded once: Markstein's correction (IBM J. Res. Dev. 34, 1990) - the remainder of the
 // product a y is exact in a fused operation, and adding its share rounds correctly while nothing over- or underflows.
-// `plain`: b is where that holds (div_plain); a value too small or too large for it is divided.
-__device__ __forceinline__ bool div_plain(float b) { return fabsf(b) >= 1e-12f && fabsf(b) <= 1e12f; }
-__device__ __forceinline__ float div_rn_by(float a, float b, float y, bool plain) {
-  const float q = a * y, size = fabsf(a);
-  float r = fmaf(fmaf(-q, b, a), y, q);
-  if (!plain || !(size <= 1e15f) || (size < 1e-15f && a != 0.f)) r = __fdiv_rn(a, b);
-  return r;
+__device__ __forceinline__ float div_rn_by(float a, float b, float y) {
+  const float q = a * y;
+  return fmaf(fmaf(-q, b, a), y, q);
+}
+// The reciprocal for a dimension's codes, or NaN where the correction does not hold for all of them: a code less the offset is 0 or
+// no smaller than the smaller of |offset| and one unit in the last place of it.
+__device__ __forceinline__ float div_reciprocal(float scale, float offset) {
+  const float s = fabsf(scale), o = fabsf(offset);
+  const bool plain = s >= 1e-12f && s <= 1e12f && (o == 0.f || o >= 1e-15f) && o <= 1e14f;
+  return plain ? __frcp_rn(scale) : CUDART_NAN_F;
 }
 
-// Sums of RR rows of codes against the query in shared memory: the metric between the fp32 query and x^ = (code - offset)/scale,
-// every operation of x^ rounded by itself (ScalarQuantizer.swift:576-578).  A lane's dimensions are lane, lane + 32, ..; the
-// parameters of a dimension serve all rows, and their reciprocal replaces the rows' divisions.
+// Sums of RR rows of codes against the query in shared memory (qs, and behind it the dimensions' reciprocals): the metric between
+// the fp32 query and x^ = (code - offset)/scale, every operation of x^ rounded by itself (ScalarQuantizer.swift:576-578).  A lane's
+// dimensions are lane, lane + 32, ..; the parameters of a dimension serve all rows, its reciprocal replaces the rows' divisions, and a
+// code becomes a number by its place in a mantissa (8 388 608 + 128 + code; conversions run at an eighth of the rate).
 template <int METRIC, int RR>
 __device__ __forceinline__ void i8_row_sums(const float* qs, const int8_t* __restrict__ codes, int dim, const float* __restrict__ scale,
                                             const float* __restrict__ offset, const uint32_t (&id)[RR], int lane, float (&sum)[RR]) {
-  const int8_t* xr[RR];
+  const uint8_t* xr[RR];
 #pragma unroll
   for (int r = 0; r < RR; ++r) {
-    xr[r] = codes + (int64_t)id[r] * dim;
+    xr[r] = reinterpret_cast<const uint8_t*>(codes) + (int64_t)id[r] * dim;
     sum[r] = 0.f;
   }
 #pragma unroll 2
   for (int i = lane; i < dim; i += 32) {
-    int8_t code[RR];
+    uint32_t code[RR];
 #pragma unroll
     for (int r = 0; r < RR; ++r) code[r] = __ldg(xr[r] + i);
-    const float sc = __ldg(scale + i), of = __ldg(offset + i), qv = qs[i], y = __frcp_rn(sc);
-    const bool plain = div_plain(sc);
+    const float sc = __ldg(scale + i), of = __ldg(offset + i), qv = qs[i], y = qs[dim + i];
+    float xv[RR];
+#pragma unroll
+    for (int r = 0; r < RR; ++r) xv[r] = __fsub_rn(__uint_as_float(code[r] ^ 0x4b000080u) - 8388736.0f, of);
+    if (y == y) {
+#pragma unroll
+      for (int r = 0; r < RR; ++r) xv[r] = div_rn_by(xv[r], sc, y);
+    } else {
+#pragma unroll
+      for (int r = 0; r < RR; ++r) xv[r] = __fdiv_rn(xv[r], sc);
+    }
 #pragma unroll
     for (int r = 0; r < RR; ++r) {
-      const float xv = div_rn_by(__fsub_rn((float)code[r], of), sc, y, plain);
       if (METRIC == VSK_METRIC_EUCLIDEAN) {
-        const float d = qv - xv;
+        const float d = qv - xv[r];
         sum[r] = fmaf(d, d, sum[r]);
       } else {
-        sum[r] = fmaf(qv, xv, sum[r]);
+        sum[r] = fmaf(qv, xv[r], sum[r]);
       }
     }
   }
@@ -1939,7 +1951,10 @@ __global__ void __launch_bounds__(256) rerank_i8_kernel(const float* __restrict_
   const int64_t qi = blockIdx.x;
   const int cnt = min(cand.count[qi], kCandCap);
   uint64_t* keys = cand.keys + qi * kCandCap;
-  for (int i = threadIdx.x; i < dim; i += blockDim.x) qs[i] = q[qi * dim + i];
+  for (int i = threadIdx.x; i < dim; i += blockDim.x) {
+    qs[i] = q[qi * dim + i];
+    qs[dim + i] = div_reciprocal(__ldg(scale + i), __ldg(offset + i));
+  }
   if (threadIdx.x == 0) atomicAdd(total, (unsigned long long)cnt);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
@@ -2056,7 +2071,10 @@ __global__ void __launch_bounds__(NT, kFinishMinBlocks<NT>) finish_kernel(Finish
     key[i] = idx < c ? *VSK_CHK(keys + idx) : kEmptyKey;
     nvalid += key[i] != kEmptyKey;
   }
-  for (int i = threadIdx.x; i < a.dim; i += NT) qs[i] = *VSK_CHK(a.q + qi * a.dim + i);
+  for (int i = threadIdx.x; i < a.dim; i += NT) {
+    qs[i] = *VSK_CHK(a.q + qi * a.dim + i);
+    if (I8) qs[a.dim + i] = div_reciprocal(__ldg(a.sq_scale + i), __ldg(a.sq_offset + i));
+  }
   if (threadIdx.x == 0) { s_valid = 0; s_out = 0; }
   __syncthreads();
   nvalid = __reduce_add_sync(0xffffffffu, nvalid);
@@ -2878,7 +2896,7 @@ bool finish_applies(int dim) { return (size_t)dim * sizeof(float) <= 160 * 1024;
 
 template <int METRIC, int NT, bool I8>
 int32_t launch_finish_as(Ctx* ctx, const FinishArgs& f, int64_t nq) {
-  const size_t smem = (size_t)NT * SEL_ITEMS * sizeof(uint64_t) + (size_t)f.dim * sizeof(float);
+  const size_t smem = (size_t)NT * SEL_ITEMS * sizeof(uint64_t) + (size_t)f.dim * sizeof(float) * (I8 ? 2 : 1);
   if (smem > 48 * 1024) VSK_CUDA(ctx, cudaFuncSetAttribute(finish_kernel<METRIC, NT, I8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   finish_kernel<METRIC, NT, I8><<<(unsigned)nq, NT, smem, ctx->stream>>>(f);
   tl_mark(ctx, "finish");
@@ -4291,7 +4309,9 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
     for (int64_t i = 0; i < nq; ++i) bad += hflags[i] != 0 && !(hflags[i] & kFlagDegenerate);
     return bad;
   };
-  const size_t qsm = (size_t)dim * sizeof(float);
+  const size_t qsm = (size_t)dim * sizeof(float);   // (i8_search_applicable: at most 48 KB)
+  if (2 * qsm > 48 * 1024)
+    VSK_CUDA(ctx, cudaFuncSetAttribute(rerank_i8_kernel<VSK_METRIC_DOT_PRODUCT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * qsm)));
   const int64_t growth = nq <= 2048 ? std::max(16, ctx->tuning.chunk_growth) : std::max(1, ctx->tuning.chunk_growth);
   bool looked = nq < 256;   // a small batch is cheap to scan twice: no look between its chunks
   while (seen < n) {
@@ -4330,7 +4350,7 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
       VSK_TRY(launch_list_scan<true>(ctx, mx, mq, mx, mb, la, stride));
     } else if (tc_epilogue_warps(a.kblocks, false) == 16) VSK_TRY((launch_tc_ew<SCAN_THRESHOLD, 16, true>(ctx, mq, mx, a, false)));
     else VSK_TRY((launch_tc_ew<SCAN_THRESHOLD, 8, true>(ctx, mq, mx, a, false)));
-    rerank_i8_kernel<VSK_METRIC_DOT_PRODUCT><<<(unsigned)nq, 256, qsm, ctx->stream>>>(q, ix->codes, dim, ix->sq_scale, ix->sq_offset, cand, rr_total);
+    rerank_i8_kernel<VSK_METRIC_DOT_PRODUCT><<<(unsigned)nq, 256, 2 * qsm, ctx->stream>>>(q, ix->codes, dim, ix->sq_scale, ix->sq_offset, cand, rr_total);
     ctx->stats.kernel_launches++;
     VSK_CUDA(ctx, cudaGetLastError());
     tl_mark(ctx, "rerank");
