@@ -138,6 +138,37 @@ def test_one_filter_group_that_overflows_does_not_shut_out_the_others(vsk, dev):
     ix.close()
 
 
+def test_filter_groups_take_turns_on_two_lanes(vsk, dev):
+    """Groups of different sizes, one that no row passes, one too small for the byte filter and one whose lists overflow, on both
+    lanes of the context: the fp32 scan's results, and the same again."""
+    rng = np.random.default_rng(36)
+    n, d = 480_000, 256
+    x = rng.uniform(-1, 1, (n, d)).astype(np.float32)
+    rm = np.uint64(1) << rng.integers(0, 6, n).astype(np.uint64)
+    sizes = [300, 240, 9, 80, 200, 66, 64]                       # the seventh group's bit is on no row
+    qm = np.concatenate([np.full(m, 1 << g, np.uint64) for g, m in enumerate(sizes)])
+    q = rng.uniform(-1, 1, (len(qm), d)).astype(np.float32)
+    late = np.arange(400_000, n)
+    x[late[rm[late] == 16]] = 0.02                               # 13 000 equal rows, nearest to some of the fifth group's queries
+    q[630:660] = 0.0
+    order = rng.permutation(len(qm))
+    q, qm = np.ascontiguousarray(q[order]), np.ascontiguousarray(qm[order])
+    ix = _index(vsk, dev, x, rm)
+    dev.set_search_path(1)
+    ref = ix.batchSearch(q, 20, qm)
+    dev.set_search_path(0)
+    for call in range(3):
+        dev.timeline(True)
+        dev.timeline_read()
+        got = ix.batchSearch(q, 20, qm)
+        lanes = {lane for lane, what, _ in dev.timeline_read() if what == "l1_scan"}
+        dev.timeline(False)
+        assert call == 0 or {int(v) for v in lanes} == {0, 1}    # (the first batch does not pay for the byte copy)
+        assert np.array_equal(got[1], ref[1]) and np.array_equal(got[0], ref[0])
+    assert np.all(got[1][qm == 64] == -1)
+    ix.close()
+
+
 def test_only_rows_that_are_re_scored_are_counted(vsk, dev):
     """The k rows kept from chunk to chunk carry their exact values already."""
     rng = np.random.default_rng(33)

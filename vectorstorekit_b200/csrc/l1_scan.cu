@@ -378,6 +378,13 @@ static bool l1_pays(Index* ix, int64_t n, int64_t nq, L1Call* call) {
 
 int32_t l1_topk(Index* ix, const ExactScanArgs& proto, int64_t n, int64_t nq, const int32_t* sub_dev, int32_t k, float* out_dist,
                 int64_t* out_ids, L1Call* call, bool* handled) {
+  L1Pending pending;
+  VSK_TRY(l1_issue(ix, proto, n, nq, sub_dev, k, out_dist, out_ids, call, handled, &pending));
+  return *handled ? l1_collect(ix, &pending, call) : VSK_OK;
+}
+
+int32_t l1_issue(Index* ix, const ExactScanArgs& proto, int64_t n, int64_t nq, const int32_t* sub_dev, int32_t k, float* out_dist,
+                 int64_t* out_ids, L1Call* call, bool* handled, L1Pending* pending) {
   VSK_TRACE("vsk:l1_scan");
   Ctx* ctx = ix->ctx;
   *handled = false;
@@ -482,23 +489,43 @@ int32_t l1_topk(Index* ix, const ExactScanArgs& proto, int64_t n, int64_t nq, co
   VSK_CUDA(ctx, cudaMemcpyAsync(hb.p, total, 8, cudaMemcpyDeviceToHost, ctx->stream));
   VSK_CUDA(ctx, cudaMemcpyAsync(hflags, cand.flags, (size_t)nq * 4, cudaMemcpyDeviceToHost, ctx->stream));
   if (sub_dev) VSK_CUDA(ctx, cudaMemcpyAsync(hsub, sub_dev, (size_t)nq * 4, cudaMemcpyDeviceToHost, ctx->stream));
+  pending->active = true;
+  pending->proto = proto;
+  pending->n = n;
+  pending->nq = nq;
+  pending->sub_dev = sub_dev;
+  pending->k = k;
+  pending->out_dist = out_dist;
+  pending->out_ids = out_ids;
+  *handled = true;
+  return VSK_OK;
+}
+
+// Waits for the lane's stream, and runs the queries whose list overflowed again on the fp32 scan.
+int32_t l1_collect(Index* ix, L1Pending* pending, L1Call* call) {
+  Ctx* ctx = ix->ctx;
+  const L1Pending pd = *pending;
+  pending->active = false;
   VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  const PinnedBuf& hb = ctx->host_flags[ctx->lane];
+  const int32_t* hflags = (const int32_t*)((const char*)hb.p + 16);
+  const int32_t* hsub = hflags + pd.nq;
   unsigned long long hrr;
   memcpy(&hrr, hb.p, 8);
   ctx->stats.reranked_rows += (int64_t)hrr;
   std::vector<int32_t> bad;
-  for (int64_t i = 0; i < nq; ++i) {
-    if (hflags[i]) bad.push_back(sub_dev ? hsub[i] : (int32_t)i);
+  for (int64_t i = 0; i < pd.nq; ++i) {
+    if (hflags[i]) bad.push_back(pd.sub_dev ? hsub[i] : (int32_t)i);
     call->bad += hflags[i] != 0 && !(hflags[i] & kFlagDegenerate);
   }
-  call->seen += nq;
-  *handled = true;
+  call->seen += pd.nq;
   if (bad.empty()) return VSK_OK;
+  void* p;
   VSK_TRY(scratch(ctx, SLOT_SUBSET, bad.size() * sizeof(int32_t), &p));
   VSK_CUDA(ctx, cudaMemcpyAsync(p, bad.data(), bad.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
   VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   ctx->stats.fallback_queries += (int64_t)bad.size();
-  return fp32_topk(ctx, proto, n, (int64_t)bad.size(), (const int32_t*)p, k, ix->id_base, out_dist, out_ids, 0);
+  return fp32_topk(ctx, pd.proto, pd.n, (int64_t)bad.size(), (const int32_t*)p, pd.k, ix->id_base, pd.out_dist, pd.out_ids, 0);
 }
 
 }  // namespace vsk

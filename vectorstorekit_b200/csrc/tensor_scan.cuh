@@ -64,6 +64,21 @@ constexpr int kL1RestOneIn = 4;
 bool l1_applicable(const Index* ix, int64_t n, int64_t nq, int32_t k);
 int32_t l1_topk(Index* ix, const ExactScanArgs& proto, int64_t n, int64_t nq, const int32_t* sub_dev, int32_t k, float* out_dist,
                 int64_t* out_ids, L1Call* call, bool* handled);
+// The same in two steps, so that the groups of a batch can take turns on the context's lanes: everything enqueued on the current
+// lane, its flag words on their way to the lane's pinned buffer, and, on the same lane before its next group, the wait and what is
+// to be run again.
+struct L1Pending {
+  bool active = false;
+  ExactScanArgs proto{};
+  int64_t n = 0, nq = 0;
+  const int32_t* sub_dev = nullptr;
+  int32_t k = 0;
+  float* out_dist = nullptr;
+  int64_t* out_ids = nullptr;
+};
+int32_t l1_issue(Index* ix, const ExactScanArgs& proto, int64_t n, int64_t nq, const int32_t* sub_dev, int32_t k, float* out_dist,
+                 int64_t* out_ids, L1Call* call, bool* handled, L1Pending* pending);
+int32_t l1_collect(Index* ix, L1Pending* pending, L1Call* call);
 // Candidate lists for nq queries in the current lane's scratch.
 int32_t cand_lists(Ctx* ctx, int64_t nq, CandLists* cand);
 // Drops the operand copies after rows were added; makes it (once per index state).
