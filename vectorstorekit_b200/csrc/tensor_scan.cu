@@ -1707,6 +1707,52 @@ __global__ void prep_rows_kernel(const float* __restrict__ x, int64_t n, int dim
   }
 }
 
+// The same for rows of at most 256 dimensions in 16-byte pieces (no fold, no metric of its own): a lane holds its pieces between
+// the two passes, so the row is read once, and stores four halves at a time.  10 million x 128, 192 operand columns: 3.4 - 3.9 ms
+// for the form above (its 64-byte stores), 1.6 here.
+__global__ void __launch_bounds__(256) prep_rows_wide_kernel(const float* __restrict__ x, int64_t n, int dim, int dim16, const float* scale_p,
+                                                             __half* __restrict__ out, float* __restrict__ nrm16, float* __restrict__ err16,
+                                                             float* __restrict__ nrm) {
+  const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= n) return;
+  const int lane = threadIdx.x & 31, nv = dim >> 2;
+  const float s = __ldg(scale_p);
+  const float4* p = reinterpret_cast<const float4*>(x + row * dim);
+  float4 v[2];
+#pragma unroll
+  for (int c = 0; c < 2; ++c) v[c] = lane + 32 * c < nv ? __ldg(p + lane + 32 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  float ss = 0.f, n2 = 0.f, e2 = 0.f;
+  uint2* o = reinterpret_cast<uint2*>(out + row * dim16);
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const float f[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
+    __half2 h[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const float t0 = f[2 * u] * s, t1 = f[2 * u + 1] * s;
+      h[u] = __floats2half2_rn(t0, t1);
+      const float2 b = __half22float2(h[u]);
+      ss = fmaf(f[2 * u], f[2 * u], fmaf(f[2 * u + 1], f[2 * u + 1], ss));
+      n2 = fmaf(b.x, b.x, fmaf(b.y, b.y, n2));
+      e2 = fmaf(t0 - b.x, t0 - b.x, fmaf(t1 - b.y, t1 - b.y, e2));
+    }
+    if (lane + 32 * c < dim16 >> 2) *VSK_CHK_W(o + lane + 32 * c) = make_uint2(*reinterpret_cast<uint32_t*>(&h[0]), *reinterpret_cast<uint32_t*>(&h[1]));
+  }
+  for (int c = lane + 64; c < dim16 >> 2; c += 32) *VSK_CHK_W(o + c) = make_uint2(0u, 0u);
+#pragma unroll
+  for (int k = 16; k > 0; k >>= 1) {
+    ss += __shfl_xor_sync(0xffffffffu, ss, k);
+    n2 += __shfl_xor_sync(0xffffffffu, n2, k);
+    e2 += __shfl_xor_sync(0xffffffffu, e2, k);
+  }
+  if (lane == 0) {
+    const float up = 1.0f + 1e-5f;   // the measured norms are used as upper bounds
+    *VSK_CHK_W(nrm16 + row) = sqrtf(n2) * up;
+    *VSK_CHK_W(err16 + row) = sqrtf(e2) * up;
+    *VSK_CHK_W(nrm + row) = sqrtf(ss);
+  }
+}
+
 struct BoundConsts {
   float scale_x;       // s_x
   float max_norm16;    // X' = max |x'|
@@ -4415,7 +4461,12 @@ int32_t tensor_assign_prepare(Ctx* ctx, const float* rows, int64_t n, int32_t di
   absmax_kernel<<<1184, 256, 0, ctx->stream>>>(rows, n * (int64_t)dim, sm + 0);
   choose_scale_kernel<<<1, 1, 0, ctx->stream>>>(sm + 0, 0, (float*)sm + 1);
   float* st = (float*)ta->stats;
-  launch_prep<VSK_METRIC_DOT_PRODUCT>(ctx, rows, n, dim, ta->dim16, (float*)sm + 1, ta->rows16, nullptr, st, st + n, st + 2 * n, nullptr);
+  if (dim % 4 == 0 && dim <= 256 && (reinterpret_cast<uintptr_t>(rows) & 15) == 0) {
+    prep_rows_wide_kernel<<<(unsigned)ceil_div(n, 8), 256, 0, ctx->stream>>>(rows, n, dim, ta->dim16, (float*)sm + 1, ta->rows16, st, st + n, st + 2 * n);
+    ctx->stats.kernel_launches++;
+  } else {
+    launch_prep<VSK_METRIC_DOT_PRODUCT>(ctx, rows, n, dim, ta->dim16, (float*)sm + 1, ta->rows16, nullptr, st, st + n, st + 2 * n, nullptr);
+  }
   ctx->stats.kernel_launches += 2;
   VSK_CUDA(ctx, cudaGetLastError());
   VSK_TRY(make_map(ctx, ta->rows16, n, ta->dim16, TM, (CUtensorMap*)ta->map_rows));
