@@ -438,3 +438,32 @@ def test_kmeans_plusplus_degenerate_data_is_refused(vsk, dev):
     x = np.ones((50, 4), np.float32)
     with pytest.raises(vsk.InvalidInput):
         vsk.KMeansClustering(dev, seed=1).initializeKMeansPlusPlus(x, 3)
+
+
+def test_the_training_block_is_kept_and_given_back(vsk):
+    """K-means keeps its work buffers for the next call (the same result again, also after a call of another size), and a large
+    allocation of the library gets them back first."""
+    import torch
+    if os.environ.get("VSK_CHECKED", "0") not in ("", "0"):
+        pytest.skip("the checked build allocates every buffer by itself")
+    dev = vsk.CUDAAcceleratorStrategy(0).initialize()
+    try:
+        gen = torch.Generator(device="cuda").manual_seed(11)
+        rows = torch.empty((400_000, 128), device="cuda").normal_(generator=gen)
+        trainer = vsk.KMeansClustering(dev, maxIterations=3, tolerance=-1.0)
+
+        def run(n, k):
+            c, a, _, _ = trainer.cluster(rows[:n], k, rows[:k].clone())
+            torch.cuda.synchronize()
+            return c, a
+        first = run(400_000, 512)
+        for n, k in ((400_000, 512), (90_000, 300), (400_000, 512)):
+            again = run(n, k)
+        assert torch.equal(first[0], again[0]) and torch.equal(first[1], again[1])
+        free = torch.cuda.mem_get_info()[0]
+        ix = vsk.FlatIndex(dev, 128, vsk.DistanceMetric.dotProduct)
+        ix.add(rows)                                             # 205 MB, less what training held: over 150 MB
+        assert free - torch.cuda.mem_get_info()[0] < 100 << 20
+        ix.close()
+    finally:
+        dev.close()

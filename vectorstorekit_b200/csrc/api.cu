@@ -26,10 +26,23 @@ int32_t fail(Ctx* ctx, int32_t status, const char* fmt, ...) {
   return status;
 }
 
+static void arena_drop(Ctx* ctx) {
+  if (!ctx->arena || ctx->arena_busy) return;
+  dev_free(ctx->arena);   // (idle: the call that used it has drained its stream)
+  ctx->arena = nullptr;
+  ctx->arena_bytes = 0;
+}
+
 int32_t dev_alloc(Ctx* ctx, void** p, size_t bytes) {
   *p = nullptr;
   if (bytes == 0) return VSK_OK;
+  if (ctx && bytes >= kArenaYield) arena_drop(ctx);
   cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess && ctx && ctx->arena && !ctx->arena_busy) {
+    cudaGetLastError();
+    arena_drop(ctx);
+    e = cudaMalloc(p, bytes);
+  }
   if (e != cudaSuccess) {
     size_t fr = 0, tot = 0;
     cudaMemGetInfo(&fr, &tot);
@@ -52,6 +65,22 @@ void dev_free(void* p) {
     cudaGetLastError();
   }
 }
+
+void* arena_take(Ctx* ctx, size_t bytes) {
+#ifdef VSK_CHECKED
+  return nullptr;   // every buffer a range of its own
+#else
+  if (ctx->arena_busy || bytes == 0 || bytes > kArenaMax) return nullptr;
+  if (ctx->arena_bytes < bytes || ctx->arena_bytes / 4 > bytes) {   // (a block much too large is not held for small calls)
+    arena_drop(ctx);
+    if (dev_alloc(ctx, &ctx->arena, bytes) != VSK_OK) return nullptr;
+    ctx->arena_bytes = bytes;
+  }
+  ctx->arena_busy = true;
+  return ctx->arena;
+#endif
+}
+void arena_return(Ctx* ctx) { ctx->arena_busy = false; }
 
 int32_t lanes_fork(Ctx* ctx) {
   VSK_CUDA(ctx, cudaEventRecord(ctx->ev_fork, ctx->stream_main));
@@ -471,8 +500,35 @@ static int32_t filtered_grouped_search(Index* ix, const float* q, int64_t nq, in
   Ctx* ctx = ix->ctx;
   *handled = false;
   std::vector<uint64_t> hm((size_t)nq);
-  VSK_CUDA(ctx, cudaMemcpyAsync(hm.data(), qmasks, (size_t)nq * 8, cudaMemcpyDeviceToHost, ctx->stream));
-  VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  if (ctx->masks_dev && qmasks >= ctx->masks_dev) {   // (a batch of a host call's queries)
+    memcpy(hm.data(), ctx->masks_host + (qmasks - ctx->masks_dev), (size_t)nq * 8);
+  } else {
+    VSK_CUDA(ctx, cudaMemcpyAsync(hm.data(), qmasks, (size_t)nq * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    VSK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  }
+  // The sizes of the groups of equal masks, before anything is ordered: most batches on the tensor path end here.
+  constexpr int kTable = 1024;   // (at most 257 masks are entered)
+  struct Entry { uint64_t mask; int32_t count; };
+  std::vector<Entry> table((size_t)kTable, Entry{0, 0});
+  int64_t groups = 0;
+  for (int64_t i = 0; i < nq && groups <= 256; ++i) {
+    size_t at = (size_t)((hm[(size_t)i] * 0x9e3779b97f4a7c15ull) >> 54);
+    while (table[at].count && table[at].mask != hm[(size_t)i]) at = (at + 1) % kTable;
+    groups += table[at].count++ == 0;
+    table[at].mask = hm[(size_t)i];
+  }
+  // Worth it?  Cost is proportional to (padded queries) x (rows scanned).  Grouped: each group's queries padded
+  // to its query tile, over its eligible rows (assumed to be at most 60 % of the rows); ungrouped: all queries
+  // padded to 128, over all rows.
+  if (groups > (max_fraction >= 0.0 ? 64 : 256)) return VSK_OK;
+  int64_t padded = 0;
+  for (const Entry& t : table)
+    if (t.count) padded += ceil_div(t.count, pick_query_tile(t.count)) * pick_query_tile(t.count);
+  if ((double)padded * 0.6 > (double)(ceil_div(nq, 128) * 128)) return VSK_OK;
+  // A batch small enough for the streaming scan is bound by the bytes it reads: one pass over all rows (rows that
+  // no query may see are skipped there too) beats one pass over the eligible rows per group, unless there is
+  // only one group.
+  if (nq <= kStreamScanMaxQueries && groups > 1) return VSK_OK;
   std::vector<int32_t> perm((size_t)nq);
   for (int64_t i = 0; i < nq; ++i) perm[(size_t)i] = (int32_t)i;
   std::stable_sort(perm.begin(), perm.end(), [&](int32_t a, int32_t b) { return hm[(size_t)a] < hm[(size_t)b]; });
@@ -480,26 +536,11 @@ static int32_t filtered_grouped_search(Index* ix, const float* q, int64_t nq, in
   for (int64_t i = 0; i < nq; ++i)
     if (i == 0 || hm[(size_t)perm[(size_t)i]] != hm[(size_t)perm[(size_t)i - 1]]) starts.push_back(i);
   starts.push_back(nq);
-  const int64_t groups = (int64_t)starts.size() - 1;
-  // Worth it?  Cost is proportional to (padded queries) x (rows scanned).  Grouped: each group's queries padded
-  // to its query tile, over its eligible rows (assumed to be at most 60 % of the rows); ungrouped: all queries
-  // padded to 128, over all rows.
-  int64_t padded = 0;
-  for (int64_t g = 0; g < groups; ++g) {
-    const int64_t sz = starts[(size_t)g + 1] - starts[(size_t)g];
-    padded += ceil_div(sz, pick_query_tile(sz)) * pick_query_tile(sz);
-  }
-  if (groups > 256 || (double)padded * 0.6 > (double)(ceil_div(nq, 128) * 128)) return VSK_OK;
-  // A batch small enough for the streaming scan is bound by the bytes it reads: one pass over all rows (rows that
-  // no query may see are skipped there too) beats one pass over the eligible rows per group, unless there is
-  // only one group.
-  if (nq <= kStreamScanMaxQueries && groups > 1) return VSK_OK;
   // Manhattan groups take turns on the context's two lanes, so that one group's first rows, re-scoring and selections run beside
   // the other's byte scan: alone they leave the machine idle (64 groups of 156 queries over 2.5 million rows each: 15 of 150 ms).
   const bool two = max_fraction < 0.0 && ix->metric == VSK_METRIC_MANHATTAN && groups > 1 && groups <= 64 && ctx->lane == 0 && !ctx->profile;
   void *dperm, *dcount;
   std::vector<unsigned long long> cnt;
-  if (max_fraction >= 0.0 && groups > 64) return VSK_OK;
   if (max_fraction >= 0.0 || two) {
     std::vector<uint64_t> gm((size_t)groups);
     for (int64_t g = 0; g < groups; ++g) gm[(size_t)g] = hm[(size_t)perm[(size_t)starts[(size_t)g]]];
@@ -820,6 +861,7 @@ int32_t vsk_close(vsk_ctx* c) {
   cudaStreamSynchronize(ctx->stream_aux);
   comm_release(ctx);
   for (auto& p : ctx->scratch) dev_free(p);
+  dev_free(ctx->arena);
   for (auto& p : ctx->few_tickets) dev_free(p);
   for (auto& b : ctx->host_flags)
     if (b.p) {
@@ -1213,7 +1255,10 @@ int32_t vsk_search(vsk_index* i, const float* q, int64_t nq, int32_t k, const ui
   if (!q || !out_dist || !out_ids) return fail(ctx, VSK_ERR_INVALID_INPUT, "null pointer");
   HostCall c;
   VSK_TRY(host_call_begin(ctx, q, nq, ix->dim, qmasks, k, &c, ix->kind == INDEX_FLAT_F32));
+  ctx->masks_dev = c.masks;
+  ctx->masks_host = qmasks;
   const int32_t st = vsk_search_dev(i, c.q, nq, k, c.masks, c.dist, c.ids);
+  ctx->masks_dev = ctx->masks_host = nullptr;
   ctx->host_query.pending = false;
   VSK_TRY(st);
   VSK_TRY(host_call_end(ctx, c, nq, ix->dim, k, out_dist, out_ids));

@@ -190,6 +190,15 @@ struct Ctx {
     size_t bytes = 0;
     bool pending = false;
   } host_query;
+  // The filter masks of a host-pointer call in progress, on the device and where the caller has them.
+  const uint64_t* masks_dev = nullptr;
+  const uint64_t* masks_host = nullptr;
+  // One block kept between calls that take a lot of device memory for their own duration only (k-means): 10 ms of a 110 ms
+  // training call over 10 million x 128 went into 5 GB of allocations and frees.  At most kArenaMax, one user at a time; given
+  // back before any other large allocation of the context (dev_alloc), and with the context.
+  void* arena = nullptr;
+  size_t arena_bytes = 0;
+  bool arena_busy = false;
   PinnedBuf host_io;         // staging of small host-pointer calls (HostCall)
   PinnedBuf host_flags[2];   // per lane: the flag words a finished half-search hands to the host
   std::vector<const void*> configured;   // kernels that have their shared memory on this device (opt_in_shared) ...
@@ -533,6 +542,11 @@ void chk_add(const void* p, size_t bytes);
 void chk_remove(const void* p);
 void worker_release(Ctx* ctx);
 int32_t dev_alloc(Ctx* ctx, void** p, size_t bytes);
+// `bytes` of the context's kept block, or null (in use, too large, no memory): the caller allocates for itself.  arena_return
+// when the work that uses it has drained.
+constexpr size_t kArenaMax = 8ull << 30, kArenaYield = 64ull << 20;
+void* arena_take(Ctx* ctx, size_t bytes);
+void arena_return(Ctx* ctx);
 void dev_free(void* p);
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }

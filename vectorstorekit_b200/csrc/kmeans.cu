@@ -160,7 +160,7 @@ int32_t assign_rows(Ctx* ctx, const float* rows, int64_t n, int32_t dim, const f
                     int32_t* assign, float* dist) {
   if (use_tensor_assign(ctx, n, k)) {
     TensorAssign ta;
-    int32_t st = tensor_assign_prepare(ctx, rows, n, dim, &ta);
+    int32_t st = tensor_assign_prepare(ctx, rows, n, dim, &ta, true);
     if (st == VSK_OK) st = tensor_assign(ctx, &ta, rows, centroids, k, assign, dist, false);
     if (st == VSK_OK && cudaStreamSynchronize(ctx->stream) != cudaSuccess) st = VSK_ERR_EXECUTION_FAILED;
     tensor_assign_release(&ta);
@@ -260,7 +260,7 @@ int32_t kmeans_dev(Ctx* ctx, const float* rows, int64_t n, int32_t dim, int32_t 
     TensorAssign* t;
     ~Release() { tensor_assign_release(t); }
   } release{&ta};
-  if (tc) VSK_TRY(tensor_assign_prepare(ctx, rows, n, dim, &ta));
+  if (tc) VSK_TRY(tensor_assign_prepare(ctx, rows, n, dim, &ta, true));
   while (it < max_iters && !converged) {
     if (tc) VSK_TRY(tensor_assign(ctx, &ta, rows, (const float*)cur, k, assign, (float*)dist, it > 0));
     else VSK_TRY(assign_rows_fp32(ctx, rows, n, dim, (const float*)cur, k, assign, (float*)dist));

@@ -4439,22 +4439,35 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
 }
 
 // ---- public: tensor-core nearest-centroid assignment (used by kmeans.cu) ---------------------------
-int32_t tensor_assign_prepare(Ctx* ctx, const float* rows, int64_t n, int32_t dim, TensorAssign* ta) {
+int32_t tensor_assign_prepare(Ctx* ctx, const float* rows, int64_t n, int32_t dim, TensorAssign* ta, bool one_call) {
   ta->n = n;
   ta->dim = dim;
   // Short contractions keep a block of centroids resident (assign_scan_kernel): the operands then carry 16 more
   // columns for the folded |c|^2 / 2 term.  Longer ones (more than four k-blocks with those columns) take the general kernel.
   ta->stationary = fold_col0(dim) + kFoldCols <= AS_MAX_KB * TK;
   ta->dim16 = (int32_t)(ceil_div(ta->stationary ? fold_col0(dim) + kFoldCols : dim, TK) * TK);
-  VSK_TRY(dev_alloc(ctx, (void**)&ta->rows16, (size_t)n * ta->dim16 * sizeof(__half)));
-  VSK_TRY(dev_alloc(ctx, (void**)&ta->stats, (size_t)n * 4 * sizeof(float)));
   // stationary kernel: `keys` is the hit log (a hit or two per row as a rule; six entries per row of room)
-  VSK_TRY(dev_alloc(ctx, (void**)&ta->keys, (size_t)n * (ta->stationary ? kAssignLogPerRow : kAssignCap) * sizeof(uint64_t)));
-  VSK_TRY(dev_alloc(ctx, (void**)&ta->best, (size_t)n * sizeof(unsigned long long)));
-  VSK_TRY(dev_alloc(ctx, (void**)&ta->count, (size_t)n * sizeof(int32_t)));
-  VSK_TRY(dev_alloc(ctx, (void**)&ta->thr, (size_t)n * sizeof(float)));
-  VSK_TRY(dev_alloc(ctx, (void**)&ta->bad_rows, (size_t)n * sizeof(int32_t)));
-  VSK_TRY(dev_alloc(ctx, (void**)&ta->small, 256));
+  const struct { void** p; size_t bytes; } need[] = {
+      {(void**)&ta->rows16, (size_t)n * ta->dim16 * sizeof(__half)},
+      {(void**)&ta->stats, (size_t)n * 4 * sizeof(float)},
+      {(void**)&ta->keys, (size_t)n * (ta->stationary ? kAssignLogPerRow : kAssignCap) * sizeof(uint64_t)},
+      {(void**)&ta->best, (size_t)n * sizeof(unsigned long long)},
+      {(void**)&ta->count, (size_t)n * sizeof(int32_t)},
+      {(void**)&ta->thr, (size_t)n * sizeof(float)},
+      {(void**)&ta->bad_rows, (size_t)n * sizeof(int32_t)},
+      {&ta->small, 256}};
+  size_t total = 0;
+  for (const auto& b : need) total += (b.bytes + 255) / 256 * 256;
+  char* block = one_call ? (char*)arena_take(ctx, total) : nullptr;
+  if (block) {
+    ta->arena = ctx;
+    for (const auto& b : need) {
+      *b.p = block;
+      block += (b.bytes + 255) / 256 * 256;
+    }
+  } else {
+    for (const auto& b : need) VSK_TRY(dev_alloc(ctx, b.p, b.bytes));
+  }
   VSK_CUDA(ctx, cudaMemsetAsync(ta->small, 0, 256, ctx->stream));
   // small: [0] absmax(rows) [1] scale_x [2] absmax(cent) [3] scale_c [4] alpha [5] err [6] bad_count, then PrepStats at +64
   unsigned* sm = (unsigned*)ta->small;
@@ -4475,8 +4488,14 @@ int32_t tensor_assign_prepare(Ctx* ctx, const float* rows, int64_t n, int32_t di
 }
 
 void tensor_assign_release(TensorAssign* ta) {
-  dev_free(ta->rows16); dev_free(ta->stats); dev_free(ta->keys); dev_free(ta->best); dev_free(ta->count);
-  dev_free(ta->thr); dev_free(ta->bad_rows); dev_free(ta->small); dev_free(ta->prev_cent); dev_free(ta->shift);
+  if (ta->arena) {
+    cudaStreamSynchronize(ta->arena->stream);   // (a call that failed part-way may have left work behind)
+    arena_return(ta->arena);
+  } else {
+    dev_free(ta->rows16); dev_free(ta->stats); dev_free(ta->keys); dev_free(ta->best); dev_free(ta->count);
+    dev_free(ta->thr); dev_free(ta->bad_rows); dev_free(ta->small);
+  }
+  dev_free(ta->prev_cent); dev_free(ta->shift);
   *ta = TensorAssign{};
 }
 

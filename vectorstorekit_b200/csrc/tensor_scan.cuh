@@ -106,6 +106,7 @@ struct TensorAssign {
   float* thr = nullptr;               // [n]
   int32_t* bad_rows = nullptr;        // [n] rows handed to the fp32 tile
   void* small = nullptr;              // scalars and centroid-operand statistics
+  Ctx* arena = nullptr;               // the buffers above are the kept block of this context, not allocations of their own
   bool stationary = false;            // short contraction: resident centroid block, |c|^2 / 2 folded into the operands
   float* prev_cent = nullptr;         // [prev_k][dim] the centroids of the previous call (stationary path) ...
   float* shift = nullptr;             // [prev_k] ... and how far each has moved since
@@ -115,7 +116,8 @@ struct TensorAssign {
   alignas(64) unsigned char map_rows[128] = {};  // TMA tensor map of rows16
   alignas(64) unsigned char map_rows_narrow[128] = {};  // the same through a 16-column box (the fold columns' K16 step)
 };
-int32_t tensor_assign_prepare(Ctx* ctx, const float* rows, int64_t n, int32_t dim, TensorAssign* ta);
+// one_call: the buffers serve one library call, which drains its stream before it releases them (the context's kept block).
+int32_t tensor_assign_prepare(Ctx* ctx, const float* rows, int64_t n, int32_t dim, TensorAssign* ta, bool one_call = false);
 // assign_holds_previous: `assign` holds, for every row, a valid centroid index (the previous iteration's
 // assignment), which gives the candidate threshold without the coarse arg-min pass.
 int32_t tensor_assign(Ctx* ctx, TensorAssign* ta, const float* rows, const float* centroids, int32_t k,

@@ -147,6 +147,15 @@ def _host(a, dtype):
     return np.ascontiguousarray(a, dtype=dtype)
 
 
+def _ptrs(*arrays):
+    """Addresses of the arrays of one call: torch's streams are waited for once, not once per array (see _ptr)."""
+    for device in {a.device for a in arrays if a is not None and _is_dev(a)}:
+        torch.cuda.current_stream(device).synchronize()
+    if _lib.CHECKED:
+        return [_ptr(a) for a in arrays]
+    return [None if a is None else C.c_void_p(a.data_ptr() if _is_dev(a) else a.ctypes.data) for a in arrays]
+
+
 def _ptr(a):
     """Address of an array for the C ABI.  The library works on its own CUDA stream, which does not wait for
     torch's: a CUDA tensor is handed over only after the torch stream that produced it has drained."""
@@ -447,7 +456,8 @@ class _IndexBase:
             od = torch.empty((nq, k), dtype=torch.float32, device=q.device)
             oi = torch.empty((nq, k), dtype=torch.int64, device=q.device)
             qm = qmasks.contiguous() if qmasks is not None else None
-            self.dev.check(self._lib.vsk_search_dev(self._h, _ptr(q), nq, k, _ptr(qm), _ptr(od), _ptr(oi)))
+            pq, pm, pd, pi = _ptrs(q, qm, od, oi)
+            self.dev.check(self._lib.vsk_search_dev(self._h, pq, nq, k, pm, pd, pi))
             return od, oi
         q = _host(queries, np.float32)
         od = np.empty((nq, k), np.float32)
@@ -932,7 +942,8 @@ class IVFIndex(_IndexBase, _ShardedSearchMixin):
             od = torch.empty((nq, k), dtype=torch.float32, device=q.device)
             oi = torch.empty((nq, k), dtype=torch.int64, device=q.device)
             qm = filter_masks.contiguous() if filter_masks is not None else None
-            self.dev.check(self._lib.vsk_ivf_search_filtered_dev(self._h, _ptr(q), nq, k, nprobe, _ptr(qm), _ptr(od), _ptr(oi)))
+            pq, pm, pd, pi = _ptrs(q, qm, od, oi)
+            self.dev.check(self._lib.vsk_ivf_search_filtered_dev(self._h, pq, nq, k, nprobe, pm, pd, pi))
             return od, oi
         q = _host(queries, np.float32)
         od = np.empty((nq, k), np.float32)
