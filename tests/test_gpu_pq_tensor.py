@@ -62,6 +62,23 @@ def test_tensor_batches_equal_table_sums(vsk, dev, cpu_oracle, shape):
     assert np.array_equal(i1, ri[:63]) and np.array_equal(d1, rd[:63])
 
 
+# tables of sixteen queries to a block (from 256 queries on): every segment length with a kernel of its own, one of the general
+# kernel, remainders of 0, 1 and 15 queries, few codewords; and operand rows of 128, 129 and more 16-byte pieces
+@pytest.mark.parametrize("m,ds,ksub,nq", [(8, 2, 256, 256), (8, 4, 256, 257), (8, 8, 32, 271), (4, 16, 256, 255), (4, 16, 256, 256),
+                                          (8, 3, 256, 272), (63, 16, 16, 64), (129, 8, 16, 64), (131, 8, 16, 70)])
+def test_tables_and_wide_rows(vsk, dev, cpu_oracle, m, ds, ksub, nq):
+    rng = np.random.default_rng(m * ds + nq)
+    q, cb, x = _clustered(rng, 16_411, nq, m, ksub, ds)
+    codes = cpu_oracle.pq_encode(x, cb)
+    ix = _index(vsk, dev, cb, codes)
+    before = dev.stats()["tensor_tiles"]
+    dist, ids = ix.batchSearch(q, 10)
+    assert dev.stats()["tensor_tiles"] > before
+    rd, ri = cpu_oracle.pq_search(q, codes, cb, 10)
+    assert np.array_equal(ids, ri)
+    assert np.array_equal(dist, rd)
+
+
 @pytest.mark.parametrize("offset", [30.0, 3000.0])
 def test_rows_far_from_the_origin(vsk, dev, cpu_oracle, offset):
     """The error bound grows with the rows' norms: lists get longer, and where they overflow the table scan answers."""

@@ -2017,6 +2017,45 @@ __global__ void __launch_bounds__(256) rerank_i8_kernel(const float* __restrict_
   }
 }
 
+// Sums of RR fp32 rows against the query in shared memory (direct formulas; a lane's dimensions are lane, lane + 32, .., added in
+// that order), four loads of every row in flight.  Bound by the gathered rows; with one load of each row in flight the re-scoring
+// of the list search was bound by their latency (1 000 queries of 128 dimensions: 690 us in two launches, 468 with four).
+template <int METRIC, int RR>
+__device__ __forceinline__ void f32_row_sums(const float* qs, const float* __restrict__ x, int dim, const uint32_t (&id)[RR], int lane,
+                                             float (&sum)[RR]) {
+  constexpr int U = 4;
+  const float* xr[RR];
+#pragma unroll
+  for (int r = 0; r < RR; ++r) {
+    xr[r] = x + (int64_t)id[r] * dim;
+    sum[r] = 0.f;
+  }
+  for (int i0 = lane; i0 < dim; i0 += 32 * U) {
+    float xv[RR][U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int r = 0; r < RR; ++r) xv[r][u] = i0 + 32 * u < dim ? __ldg(xr[r] + i0 + 32 * u) : 0.f;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const float qv = i0 + 32 * u < dim ? qs[i0 + 32 * u] : 0.f;
+#pragma unroll
+      for (int r = 0; r < RR; ++r) {
+        if (METRIC == VSK_METRIC_EUCLIDEAN) {
+          const float d = qv - xv[r][u];
+          sum[r] = fmaf(d, d, sum[r]);
+        } else {
+          sum[r] = fmaf(qv, xv[r][u], sum[r]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < RR; ++r)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o);
+}
+
 // ---- exact rerank -------------------------------------------------------------------------
 // One CTA per query: replaces every kept candidate's coarse value with the reference's direct fp32 value:
 //   euclidean sum (q-x)^2 (rooted at output), cosine 1 - q.x/(|q||x| + 1e-8), dotProduct -(q.x).
@@ -2038,31 +2077,12 @@ __global__ void __launch_bounds__(256) rerank_kernel(const float* __restrict__ q
   constexpr int RR = 4;
   for (int c0 = warp * RR; c0 < cnt; c0 += nwarps * RR) {
     uint32_t id[RR];
-    const float* xr[RR];
     float s[RR];
 #pragma unroll
-    for (int r = 0; r < RR; ++r) {
-      id[r] = c0 + r < cnt ? (uint32_t)keys[c0 + r] : 0u;
-      xr[r] = x + (int64_t)id[r] * dim;
-      s[r] = 0.f;
-    }
-    for (int i = lane; i < dim; i += 32) {
-      const float qv = qs[i];
-#pragma unroll
-      for (int r = 0; r < RR; ++r) {
-        const float xv = __ldg(xr[r] + i);
-        if (METRIC == VSK_METRIC_EUCLIDEAN) {
-          const float d = qv - xv;
-          s[r] = fmaf(d, d, s[r]);
-        } else {
-          s[r] = fmaf(qv, xv, s[r]);
-        }
-      }
-    }
+    for (int r = 0; r < RR; ++r) id[r] = (uint32_t)keys[min(c0 + r, cnt - 1)];
+    f32_row_sums<METRIC, RR>(qs, x, dim, id, lane, s);
 #pragma unroll
     for (int r = 0; r < RR; ++r) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
       if (lane == 0 && c0 + r < cnt) {
         float v;
         if (METRIC == VSK_METRIC_COSINE) v = 1.0f - s[r] / (qn * xnorm[id[r]] + 1e-8f);
@@ -2157,7 +2177,7 @@ __global__ void __launch_bounds__(NT, kFinishMinBlocks<NT>) finish_kernel(Finish
   }
   // exact values: four rows per warp step, four loads of each in flight
   const float qn = (METRIC == VSK_METRIC_COSINE) ? *VSK_CHK(a.qnorm + qi) : 0.f;
-  constexpr int RR = 4, U = 4;
+  constexpr int RR = 4;
   for (int c0 = warp * RR; c0 < cnt; c0 += (NT / 32) * RR) {
     if constexpr (I8) {
       uint32_t id[RR];
@@ -2172,39 +2192,13 @@ __global__ void __launch_bounds__(NT, kFinishMinBlocks<NT>) finish_kernel(Finish
       continue;
     }
     uint32_t id[RR];
-    const float* xr[RR];
     float sum[RR];
 #pragma unroll
-    for (int r = 0; r < RR; ++r) {
-      id[r] = (uint32_t)s_keys[min(c0 + r, cnt - 1)];
-      xr[r] = a.x + (int64_t)id[r] * a.dim;
-      sum[r] = 0.f;
-    }
-    for (int i0 = lane; i0 < a.dim; i0 += 32 * U) {
-      float xv[RR][U];
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-#pragma unroll
-        for (int r = 0; r < RR; ++r) xv[r][u] = i0 + 32 * u < a.dim ? __ldg(xr[r] + i0 + 32 * u) : 0.f;
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const float qv = i0 + 32 * u < a.dim ? qs[i0 + 32 * u] : 0.f;
-#pragma unroll
-        for (int r = 0; r < RR; ++r) {
-          if (METRIC == VSK_METRIC_EUCLIDEAN) {
-            const float d = qv - xv[r][u];
-            sum[r] = fmaf(d, d, sum[r]);
-          } else {
-            sum[r] = fmaf(qv, xv[r][u], sum[r]);
-          }
-        }
-      }
-    }
+    for (int r = 0; r < RR; ++r) id[r] = (uint32_t)s_keys[min(c0 + r, cnt - 1)];
+    f32_row_sums<METRIC, RR>(qs, a.x, a.dim, id, lane, sum);
     __syncwarp();
 #pragma unroll
     for (int r = 0; r < RR; ++r) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o);
       if (lane == 0 && c0 + r < cnt) {
         float v;
         if (METRIC == VSK_METRIC_COSINE) v = 1.0f - sum[r] / (qn * __ldg(a.xnorm + id[r]) + 1e-8f);
@@ -3766,7 +3760,9 @@ constexpr int64_t kPqBlockBytes = 512ll << 20;   // decoded operand rows held at
 constexpr int PQ_DEC_ROWS = 64;                  // rows per CTA of the decode kernel
 
 // One CTA decodes PQ_DEC_ROWS rows: codes and |x^|^2 (segment sums of the codewords' norms) are staged in shared
-// memory, then every thread writes 16-byte pieces of the operand rows.  Bound by the 2 dim16 bytes a row writes.
+// memory, then every thread writes 16-byte pieces of the operand rows.  Bound by the issue of the pieces (a gather from the
+// codebook and a store each): 10 000 000 rows of 128 in 12 blocks take 1.22 ms, against 0.45 ms for their 2.9 GB; it was 1.88 ms
+// with a division per piece and the 48 columns of padding written as well.
 // DS: 2, 4, 8 = the segment length; 16 = any multiple of 8 (a piece lies inside one codeword); 0 = any length.
 template <int DS>
 __global__ void __launch_bounds__(256) pq_decode16_kernel(const uint8_t* __restrict__ codes, int64_t n, int dim, int dim16, int m,
@@ -3794,9 +3790,13 @@ __global__ void __launch_bounds__(256) pq_decode16_kernel(const uint8_t* __restr
     }
   }
   __syncthreads();
-  const int pieces = dim16 >> 3;
+  // Columns past the last K16 step that the contraction takes are not written: no MMA reads them (k16_last_of).
+  // The division by the pieces of a row is a multiplication: with inv = (2^20 + e) / pieces, e < pieces, the quotient is exact
+  // while t e < 2^20, and t is below 64 pieces: for up to 128 pieces (rows of up to 1 024 columns).
+  const int pieces = (fold ? col0 + kFoldCols : (dim + 15) / 16 * 16) >> 3;
+  const uint32_t inv = ((1u << 20) + (uint32_t)pieces - 1u) / (uint32_t)pieces;
   for (int t = threadIdx.x; t < rows * pieces; t += blockDim.x) {
-    const int r = t / pieces, c = (t - r * pieces) * 8;
+    const int r = pieces <= 128 ? (int)(((uint32_t)t * inv) >> 20) : t / pieces, c = (t - r * pieces) * 8;
     __align__(16) __half h[8];
     if (fold && c >= col0 && c < col0 + kFoldCols) {
       // pieces of R = s (|x^|^2 / 2) 2^exp as in prep_rows_kernel
