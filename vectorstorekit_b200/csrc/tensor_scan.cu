@@ -19,9 +19,10 @@
 // so that concurrently running CTAs share the same rows in L2):
 //   warp 0      TMA producer: 4-stage ring of {128 x 64 query, 256 x 64 row} fp16 tiles
 //   warp 1      tensor-memory allocation; one lane issues tcgen05.mma (M128 N256 K16 x 4 per stage)
-//   warps 2..   epilogue (8 warps for long contractions, 16 up to d = 256): tcgen05.ld of the thread's
-//               accumulator row (one query per thread; the warps of a lane quarter split the tile's columns),
-//               threshold filter, candidate append; double-buffered accumulators (2 x 256 columns)
+//   warps 2..   epilogue (8 warps for long contractions and with a per-row term, 16 up to four K blocks without one):
+//               tcgen05.ld of the thread's accumulator row (one query per thread; the warps of a lane quarter split the
+//               tile's columns), threshold filter on the maxima of eight columns, hits queued in shared memory and
+//               appended under the next tile's loads; double-buffered accumulators (2 x 256 columns)
 // The same kernel scans the probed lists of an IVF index (tile-table mode: an explicit list of tiles over a
 // query operand gathered per (query, list) pair) and assigns rows to centroids for k-means (argmin mode and a
 // threshold mode whose tiles walk the centroids for a fixed block of rows).
@@ -50,8 +51,9 @@ constexpr int RING_BYTES = STAGES * STAGE_BYTES;
 // operand traffic from L2.  It was removed.)
 // Warp 0 is the TMA producer, warp 1 the MMA issuer, then EW epilogue warps: EW / 4 per tensor-memory lane quarter,
 // each taking one of EW / 4 equal parts of the tile's columns.  EW = 8 for long contractions (the epilogue hides
-// behind the MMAs, and fewer warps cost less issue and power); EW = 16 for short ones (d <= 256), where a tile's
-// MMAs take about a microsecond and the epilogue warps' serial chain of tensor-memory loads sets the pace.
+// behind the MMAs, and fewer warps cost less issue and power) and with a per-row term (tc_epilogue_warps); EW = 16 for
+// short ones (d <= 256), where a tile's MMAs take about a microsecond and the epilogue warps' serial chain of
+// tensor-memory loads sets the pace.
 template <int EW> struct Epi {
   static constexpr int WARPS = EW;
   static constexpr int PARTS = EW / 4;
