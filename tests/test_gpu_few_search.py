@@ -199,3 +199,32 @@ def test_probes_of_short_rows_take_one_launch(vsk, dev, cpu_oracle):
     for nq in (3, 8, 16):
         q = rng.standard_normal((nq, 24)).astype(np.float32)
         assert_topk_parity(*ivf.batchSearch(q, 20), *cpu_oracle.flat_search(oracle.EUCLIDEAN, q, x, 20))
+
+
+# 1, 2, 8 and 16 queries walk both lists in several rounds per CTA (the launch's CTAs, three per SM, are shared by the queries, and
+# a round is 512 rows of a CTA): on 148 SMs the nearer list takes 3.5 rounds, 4, 5 and 5.
+@pytest.mark.parametrize("nq,d,n,launches", [(1, 8, 1_200_000, 2), (2, 8, 700_000, 3), (8, 36, 210_000, 3), (16, 36, 105_000, 5)])
+def test_listed_rows_get_their_ids_in_every_round(vsk, dev, nq, d, n, launches):
+    """Every row of the nearer list is nearer than all before it, so that each is listed, most of them in the rounds after the
+    first; every third row belongs to the other list, so that no stored row's number is its id.  Against the order of insertion."""
+    import torch
+    k = 100
+    far = np.arange(n) % 3 == 0
+    x = np.zeros((n, d), np.float32)
+    x[~far, 1] = np.arange((~far).sum(), 0, -1)                  # whole numbers; the last rows are the nearest
+    x[far, 1] = 2e7
+    cent = np.zeros((2, d), np.float32)
+    cent[1, 1] = 2e7
+    q = np.zeros((nq, d), np.float32)
+    q[:, 2] = np.arange(nq)                                      # (off the rows' line: the same order for every query)
+    ix = vsk.IVFIndex(dev, d, numberOfCentroids=2, numberOfProbes=2)
+    ix.centroids, ix.trained = cent, True
+    ix.insert(x)
+    ids = np.nonzero(~far)[0][:-k - 1:-1]
+    dist = np.sqrt(np.arange(1, k + 1) ** 2 + np.arange(nq)[:, None] ** 2).astype(np.float32)   # (sums below 2^24)
+    for _ in range(20):
+        before = dev.stats()["kernel_launches"]
+        gd, gi = (a.cpu().numpy() for a in ix.batchSearch(torch.from_numpy(q).cuda(), k))
+        assert dev.stats()["kernel_launches"] - before == launches   # the probe list (merged apart from two queries on), and the walk
+        assert np.array_equal(gi, np.tile(ids, (nq, 1))) and np.allclose(gd, dist, rtol=2e-7, atol=0)
+    ix.close()

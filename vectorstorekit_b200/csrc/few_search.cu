@@ -408,7 +408,10 @@ __global__ void __launch_bounds__(FEW_THREADS, NQ > 4 ? 2 : 3) few_topk_kernel(c
         lists[j] = (lists[j] & 0xffffffff00000000ull) | (uint32_t)*VSK_CHK(a.id_remap + (uint32_t)lists[j]);
     }
     few_end_round(lists, nq_here, k, ka.stride, r0 + stride >= n, s_cnt, s_thr, fs);
-    done = s_cnt[0];
+    if (NQ == 1 && a.id_remap) {
+      done = s_cnt[0];
+      __syncthreads();   // the next round's first keys are counted in s_cnt: not before every thread has read it
+    }
   }
   // ---- this CTA's lists, and the merge by the last one to arrive ----
   few_write_lists(ka, lists, qp, nq_here, s_cnt);
