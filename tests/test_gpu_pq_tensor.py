@@ -216,7 +216,7 @@ def test_encoding_on_the_tensor_cores_equals_the_exact_sums(vsk, dev, cpu_oracle
     assert np.array_equal(_encode(dev, cb, x), cpu_oracle.pq_encode(x, cb))
 
 
-@pytest.mark.parametrize("what", ["equal", "tiny", "huge", "nan"])
+@pytest.mark.parametrize("what", ["equal", "tiny", "huge", "largest", "nan"])
 def test_encoding_with_unusual_codebooks(vsk, dev, cpu_oracle, what):
     rng = np.random.default_rng(8)
     m, ksub, ds, n = 5, 256, 8, 13_200
@@ -230,6 +230,11 @@ def test_encoding_with_unusual_codebooks(vsk, dev, cpu_oracle, what):
     elif what == "huge":
         cb[1] *= np.float32(1e20)
         x[:, ds:2 * ds] *= np.float32(1e18)
+    elif what == "largest":                                       # one codeword of every four near fp32's limit, the mean is not
+        cb[1] *= np.float32(1e37)
+        big = np.arange(0, ksub, 4)
+        cb[1, big] = np.where(big // 32 % 2, -1, 1)[:, None] * (2.9e38 * (1 + 0.01 * rng.random((len(big), ds)))).astype(np.float32)
+        x[:, ds:2 * ds] = cb[1, rng.integers(0, ksub, n)]
     else:
         cb[1, 9, 3], cb[2, 200, 0] = np.nan, np.inf
     assert np.array_equal(_encode(dev, cb, x), cpu_oracle.pq_encode(x, cb))

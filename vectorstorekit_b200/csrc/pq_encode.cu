@@ -250,8 +250,8 @@ __global__ void __launch_bounds__(PE_THREADS, 1) pq_encode_tensor_kernel(const _
     float s = 1.f;
     if (top > 0.f && top < CUDART_INF_F) {
       int e;
-      frexpf(top, &e);                                  // the largest entry becomes 8 .. 16
-      s = ldexpf(1.f, max(-120, min(120, 4 - e)));
+      frexpf(top, &e);                                  // the largest entry becomes 8 .. 16, so that |c|^2 / 2 fits fp16
+      s = ldexpf(1.f, min(120, 4 - e));                 // (e is at most 128: 2^-124 at least, a normal number)
     }
 #pragma unroll
     for (int i = 0; i < DS; ++i)
