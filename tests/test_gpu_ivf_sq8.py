@@ -467,3 +467,38 @@ def test_the_training_block_is_kept_and_given_back(vsk):
         ix.close()
     finally:
         dev.close()
+
+
+def test_the_training_block_leaves_the_device_to_others(vsk):
+    """A block of a gigabyte or more that is more than a sixteenth of the free memory goes back when its call ends; others on
+    request."""
+    import torch
+    if os.environ.get("VSK_CHECKED", "0") not in ("", "0"):
+        pytest.skip("the checked build allocates every buffer by itself")
+    dev = vsk.CUDAAcceleratorStrategy(0).initialize()
+    filler = None
+    try:
+        gen = torch.Generator(device="cuda").manual_seed(12)
+        rows = torch.empty((3_000_000, 128), device="cuda").normal_(generator=gen)
+        trainer = vsk.KMeansClustering(dev, maxIterations=2, tolerance=-1.0)
+
+        def held():
+            torch.cuda.synchronize()
+            free = torch.cuda.mem_get_info()[0]
+            out = trainer.cluster(rows, 512, rows[:512].clone())
+            torch.cuda.synchronize()
+            return free - torch.cuda.mem_get_info()[0], out
+        _, first = held()                                        # the context's scratch, torch's blocks
+        dev.trim()
+        size, _ = held()
+        assert 1 << 30 < size < 3 << 30
+        dev.trim()
+        free = torch.cuda.mem_get_info()[0]
+        filler = torch.empty(free - 8 * size, dtype=torch.uint8, device="cuda")
+        size, again = held()
+        assert size < 32 << 20
+        assert all(torch.equal(a, b) for a, b in zip(first[:2], again[:2]))
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+        dev.close()

@@ -62,6 +62,7 @@ SIGNATURES = {
     "vsk_stats_get": (C.c_int32, [vp, C.POINTER(Stats)]),
     "vsk_last_error": (C.c_char_p, [vp]),
     "vsk_status_string": (C.c_char_p, [C.c_int32]),
+    "vsk_trim": (C.c_int32, [vp]),
     "vsk_set_search_path": (C.c_int32, [vp, C.c_int32]),
     "vsk_stream": (vp, [vp]),
     "vsk_profile": (C.c_int32, [vp, C.c_int32]),

@@ -73,14 +73,28 @@ void* arena_take(Ctx* ctx, size_t bytes) {
   if (ctx->arena_busy || bytes == 0 || bytes > kArenaMax) return nullptr;
   if (ctx->arena_bytes < bytes || ctx->arena_bytes / 4 > bytes) {   // (a block much too large is not held for small calls)
     arena_drop(ctx);
-    if (dev_alloc(ctx, &ctx->arena, bytes) != VSK_OK) return nullptr;
+    if (cudaMalloc(&ctx->arena, bytes) != cudaSuccess) {   // (no error of the call: its own buffers may still fit)
+      cudaGetLastError();
+      ctx->arena = nullptr;
+      return nullptr;
+    }
     ctx->arena_bytes = bytes;
   }
   ctx->arena_busy = true;
   return ctx->arena;
 #endif
 }
-void arena_return(Ctx* ctx) { ctx->arena_busy = false; }
+
+void arena_return(Ctx* ctx) {
+  ctx->arena_busy = false;
+  if (ctx->arena_bytes < kArenaAsk) return;
+  size_t fr = 0, tot = 0;
+  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+    cudaGetLastError();
+    fr = 0;
+  }
+  if (ctx->arena_bytes > fr / kArenaShare) arena_drop(ctx);
+}
 
 int32_t lanes_fork(Ctx* ctx) {
   VSK_CUDA(ctx, cudaEventRecord(ctx->ev_fork, ctx->stream_main));
@@ -878,6 +892,14 @@ int32_t vsk_close(vsk_ctx* c) {
   cudaStreamDestroy(ctx->stream_main);
   cudaStreamDestroy(ctx->stream_aux);
   delete ctx;
+  return VSK_OK;
+}
+
+int32_t vsk_trim(vsk_ctx* c) {
+  Ctx* ctx = reinterpret_cast<Ctx*>(c);
+  if (!ctx) return VSK_ERR_INVALID_INPUT;
+  VSK_CUDA(ctx, cudaSetDevice(ctx->device));
+  arena_drop(ctx);
   return VSK_OK;
 }
 

@@ -239,6 +239,10 @@ class CUDAComputeDevice:
     def profile(self, enable: bool):
         self.check(self._lib.vsk_profile(self._h, 1 if enable else 0))
 
+    def trim(self):
+        """``vsk_trim``: device memory kept between training calls goes back, for other allocators on the device."""
+        self.check(self._lib.vsk_trim(self._h))
+
     def set_search_path(self, path: int):
         self.check(self._lib.vsk_set_search_path(self._h, path))
 
