@@ -57,6 +57,38 @@ def test_a_read_past_the_announced_end_is_refused_and_reported():
         dev.close()
 
 
+@pytest.mark.skipif(not CHECKED, reason="needs the checked build (VSK_CHECKED=1)")
+def test_buffers_announced_while_a_kernel_runs_refuse_nothing():
+    """A trainer's rows are still being prepared when its constructor returns; each announcement then moves the entries of the
+    range table that lie behind it."""
+    import ctypes as C
+
+    import torch
+    import vectorstorekit_b200 as vsk
+    dev = vsk.CUDAComputeDevice(0)
+    try:
+        x = torch.randn((200_000, 240), device="cuda", generator=torch.Generator(device="cuda").manual_seed(5))
+        c = x[:256].clone()
+        low, high = (torch.empty(1 << 20, dtype=torch.uint8, device="cuda") for _ in range(2))
+        spots = [t.data_ptr() + (i << 12) for t in sorted((low, high), key=lambda t: -t.data_ptr()) for i in reversed(range(100))]
+        dev.checked_faults()
+        first = None
+        for _ in range(3):
+            tr = vsk.KMeansTrainer(dev, x, 256)
+            for p in spots:
+                assert dev._lib.vsk_checked_register(C.c_void_p(p), 16) == 0
+            tr.step(c)
+            got = tr.assignments()
+            assert dev.checked_faults()[0] == 0
+            first = got if first is None else first
+            assert torch.equal(first, got)
+            for p in spots:
+                dev._lib.vsk_checked_unregister(C.c_void_p(p))
+            tr.close()
+    finally:
+        dev.close()
+
+
 @pytest.mark.skipif(CHECKED, reason="the normal library")
 def test_the_normal_library_answers_that_it_is_not_checked():
     import vectorstorekit_b200 as vsk

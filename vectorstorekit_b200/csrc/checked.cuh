@@ -22,8 +22,8 @@ struct Range {
   unsigned long long lo, hi;   // [lo, hi)
 };
 
-// Lives in device memory, one per GPU.  The host rewrites table (version + 1) % kTables and then publishes `version`;
-// a kernel in flight keeps reading the table it started with.
+// Lives in device memory, one per GPU.  The host rewrites table (version + 1) % kTables and then publishes `version`:
+// an access in flight keeps reading the table it started with.
 struct State {
   int version;
   int count[kTables];
@@ -54,18 +54,26 @@ static __device__ __noinline__ unsigned long long vsk_chk_access(unsigned long l
   if (s == nullptr) return addr;                                       // no table yet (a launch before vsk_open)
   const unsigned bytes = info & 0xffu;
   const bool misaligned = (addr & (unsigned long long)(bytes - 1u)) != 0ull;   // every access size is a power of two
-  const int t = *reinterpret_cast<volatile int*>(&s->version) & (kTables - 1);
-  const Range* r = s->ranges[t];
-  int lo = 0, hi = s->count[t];   // first range with r.lo > addr
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (r[mid].lo <= addr) lo = mid + 1; else hi = mid;
-  }
-  const bool inside = lo > 0 && addr + bytes <= r[lo - 1].hi;
   // the state itself (the sink included) is always a legal target
   const unsigned long long sb = reinterpret_cast<unsigned long long>(s);
   const bool own = addr >= sb && addr + bytes <= sb + sizeof(State);
-  if ((inside || own) && !misaligned) return addr;
+  // The first look may take the table from this SM's L1, which keeps lines of a slot that has been written again since the kernel
+  // began (kTables announcements on: training that is still preparing its rows while the caller announces the next call's buffers).
+  // An access is refused only by a look past L1 at a version that is still the published one after it.
+  for (int look = 0; !misaligned; ++look) {
+    const int v = *reinterpret_cast<volatile int*>(&s->version);
+    const Range* r = s->ranges[v & (kTables - 1)];
+    const int* count = &s->count[v & (kTables - 1)];
+    const bool fresh = look > 0;
+    int lo = 0, hi = fresh ? *reinterpret_cast<const volatile int*>(count) : *count;   // first range with r.lo > addr
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if ((fresh ? *reinterpret_cast<const volatile unsigned long long*>(&r[mid].lo) : r[mid].lo) <= addr) lo = mid + 1; else hi = mid;
+    }
+    if (own || (lo > 0 && addr + bytes <= (fresh ? *reinterpret_cast<const volatile unsigned long long*>(&r[lo - 1].hi) : r[lo - 1].hi)))
+      return addr;
+    if (fresh && (v == *reinterpret_cast<volatile int*>(&s->version) || look == 64)) break;
+  }
   if (atomicAdd(&s->faults, 1ull) == 0ull) {
     s->first_addr = addr;
     s->first_info = (unsigned long long)info | (misaligned ? 0x200ull : 0ull);
