@@ -169,6 +169,42 @@ def test_filter_groups_take_turns_on_two_lanes(vsk, dev):
     ix.close()
 
 
+def test_filter_groups_take_one_lane_where_two_have_no_room(vsk):
+    """With less free memory than the second lane's row list takes (90 MB), the groups take the first lane in turn."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(41)
+    n, d, per, k = 20_000_000, 4, 40, 10
+    x = torch.empty((n, d), device="cuda").uniform_(-1.0, 1.0, generator=gen)
+    q = torch.empty((2 * per, d), device="cuda").uniform_(-1.0, 1.0, generator=gen)
+    rm = (torch.arange(n, device="cuda") & 1) + 1
+    qm = torch.arange(2 * per, device="cuda") // per + 1
+    filler = None
+    try:
+        found = []
+        for tight in (False, True):
+            dev = vsk.CUDAAcceleratorStrategy(0).initialize()
+            try:
+                ix = _index(vsk, dev, x, rm)
+                for group in (slice(0, per), slice(per, 2 * per)):   # one group at a time: the first lane's buffers
+                    ix.batchSearch(q[group], k, qm[group])
+                if tight:
+                    filler = torch.empty(torch.cuda.mem_get_info()[0] - (72 << 20), dtype=torch.uint8, device="cuda")
+                dev.timeline(True)
+                dev.timeline_read()
+                found.append(ix.batchSearch(q, k, qm))
+                found[-1] += ({int(lane) for lane, _, _ in dev.timeline_read()},)
+                dev.timeline(False)
+                ix.close()
+            finally:
+                dev.close()
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    (d0, i0, lanes0), (d1, i1, _) = found
+    assert lanes0 == {0, 1}
+    assert torch.equal(i0, i1) and torch.equal(d0, d1) and bool((i1[:per] % 2 == 0).all()) and bool((i1[per:] % 2 == 1).all())
+
+
 def test_only_rows_that_are_re_scored_are_counted(vsk, dev):
     """The k rows kept from chunk to chunk carry their exact values already."""
     rng = np.random.default_rng(33)

@@ -622,17 +622,39 @@ static int32_t filtered_grouped_search(Index* ix, const float* q, int64_t nq, in
     }
     return fp32_topk(ctx, a, rows, e - b, qpos, k, ix->id_base, out_dist, out_ids, 0);
   };
-  int32_t st = VSK_OK;
-  if (two) VSK_TRY(lanes_fork(ctx));
-  for (int64_t g = 0; g < groups && st == VSK_OK; ++g) st = run_group(g, two ? (int)(g & 1) : 0);
-  for (int lane = 0; lane < 2 && st == VSK_OK; ++lane) st = collect(lane);
-  if (two) {
-    const int32_t jst = lanes_join(ctx);
-    if (st != VSK_OK || jst != VSK_OK) {   // nothing of either lane may be left running over the caller's buffers
-      cudaStreamSynchronize(ctx->stream_main);
-      cudaStreamSynchronize(ctx->stream_aux);
-      return st != VSK_OK ? st : jst;
+  auto run_all = [&](bool lanes) -> int32_t {
+    int32_t rs = VSK_OK;
+    if (lanes) VSK_TRY(lanes_fork(ctx));
+    for (int64_t g = 0; g < groups && rs == VSK_OK; ++g) rs = run_group(g, lanes ? (int)(g & 1) : 0);
+    for (int lane = 0; lane < 2 && rs == VSK_OK; ++lane) rs = collect(lane);
+    if (lanes) {
+      const int32_t jst = lanes_join(ctx);
+      if (rs != VSK_OK || jst != VSK_OK) {   // nothing of either lane may be left running over the caller's buffers
+        cudaStreamSynchronize(ctx->stream_main);
+        cudaStreamSynchronize(ctx->stream_aux);
+        return rs != VSK_OK ? rs : jst;
+      }
     }
+    return rs;
+  };
+  const L1Call l1_before = *l1;
+  const double work_before = ix->l1_work;
+  const int64_t reranked = ctx->stats.reranked_rows, fallback = ctx->stats.fallback_queries;
+  int32_t st = run_all(two);
+  if (two && st == VSK_ERR_OUT_OF_MEMORY) {
+    // No room for the buffers of two groups at a time: the second lane's go back, and every group takes the first lane.
+    for (int i = 64; i < 2 * 64; ++i) {
+      dev_free(ctx->scratch[i]);
+      ctx->scratch[i] = nullptr;
+      ctx->scratch_bytes[i] = 0;
+    }
+    pending[0] = pending[1] = L1Pending{};
+    *l1 = l1_before;
+    ix->l1_work = work_before;
+    ctx->stats.reranked_rows = reranked;
+    ctx->stats.fallback_queries = fallback;
+    ctx->err.clear();
+    st = run_all(false);
   }
   VSK_TRY(st);
   VSK_CUDA(ctx, cudaGetLastError());
