@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 import oracle
-from parity import assert_topk_parity
+from parity import assert_topk_parity, logged_launches
 
 pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -628,3 +628,82 @@ def test_no_small_last_chunk_in_a_small_batch(vsk, dev, cpu_oracle, n, nq, k):
     ix.close()
     assert dev.stats()["fallback_queries"] - before <= nq // 20
     assert_topk_parity(*got, *cpu_oracle.flat_search(oracle.COSINE, q, x, k))
+
+
+@pytest.mark.parametrize("metric", ["euclidean", "cosine", "dotProduct"])
+def test_unusual_queries_do_not_disturb_the_others(vsk, dev, cpu_oracle, metric):
+    """Queries that are not numbers, not finite, denormal, zero, tiny and huge in one batch, each with an operand scale of its own:
+    the others are answered without a re-run, and the finite ones as the oracle answers them."""
+    rng = np.random.default_rng(51)
+    n, d, nq, k = 30_000, 96, 300, 10
+    x = rng.standard_normal((n, d)).astype(np.float32)
+    q = rng.standard_normal((nq, d)).astype(np.float32)
+    plain = np.arange(nq) % 50 >= 6
+    q[3, 5], q[53, :] = np.nan, np.nan
+    q[4, 7], q[54, 0] = np.inf, -np.inf
+    q[0] *= np.float32(1e-41)
+    q[1] *= np.float32(1e-25)
+    q[2] *= np.float32(1e15)
+    q[5] = 0.0
+    ix = _flat(vsk, dev, metric, x)
+    try:
+        before = dev.stats()["fallback_queries"]
+        gd, gi = ix.batchSearch(q, k)
+        assert dev.stats()["fallback_queries"] - before <= (~plain).sum()
+        dev.set_search_path(1)
+        fd, fi = ix.batchSearch(q, k)
+    finally:
+        dev.set_search_path(0)
+        ix.close()
+    finite = np.isfinite(q).all(axis=1)
+    rd, ri = cpu_oracle.flat_search(oracle.METRIC_IDS[metric], q[finite], x, k)
+    assert_topk_parity(gd[finite], gi[finite], rd, ri)
+    odd = ~finite
+    assert np.array_equal(gi[odd], fi[odd]) and np.array_equal(gd[odd], fd[odd], equal_nan=True)
+
+
+@pytest.mark.parametrize("metric", ["euclidean", "cosine", "dotProduct"])
+def test_rows_too_wide_for_the_one_launch_finish(vsk, metric):
+    """41 001 dimensions: a query row and a candidate list do not fit in one CTA's shared memory, so the last compaction, the
+    re-scoring and the final order are launches of their own; unsharded and as two shards.  Every query has ten rows near it: the
+    bound of so wide a contraction is a hundredth of |q| |x|, and rows without structure would all lie within it."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(61)
+    n, d, nq, k = 2_600, 41_001, 20, 10
+    x = torch.empty((n, d), device="cuda").normal_(generator=gen)
+    q = torch.empty((nq, d), device="cuda").normal_(generator=gen)
+    for j, rows in enumerate(torch.randperm(n, device="cuda", generator=gen)[:nq * k].view(k, nq)):
+        x[rows] = (1 + 0.02 * j) * q + 0.05 * (j + 1) * x[rows]
+    devs, bounds, shards = [], [], []
+    try:
+        whole = vsk.CUDAAcceleratorStrategy(0).initialize()
+        devs.append(whole)
+        ix = _flat(vsk, whole, metric, x)
+        (gd, gi), names = logged_launches(whole, lambda: ix.batchSearch(q, k))
+        assert names.count("rerank") == 1 and "finish" not in names and whole.stats()["fallback_queries"] == 0
+        for s in range(2):
+            devs.append(vsk.CUDAAcceleratorStrategy(0).initialize())
+            shards.append(vsk.FlatIndex(devs[-1], d, metric))
+            shards[-1].add(x[s * n // 2:(s + 1) * n // 2])
+            shards[-1].set_id_base(s * n // 2)
+            bounds.append(shards[-1].shardSearchBegin(q, k, 2))
+        torch.cuda.synchronize()
+        g = torch.stack(bounds).max(dim=0).values
+        parts = [sh.shardSearchFinish(g) for sh in shards]
+        md, mi = vsk.CUDAAccelerationEngine(whole).mergeTopK(torch.stack([p[0] for p in parts]), torch.stack([p[1] for p in parts]))
+    finally:
+        for dv in devs:
+            dv.close()
+    dot = q.double() @ x.double().T
+    if metric == "euclidean":
+        ref = (q.double().square().sum(1)[:, None] + x.double().square().sum(1) - 2 * dot).clamp(min=0).sqrt()
+    else:
+        ref = -dot if metric == "dotProduct" else 1 - dot / (q.double().norm(dim=1)[:, None] * x.double().norm(dim=1) + 1e-8)
+    rd, ri = torch.topk(ref, k, dim=1, largest=False)
+    for dist, ids in ((gd, gi), (md, mi)):
+        if metric == "cosine":
+            # one less a quotient: the absolute error of the product and of the norms remains, each a lane's d / 32 terms and five
+            # sums over the lanes, every one rounded to 2^-24 of at most |q| |x| (1.5e-4; the planted rows lie 3e-3 apart)
+            assert torch.equal(ids, ri) and float((dist.double() - rd).abs().max()) <= 2 * (d / 32 + 5) * 2 ** -24
+        else:
+            assert_topk_parity(dist.cpu().numpy(), ids.cpu().numpy(), rd.float().cpu().numpy(), ri.cpu().numpy())

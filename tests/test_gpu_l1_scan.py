@@ -205,6 +205,27 @@ def test_filter_groups_take_one_lane_where_two_have_no_room(vsk):
     assert torch.equal(i0, i1) and torch.equal(d0, d1) and bool((i1[:per] % 2 == 0).all()) and bool((i1[per:] % 2 == 1).all())
 
 
+def test_more_filter_groups_than_are_counted_in_one_pass(vsk, dev, cpu_oracle):
+    """105 distinct masks of two bits: the groups' rows are counted group by group, on one lane."""
+    rng = np.random.default_rng(37)
+    n, d, per, k = 60_000, 256, 100, 10                          # 1.1e9 steps a group: the byte filter pays
+    x = rng.uniform(-1, 1, (n, d)).astype(np.float32)
+    rm = rng.integers(0, 2 ** 15, n, dtype=np.uint64)
+    masks = np.array([(1 << a) | (1 << b) for a in range(15) for b in range(a)], np.uint64)
+    qm = rng.permutation(np.repeat(masks, per))
+    q = rng.uniform(-1, 1, (len(qm), d)).astype(np.float32)
+    ix = _index(vsk, dev, x, rm)
+    dev.set_search_path(1)
+    ref = ix.batchSearch(q, k, qm)
+    dev.set_search_path(0)
+    got, names = logged_launches(dev, lambda: ix.batchSearch(q, k, qm))
+    ix.close()
+    assert names.count("l1_dense") == len(masks)
+    assert np.array_equal(got[1], ref[1]) and np.array_equal(got[0], ref[0])
+    some = rng.choice(len(qm), 64, replace=False)
+    assert_topk_parity(got[0][some], got[1][some], *cpu_oracle.flat_search(oracle.MANHATTAN, q[some], x, k, rm, qm[some]))
+
+
 def test_only_rows_that_are_re_scored_are_counted(vsk, dev):
     """The k rows kept from chunk to chunk carry their exact values already."""
     rng = np.random.default_rng(33)

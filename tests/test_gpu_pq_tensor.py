@@ -197,7 +197,9 @@ def test_encoding_equals_the_exact_sums(vsk, dev, cpu_oracle, ds, ksub, offset):
 # The contraction takes 129 or more codewords from 65 536 (row, segment) pairs on (131 072 for two dimensions): whole and ragged
 # row tiles, whole and partial groups of segments.
 @pytest.mark.parametrize("ds,m,ksub,n", [(2, 8, 256, 16_384), (2, 10, 129, 13_185), (4, 8, 256, 8_319), (4, 9, 200, 8_000), (8, 4, 256, 20_001),
-                                         (8, 5, 255, 13_185), (8, 16, 256, 19_072), (16, 2, 256, 32_896), (16, 3, 130, 22_007)])
+                                         (8, 5, 255, 13_185), (8, 16, 256, 19_072), (16, 2, 256, 32_896), (16, 3, 130, 22_007),
+                                         # rows narrower than the 32 (16) columns that are fetched of them
+                                         (2, 2, 256, 65_537), (4, 2, 200, 33_001), (8, 2, 256, 32_896), (8, 3, 129, 22_003), (16, 1, 256, 65_600)])
 def test_encoding_on_the_tensor_cores_equals_the_exact_sums(vsk, dev, cpu_oracle, ds, m, ksub, n):
     rng = np.random.default_rng(ds * 100 + m)
     x = (rng.standard_normal((n, m * ds)) + 2.0 * rng.standard_normal(m * ds)).astype(np.float32)
