@@ -552,6 +552,8 @@ static int32_t filtered_grouped_search(Index* ix, const float* q, int64_t nq, in
   starts.push_back(nq);
   // Manhattan groups take turns on the context's two lanes, so that one group's first rows, re-scoring and selections run beside
   // the other's byte scan: alone they leave the machine idle (64 groups of 156 queries over 2.5 million rows each: 15 of 150 ms).
+  // Both lanes' groups are issued without a wait in between, so their row counts are taken beforehand: mask_count_kernel counts up
+  // to 64 groups in its one pass (two totals to a lane).  A batch of more groups reads each count as it comes, on one lane.
   const bool two = max_fraction < 0.0 && ix->metric == VSK_METRIC_MANHATTAN && groups > 1 && groups <= 64 && ctx->lane == 0 && !ctx->profile;
   void *dperm, *dcount;
   std::vector<unsigned long long> cnt;

@@ -748,7 +748,8 @@ int32_t few_launch_as(Ctx* ctx, FewKernelArgs ka, const float* host_q) {
 }
 
 // One query over rows of at most 256 dimensions: four 16-byte loads per lane and step, the next step's already on their way
-// (the general form takes two rows per step and waits for them).
+// (the general form takes two rows per step and waits for them).  Whole call, general form / this, rows of 256 dimensions: 400 000
+// rows 104 / 94 us (cosine 115 / 99), 100 000 rows 46.6 / 43.4; of 160: 100 000 rows 42.5 / 41.8; 10 000 rows, stored or probed: the same.
 template <int METRIC, int NQ, bool VEC, bool SEG, bool INL>
 int32_t few_launch_one(Ctx* ctx, const FewKernelArgs& ka, const float* host_q) {
   if constexpr (VEC) {

@@ -1711,7 +1711,7 @@ __global__ void prep_rows_kernel(const float* __restrict__ x, int64_t n, int dim
 
 // The same for rows of at most 256 dimensions in 16-byte pieces (no fold, no metric of its own): a lane holds its pieces between
 // the two passes, so the row is read once, and stores four halves at a time.  10 million x 128, 192 operand columns: 3.4 - 3.9 ms
-// for the form above (its 64-byte stores), 1.6 here.
+// for the form above (its 64-byte stores), 2.1 here.
 __global__ void __launch_bounds__(256) prep_rows_wide_kernel(const float* __restrict__ x, int64_t n, int dim, int dim16, const float* scale_p,
                                                              __half* __restrict__ out, float* __restrict__ nrm16, float* __restrict__ err16,
                                                              float* __restrict__ nrm) {
@@ -1770,7 +1770,6 @@ struct BoundConsts {
 //                                       + dim16 * 2^-22 * |q'| X'            (fp32 accumulation in the tensor core)
 //   divided by s_q s_x; doubled for euclidean (value = |x|^2 - 2 q.x) plus the fp32 rounding of |x|^2;
 //   cosine adds the effect of the reference's +1e-8 in the denominator and of normalising in fp32.
-// Also writes alpha = coefficient / (s_q s_x).
 template <int METRIC>
 __device__ __forceinline__ float query_eps(float a, float e, float qn, float inv, const BoundConsts& c) {
   float dot_err = (a * c.max_err16 + e * c.max_norm16 + e * c.max_err16) + (float)c.dim16 * 2.3841858e-7f * a * c.max_norm16;
@@ -1793,15 +1792,15 @@ __device__ __forceinline__ float query_eps(float a, float e, float qn, float inv
   return r * 1.0001f + 1e-30f;
 }
 
-template <int METRIC>
+// Inverted lists and product-quantised rows (squared distances only), with one query scale for the batch; also writes alpha.
 __global__ void bound_kernel(const float* __restrict__ qn16, const float* __restrict__ qe16,
                              const float* __restrict__ qnorm, int64_t nq, const float* scale_q, BoundConsts c,
                              float* __restrict__ eps, float* alpha) {
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const float inv = 1.0f / ((*scale_q) * c.scale_x);
-  if (q == 0) *alpha = (METRIC == VSK_METRIC_EUCLIDEAN ? -2.0f : -1.0f) * inv;
+  if (q == 0) *alpha = -2.0f * inv;
   if (q >= nq) return;
-  eps[q] = query_eps<METRIC>(qn16[q], qe16[q], qnorm[q], inv, c);
+  eps[q] = query_eps<VSK_METRIC_EUCLIDEAN>(qn16[q], qe16[q], qnorm[q], inv, c);
 }
 
 // eps for int8-coded rows (operand residual of the rows is zero; the query operand is fp16(s_q q~), q~ = q / scale):
@@ -1833,7 +1832,8 @@ struct QueryPrep {
   float *alpha, *eps, *norm;
   CandLists cand;
   uint64_t* words;          // eight words to be zeroed (error word, counters)
-  const float* sq_scale;    // I8: the operand is made from q / scale (the codes are the row operand)
+  const float* sq_scale;    // I8: the codes are the row operand, the query's is made from q~ = q / scale per dimension:
+                            // sum_i q_i x^_i = sum_i q~_i code_i - sum_i q_i offset_i / scale_i, whose second term is no row's own
 };
 
 template <int METRIC, bool I8 = false>
@@ -1927,8 +1927,6 @@ __global__ void prep_codes_kernel(const int8_t* __restrict__ codes, int64_t n, i
   }
 }
 
-// q~ = q / scale per dimension: sum_i q_i x^_i = sum_i q~_i code_i - sum_i q_i offset_i / scale_i, and the
-// second term does not depend on the row.
 // a / b rounded once, with y = 1 / b rounded once: Markstein's correction (IBM J. Res. Dev. 34, 1990) - the remainder of the
 // product a y is exact in a fused operation, and adding its share rounds correctly while nothing over- or underflows.
 __device__ __forceinline__ float div_rn_by(float a, float b, float y) {
@@ -1988,9 +1986,9 @@ __device__ __forceinline__ void i8_row_sums(const float* qs, const int8_t* __res
     for (int o = 16; o > 0; o >>= 1) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o);
 }
 
-// Exact re-scoring against dequantised rows.  Four rows per warp step share a dimension's parameters and reciprocal: a row at a
-// time, each code divided by its scale, the seven launches of 10 000 queries over 6.25 million x 384 took 2.84 ms.
-template <int METRIC>
+// Exact re-scoring against dequantised rows, dot product (the integer contraction's lists).  Four rows per warp step share a
+// dimension's parameters and reciprocal: a row at a time, each code divided by its scale, the seven launches of 10 000 queries over
+// 6.25 million x 384 took 2.84 ms.
 __global__ void __launch_bounds__(256) rerank_i8_kernel(const float* __restrict__ q, const int8_t* __restrict__ codes,
                                                         int dim, const float* __restrict__ scale,
                                                         const float* __restrict__ offset, CandLists cand,
@@ -2012,16 +2010,16 @@ __global__ void __launch_bounds__(256) rerank_i8_kernel(const float* __restrict_
     float sum[RR];
 #pragma unroll
     for (int r = 0; r < RR; ++r) id[r] = (uint32_t)keys[min(c0 + r, cnt - 1)];
-    i8_row_sums<METRIC, RR>(qs, codes, dim, scale, offset, id, lane, sum);
+    i8_row_sums<VSK_METRIC_DOT_PRODUCT, RR>(qs, codes, dim, scale, offset, id, lane, sum);
 #pragma unroll
     for (int r = 0; r < RR; ++r)
-      if (lane == r && c0 + r < cnt) *VSK_CHK_W(keys + c0 + r) = make_key(METRIC == VSK_METRIC_EUCLIDEAN ? sum[r] : -sum[r], id[r]);
+      if (lane == r && c0 + r < cnt) *VSK_CHK_W(keys + c0 + r) = make_key(-sum[r], id[r]);
   }
 }
 
 // Sums of RR fp32 rows against the query in shared memory (direct formulas; a lane's dimensions are lane, lane + 32, .., added in
 // that order), four loads of every row in flight.  Bound by the gathered rows; with one load of each row in flight the re-scoring
-// of the list search was bound by their latency (1 000 queries of 128 dimensions: 690 us in two launches, 468 with four).
+// of the list search was bound by their latency (10 000 queries of 128 dimensions: 690 us in two launches, 468 with four).
 template <int METRIC, int RR>
 __device__ __forceinline__ void f32_row_sums(const float* qs, const float* __restrict__ x, int dim, const uint32_t (&id)[RR], int lane,
                                              float (&sum)[RR]) {
@@ -2827,7 +2825,7 @@ struct QueryOperands {
 int32_t prepare_query_operands(Index* ix, const float* q, int64_t nq, QueryOperands* out) {
   VSK_TRACE("vsk:query_operands");
   Ctx* ctx = ix->ctx;
-  prefer_shared_carveout(ctx, absmax_kernel, choose_scale_kernel, prep_rows_kernel<VSK_METRIC_EUCLIDEAN>, bound_kernel<VSK_METRIC_EUCLIDEAN>);
+  prefer_shared_carveout(ctx, absmax_kernel, choose_scale_kernel, prep_rows_kernel<VSK_METRIC_EUCLIDEAN>, bound_kernel);
   const int dim = ix->dim, dim16 = ix->dim16;
   void* p;
   const int64_t nq_pad = ceil_div(nq, TN) * TN;
@@ -2853,7 +2851,7 @@ int32_t prepare_query_operands(Index* ix, const float* q, int64_t nq, QueryOpera
   choose_scale_kernel<<<1, 1, 0, ctx->stream>>>(q_absmax, 0, q_scale, fold ? 1 : 0, ix->fold_exp - 1);
   BoundConsts bc{ix->scale16, ix->max_xnorm16, ix->max_xerr16, ix->max_xnorm, ix->min_xnorm_nz, dim16, fold ? ix->fold_bmax : 0.f};
   launch_prep<VSK_METRIC_EUCLIDEAN>(ctx, q, nq, dim, dim16, q_scale, q16, nullptr, qn16, qe16, qn_tmp, nullptr, qfold);
-  bound_kernel<VSK_METRIC_EUCLIDEAN><<<(unsigned)ceil_div(nq, 256), 256, 0, ctx->stream>>>(qn16, qe16, qn_tmp, nq, q_scale, bc, eps, alpha);
+  bound_kernel<<<(unsigned)ceil_div(nq, 256), 256, 0, ctx->stream>>>(qn16, qe16, qn_tmp, nq, q_scale, bc, eps, alpha);
   ctx->stats.kernel_launches += 3;
   VSK_CUDA(ctx, cudaGetLastError());
   tl_mark(ctx, "query_operands");
@@ -3489,7 +3487,7 @@ int32_t ivf_tensor_search(Index* ix, const float* q, int64_t nq, const int64_t* 
   ctx->stats.kernel_launches += 2;
   BoundConsts bc{ix->scale16, ix->max_xnorm16, ix->max_xerr16, ix->max_xnorm, ix->min_xnorm_nz, dim16, fold ? ix->fold_bmax : 0.f};
   launch_prep<VSK_METRIC_EUCLIDEAN>(ctx, q, nq, dim, dim16, q_scale, q16, nullptr, qn16, qe16, qn_tmp, nullptr, qfold);
-  bound_kernel<VSK_METRIC_EUCLIDEAN><<<(unsigned)ceil_div(nq, 256), 256, 0, ctx->stream>>>(qn16, qe16, qn_tmp, nq, q_scale, bc, eps, alpha);
+  bound_kernel<<<(unsigned)ceil_div(nq, 256), 256, 0, ctx->stream>>>(qn16, qe16, qn_tmp, nq, q_scale, bc, eps, alpha);
   ctx->stats.kernel_launches++;
   VSK_CUDA(ctx, cudaGetLastError());
 
@@ -4359,7 +4357,7 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
   };
   const size_t qsm = (size_t)dim * sizeof(float);   // (i8_search_applicable: at most 48 KB)
   if (2 * qsm > 48 * 1024)
-    VSK_CUDA(ctx, cudaFuncSetAttribute(rerank_i8_kernel<VSK_METRIC_DOT_PRODUCT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * qsm)));
+    VSK_CUDA(ctx, cudaFuncSetAttribute(rerank_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * qsm)));
   const int64_t growth = nq <= 2048 ? std::max(16, ctx->tuning.chunk_growth) : std::max(1, ctx->tuning.chunk_growth);
   bool looked = nq < 256;   // a small batch is cheap to scan twice: no look between its chunks
   while (seen < n) {
@@ -4398,7 +4396,7 @@ int32_t i8_search(Index* ix, const float* q, int64_t nq, int32_t k, float* out_d
       VSK_TRY(launch_list_scan<true>(ctx, mx, mq, mx, mb, la, stride));
     } else if (tc_epilogue_warps(a.kblocks, false) == 16) VSK_TRY((launch_tc_ew<SCAN_THRESHOLD, 16, true>(ctx, mq, mx, a, false)));
     else VSK_TRY((launch_tc_ew<SCAN_THRESHOLD, 8, true>(ctx, mq, mx, a, false)));
-    rerank_i8_kernel<VSK_METRIC_DOT_PRODUCT><<<(unsigned)nq, 256, 2 * qsm, ctx->stream>>>(q, ix->codes, dim, ix->sq_scale, ix->sq_offset, cand, rr_total);
+    rerank_i8_kernel<<<(unsigned)nq, 256, 2 * qsm, ctx->stream>>>(q, ix->codes, dim, ix->sq_scale, ix->sq_offset, cand, rr_total);
     ctx->stats.kernel_launches++;
     VSK_CUDA(ctx, cudaGetLastError());
     tl_mark(ctx, "rerank");
