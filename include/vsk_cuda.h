@@ -155,7 +155,7 @@ typedef struct vsk_tuning {
 int32_t vsk_open(int32_t device, vsk_ctx** out_ctx);
 int32_t vsk_close(vsk_ctx* ctx);
 /* Gives back the device memory a context keeps between calls for speed only: the work buffers of k-means training and
- * assignment (at most 8 GB, and from 1 GB on at most a sixteenth of the device memory that is free when a call ends).
+ * assignment (at most 8 GB, and from 64 MB on at most a sixteenth of the device memory that was free beside them).
  * The library does so by itself before its own large allocations; for another allocator on the same device call this. */
 int32_t vsk_trim(vsk_ctx* ctx);
 int32_t vsk_device_info_get(vsk_ctx* ctx, vsk_device_info* out);

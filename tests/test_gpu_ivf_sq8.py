@@ -470,8 +470,7 @@ def test_the_training_block_is_kept_and_given_back(vsk):
 
 
 def test_the_training_block_leaves_the_device_to_others(vsk):
-    """A block of a gigabyte or more that is more than a sixteenth of the free memory goes back when its call ends; others on
-    request."""
+    """A block that is more than a sixteenth of the free memory goes back when its call ends; others on request."""
     import torch
     if os.environ.get("VSK_CHECKED", "0") not in ("", "0"):
         pytest.skip("the checked build allocates every buffer by itself")

@@ -79,6 +79,12 @@ void* arena_take(Ctx* ctx, size_t bytes) {
       return nullptr;
     }
     ctx->arena_bytes = bytes;
+    size_t fr = 0, tot = 0;
+    if (bytes >= kArenaYield && cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+      cudaGetLastError();
+      fr = 0;
+    }
+    ctx->arena_stays = bytes < kArenaYield || bytes <= fr / kArenaShare;
   }
   ctx->arena_busy = true;
   return ctx->arena;
@@ -87,13 +93,7 @@ void* arena_take(Ctx* ctx, size_t bytes) {
 
 void arena_return(Ctx* ctx) {
   ctx->arena_busy = false;
-  if (ctx->arena_bytes < kArenaAsk) return;
-  size_t fr = 0, tot = 0;
-  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
-    cudaGetLastError();
-    fr = 0;
-  }
-  if (ctx->arena_bytes > fr / kArenaShare) arena_drop(ctx);
+  if (!ctx->arena_stays) arena_drop(ctx);
 }
 
 int32_t lanes_fork(Ctx* ctx) {

@@ -196,10 +196,10 @@ struct Ctx {
   // One block kept between calls that take a lot of device memory for their own duration only (k-means): 10 ms of a 110 ms
   // training call over 10 million x 128 went into 5 GB of allocations and frees.  At most kArenaMax, one user at a time; given
   // back before any other large allocation of the context (dev_alloc), on request (vsk_trim) and with the context.  Nobody else
-  // on the device can ask for it, so a large one stays only while it is a small share of what they have left (arena_return).
+  // on the device can ask for it, so a large one stays only if it is a small share of what they have left (arena_return).
   void* arena = nullptr;
   size_t arena_bytes = 0;
-  bool arena_busy = false;
+  bool arena_busy = false, arena_stays = false;   // (stays: it may outlive the call)
   PinnedBuf host_io;         // staging of small host-pointer calls (HostCall)
   PinnedBuf host_flags[2];   // per lane: the flag words a finished half-search hands to the host
   std::vector<const void*> configured;   // kernels that have their shared memory on this device (opt_in_shared) ...
@@ -544,10 +544,11 @@ void chk_remove(const void* p);
 void worker_release(Ctx* ctx);
 int32_t dev_alloc(Ctx* ctx, void** p, size_t bytes);
 // `bytes` of the context's kept block, or null (in use, too large, no memory): the caller allocates for itself.  arena_return
-// when the work that uses it has drained: a block of kArenaAsk or more is kept only while at least kArenaShare times as much is
-// free on the device, so that other allocators lose at most a sixteenth of it.  (Asking takes 0.15 ms: a tenth of a training call
-// over 200 000 x 250, whose block is 130 MB, and a hundredth of the calls whose block is a gigabyte.)
-constexpr size_t kArenaMax = 8ull << 30, kArenaYield = 64ull << 20, kArenaAsk = 1ull << 30, kArenaShare = 16;
+// when the work that uses it has drained: a block of kArenaYield or more outlives the call only if kArenaShare times as much was free
+// on the device beside it when it was made, so that other allocators lose at most a sixteenth of that.  (Asked when the block is
+// made, not when a call returns it: the question takes 0.15 ms as a rule, a tenth of a call over 200 000 x 250, and tens of
+// milliseconds on a busy driver.)
+constexpr size_t kArenaMax = 8ull << 30, kArenaYield = 64ull << 20, kArenaShare = 16;
 void* arena_take(Ctx* ctx, size_t bytes);
 void arena_return(Ctx* ctx);
 void dev_free(void* p);
