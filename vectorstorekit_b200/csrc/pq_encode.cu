@@ -11,9 +11,9 @@
 //              (ProductQuantizerCodebook.swift:12-30), decide, so codes equal the exact encoder's bit for bit.
 //
 // 1 million x 128, 16 segments: 2.29 ms for the short-form kernel of pq.cu, 0.52 here (8 segments of 4: 0.82 -> 0.24, 32 of 2:
-// 2.57 -> 0.86, 8 of 16: 1.86 -> 0.40).  What bounds it now: the epilogue's instructions - 57 % of the cycles of the pipe that
-// does maxima, shifts and comparisons, 51 % of the shared-memory pipe (codewords of the fours, at addresses of the lanes'
-// choosing), the tensor pipe is at 21 %.  Holding the 64 maxima of a row takes the registers: with 32 columns per load, with the
+// 2.57 -> 0.86, 8 of 16: 1.86 -> 0.40).  What bounds it now: the epilogue's instructions - 62 % of the issue slots and of the
+// pipe that does maxima, shifts and comparisons, 47 % of the shared-memory pipe (codewords of the fours, at addresses of the lanes'
+// choosing), the tensor pipe is at 22 %.  Holding the 64 maxima of a row takes the registers: with 32 columns per load, with the
 // columns in two halves, or with four groups of 96 registers some of them spilled, and next to 220 KB of shared memory there
 // is no L1 left to spill to (0.61 - 0.87 ms).
 //
